@@ -155,6 +155,28 @@ def test_gemm_f32(n, k, m):
     assert torch.equal(one.cpu()[0], out.cpu()[n - 1])
 
 
+@pytest.mark.parametrize("k,m", [(256, 64), (260, 65), (512, 15), (2304, 129), (4100, 33), (52, 4800)])
+def test_gemm_f32_rows_of_every_batch_size(k, m):
+    """Segments that end in the middle, more segments than warps, columns around the tiles' edges:
+    a row has the same bits among 1, 8, 9, 16, 17, 32, 33, 64, 129 and 700 rows (all kernels and
+    tile sizes).  Bound: a chain of 256 roundings and one a segment, each of half a unit of the sum
+    of absolute terms."""
+    ops = _ops()
+    g = torch.Generator(device=DEV).manual_seed(k + m)
+    x = torch.randn(700, k, generator=g, device=DEV)
+    w = torch.randn(m, k, generator=g, device=DEV)
+    first = None
+    for n in (700, 1, 8, 9, 16, 17, 32, 33, 64, 129):
+        out = torch.full((n, m), float("nan"), device=DEV)
+        ops.gemm_f32(x[:n], w, out)
+        if first is None:
+            first = out
+            terms = x.double().abs() @ w.double().abs().t()
+            bound = (min(k, 256) + (k + 255) // 256) * 2.0 ** -24 * terms
+            assert ((out.double() - x.double() @ w.double().t()).abs() <= bound).all()
+        assert torch.equal(out, first[:n]), n
+
+
 def test_gemm_f32_is_true_32_bit():
     """Operands with 12 mantissa bits: a 10-bit (TF32) or 8-bit (bfloat16) mantissa would round
     them to 1 and give exactly k.  Every partial sum n * (1 + 2^-12), n <= 64, fits float32, so
