@@ -176,6 +176,236 @@ attn_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
     }
 }
 
+// The same attention for float32 pages whose rows are whole 16-byte pieces: tiles of keys and values
+// come through three stages of 16-byte cp.async (eight threads a key, which look its page up once
+// and a tile ahead), a warp takes RW rows and reads a key or a value from shared memory once for
+// all of them.  A row's sums have the order of the kernel above - features ascending in a score,
+// keys ascending in a weighted sum - so the two, and any RW, give the same bits.  The kernel above
+// waited for one element's page and then its key at a time: a decode step of 8 sequences of 520 keys
+// (4 kv heads of 64, ranges of 128 keys) took 53 us and takes 22; a layer with a prompt of 400 tokens
+// takes 325 us (872), one of 64 sequences of 1,900 keys and 8 kv heads of 128 747 us (1,883).
+constexpr int STAGES = 3;
+
+template <int RW, int VW, int NB>
+__global__ void __launch_bounds__(ROWS * 32)
+attn_simt_vec_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out,
+                     int out_stride, const float* __restrict__ k_pages,
+                     const float* __restrict__ v_pages, const int* __restrict__ block_table,
+                     int table_stride, int num_pages, const int* __restrict__ seq_slot,
+                     const int* __restrict__ seq_qstart, const int* __restrict__ seq_qlen,
+                     const int* __restrict__ seq_pos0, const WorkItem* __restrict__ items,
+                     float* __restrict__ partial_acc, float* __restrict__ partial_ml,
+                     int partial_limit, int heads, int kv_heads, int d, int page, float scale,
+                     int window, int aligned, int* __restrict__ status) {
+    constexpr int TROWS = ROWS * RW;
+    extern __shared__ __align__(16) float smem[];
+    const int ks = d + 4;                             // a key's stride: 16-byte reads without conflicts
+    const int stage_floats = TILE * (ks + d) + TILE;
+    float* Qs = smem + STAGES * stage_floats;         // [TROWS][d]
+
+    const WorkItem it = items[blockIdx.x];
+    if (it.kv_begin >= it.kv_end || it.partial >= partial_limit) {
+        pdl_wait();
+        return;
+    }
+    const int hk = blockIdx.y;
+    const int g = heads / kv_heads;
+    const int qlen = seq_qlen[it.seq], pos0 = seq_pos0[it.seq];
+    const int slot = seq_slot[it.seq], tok0 = seq_qstart[it.seq];
+    const int rows_total = qlen * g;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    bool active[RW], any = false;
+    int tok[RW], hq[RW], row_lo[RW], row_hi[RW];
+#pragma unroll
+    for (int i = 0; i < RW; ++i) {
+        const int r = it.row0 + warp * RW + i;
+        active[i] = r < rows_total;
+        any |= active[i];
+        tok[i] = active[i] ? r / g : 0;
+        hq[i] = hk * g + (active[i] ? r % g : 0);
+        const int pos = pos0 + tok[i];
+        row_lo[i] = it.kv_begin;
+        if (window > 0) row_lo[i] = max(row_lo[i], pos - window + 1);
+        row_hi[i] = active[i] ? min(it.kv_end, pos + 1) : 0;
+    }
+    const int last_row = min(it.row0 + TROWS, rows_total) - 1;
+    const int max_pos = pos0 + last_row / g, min_pos = pos0 + it.row0 / g;
+    const int k_hi = min(it.kv_end, max_pos + 1);
+    int k_lo_true = it.kv_begin;
+    if (window > 0) k_lo_true = max(k_lo_true, min_pos - window + 1);
+    const int k_lo = (k_lo_true / TILE) * TILE;       // tiles sit at absolute positions
+
+    const int j = threadIdx.x >> 3, part = threadIdx.x & 7;    // this thread's key of a tile
+    const int pieces = d >> 2;
+    auto page_of = [&](int kt) {                      // of the key at kt + j; -2: outside the range
+        const int kpos = kt + j;
+        if (kpos < k_lo_true || kpos >= k_hi) return -2;
+        return block_table[(size_t)slot * table_stride + kpos / page];
+    };
+    int next_page = page_of(k_lo);
+
+    pdl_wait();            // q, and the keys and values of this step's tokens, are just written
+    auto issue = [&](int kt, int stage) {
+        float* kd = smem + stage * stage_floats + j * ks;
+        float* vd = smem + stage * stage_floats + TILE * ks + j * d;
+        const int page_id = next_page;
+        next_page = page_of(kt + TILE);
+        const bool read = page_id >= 0 && page_id < num_pages;
+        const bool gone = page_id != -2 && !read;
+        const size_t off = read ? (((size_t)page_id * kv_heads + hk) * page +
+                                   (size_t)((kt + j) % page)) * d : 0;
+        const int bytes = read ? 16 : 0;
+        if (!aligned) {                               // pages that do not start at 16 bytes
+            for (int c = part; c < d; c += 8) {
+                kd[c] = read ? k_pages[off + c] : 0.0f;
+                vd[c] = read ? v_pages[off + c] : 0.0f;
+            }
+        }
+        for (int c = part; c < (aligned ? pieces : 0); c += 8) {
+            const unsigned ka = (unsigned)__cvta_generic_to_shared(kd + 4 * c);
+            const unsigned va = (unsigned)__cvta_generic_to_shared(vd + 4 * c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(ka),
+                         "l"(k_pages + off + 4 * c), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(va),
+                         "l"(v_pages + off + 4 * c), "r"(bytes) : "memory");
+        }
+        if (part == 0) {
+            smem[stage * stage_floats + TILE * (ks + d) + j] = gone ? -INFINITY : 0.0f;
+            if (gone && status != nullptr) atomicExch(status, 2);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (k_lo + s * TILE < k_hi) issue(k_lo + s * TILE, s);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+#pragma unroll
+    for (int i = 0; i < RW; ++i)
+        for (int dd = lane; dd < d; dd += 32)
+            Qs[(warp * RW + i) * d + dd] =
+                active[i] ? q[(size_t)(tok0 + tok[i]) * q_stride + hq[i] * d + dd] : 0.0f;
+
+    float m[RW], l[RW], acc[RW][NB][VW];
+#pragma unroll
+    for (int i = 0; i < RW; ++i) {
+        m[i] = -INFINITY;
+        l[i] = 0.0f;
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int e = 0; e < VW; ++e) acc[i][b][e] = 0.0f;
+    }
+
+    int stage = 0;
+    for (int kt = k_lo; kt < k_hi; kt += TILE) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();                              // this tile has landed, the oldest is consumed
+        const int free = stage == 0 ? STAGES - 1 : stage - 1;
+        if (kt + (STAGES - 1) * TILE < k_hi) issue(kt + (STAGES - 1) * TILE, free);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const float* Ks = smem + stage * stage_floats;
+        const float* Vs = Ks + TILE * ks;
+        stage = stage == STAGES - 1 ? 0 : stage + 1;
+        if (!any) continue;
+
+        const int kpos = kt + lane;
+        const float4* kr = reinterpret_cast<const float4*>(Ks + lane * ks);
+        float s[RW];
+#pragma unroll
+        for (int i = 0; i < RW; ++i) s[i] = 0.0f;
+#pragma unroll 4
+        for (int c = 0; c < pieces; ++c) {
+            const float4 kk = kr[c];
+#pragma unroll
+            for (int i = 0; i < RW; ++i) {
+                const float4 qq = reinterpret_cast<const float4*>(Qs + (warp * RW + i) * d)[c];
+                s[i] = fmaf(qq.x, kk.x, s[i]);
+                s[i] = fmaf(qq.y, kk.y, s[i]);
+                s[i] = fmaf(qq.z, kk.z, s[i]);
+                s[i] = fmaf(qq.w, kk.w, s[i]);
+            }
+        }
+        const bool held = Vs[TILE * d + lane] == 0.0f;
+        float p[RW];
+        bool some = false;
+#pragma unroll
+        for (int i = 0; i < RW; ++i) {
+            const bool valid = kpos >= row_lo[i] && kpos < row_hi[i] && held;
+            const float sc = valid ? s[i] * scale : -INFINITY;
+            const float m_new = fmaxf(m[i], warp_max(sc));
+            p[i] = 0.0f;
+            if (m_new == -INFINITY) continue;         // nothing of this tile is visible to the row
+            p[i] = valid ? expf(sc - m_new) : 0.0f;
+            const float corr = expf(m[i] - m_new);    // 0 when m was -inf
+            l[i] = l[i] * corr + warp_sum(p[i]);
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int e = 0; e < VW; ++e) acc[i][b][e] *= corr;
+            m[i] = m_new;
+            some = true;
+        }
+        if (!some) continue;
+#pragma unroll 4
+        for (int key = 0; key < TILE; ++key) {
+            float pj[RW];
+            bool zero = true;
+#pragma unroll
+            for (int i = 0; i < RW; ++i) {
+                pj[i] = __shfl_sync(0xffffffffu, p[i], key);
+                zero &= pj[i] == 0.0f;
+            }
+            if (zero) continue;                       // uniform over the warp
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const int dd = VW * lane + 32 * VW * b;
+                if (dd >= d) continue;
+                float v[VW];
+                if (VW == 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(Vs + key * d + dd);
+                    v[0] = t.x; v[1] = t.y; v[VW - 2] = t.z; v[VW - 1] = t.w;
+                } else {
+                    const float2 t = *reinterpret_cast<const float2*>(Vs + key * d + dd);
+                    v[0] = t.x; v[1] = t.y;
+                }
+#pragma unroll
+                for (int i = 0; i < RW; ++i) {
+                    if (pj[i] == 0.0f) continue;
+#pragma unroll
+                    for (int e = 0; e < VW; ++e) acc[i][b][e] = fmaf(pj[i], v[e], acc[i][b][e]);
+                }
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < RW; ++i) {
+        if (!active[i]) continue;
+        float* o;
+        float factor = 1.0f;
+        if (it.partial < 0) {
+            factor = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
+            o = out + (size_t)(tok0 + tok[i]) * out_stride + hq[i] * d;
+        } else {
+            const size_t idx = ((size_t)it.partial * kv_heads + hk) * TROWS + warp * RW + i;
+            o = partial_acc + idx * d;
+            if (lane == 0) {
+                partial_ml[idx * 2] = m[i];
+                partial_ml[idx * 2 + 1] = l[i];
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int e = 0; e < VW; ++e) {
+                const int dd = VW * lane + 32 * VW * b + e;
+                if (dd < d) o[dd] = it.partial < 0 ? acc[i][b][e] * factor : acc[i][b][e];
+            }
+    }
+}
+
 // Merge the chunks of each row, in ascending order of the chunks.
 template <typename T>
 __global__ void __launch_bounds__(ROWS * 32)
@@ -243,7 +473,7 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
                        const int* seq_qstart, const int* seq_qlen, const int* seq_pos0,
                        const int* items, int num_items, float* partial_acc, float* partial_ml,
                        int partial_limit, int heads, int kv_heads, int d, int page, float scale,
-                       int window, int* status, void* stream);
+                       int window, int* status, void* stream, int tile_rows = ROWS);
 static int launch_combine(int dtype, void* out, int out_stride, const int* seq_qstart,
                           const int* seq_qlen, const int* items, int num_items,
                           const float* partial_acc, const float* partial_ml, int partial_limit,
@@ -255,11 +485,11 @@ DE_EXPORT int de_attn_simt(int dtype, const void* q, int q_stride, void* out, in
                            const int* seq_qstart, const int* seq_qlen, const int* seq_pos0,
                            const int* items, int num_items, float* partial_acc, float* partial_ml,
                            int heads, int kv_heads, int d, int page, float scale, int window,
-                           int* status, void* stream) {
+                           int tile_rows, int* status, void* stream) {
     return launch_simt(dtype, q, q_stride, out, out_stride, k_pages, v_pages, block_table,
                        table_stride, num_pages, seq_slot, seq_qstart, seq_qlen, seq_pos0, items,
                        num_items, partial_acc, partial_ml, 0x7fffffff, heads, kv_heads, d, page,
-                       scale, window, status, stream);
+                       scale, window, status, stream, tile_rows);
 }
 
 // `partial_limit`: partial slots that the scratch holds (work items that name a slot beyond it are
@@ -270,10 +500,41 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
                        const int* seq_qstart, const int* seq_qlen, const int* seq_pos0,
                        const int* items, int num_items, float* partial_acc, float* partial_ml,
                        int partial_limit, int heads, int kv_heads, int d, int page, float scale,
-                       int window, int* status, void* stream) {
+                       int window, int* status, void* stream, int tile_rows) {
     if (num_items <= 0) return 0;
     if (d <= 0 || d > MAX_D || heads % kv_heads != 0) return -2;
     cudaStream_t s = (cudaStream_t)stream;
+    const bool vec = dtype == DE_F32 && d % 4 == 0;
+    const int aligned = (uintptr_t)k_pages % 16 == 0 && (uintptr_t)v_pages % 16 == 0;
+    if (tile_rows != ROWS && !(vec && tile_rows == 4 * ROWS)) return -5;
+    if (vec) {
+        const size_t bytes = (size_t)(STAGES * (TILE * (2 * d + 4) + TILE) + tile_rows * d) *
+                             sizeof(float);
+#define LAUNCH_VEC(RW, VW, NB)                                                                  \
+    do {                                                                                        \
+        auto kernel = attn_simt_vec_kernel<RW, VW, NB>;                                         \
+        if (bytes > 48 * 1024) {                                                                \
+            const cudaError_t e = cudaFuncSetAttribute(                                         \
+                kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);               \
+            if (e != cudaSuccess) return (int)e;                                                \
+        }                                                                                       \
+        return de_launch(kernel, dim3(num_items, kv_heads), dim3(ROWS * 32), bytes, s,          \
+                         (const float*)q, q_stride, (float*)out, out_stride,                    \
+                         (const float*)k_pages, (const float*)v_pages, block_table,             \
+                         table_stride, num_pages, seq_slot, seq_qstart, seq_qlen, seq_pos0,     \
+                         (const WorkItem*)items, partial_acc, partial_ml, partial_limit, heads, \
+                         kv_heads, d, page, scale, window, aligned, status);                    \
+    } while (0)
+        if (tile_rows == ROWS) {
+            if (d <= 64) LAUNCH_VEC(1, 2, 1);
+            if (d <= 128) LAUNCH_VEC(1, 4, 1);
+            LAUNCH_VEC(1, 4, 2);
+        }
+        if (d <= 64) LAUNCH_VEC(4, 2, 1);
+        if (d <= 128) LAUNCH_VEC(4, 4, 1);
+        LAUNCH_VEC(4, 4, 2);
+#undef LAUNCH_VEC
+    }
     const size_t smem = (size_t)(TILE * (d + 1) + TILE * d + ROWS * d) * sizeof(float);
     dim3 grid(num_items, kv_heads);
     cudaError_t e;

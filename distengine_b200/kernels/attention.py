@@ -5,8 +5,9 @@ items on the host and launches them.
   (``csrc/attention_mma.cu``, compiled for that head size at first use).  Sequences with many query
   rows in the step use its wide tile (64 rows), sequences with at most 16 rows (decoded tokens)
   its narrow tile (16 rows, the keys of a tile split over the warps).
-* float32, or any other even head size up to 256: the CUDA-core kernel in float32 arithmetic
-  (``csrc/attention_simt.cu``), 8 rows a tile.
+* float32, or any other even head size up to 256: the CUDA-core kernels in float32 arithmetic
+  (``csrc/attention_simt.cu``), 8 rows a tile; in float32 with head sizes that are a multiple of 4
+  32 rows a tile for sequences with many query rows.
 
 Long key ranges of a step with few tiles are cut into chunks; ``de_attn_combine`` merges the
 partial results (``attention_plan``).  In float32 the chunk length is fixed (``F32_CHUNK`` keys,
@@ -91,6 +92,10 @@ class AttentionLauncher:
                 self.shapes[0] = _Shape("wide", 256 if head_dim == 64 else 128, 2)
         else:
             self.shapes = [_Shape("rows8", 8, -1)]
+            if dtype == torch.float32 and head_dim % 4 == 0:
+                # rows of whole 16-byte pieces: sequences with many rows take tiles of 32 (a row's
+                # result is the same bits in either)
+                self.shapes.insert(0, _Shape("rows32", 32, -1))
             self.module = ("attention_simt", ())
         self.fixed_chunk = F32_CHUNK if dtype == torch.float32 else None
         # steps of decoded tokens only: rotation, cache write, attention and merge in one launch;
@@ -355,7 +360,7 @@ def launch_items(code: int, module, q, out, k_pages, v_pages, block_table, seq_s
             _status_fallback = torch.zeros(1, dtype=torch.int32, device=q.device)
         status = _status_fallback
     if code < 0:
-        _check(lib.de_attn_simt(_tag(q.dtype), *common, status.data_ptr(), _stream()),
+        _check(lib.de_attn_simt(_tag(q.dtype), *common, tile_rows, status.data_ptr(), _stream()),
                "paged attention")
     elif code == 2:
         _check(lib.de_attn_tcgen05(*common, status.data_ptr(), _stream()),

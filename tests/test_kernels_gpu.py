@@ -155,6 +155,34 @@ def test_gemm_f32(n, k, m):
     assert torch.equal(one.cpu()[0], out.cpu()[n - 1])
 
 
+@pytest.mark.parametrize("head_dim,heads,kv_heads,window,page", [
+    (4, 2, 1, None, 4), (60, 6, 2, 40, 8), (64, 8, 1, None, 16), (100, 3, 3, None, 16),
+    (128, 4, 2, 129, 16), (132, 2, 1, None, 64), (256, 2, 2, 33, 16)])
+@pytest.mark.parametrize("chunk", [0, 128])
+def test_attention_f32_tiles_of_8_and_32_rows_agree_bit_for_bit(head_dim, heads, kv_heads, window,
+                                                                page, chunk):
+    """Rows around a tile's 32, keys around tiles of 32 and ranges of 128, at sizes around what a
+    lane takes of a value's row; the larger tiles give the bits of the smaller."""
+    fx = PagedFixture([70, 1, 33, 290, 128], kv_heads, head_dim, page, torch.float32, DEV)
+    g = torch.Generator().manual_seed(head_dim)
+    q = [torch.randn(n, heads, head_dim, generator=g) for n in (37, 1, 33, 9, 2)]
+    args = (heads, kv_heads, head_dim, head_dim ** -0.5, window or 0)
+    few, _ = run_paged_attention(fx, q, *args, chunk=chunk, shape="rows8")
+    many, _ = run_paged_attention(fx, q, *args, chunk=chunk, shape="rows32")
+    assert torch.equal(few, many)
+    group, at = heads // kv_heads, 0
+    for i, (keys, qi) in enumerate(zip(fx.kv_lens, q)):
+        n = qi.shape[0]
+        dist = (torch.arange(keys - n, keys)[:, None] - torch.arange(keys)[None, :])
+        seen = (dist >= 0) if window is None else (dist >= 0) & (dist < window)
+        for h in range(heads):
+            s = qi[:, h].double() @ fx.k[i][:, h // group].double().t() * head_dim ** -0.5
+            want = torch.softmax(s.masked_fill(~seen, float("-inf")), 1) @ fx.v[i][:, h // group].double()
+            got = many[at: at + n, h * head_dim: (h + 1) * head_dim]
+            assert_close(got, want.float(), torch.float32, f"sequence {i}, head {h}")
+        at += n
+
+
 @pytest.mark.parametrize("k,m", [(256, 64), (260, 65), (512, 15), (2304, 129), (4100, 33), (52, 4800)])
 def test_gemm_f32_rows_of_every_batch_size(k, m):
     """Segments that end in the middle, more segments than warps, columns around the tiles' edges:
