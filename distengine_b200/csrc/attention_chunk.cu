@@ -1305,6 +1305,426 @@ attn_chunk_tiled_kernel(const T* __restrict__ q, int q_stride, void* __restrict_
 
 
 // ------------------------------------------------------------------------------------------
+// The same attention on the tensor cores, for bfloat16 rows of D = 64 or 128 features (keys and
+// values alike): mma.sync m16n8k16, a block of four warps takes 64 rows, a warp 16 of them against
+// tiles of 64 keys that come through two stages of cp.async.  Nothing loses precision against the
+// kernels above: the products of bfloat16 queries and keys are exact, and a softmax weight enters
+// its product with the values as three bfloat16 terms whose sum is the float32 weight.  What the
+// tensor cores add up is a tile's share only, the small terms first; the running sums of a row are
+// float32 multiply-adds (acc <- acc * correction + tile's share).  Scores, cap, penalty, maximum and
+// exponentials are those of the kernels above.  A row's tiles lie at absolute multiples of 32, so its result does not depend on what shares its block or its step.
+// The kernel above runs the same work on the CUDA cores, where a prompt of 2,048 tokens of 16 heads
+// of 128 on 4 kv heads takes 734 us with a window of 1,024 and a cap, 147 us here, 39 us of
+// 512 tokens against 221 (its distance from 64 bits 2.5e-7 of the result against 4.7e-7); without
+// window and cap 202 us against 1,141.  What bounds it: twelve warps an SM, each a chain of two
+// products, a maximum and exponentials a tile; the tensor pipe is busy a third of the time.
+// ------------------------------------------------------------------------------------------
+__device__ __forceinline__ void ldmatrix4(unsigned (&r)[4], const void* p) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void ldmatrix4_trans(unsigned (&r)[4], const void* p) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], unsigned b0,
+                                         unsigned b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+        "{%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ unsigned pack2(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const unsigned*>(&v);
+}
+// x and y as sums of three bfloat16 numbers each: all 24 bits of a float32 mantissa
+__device__ __forceinline__ void split3(float x, float y, unsigned& a, unsigned& b, unsigned& c) {
+    a = pack2(x, y);
+    const float rx = x - __uint_as_float(a << 16), ry = y - __uint_as_float(a & 0xffff0000u);
+    b = pack2(rx, ry);
+    c = pack2(rx - __uint_as_float(b << 16), ry - __uint_as_float(b & 0xffff0000u));
+}
+
+// tanh(x) for |x| <= TANH_NEAR to 7e-8 of its value (as good as tanhf and a third of its
+// instructions): x + x^3 P(x^2), P of degree 4 fitted to tanh at Chebyshev nodes by reweighted
+// least squares (3e-9 but for float32's rounding).  Scores under a cap mostly lie here.
+constexpr float TANH_NEAR = 0.6f;
+__device__ __forceinline__ float tanh_near(float x) {
+    const float u = x * x;
+    float p = fmaf(u, -0.00589515036f, 0.0207959637f);
+    p = fmaf(u, p, -0.0537838265f);
+    p = fmaf(u, p, 0.133319244f);
+    p = fmaf(u, p, -0.333332986f);
+    return fmaf(x * u, p, x);
+}
+
+constexpr int MKT = 32;           // keys of a tile
+
+template <int D, int HALVES> constexpr size_t mma_smem() {
+    return (size_t)4 * HALVES * MKT * (D + 8) * sizeof(__nv_bfloat16);
+}
+
+template <int D, int HALVES>
+__global__ void __launch_bounds__(128, 3)
+attn_chunk_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, void* __restrict__ out,
+                      int out_stride, const __nv_bfloat16* __restrict__ k_pages,
+                      const __nv_bfloat16* __restrict__ v_pages,
+                      const int* __restrict__ block_table, int table_stride, int num_pages,
+                      const int* __restrict__ seq_slot, const int* __restrict__ seq_qstart,
+                      const int* __restrict__ seq_qlen, const int* __restrict__ seq_pos0,
+                      const WorkItem* __restrict__ items, const float* __restrict__ r1,
+                      const float* __restrict__ r2, int heads, int kv_heads, int page, float scale,
+                      Sight sight, int out_f32, int* __restrict__ status) {
+    using T = __nv_bfloat16;
+    constexpr int LD = D + 8;                        // a row's stride: ldmatrix without conflicts
+    constexpr int NT = MKT / 8, DT = D / 8, CH = D / 8;
+    constexpr int TEAM = 128 / HALVES, WARPS = 4 / HALVES, MROWS = 16 * WARPS;
+    extern __shared__ __align__(16) float smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int half = warp / WARPS, tid = threadIdx.x % TEAM;  // which tiles; thread of the half
+    T* k_s = reinterpret_cast<T*>(smem) + half * 4 * MKT * LD;       // [2][MKT][LD]
+    T* v_s = k_s + 2 * MKT * LD;                     // [2][MKT][LD]
+    __shared__ int pages_all[HALVES][3][MKT];             // the pages of three tiles in a row
+    __shared__ int gone_s;                           // a key inside the range had no page
+    int (*pages_s)[MKT] = pages_all[half];
+    auto half_sync = [&]() {
+        asm volatile("bar.sync %0, %1;\n" ::"r"(1 + half), "n"(TEAM) : "memory");
+    };
+
+    const WorkItem it = items[blockIdx.x];
+    if (it.kv_begin >= it.kv_end) {
+        pdl_wait();
+        return;
+    }
+    const int hk = blockIdx.y;
+    const int g = heads / kv_heads;
+    const int qlen = seq_qlen[it.seq], pos0 = seq_pos0[it.seq];
+    const int slot = seq_slot[it.seq], tok0 = seq_qstart[it.seq];
+    const int rows_total = qlen * g;
+    const int gid = lane >> 2, tig = lane & 3;
+    const bool penalty = r1 != nullptr;
+
+    // the rows of this thread: gid and gid + 8 of the warp's sixteen
+    bool active[2];
+    int tok[2], hq[2], pos[2], row_lo[2], row_hi[2], row_first[2];
+    float pen1[2], pen2[2], m[2], l[2];
+    int all_lo = 0, all_hi = 0x7fffffff;             // keys [all_lo, all_hi) are seen by every row
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int r = it.row0 + warp % WARPS * 16 + gid + 8 * e;
+        active[e] = r < rows_total;
+        tok[e] = active[e] ? r / g : 0;
+        hq[e] = hk * g + (active[e] ? r % g : 0);
+        pos[e] = pos0 + tok[e];
+        pen1[e] = penalty ? r1[hq[e]] : 0.0f;
+        pen2[e] = penalty ? r2[hq[e]] : 0.0f;
+        row_lo[e] = max(it.kv_begin, sight_lo(sight, pos[e]));
+        row_first[e] = it.kv_begin > 0 ? 0 : sight_first(sight, row_lo[e]);
+        row_hi[e] = active[e] ? min(it.kv_end, pos[e] + 1) : 0;
+        if (active[e]) {
+            all_lo = max(all_lo, row_lo[e]);
+            all_hi = min(all_hi, row_hi[e]);
+        }
+        m[e] = -INFINITY;
+        l[e] = 0.0f;
+    }
+    const bool any = it.row0 + warp % WARPS * 16 < rows_total;
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+        all_lo = max(all_lo, __shfl_xor_sync(0xffffffffu, all_lo, o));
+        all_hi = min(all_hi, __shfl_xor_sync(0xffffffffu, all_hi, o));
+    }
+    const int last_row = min(it.row0 + MROWS, rows_total) - 1;
+    const int max_pos = pos0 + last_row / g, min_pos = pos0 + it.row0 / g;
+    const int k_hi = min(it.kv_end, max_pos + 1);
+    const int k_lo_true = max(it.kv_begin, sight_lo(sight, min_pos));
+    const int k_first = it.kv_begin > 0 ? 0 : sight_first(sight, k_lo_true);
+    const TileWalk walk(k_lo_true, k_first, MKT);
+    // two halves: the first two warps take the tiles of even number, the others those of odd number
+    // (by absolute place, so that a tile's half does not depend on what else the block holds)
+    auto mine = [&](int kt) {
+        while (HALVES == 2 && kt < k_hi && ((kt / MKT) & 1) != half) kt = walk.next(kt, MKT);
+        return kt;
+    };
+    auto after = [&](int kt) { return mine(walk.next(kt, MKT)); };
+
+    // the page of key kt + thread; -1 for keys that no row sees, -2 for a seen key without a page
+    auto page_of = [&](int kt) {
+        const int kpos = kt + tid;
+        if (tid >= MKT || kt >= k_hi || (kpos < k_lo_true && kpos >= k_first) || kpos >= k_hi) return -1;
+        const int id = block_table[(size_t)slot * table_stride + kpos / page];
+        return id >= 0 && id < num_pages ? id : -2;
+    };
+    auto put_page = [&](int id, int which) {
+        if (tid < MKT) pages_s[which][tid] = id;
+        if (id == -2) {
+            gone_s = 1;
+            if (status != nullptr) atomicExch(status, 2);
+        }
+    };
+    auto load_tile = [&](int kt, int which, int stage) {
+        T* kd = k_s + stage * MKT * LD;
+        T* vd = v_s + stage * MKT * LD;
+#pragma unroll
+        for (int i = 0; i < MKT * CH / TEAM; ++i) {
+            const int c = tid + TEAM * i, j = c / CH, ch = c % CH;
+            const int id = pages_s[which][j];
+            const size_t at = id >= 0 ? ((size_t)id * kv_heads + hk) * page +
+                                            (size_t)((kt + j) % page) : 0;
+            const int bytes = id >= 0 ? 16 : 0;
+            const unsigned ka = (unsigned)__cvta_generic_to_shared(kd + j * LD + ch * 8);
+            const unsigned va = (unsigned)__cvta_generic_to_shared(vd + j * LD + ch * 8);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(ka),
+                         "l"(k_pages + at * D + ch * 8), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(va),
+                         "l"(v_pages + at * sight.v_stride + ch * 8), "r"(bytes) : "memory");
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+
+    if (threadIdx.x == 0) gone_s = 0;
+    const int start = mine(walk.start), second = after(start);
+    const int page_a = page_of(start), page_b = page_of(second);
+    __syncthreads();
+    put_page(page_a, 0);
+    put_page(page_b, 1);
+    __syncthreads();
+    pdl_wait();            // q, and the keys and values of this step's tokens, are just written
+    load_tile(start, 0, 0);
+
+    // q fragments straight from global memory (read once)
+    unsigned qf[D / 16][4];
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const T* p = q + (size_t)(tok0 + tok[e]) * q_stride + hq[e] * D + kk * 16 + 2 * tig;
+            qf[kk][e] = active[e] ? *reinterpret_cast<const unsigned*>(p) : 0u;
+            qf[kk][e + 2] = active[e] ? *reinterpret_cast<const unsigned*>(p + 8) : 0u;
+        }
+    float acc[DT][4];
+#pragma unroll
+    for (int j = 0; j < DT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = 0.0f;
+
+    const int mat = lane >> 3, mr = lane & 7;
+    const float inv_cap = sight.softcap > 0.0f ? 1.0f / sight.softcap : 0.0f;
+    int stage = 0, which = 0;
+    for (int kt = start; kt < k_hi; stage ^= 1) {
+        const int next = after(kt), which_next = which == 2 ? 0 : which + 1;
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        half_sync();                 // this tile has landed, the one before it has been used
+        int ahead = -1;
+        if (next < k_hi) {
+            load_tile(next, which_next, stage ^ 1);
+            ahead = page_of(after(next));
+        }
+        if (any) {
+            const T* kb = k_s + stage * MKT * LD;
+            const T* vb = v_s + stage * MKT * LD;
+            // q . k in two chains of half the features each, added in float32
+            float s[NT][4];
+#pragma unroll
+            for (int j = 0; j < NT; j += 2) {
+                float c[2][2][4];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) c[i >> 3][(i >> 2) & 1][i & 3] = 0.0f;
+#pragma unroll
+                for (int kk = 0; kk < D / 16; ++kk) {
+                    unsigned b[4];
+                    ldmatrix4(b, kb + ((j + (mat >> 1)) * 8 + mr) * LD + kk * 16 + (mat & 1) * 8);
+                    mma16816(c[kk & 1][0], qf[kk], b[0], b[1]);
+                    mma16816(c[kk & 1][1], qf[kk], b[2], b[3]);
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    s[j][x] = c[0][0][x] + c[1][0][x];
+                    s[j + 1][x] = c[0][1][x] + c[1][1][x];
+                }
+            }
+            const bool inside = kt >= all_lo && kt + MKT <= all_hi && gone_s == 0;
+            // as sight_score: scale, penalty, cap
+            if (!penalty) {
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) s[j][x] *= scale;
+            } else {
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const int e = x >> 1;
+                        const float dist = (float)(pos[e] - (kt + j * 8 + 2 * tig + (x & 1)));
+                        s[j][x] *= scale;
+                        s[j][x] -= sight.linear ? pen1[e] * dist : pen1[e] * log1pf(pen2[e] * dist);
+                    }
+            }
+            if (sight.softcap > 0.0f) {
+                float far = 0.0f;
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        s[j][x] *= inv_cap;
+                        far = fmaxf(far, fabsf(s[j][x]));
+                    }
+                if (__any_sync(0xffffffffu, far > TANH_NEAR)) {
+#pragma unroll
+                    for (int j = 0; j < NT; ++j)
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) {
+                            const float y = s[j][x], a = fabsf(y);
+                            const float t = 1.0f - __fdividef(2.0f, 1.0f + expf(2.0f * a));
+                            s[j][x] = sight.softcap *
+                                      (a > TANH_NEAR ? copysignf(t, y) : tanh_near(y));
+                        }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < NT; ++j)
+#pragma unroll
+                        for (int x = 0; x < 4; ++x)
+                            s[j][x] = sight.softcap * tanh_near(s[j][x]);
+                }
+            }
+            if (!inside) {
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const int e = x >> 1, key = j * 8 + 2 * tig + (x & 1), kpos = kt + key;
+                        const bool valid = (kpos >= row_lo[e] || kpos < row_first[e]) &&
+                                           kpos < row_hi[e] && pages_s[which][key] >= 0;
+                        if (!valid) s[j][x] = -INFINITY;
+                    }
+            }
+            float corr[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float top = m[e];
+#pragma unroll
+                for (int j = 0; j < NT; ++j) top = fmaxf(top, fmaxf(s[j][2 * e], s[j][2 * e + 1]));
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+                // (a row that has seen nothing yet: every weight is exp(-inf) = 0)
+                const float use = top == -INFINITY ? 0.0f : top;
+                corr[e] = expf(m[e] - use);
+                m[e] = top;
+                float sum = 0.0f;
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int x = 2 * e; x < 2 * e + 2; ++x) {
+                        s[j][x] = expf(s[j][x] - use);
+                        sum += s[j][x];
+                    }
+                l[e] = l[e] * corr[e] + sum;
+            }
+            unsigned pw[3][MKT / 16][4];             // the weights' terms, largest first
+#pragma unroll
+            for (int ks = 0; ks < MKT / 16; ++ks)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float* p = &s[2 * ks + (i >> 1)][2 * (i & 1)];
+                    split3(p[0], p[1], pw[0][ks][i], pw[1][ks][i], pw[2][ks][i]);
+                }
+#pragma unroll
+            for (int jd = 0; jd < DT; jd += 2) {
+                unsigned b[MKT / 16][4];
+                float t0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, t1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int ks = 0; ks < MKT / 16; ++ks)
+                    ldmatrix4_trans(b[ks], vb + (ks * 16 + (mat & 1) * 8 + mr) * LD +
+                                               (jd + (mat >> 1)) * 8);
+#pragma unroll
+                for (int term = 2; term >= 0; --term)
+#pragma unroll
+                    for (int ks = 0; ks < MKT / 16; ++ks) {
+                        mma16816(t0, pw[term][ks], b[ks][0], b[ks][1]);
+                        mma16816(t1, pw[term][ks], b[ks][2], b[ks][3]);
+                    }
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    acc[jd][x] = fmaf(acc[jd][x], corr[x >> 1], t0[x]);
+                    acc[jd + 1][x] = fmaf(acc[jd + 1][x], corr[x >> 1], t1[x]);
+                }
+            }
+        }
+        // (the pages of the tile before this one were last read before the barrier above)
+        put_page(ahead, which == 0 ? 2 : which - 1);
+        which = which_next;
+        kt = next;
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (HALVES == 1) pdl_trigger();
+    // the second half's sums join the first's
+    float* joint = smem + tid;                       // [DT * 4 + 4][64]
+    if (HALVES == 2) __syncthreads();
+    if (half == 1) {
+#pragma unroll
+        for (int j = 0; j < DT; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) joint[(4 * j + x) * 64] = acc[j][x];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            joint[(4 * DT + e) * 64] = m[e];
+            joint[(4 * DT + 2 + e) * 64] = l[e];
+        }
+    }
+    if (HALVES == 2) {
+        __syncthreads();
+        pdl_trigger();
+        if (half == 1) return;
+        float mine_f[2], other_f[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float mo = joint[(4 * DT + e) * 64], top = fmaxf(m[e], mo);
+            const float use = top == -INFINITY ? 0.0f : top;
+            mine_f[e] = expf(m[e] - use);
+            other_f[e] = expf(mo - use);
+            l[e] = l[e] * mine_f[e] + joint[(4 * DT + 2 + e) * 64] * other_f[e];
+            m[e] = top;
+        }
+#pragma unroll
+        for (int j = 0; j < DT; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+                acc[j][x] = fmaf(acc[j][x], mine_f[x >> 1],
+                                 joint[(4 * j + x) * 64] * other_f[x >> 1]);
+    }
+    const bool pairs = out_stride % 2 == 0 && (uintptr_t)out % (out_f32 ? 8 : 4) == 0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 1);
+        l[e] += __shfl_xor_sync(0xffffffffu, l[e], 2);
+        if (!active[e]) continue;
+        const float inv = sight_inverse(sight, hq[e], m[e], l[e]);
+        const size_t token = (size_t)(tok0 + tok[e]);
+        const size_t o = token * out_stride + hq[e] * D;
+#pragma unroll
+        for (int j = 0; j < DT; ++j) {
+            const int col = j * 8 + 2 * tig;
+            const float a = acc[j][2 * e] * inv * sight_gate<T>(sight, token, hq[e], D, col);
+            const float b = acc[j][2 * e + 1] * inv *
+                            sight_gate<T>(sight, token, hq[e], D, col + 1);
+            if (!pairs) {
+                store_out<T>(out, out_f32, o + col, a);
+                store_out<T>(out, out_f32, o + col + 1, b);
+            } else if (out_f32) {
+                store_pair((float*)out + o + col, a, b);
+            } else {
+                store_pair((T*)out + o + col, a, b);
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
 // Steps in which every sequence brings one token.  A block takes a sequence and a kv head; its
 // eight warps share the key tiles of the token's chunk out among themselves (warp w takes tiles
 // w, w + 8, ...) and each works alone: it asks for its tile's 32 key rows and 32 value rows at
@@ -1636,10 +2056,19 @@ static size_t tiled_smem(int dk, int dv) {
     return (size_t)(TILE * (dk + 4) + TILE * dv + TROWS * (dk + 4) + 4 * TILE * 16 + TILE) *
            sizeof(float);
 }
+// the tensor-core kernel's sizes: bfloat16, keys and values of 64 or of 128 features
+static bool mma_ok(int dtype, int dk, int dv) {
+    return dtype == DE_BF16 && dk == dv && (dk == 64 || dk == 128);
+}
 // `wide`: 0 for steps of single tokens, else the rows (tokens times query heads a kv head) of the
-// step's longest portion (1: some portion): from 48 rows on the register-tiled kernel's 64.
+// step's longest portion (1: some portion): from 48 rows on 64 (the register-tiled kernel's,
+// or the tensor-core kernel's first form), else 32; callers give a portion's rows only where tiles of
+// 64 give every SM two blocks (tensor cores, 16 heads on 4 kv heads of 128: 1,024 tokens of 8 heads
+// on 2, 128 blocks of 64 rows or 256 of 32, 100 against 79 us; 2,048 tokens of 16 heads, 512 or
+// 1,024 blocks, 199 against 231).
 DE_EXPORT int de_attn_chunk_rows(int dtype, int dk, int dv, int wide) {
     if (!(vec_ok(dtype, dk, dv) && wide)) return ROWS;
+    if (mma_ok(dtype, dk, dv)) return wide >= 48 ? TROWS : TROWS / 2;
     if (wide >= 48 && tiled_smem(dk, dv) <= 200 * 1024) return TROWS;
     return vec_fits(dtype, dk, dv) ? ROWS * 4 : ROWS;
 }
@@ -1869,6 +2298,31 @@ DE_EXPORT int de_attn_chunk(int dtype, const void* q, int q_stride, void* out, i
     if (tile_rows != ROWS && !((tile_rows == ROWS * 4 && vec_fits(dtype, dk, dv)) ||
                                (tile_rows == TROWS && vec_ok(dtype, dk, dv))))
         return -5;
+    if ((tile_rows == TROWS || tile_rows == TROWS / 2) && mma_ok(dtype, dk, dv) &&
+        q_stride % 2 == 0 && (uintptr_t)q % 4 == 0 && (uintptr_t)k_pages % 16 == 0 &&
+        (uintptr_t)v_pages % 16 == 0) {
+        dim3 mgrid(num_items, kv_heads);
+#define MMA(D, HALVES)                                                                          \
+    do {                                                                                        \
+        auto kernel = attn_chunk_mma_kernel<D, HALVES>;                                         \
+        const size_t bytes = mma_smem<D, HALVES>();                                             \
+        const cudaError_t me = cudaFuncSetAttribute(                                            \
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);                   \
+        if (me != cudaSuccess) return (int)me;                                                  \
+        return de_launch(kernel, mgrid, dim3(128), bytes, s, (const __nv_bfloat16*)q, q_stride, \
+                         out, out_stride, (const __nv_bfloat16*)k_pages,                        \
+                         (const __nv_bfloat16*)v_pages, block_table, table_stride, num_pages,   \
+                         seq_slot, seq_qstart, seq_qlen, seq_pos0, (const WorkItem*)items, r1,  \
+                         r2, heads, kv_heads, page, scale, sight, out_f32, status);             \
+    } while (0)
+        if (tile_rows == TROWS) {
+            if (dk == 64) MMA(64, 1);
+            MMA(128, 1);
+        }
+        if (dk == 64) MMA(64, 2);
+        MMA(128, 2);
+#undef MMA
+    }
     if (tile_rows == TROWS) {
         if ((uintptr_t)k_pages % 16 != 0 || (uintptr_t)v_pages % 16 != 0) return -5;
         const size_t tsmem = tiled_smem(dk, dv);

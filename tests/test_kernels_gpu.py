@@ -650,3 +650,70 @@ def test_products_of_many_rows_take_the_tcgen05_kernel():
     up = plain.plain_linear(x.float(), wg[inner:].float(), torch.bfloat16)
     assert_close(act, plain.plain_swiglu(gate, up, torch.bfloat16), torch.bfloat16,
                  "linear_gated, many rows")
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("rows", [32, 64])
+@pytest.mark.parametrize("form", ["window", "slopes", "chunk"])
+def test_chunk_attention_on_tensor_cores(dim, rows, form):
+    """Rows around a tile's 32 and 64, keys around tiles of 32, both halves of a block, pages that a
+    window has passed, far and near scores under a cap: float32 results against 64 bits.  Bound: as
+    float32 sums of up to 400 terms (the exact products of bfloat16 operands)."""
+    from types import SimpleNamespace
+    from distengine_b200.kernels import recurrent as rk
+    from distengine_b200.kernels.attention_plan import build_plan
+    heads, kv_heads, page = 6, 2, 16
+    fx = PagedFixture([70, 1, 33, 390, 128], kv_heads, dim, page, torch.bfloat16, DEV)
+    qlen = np.array([37, 1, 33, 23, 65], dtype=np.int32)
+    pos0 = np.array(fx.kv_lens, dtype=np.int32) - qlen
+    g = torch.Generator().manual_seed(dim)
+    n, group = int(qlen.sum()), heads // kv_heads
+    q = (torch.randn(n, heads, dim, generator=g) * 3).to(torch.bfloat16)
+    window, keep, chunk, cap = (40, 3, 0, 4.0) if form == "window" else (
+        (0, 0, 50, 0.0) if form == "chunk" else (0, 0, 0, 0.0))
+    r = torch.rand(heads, generator=g) * 0.3
+    sink = torch.randn(heads, generator=g)
+    gate = torch.randn(n, heads, generator=g).to(torch.bfloat16)
+    if form == "window":                    # the pages between the kept keys and the first window
+        for p in range(1, (int(pos0[3]) - window + 1) // page):
+            fx.block_table[fx.slots[3], p] = -1
+    k_pages, v_pages, table = fx.to_device()
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).to(DEV)
+    qstart = (np.cumsum(qlen) - qlen).astype(np.int32)
+    ctx = SimpleNamespace(seq_slot=t(np.array(fx.slots)), seq_qstart=t(qstart), seq_qlen=t(qlen),
+                          seq_pos0=t(pos0), status=torch.zeros(1, dtype=torch.int32, device=DEV))
+    items = t(build_plan(qlen, pos0, group, kv_heads, rows, 0, chunk=0).items)
+    out = torch.full((n, heads * dim), float("nan"), device=DEV)
+    extras = {} if form != "slopes" else dict(slopes=r.to(DEV), sink=sink.to(DEV), gate_per_head=True,
+                                              gate=gate.to(DEV), out_scale=1.5)
+    pen = (r.to(DEV), (4 * r).to(DEV)) if form == "chunk" else (None, None)
+    rk.chunk_attention(q.view(n, -1).to(DEV), out, k_pages, v_pages, table, items, *pen, heads,
+                       kv_heads, dim, dim, dim ** -0.5, chunk, ctx, tile_rows=rows, window=window,
+                       keep_first=keep, softcap=cap, **extras)
+    assert int(ctx.status.item()) == 0
+    got = out.double().cpu().view(n, heads, dim)
+    for i, keys in enumerate(fx.kv_lens):
+        pos = torch.arange(int(pos0[i]), keys)
+        j = torch.arange(keys)
+        dist = pos[:, None] - j[None, :]
+        seen = dist >= 0
+        if window:
+            seen &= (dist < window) | (j < keep)[None, :]
+        if chunk:
+            seen &= (pos[:, None] // chunk) == (j[None, :] // chunk)
+        at = slice(int(qstart[i]), int(qstart[i] + qlen[i]))
+        for h in range(heads):
+            s = q[at, h].double() @ fx.k[i][:, h // group].double().t() * dim ** -0.5
+            if form == "slopes":
+                s = s - r[h].double() * dist
+            if form == "chunk":
+                s = s - r[h].double() * torch.log1p(4 * r[h].double() * dist.clamp(min=0))
+            if cap:
+                s = cap * torch.tanh(s / cap)
+            e = torch.exp(s.masked_fill(~seen, float("-inf")))
+            total = e.sum(1, keepdim=True) + (sink[h].double().exp() if form == "slopes" else 0.0)
+            want = e / total @ fx.v[i][:, h // group].double()
+            if form == "slopes":
+                want = want * 1.5 * torch.sigmoid(gate[at, h].double())[:, None]
+            err = (got[at, h] - want).abs().max().item()
+            assert err <= 4e-6 * max(1.0, want.abs().max().item()), (i, h, err)
