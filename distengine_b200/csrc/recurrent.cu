@@ -269,7 +269,7 @@ scan_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, i
             float* __restrict__ state, long long slot_stride, float* __restrict__ out,
             const int* __restrict__ seq_slot, const int* __restrict__ seq_qstart,
             const int* __restrict__ seq_qlen, int H, int rep, int dk, int dv, int vec16,
-            ConvKeep keep) {
+            int longest, ConvKeep keep) {
     constexpr int PD = LANES * (R + 4);                  // a token's vector in shared memory
     constexpr bool DELTA = MODE == 1;
     constexpr int VECS = MODE == 0 ? 2 : (MODE == 1 ? 3 : 4);      // q, k (, g (, z))
@@ -302,6 +302,7 @@ scan_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, i
                 cs[(size_t)i * keep.C + c] = x;
             }
     }
+    if (qlen > longest) return;                      // such portions go by chunks (recurrent_chunks.cu)
     float* S_g = slot_state + (size_t)h * dk * dv;
     float S[R];
 #pragma unroll
@@ -578,7 +579,7 @@ int launch_scan_cols(int R, dim3 grid, cudaStream_t s, const float* q, int ldq, 
                      int ldk, const VT* v, int ldv, const float* g, int ldg, const float* beta,
                      int ldb, const float* z, int ldz, const float* decay, float* state, long long slot_stride, float* out,
                      const int* seq_slot, const int* seq_qstart, const int* seq_qlen, int H,
-                     int rep, int dk, int dv, int vec16, ConvKeep keep) {
+                     int rep, int dk, int dv, int vec16, int longest, ConvKeep keep) {
 #define SCAN(RR)                                                                                \
     do {                                                                                        \
         const size_t smem = (size_t)2 * TB * (MODE + 2) * LANES * (RR + 4) * sizeof(float);     \
@@ -591,7 +592,7 @@ int launch_scan_cols(int R, dim3 grid, cudaStream_t s, const float* q, int ldq, 
         return de_launch(scan_kernel<VT, RR, MODE, COLS, LANES>, grid, dim3(COLS * LANES),      \
                          smem, s, q, ldq, k, ldk, v, ldv, g, ldg, beta, ldb, z, ldz, decay, state, \
                          slot_stride, out, seq_slot, seq_qstart, seq_qlen, H, rep, dk, dv,      \
-                         vec16, keep);                                                          \
+                         vec16, longest, keep);                                                          \
     } while (0)
     if (R <= 8) SCAN(8);
     if (R <= 16) SCAN(16);
@@ -618,7 +619,7 @@ int launch_scan(cudaStream_t s, const float* q, int ldq, const float* k, int ldk
                 int ldz, const float* decay,
                 float* state, long long slot_stride, float* out, const int* seq_slot,
                 const int* seq_qstart, const int* seq_qlen, int n_seqs, int H, int rep, int dk,
-                int dv, ConvKeep keep) {
+                int dv, int longest, ConvKeep keep) {
     const int vec16 = (dk % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && (MODE == 0 || ldg % 4 == 0) &&
                        (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 &&
                        (MODE == 0 || (uintptr_t)g % 16 == 0) &&
@@ -628,7 +629,7 @@ int launch_scan(cudaStream_t s, const float* q, int ldq, const float* k, int ldk
     return launch_scan_cols<VT, MODE, CC, LL>(R, grid, s, q, ldq, k, ldk, v, ldv, g, ldg,       \
                                                beta, ldb, z, ldz, decay, state, slot_stride, out, \
                                                seq_slot, seq_qstart, seq_qlen, H, rep, dk, dv, \
-                                               vec16, keep)
+                                               vec16, longest, keep)
     // (eight lanes a column - twice the warps, half the instructions a token and warp - was
     // measured for a single long prompt and is slower: 867 against 788 us for 2,048 tokens of 16
     // heads of 128 x 128; a token's time is its chain of dependent steps, which a third butterfly
@@ -715,7 +716,8 @@ DE_EXPORT int de_retention_prep(int dtype, const void* proj, int ld, const int* 
 // [N, ldz] and in beta's place the heads' (z . r, k . r) [N, 2 H] (the generalized delta rule);
 // 0: decay [H].  conv_taps > 1: the slots also keep the
 // last conv_taps - 1 rows of the first conv_channels columns of conv_proj (of type conv_dtype,
-// row stride conv_ld) at conv_offset of their state row.
+// row stride conv_ld) at conv_offset of their state row.  Sequences with more than `longest` tokens
+// only have their kept rows moved on: their states have gone by chunks.
 DE_EXPORT int de_state_scan(int mode, int v_dtype, const float* q, int ldq, const float* k,
                             int ldk, const void* v, int ldv, const float* g, int ldg,
                             const float* beta, int ldb, const float* z, int ldz,
@@ -723,7 +725,7 @@ DE_EXPORT int de_state_scan(int mode, int v_dtype, const float* q, int ldq, cons
                             const int* seq_slot, const int* seq_qstart, const int* seq_qlen,
                             int n_seqs, int H, int rep, int dk, int dv, const void* conv_proj,
                             int conv_ld, int conv_dtype, int conv_offset, int conv_channels,
-                            int conv_taps, void* stream) {
+                            int conv_taps, int longest, void* stream) {
     if (n_seqs <= 0) return 0;
     if (dk <= 0 || dk > 256 || dv <= 0 || H <= 0 || rep <= 0 || H % rep) return -2;
     if (mode < 0 || mode > 2) return -2;
@@ -732,7 +734,7 @@ DE_EXPORT int de_state_scan(int mode, int v_dtype, const float* q, int ldq, cons
                      conv_channels, conv_proj ? conv_taps : 0};
 #define SCAN_ARGS(VT)                                                                           \
     s, q, ldq, k, ldk, (const VT*)v, ldv, g, ldg, beta, ldb, z, ldz, decay, state, slot_stride, \
-        out, seq_slot, seq_qstart, seq_qlen, n_seqs, H, rep, dk, dv, keep
+        out, seq_slot, seq_qstart, seq_qlen, n_seqs, H, rep, dk, dv, longest, keep
     if (mode == 1) {
         if (v_dtype != DE_F32) return -4;
         return launch_scan<float, 1>(SCAN_ARGS(float));

@@ -1,0 +1,784 @@
+// Longer portions through the mixers that carry a matrix state per head, in chunks of 64 tokens
+// instead of token by token (recurrent.cu has the rules and the token-by-token scan): what depends
+// on a chunk's own tokens is formed for all chunks side by side, and only a short chain runs from
+// chunk to chunk.  Float32 multiply-adds throughout.
+//
+// A fixed decay per head (retention, lightning attention), S <- d S + k v^T, o = S^T q, with t and s
+// the places inside the chunk and S0 the state before it:
+//   o_t = d^(t+1) S0^T q_t + sum over s <= t of d^(t-s) (q_t . k_s) v_s
+//   S   = d^n S0 + sum over s of d^(n-1-s) k_s v_s^T
+//
+// The delta rule with a decay g_t per key channel, S <- diag(g_t) S; u_t = beta_t (v_t - S^T k_t);
+// S <- S + k_t u_t^T; o_t = S^T q_t, with b_t the product of g_0 .. g_t (channel by channel) and
+// w_ts = (b_t / b_s) k_s:
+//   A_ts = k_t . w_ts (s < t),  P_ts = q_t . w_ts (s <= t)
+//   u = X_v - X_k S0, where X solves (1 + diag(beta) A) X = diag(beta) [v | b k]
+//   o = (b q) S0 + P u,   S = diag(b_n) S0 + sum over s of (b_n / b_s) k_s u_s^T
+// No quotient is formed: b_t / b_s is the product of the decays between, walked channel by channel
+// (w_ts from w_(t-1)s), so nothing overflows however fast the state decays.
+//
+// A cut of a portion changes the order of float32 sums only.
+
+#include "common.cuh"
+
+DE_DEFINE_PDL_SWITCH
+
+namespace {
+
+constexpr int CH = 64;             // tokens of a chunk
+constexpr int LD = CH + 4;         // a row of 64 in shared memory
+
+struct Item {                      // a chunk
+    int seq, token, count, portion;
+};
+struct Portion {
+    int seq, first, chunks, pad;   // its first item and how many
+};
+
+__device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int bytes = ok ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void cp4(float* dst, const float* src, bool ok) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int bytes = ok ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+// two IEEE multiply-adds in one instruction
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a,
+                                     unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpair(unsigned long long v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ float4 four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// A tile of 64 x 64 on 128 threads: a thread has rows row .. row + 3, row + 16 .. row + 19 and
+// columns col .. col + 3.  Lanes l and l ^ 1 share rows, l and l ^ 2 columns, so that 16-byte reads
+// of shared memory pass in two wavefronts.
+struct Tile {
+    unsigned long long acc[8][2];
+    int row, col;
+    __device__ __forceinline__ Tile() {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        row = (warp >> 1) * 32 + (((lane >> 1) & 1) | ((lane >> 3) & 2)) * 4;
+        col = (warp & 1) * 32 + ((lane & 1) | ((lane >> 1) & 6)) * 4;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = 0ull;
+    }
+    // rows of a [k][LD] against columns of b [k][LD], n values of k
+    template <int N> __device__ __forceinline__ void add(const float* a, const float* b) {
+#pragma unroll 8
+        for (int k = 0; k < N; ++k) {
+            const float4 a0 = four(a + k * LD + row), a1 = four(a + k * LD + row + 16);
+            const float4 b0 = four(b + k * LD + col);
+            const float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const unsigned long long p0 = pair(b0.x, b0.y), p1 = pair(b0.z, b0.w);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const unsigned long long aa = pair(v[i], v[i]);
+                fma2(acc[i][0], aa, p0);
+                fma2(acc[i][1], aa, p1);
+            }
+        }
+    }
+    __device__ __forceinline__ int row_of(int i) const { return row + (i & 3) + (i >> 2) * 16; }
+    __device__ __forceinline__ float4 get(int i) const {
+        float4 v;
+        unpair(acc[i][0], v.x, v.y);
+        unpair(acc[i][1], v.z, v.w);
+        return v;
+    }
+};
+
+// d^0 .. d^64, products formed in double precision
+__device__ __forceinline__ void powers(float d, float* pw) {
+    if (threadIdx.x <= CH) {
+        double p = 1.0;
+        for (int i = 0; i < (int)threadIdx.x; ++i) p *= (double)d;
+        pw[threadIdx.x] = (float)p;
+    }
+}
+
+// 64 rows of 64 columns (rows beyond `rows` are zeros) into tile [64][LD]; 128 threads
+__device__ __forceinline__ void load_tile(float* tile, const float* src, size_t ld, int rows) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = threadIdx.x + 128 * i, r = e >> 4, c = (e & 15) * 4;
+        cp16(tile + r * LD + c, r < rows ? src + (size_t)r * ld + c : src, r < rows);
+    }
+}
+__device__ __forceinline__ void load_tile(float* tile, const __nv_bfloat16* src, size_t ld,
+                                          int rows) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = threadIdx.x + 128 * i, r = e >> 4, c = (e & 15) * 4;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (r < rows) {
+            const uint2 u = *reinterpret_cast<const uint2*>(src + (size_t)r * ld + c);
+            v = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
+                            __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+        }
+        *reinterpret_cast<float4*>(tile + r * LD + c) = v;
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// A decay per head.  products: pt[item][h][s][t] = d^(t-s) q_t . k_s (0 for s > t) and
+// xt[item][h][c][t] = d^(t+1) q_t[c].  grid (items, H), 128 threads.
+// ------------------------------------------------------------------------------------------
+template <int DK>
+__global__ void __launch_bounds__(128, 3)
+decay_products_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
+                      const float* __restrict__ decay, const Item* __restrict__ items,
+                      float* __restrict__ xt, float* __restrict__ pt, int H) {
+    extern __shared__ __align__(16) float sh[];
+    float* qs = sh;                                  // [DK][LD]
+    float* ks = qs + DK * LD;                        // [DK][LD]
+    __shared__ float pw[CH + 1];
+    const Item it = items[blockIdx.x];
+    const int h = blockIdx.y;
+    powers(decay[h], pw);
+    pdl_wait();
+    // turned on the way in: a warp copies 8 channels of 4 tokens at a time
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int c0 = 0; c0 < DK; c0 += 8)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = (i * 4 + warp) * 4 + (lane >> 3), c = c0 + (lane & 7);
+            const bool ok = t < it.count;
+            const size_t tok = (size_t)(it.token + (ok ? t : 0));
+            cp4(qs + c * LD + t, q + tok * ldq + h * DK + c, ok);
+            cp4(ks + c * LD + t, k + tok * ldk + h * DK + c, ok);
+        }
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();
+    Tile tile;
+    tile.add<DK>(ks, qs);
+    pdl_trigger();
+    const size_t at = (size_t)blockIdx.x * H + h;
+    float* p = pt + at * CH * CH;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int s = tile.row_of(i);
+        float4 v = tile.get(i);
+        const int d = tile.col - s;
+        v.x = d >= 0 ? v.x * pw[d] : 0.0f;
+        v.y = d >= -1 ? v.y * pw[d + 1] : 0.0f;
+        v.z = d >= -2 ? v.z * pw[d + 2] : 0.0f;
+        v.w = d >= -3 ? v.w * pw[d + 3] : 0.0f;
+        *reinterpret_cast<float4*>(p + s * CH + tile.col) = v;
+    }
+    float* x = xt + at * DK * CH;
+    for (int e = threadIdx.x; e < DK * CH / 4; e += 128) {
+        const int c = e >> 4, t = (e & 15) * 4;
+        const float4 v = four(qs + c * LD + t);
+        *reinterpret_cast<float4*>(x + c * CH + t) = make_float4(
+            v.x * pw[t + 1], v.y * pw[t + 2], v.z * pw[t + 3], v.w * pw[t + 4]);
+    }
+}
+
+// What a chunk adds to the state by itself: states[item][h][c][j] = sum_s d^(n-1-s) k_s[c] v_s[j].
+// grid (items, H, DK / 64 * dv / 64), 128 threads.
+template <typename VT>
+__global__ void __launch_bounds__(128, 4)
+decay_states_kernel(const float* __restrict__ k, int ldk, const VT* __restrict__ v, int ldv,
+                    const float* __restrict__ decay, const Item* __restrict__ items,
+                    float* __restrict__ states, int H, int dk, int dv) {
+    __shared__ __align__(16) float ks[CH * LD], vs[CH * LD];
+    __shared__ float pw[CH + 1];
+    const Item it = items[blockIdx.x];
+    const int h = blockIdx.y, cols = dv / 64;
+    const int c0 = (int)blockIdx.z / cols * 64, j0 = (int)blockIdx.z % cols * 64;
+    powers(decay[h], pw);
+    pdl_wait();
+    load_tile(ks, k + (size_t)it.token * ldk + h * dk + c0, ldk, it.count);
+    load_tile(vs, v + (size_t)it.token * ldv + h * dv + j0, ldv, it.count);
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();
+    for (int e = threadIdx.x; e < it.count * 16; e += 128) {
+        const int s = e >> 4;
+        float4* p = reinterpret_cast<float4*>(ks + s * LD + (e & 15) * 4);
+        const float f = pw[it.count - 1 - s];
+        p->x *= f; p->y *= f; p->z *= f; p->w *= f;
+    }
+    __syncthreads();
+    Tile tile;
+    tile.add<CH>(ks, vs);
+    pdl_trigger();
+    float* o = states + (((size_t)blockIdx.x * H + h) * dk + c0) * dv + j0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4*>(o + (size_t)tile.row_of(i) * dv + tile.col) = tile.get(i);
+}
+
+// The states at the chunks' starts: states[item] becomes the state before the chunk, the slot keeps
+// the one after the last.  grid (portions, elements / 1024), 256 threads with four elements each.
+__global__ void __launch_bounds__(256)
+decay_pass_kernel(float* __restrict__ states, const float* __restrict__ decay,
+                  const Item* __restrict__ items, const Portion* __restrict__ portions,
+                  float* __restrict__ state, long long slot_stride,
+                  const int* __restrict__ seq_slot, int H, int size) {
+    const Portion p = portions[blockIdx.x];
+    const int e = ((int)blockIdx.y * 256 + (int)threadIdx.x) * 4;
+    const int last = items[p.first + p.chunks - 1].count;
+    float* slot = state + (size_t)seq_slot[p.seq] * slot_stride;
+    if (e >= H * size) {
+        pdl_wait();
+        return;
+    }
+    const double d = (double)decay[e / size];
+    double f64 = 1.0, flast = 1.0;
+    for (int i = 0; i < CH; ++i) f64 *= d;
+    for (int i = 0; i < last; ++i) flast *= d;
+    const float full = (float)f64, part = (float)flast;
+    pdl_wait();
+    float4 s = four(slot + e);
+    float* base = states + (size_t)p.first * H * size + e;
+    const size_t step = (size_t)H * size;
+#pragma unroll 8
+    for (int n = 0; n < p.chunks; ++n) {
+        const float f = n == p.chunks - 1 ? part : full;
+        const float4 add = four(base + n * step);
+        *reinterpret_cast<float4*>(base + n * step) = s;
+        s.x = fmaf(f, s.x, add.x);
+        s.y = fmaf(f, s.y, add.y);
+        s.z = fmaf(f, s.z, add.z);
+        s.w = fmaf(f, s.w, add.w);
+    }
+    pdl_trigger();
+    *reinterpret_cast<float4*>(slot + e) = s;
+}
+
+// ------------------------------------------------------------------------------------------
+// The delta rule.  What a chunk's tokens give by themselves: at[item][h][s][t] = A_ts,
+// pt[item][h][s][t] = P_ts (0 for s > t), xt[item][h][c][t] = b_t q_t, kd[item][h][t][c] = b_t k_t,
+// kh[item][h][s][c] = (b_n / b_s) k_s and bn[item][h][c] = b_n.  grid (items, H), 128 threads.
+// A thread walks w of two columns s over the tokens, a quarter of the channels each (lanes 8 apart
+// share a column), as the scan walks the state; bound by the reads of a token's three vectors
+// from shared memory, which two columns share.
+// ------------------------------------------------------------------------------------------
+template <int DK>
+__global__ void __launch_bounds__(128, 2)
+delta_chunk_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
+                   const float* __restrict__ g, int ldg, const Item* __restrict__ items,
+                   float* __restrict__ at, float* __restrict__ pt, float* __restrict__ xt,
+                   float* __restrict__ kd, float* __restrict__ kh, float* __restrict__ bn, int H,
+                   int rep) {
+    constexpr int W = DK + 4, R = DK / 16;           // a row in shared memory; quads of a lane
+    extern __shared__ __align__(16) float sh[];
+    float* qs = sh;                                  // [CH][W]
+    float* ks = qs + CH * W;
+    float* gs = ks + CH * W;
+    const Item it = items[blockIdx.x];
+    const int h = blockIdx.y, hk = h / rep;
+    const size_t where = (size_t)blockIdx.x * H + h;
+    pdl_wait();
+    for (int e = threadIdx.x; e < CH * DK / 4; e += 128) {
+        const int t = e / (DK / 4), c = e % (DK / 4) * 4;
+        const bool ok = t < it.count;
+        const size_t tok = (size_t)(it.token + (ok ? t : 0));
+        cp16(qs + t * W + c, q + tok * ldq + hk * DK + c, ok);
+        cp16(ks + t * W + c, k + tok * ldk + hk * DK + c, ok);
+        if (ok) cp16(gs + t * W + c, g + tok * ldg + h * DK + c, true);
+        else *reinterpret_cast<float4*>(gs + t * W + c) = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    }
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();
+    if (threadIdx.x < DK) {
+        const int c = threadIdx.x;
+        float b = 1.0f;
+        float* x = xt + (where * DK + c) * CH;
+        float* d = kd + where * CH * DK + c;
+#pragma unroll 2
+        for (int t = 0; t < CH; t += 4) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                b *= gs[(t + i) * W + c];
+                v[i] = b * qs[(t + i) * W + c];
+                d[(size_t)(t + i) * DK] = b * ks[(t + i) * W + c];
+            }
+            *reinterpret_cast<float4*>(x + t) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+        bn[where * DK + c] = b;
+        float* o = kh + where * CH * DK + c;
+        float r = 1.0f;
+#pragma unroll 4
+        for (int t = CH - 1; t >= 0; --t) {
+            o[(size_t)t * DK] = r * ks[t * W + c];
+            r *= gs[t * W + c];
+        }
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int share = lane >> 3, s0 = warp * 16 + (lane & 7) * 2, s1 = s0 + 1;
+    float w0[4 * R], w1[4 * R];
+#pragma unroll
+    for (int i = 0; i < 4 * R; ++i) w0[i] = w1[i] = 0.0f;
+    float* rows = (share < 2 ? at : pt) + (where * CH + (share & 1 ? s1 : s0)) * CH;
+    for (int t = 0; t < warp * 16; t += 4)
+        *reinterpret_cast<float4*>(rows + t) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int t = warp * 16; t < CH; t += 4) {
+        float keep[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int tt = t + i;
+            float a0 = 0.0f, a1 = 0.0f, p0 = 0.0f, p1 = 0.0f;
+            float c0 = 0.0f, c1 = 0.0f, e0 = 0.0f, e1 = 0.0f;
+            const bool near = tt < warp * 16 + 16;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int o = tt * W + 16 * r + 4 * share;
+                const float4 gg = four(gs + o), kk = four(ks + o), qq = four(qs + o);
+                const float gv[4] = {gg.x, gg.y, gg.z, gg.w}, kv[4] = {kk.x, kk.y, kk.z, kk.w};
+                const float qv[4] = {qq.x, qq.y, qq.z, qq.w};
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    w0[4 * r + x] *= gv[x];
+                    w1[4 * r + x] *= gv[x];
+                }
+                if (near) {                          // (a column begins inside its warp's 16 tokens)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        if (tt == s0) w0[4 * r + x] = kv[x];
+                        if (tt == s1) w1[4 * r + x] = kv[x];
+                    }
+                }
+#pragma unroll
+                for (int x = 0; x < 4; x += 2) {
+                    a0 = fmaf(kv[x], w0[4 * r + x], a0);
+                    c0 = fmaf(kv[x + 1], w0[4 * r + x + 1], c0);
+                    a1 = fmaf(kv[x], w1[4 * r + x], a1);
+                    c1 = fmaf(kv[x + 1], w1[4 * r + x + 1], c1);
+                    p0 = fmaf(qv[x], w0[4 * r + x], p0);
+                    e0 = fmaf(qv[x + 1], w0[4 * r + x + 1], e0);
+                    p1 = fmaf(qv[x], w1[4 * r + x], p1);
+                    e1 = fmaf(qv[x + 1], w1[4 * r + x + 1], e1);
+                }
+            }
+            a0 += c0; a1 += c1; p0 += e0; p1 += e1;
+#pragma unroll
+            for (int m = 8; m < 32; m <<= 1) {
+                a0 += __shfl_xor_sync(0xffffffffu, a0, m);
+                a1 += __shfl_xor_sync(0xffffffffu, a1, m);
+                p0 += __shfl_xor_sync(0xffffffffu, p0, m);
+                p1 += __shfl_xor_sync(0xffffffffu, p1, m);
+            }
+            if (tt <= s0) a0 = 0.0f;                 // A is strictly below the diagonal
+            if (tt <= s1) a1 = 0.0f;
+            keep[i] = share == 0 ? a0 : share == 1 ? a1 : share == 2 ? p0 : p1;
+        }
+        *reinterpret_cast<float4*>(rows + t) = make_float4(keep[0], keep[1], keep[2], keep[3]);
+    }
+    pdl_trigger();
+}
+
+// X of (1 + diag(beta) A) X = diag(beta) [v | b k]: xv[item][h][t][j] and, turned, xkt[item][h][c][t].
+// grid (items, H, ceil((dv + DK) / 128)), 64 threads with two columns each: forward substitution by
+// blocks of 16 tokens, a thread's earlier rows in shared memory of its own.
+template <int DK>
+__global__ void __launch_bounds__(64)
+delta_solve_kernel(const float* __restrict__ at, const float* __restrict__ v, int ldv,
+                   const float* __restrict__ kd, const float* __restrict__ beta, int ldb,
+                   const Item* __restrict__ items, float* __restrict__ xv,
+                   float* __restrict__ xkt, int H, int dv) {
+    extern __shared__ __align__(16) float sh[];
+    float* as = sh;                                  // [CH][LD]: [s][t]
+    float* xs = as + CH * LD;                        // [CH][128]
+    __shared__ float bs[CH];
+    const Item it = items[blockIdx.x];
+    const int h = blockIdx.y;
+    const size_t where = (size_t)blockIdx.x * H + h;
+    const int j = blockIdx.z * 128 + 2 * threadIdx.x;          // columns j, j + 1 of [v | k]
+    const bool live = j < dv + DK, is_v = j < dv;
+    pdl_wait();
+    for (int e = threadIdx.x; e < CH * 16; e += 64)
+        cp16(as + (e >> 4) * LD + (e & 15) * 4, at + where * CH * CH + e * 4, true);
+    cp_commit();
+    bs[threadIdx.x] = (int)threadIdx.x < it.count
+                          ? beta[(size_t)(it.token + threadIdx.x) * ldb + h] : 0.0f;
+    cp_wait<0>();
+    __syncthreads();
+    float* mine = xs + 2 * threadIdx.x;
+    for (int t0 = 0; t0 < CH; t0 += 16) {
+        float2 rhs[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            const int t = t0 + r;
+            rhs[r] = make_float2(0.0f, 0.0f);
+            if (live && t < it.count)
+                rhs[r] = is_v ? *reinterpret_cast<const float2*>(
+                                    v + (size_t)(it.token + t) * ldv + h * dv + j)
+                              : *reinterpret_cast<const float2*>(kd + (where * CH + t) * DK + j - dv);
+        }
+        unsigned long long acc[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) acc[r] = 0ull;
+#pragma unroll 4
+        for (int s = 0; s < t0; ++s) {
+            const unsigned long long x = *reinterpret_cast<const unsigned long long*>(mine + s * 128);
+#pragma unroll
+            for (int r = 0; r < 16; r += 4) {
+                const float4 a = four(as + s * LD + t0 + r);
+                fma2(acc[r], pair(a.x, a.x), x);
+                fma2(acc[r + 1], pair(a.y, a.y), x);
+                fma2(acc[r + 2], pair(a.z, a.z), x);
+                fma2(acc[r + 3], pair(a.w, a.w), x);
+            }
+        }
+        float o0[16], o1[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            float s0, s1;
+            unpair(acc[r], s0, s1);
+            const float b = bs[t0 + r];
+            o0[r] = b * (rhs[r].x - s0);
+            o1[r] = b * (rhs[r].y - s1);
+            const unsigned long long x = pair(o0[r], o1[r]);
+            *reinterpret_cast<unsigned long long*>(mine + (t0 + r) * 128) = x;
+#pragma unroll
+            for (int i = r + 1; i < 16; ++i) {
+                const float a = as[(t0 + r) * LD + t0 + i];
+                fma2(acc[i], pair(a, a), x);
+            }
+        }
+        if (!live) continue;
+        if (is_v) {
+#pragma unroll
+            for (int r = 0; r < 16; ++r)
+                *reinterpret_cast<float2*>(xv + (where * CH + t0 + r) * dv + j) =
+                    make_float2(o0[r], o1[r]);
+        } else {
+            float* o = xkt + (where * DK + j - dv) * CH + t0;
+#pragma unroll
+            for (int r = 0; r < 16; r += 4) {
+                *reinterpret_cast<float4*>(o + r) = make_float4(o0[r], o0[r + 1], o0[r + 2], o0[r + 3]);
+                *reinterpret_cast<float4*>(o + CH + r) =
+                    make_float4(o1[r], o1[r + 1], o1[r + 2], o1[r + 3]);
+            }
+        }
+    }
+    pdl_trigger();
+}
+
+// The chain from chunk to chunk: states[item] = the state before the chunk, u = X_v - X_k S0 in
+// X_v's place, then the state after it.  grid (portions, H, dv / 16), DK threads: a block has 16
+// columns of a head's state, a warp 32 of its rows in registers.  For u every warp sums over its own
+// rows; the warps' parts meet in shared memory.  The next chunk's operands arrive meanwhile.
+constexpr int PC = 16, PLD = PC + 4;
+template <int DK> struct Pass {
+    static constexpr int W = DK + 4;
+    static constexpr int STAGE = DK * LD + CH * W + CH * PLD;  // xkt, kh, xv
+    static constexpr int WARPS = DK / 32;
+    static constexpr size_t SMEM =
+        (size_t)(2 * STAGE + DK * PLD + CH * PLD + WARPS * CH * PLD) * sizeof(float);
+};
+
+template <int DK>
+__global__ void __launch_bounds__(DK)
+delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
+                  const float* __restrict__ bn, float* __restrict__ xv, float* __restrict__ states,
+                  const Portion* __restrict__ portions, float* __restrict__ state,
+                  long long slot_stride, const int* __restrict__ seq_slot, int H, int dv) {
+    constexpr int W = Pass<DK>::W, STAGE = Pass<DK>::STAGE, WARPS = Pass<DK>::WARPS;
+    extern __shared__ __align__(16) float sh[];
+    float* ss = sh + 2 * STAGE;                      // [DK][PLD]: the state before the chunk
+    float* us = ss + DK * PLD;                       // [CH][PLD]
+    float* red = us + CH * PLD;                      // [WARPS][CH][PLD]
+    const Portion p = portions[blockIdx.x];
+    const int h = blockIdx.y, j0 = blockIdx.z * PC;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // eight groups of four rows (or of four tokens and four more 32 on) by four of four columns; lanes
+    // l and l ^ 2 share the former, l and l ^ 1 the latter
+    const int a4 = ((lane & 1) | ((lane >> 1) & 6)) * 4, j4 = (((lane >> 1) & 1) | ((lane >> 3) & 2)) * 4;
+    const int c0 = warp * 32 + a4;
+    pdl_wait();
+    float* slot = state + (size_t)seq_slot[p.seq] * slot_stride + (size_t)h * DK * dv + j0;
+    auto load = [&](int n) {
+        float* st = sh + (n & 1) * STAGE;
+        const size_t where = (size_t)(p.first + n) * H + h;
+        const float* a = xkt + where * DK * CH;
+        const float* b = kh + where * CH * DK;
+        const float* x = xv + where * CH * dv + j0;
+        for (int e = threadIdx.x; e < DK * 16; e += DK)
+            cp16(st + (e >> 4) * LD + (e & 15) * 4, a + e * 4, true);
+        for (int e = threadIdx.x; e < CH * DK / 4; e += DK)
+            cp16(st + DK * LD + e / (DK / 4) * W + e % (DK / 4) * 4, b + e * 4, true);
+        for (int e = threadIdx.x; e < CH * 4; e += DK)
+            cp16(st + DK * LD + CH * W + (e >> 2) * PLD + (e & 3) * 4,
+                 x + (size_t)(e >> 2) * dv + (e & 3) * 4, true);
+        cp_commit();
+    };
+    load(0);
+    float4 S[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S[i] = four(slot + (size_t)(c0 + i) * dv + j4);
+    for (int n = 0; n < p.chunks; ++n) {
+        const size_t where = (size_t)(p.first + n) * H + h;
+        const float4 b = four(bn + where * DK + c0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            *reinterpret_cast<float4*>(states + (where * DK + c0 + i) * dv + j0 + j4) = S[i];
+            *reinterpret_cast<float4*>(ss + (c0 + i) * PLD + j4) = S[i];
+        }
+        cp_wait<0>();
+        __syncthreads();                 // the chunk has landed, the one before it has been used
+        if (n + 1 < p.chunks) load(n + 1);
+        const float* st = sh + (n & 1) * STAGE;
+        {
+            // X_k S0 over this warp's rows of the state
+            unsigned long long acc[8][2];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = 0ull;
+            const float* xa = st + warp * 32 * LD + a4;
+            const float* sb = ss + warp * 32 * PLD + j4;
+#pragma unroll 8
+            for (int c = 0; c < 32; ++c) {
+                const float4 t0 = four(xa + c * LD), t1 = four(xa + c * LD + 32);
+                const float4 y = four(sb + c * PLD);
+                const float v[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+                const unsigned long long y0 = pair(y.x, y.y), y1 = pair(y.z, y.w);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const unsigned long long vv = pair(v[i], v[i]);
+                    fma2(acc[i][0], vv, y0);
+                    fma2(acc[i][1], vv, y1);
+                }
+            }
+            float* rd = red + warp * CH * PLD + j4;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float4 r;
+                unpair(acc[i][0], r.x, r.y);
+                unpair(acc[i][1], r.z, r.w);
+                *reinterpret_cast<float4*>(rd + (a4 + (i & 3) + (i >> 2) * 32) * PLD) = r;
+            }
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < CH * 4; e += DK) {
+            const int t = e >> 2, c = (e & 3) * 4;
+            float4 u = four(st + DK * LD + CH * W + t * PLD + c);
+            float4 sum = four(red + t * PLD + c);
+#pragma unroll
+            for (int w = 1; w < WARPS; ++w) {
+                const float4 r = four(red + (w * CH + t) * PLD + c);
+                sum.x += r.x; sum.y += r.y; sum.z += r.z; sum.w += r.w;
+            }
+            u.x -= sum.x; u.y -= sum.y; u.z -= sum.z; u.w -= sum.w;
+            *reinterpret_cast<float4*>(us + t * PLD + c) = u;
+            *reinterpret_cast<float4*>(xv + (where * CH + t) * dv + j0 + c) = u;
+        }
+        __syncthreads();
+        {
+            // S <- diag(b_n) S + sum over the tokens of kh u
+            unsigned long long acc[4][2];
+            const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
+            const float* ka = st + DK * LD + c0;
+#pragma unroll 8
+            for (int s = 0; s < CH; ++s) {
+                const float4 kk = four(ka + s * W), u = four(us + s * PLD + j4);
+                const float v[4] = {kk.x, kk.y, kk.z, kk.w};
+                const unsigned long long u0 = pair(u.x, u.y), u1 = pair(u.z, u.w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const unsigned long long vv = pair(v[i], v[i]);
+                    fma2(acc[i][0], vv, u0);
+                    fma2(acc[i][1], vv, u1);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float4 d;
+                unpair(acc[i][0], d.x, d.y);
+                unpair(acc[i][1], d.z, d.w);
+                S[i].x = fmaf(bv[i], S[i].x, d.x);
+                S[i].y = fmaf(bv[i], S[i].y, d.y);
+                S[i].z = fmaf(bv[i], S[i].z, d.z);
+                S[i].w = fmaf(bv[i], S[i].w, d.w);
+            }
+        }
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(slot + (size_t)(c0 + i) * dv + j4) = S[i];
+}
+
+// ------------------------------------------------------------------------------------------
+// The read-outs, both rules: out[t][j] = sum_c xt[c][t] S0[c][j] + sum_s pt[s][t] u_s[j].
+// grid (items, H, dv / 64), 128 threads; steps of 64 through two stages.  u: rows of the step
+// (u_by_item 0) or of the chunks' own rows [item][h][64][dv].
+// ------------------------------------------------------------------------------------------
+template <typename VT>
+__global__ void __launch_bounds__(128, 3)
+chunk_out_kernel(const float* __restrict__ xt, const float* __restrict__ states,
+                 const float* __restrict__ pt, const VT* __restrict__ u, int ldu, int u_by_item,
+                 const Item* __restrict__ items, float* __restrict__ out, int H, int dk, int dv) {
+    extern __shared__ __align__(16) float sh[];      // [2][2][64][LD]
+    const Item it = items[blockIdx.x];
+    const int h = blockIdx.y, j0 = blockIdx.z * 64;
+    const size_t at = (size_t)blockIdx.x * H + h;
+    const int steps = dk / 64 + 1;
+    pdl_wait();
+    auto load = [&](int step) {
+        float* a = sh + (step & 1) * 2 * CH * LD;
+        float* b = a + CH * LD;
+        if (step + 1 < steps) {
+            load_tile(a, xt + (at * dk + step * 64) * CH, CH, 64);
+            load_tile(b, states + (at * dk + step * 64) * dv + j0, dv, 64);
+        } else {
+            load_tile(a, pt + at * CH * CH, CH, 64);
+            if (u_by_item) load_tile(b, u + at * CH * dv + j0, dv, it.count);
+            else load_tile(b, u + (size_t)it.token * ldu + h * dv + j0, ldu, it.count);
+        }
+        cp_commit();
+    };
+    load(0);
+    Tile tile;
+    for (int step = 0; step < steps; ++step) {
+        if (step + 1 < steps) load(step + 1);
+        else cp_commit();
+        cp_wait<1>();
+        __syncthreads();
+        const float* a = sh + (step & 1) * 2 * CH * LD;
+        tile.add<CH>(a, a + CH * LD);
+        __syncthreads();
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = tile.row_of(i);
+        if (t < it.count)
+            *reinterpret_cast<float4*>(out + (size_t)(it.token + t) * (H * dv) + h * dv + j0 +
+                                       tile.col) = tile.get(i);
+    }
+}
+
+}  // namespace
+
+DE_EXPORT int de_chunk_tokens() { return CH; }
+
+// Whether portions of these sizes go by chunks: the state's rows are 64 or 128 key channels and its
+// columns whole tiles of 64.
+DE_EXPORT int de_chunk_ok(int dk, int dv) { return (dk == 64 || dk == 128) && dv > 0 && dv % 64 == 0; }
+
+static int need_smem(const void* kernel, size_t bytes) {
+    return bytes > 48 * 1024
+               ? (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)bytes)
+               : 0;
+}
+
+// The read-outs and the new states of the portions in `items` / `portions` under a decay per head.
+// Workspaces: xt [m, H, dk, 64], pt [m, H, 64, 64], states [m, H, dk, dv].
+DE_EXPORT int de_decay_chunks(int v_dtype, const float* q, int ldq, const float* k, int ldk,
+                              const void* v, int ldv, const float* decay, const int* items, int m,
+                              const int* portions, int n_portions, float* xt, float* pt,
+                              float* states, float* state, long long slot_stride,
+                              const int* seq_slot, float* out, int H, int dk, int dv, void* stream) {
+    if (m <= 0 || n_portions <= 0) return 0;
+    if (!de_chunk_ok(dk, dv) || ldk % 4 || ldv % 4 || (uintptr_t)k % 16 ||
+        (uintptr_t)v % (v_dtype == DE_BF16 ? 8 : 16) || slot_stride % 4 || (uintptr_t)state % 16)
+        return -2;
+    cudaStream_t s = (cudaStream_t)stream;
+    const Item* it = (const Item*)items;
+    const Portion* po = (const Portion*)portions;
+    const size_t psmem = (size_t)2 * dk * LD * sizeof(float);
+    int e;
+#define RUN(...)                                                                                \
+    do {                                                                                        \
+        if ((e = (__VA_ARGS__)) != 0) return e;                                                 \
+    } while (0)
+    if (dk == 64) {
+        RUN(need_smem((const void*)decay_products_kernel<64>, psmem));
+        RUN(de_launch(decay_products_kernel<64>, dim3(m, H), dim3(128), psmem, s, q, ldq, k, ldk,
+                      decay, it, xt, pt, H));
+    } else {
+        RUN(need_smem((const void*)decay_products_kernel<128>, psmem));
+        RUN(de_launch(decay_products_kernel<128>, dim3(m, H), dim3(128), psmem, s, q, ldq, k, ldk,
+                      decay, it, xt, pt, H));
+    }
+    const dim3 grid(m, H, dk / 64 * (dv / 64)), ogrid(m, H, dv / 64);
+    const size_t osmem = (size_t)4 * CH * LD * sizeof(float);
+    const dim3 pgrid(n_portions, (H * dk * dv / 4 + 255) / 256);
+    if (v_dtype == DE_BF16)
+        RUN(de_launch(decay_states_kernel<__nv_bfloat16>, grid, dim3(128), 0, s, k, ldk,
+                      (const __nv_bfloat16*)v, ldv, decay, it, states, H, dk, dv));
+    else
+        RUN(de_launch(decay_states_kernel<float>, grid, dim3(128), 0, s, k, ldk, (const float*)v,
+                      ldv, decay, it, states, H, dk, dv));
+    RUN(de_launch(decay_pass_kernel, pgrid, dim3(256), 0, s, states, decay, it, po, state,
+                  slot_stride, seq_slot, H, dk * dv));
+    if (v_dtype == DE_BF16) {
+        RUN(need_smem((const void*)chunk_out_kernel<__nv_bfloat16>, osmem));
+        RUN(de_launch(chunk_out_kernel<__nv_bfloat16>, ogrid, dim3(128), osmem, s, xt, states, pt,
+                      (const __nv_bfloat16*)v, ldv, 0, it, out, H, dk, dv));
+    } else {
+        RUN(need_smem((const void*)chunk_out_kernel<float>, osmem));
+        RUN(de_launch(chunk_out_kernel<float>, ogrid, dim3(128), osmem, s, xt, states, pt,
+                      (const float*)v, ldv, 0, it, out, H, dk, dv));
+    }
+    return 0;
+}
+
+// The same for the delta rule: g [N, ldg] decays, beta [N, ldb], v float32.  Workspaces: at, pt
+// [m, H, 64, 64], xt, kd, kh, xkt [m, H, dk, 64], bn [m, H, dk], xv [m, H, 64, dv], states
+// [m, H, dk, dv].
+DE_EXPORT int de_delta_chunks(const float* q, int ldq, const float* k, int ldk, const float* v,
+                              int ldv, const float* g, int ldg, const float* beta, int ldb,
+                              const int* items, int m, const int* portions, int n_portions,
+                              float* at, float* pt, float* xt, float* kd, float* kh, float* xkt,
+                              float* bn, float* xv, float* states, float* state,
+                              long long slot_stride, const int* seq_slot, float* out, int H,
+                              int rep, int dk, int dv, void* stream) {
+    if (m <= 0 || n_portions <= 0) return 0;
+    if (!de_chunk_ok(dk, dv) || ldq % 4 || ldk % 4 || ldg % 4 || ldv % 2 || (uintptr_t)q % 16 ||
+        (uintptr_t)k % 16 || (uintptr_t)g % 16 || (uintptr_t)v % 8 || slot_stride % 4 ||
+        (uintptr_t)state % 16 || rep <= 0 || H % rep)
+        return -2;
+    cudaStream_t s = (cudaStream_t)stream;
+    const Item* it = (const Item*)items;
+    const Portion* po = (const Portion*)portions;
+    const size_t csmem = (size_t)3 * CH * (dk + 4) * sizeof(float);
+    const size_t ssmem = (size_t)(CH * LD + CH * 128) * sizeof(float);
+    const size_t osmem = (size_t)4 * CH * LD * sizeof(float);
+    const dim3 sgrid(m, H, (dv + dk + 127) / 128), pgrid(n_portions, H, dv / PC);
+    int e;
+#define DELTA(DK)                                                                               \
+    do {                                                                                        \
+        RUN(need_smem((const void*)delta_chunk_kernel<DK>, csmem));                             \
+        RUN(de_launch(delta_chunk_kernel<DK>, dim3(m, H), dim3(128), csmem, s, q, ldq, k, ldk,  \
+                      g, ldg, it, at, pt, xt, kd, kh, bn, H, rep));                             \
+        RUN(need_smem((const void*)delta_solve_kernel<DK>, ssmem));                             \
+        RUN(de_launch(delta_solve_kernel<DK>, sgrid, dim3(64), ssmem, s, (const float*)at, v,   \
+                      ldv, (const float*)kd, beta, ldb, it, xv, xkt, H, dv));                   \
+        RUN(need_smem((const void*)delta_pass_kernel<DK>, Pass<DK>::SMEM));                     \
+        RUN(de_launch(delta_pass_kernel<DK>, pgrid, dim3(DK), Pass<DK>::SMEM, s,                \
+                      (const float*)xkt, (const float*)kh, (const float*)bn, xv, states, po,    \
+                      state, slot_stride, seq_slot, H, dv));                                    \
+    } while (0)
+    if (dk == 64) DELTA(64);
+    else DELTA(128);
+    RUN(need_smem((const void*)chunk_out_kernel<float>, osmem));
+    RUN(de_launch(chunk_out_kernel<float>, dim3(m, H, dv / 64), dim3(128), osmem, s,
+                  (const float*)xt, (const float*)states, (const float*)pt, (const float*)xv, 0, 1,
+                  it, out, H, dk, dv));
+    return 0;
+}

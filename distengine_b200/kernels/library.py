@@ -93,11 +93,17 @@ SIGNATURES: dict[str, dict[str, list]] = {
         "de_conv_state": [I, P, I, P, L, I, P, P, P, I, I, I, P],
         "de_retention_prep": [I, P, I, P, P, I, I, I, P, P, I, P],
         "de_state_scan": [I, I, P, I, P, I, P, I, P, I, P, I, P, I, P, P, L, P, P, P, P, I, I, I,
-                          I, I, P, I, I, I, I, I, P],
+                          I, I, P, I, I, I, I, I, I, P],
         "de_gdelta_prep": [I, P, I, I, I, I, P, P, P, P, P, P, P, P, I, I, I, P],
         "de_silu_rows": [I, P, I, P, I, I, P],
         "de_head_gate": [I, P, P, I, P, P, I, I, I, F, I, P],
         "de_mean_of_normed": [I, P, P, P, P, P, I, I, F, P],
+    },
+    "recurrent_chunks": {
+        "de_chunk_tokens": [], "de_chunk_ok": [I, I],
+        "de_decay_chunks": [I, P, I, P, I, P, I, P, P, I, P, I, P, P, P, P, L, P, P, I, I, I, P],
+        "de_delta_chunks": [P, I, P, I, P, I, P, I, P, I, P, I, P, I, P, P, P, P, P, P, P, P, P, P,
+                            L, P, P, I, I, I, I, P],
     },
     "ssm": {
         "de_ssm_max_state": [], "de_ssm_chunk": [],

@@ -92,7 +92,8 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
                out: torch.Tensor, heads: int, qk_heads: int, key_dim: int, value_dim: int, ctx,
                g: "torch.Tensor | None" = None, beta: "torch.Tensor | None" = None,
                decay: "torch.Tensor | None" = None, keep: "tuple | None" = None,
-               z: "torch.Tensor | None" = None, dots: "torch.Tensor | None" = None) -> None:
+               z: "torch.Tensor | None" = None, dots: "torch.Tensor | None" = None,
+               longest: int = 0) -> None:
     """Walk every sequence's tokens of the step through its state ``state`` [slots, >= H dk dv]
     (float32, rows [h][key channel][value channel] at the front) and write the read-outs, float32
     [N, H dv].  With ``g`` [N, H dk] and ``beta`` [N, H]: the delta rule with a decay per key
@@ -103,7 +104,9 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     float32 or the activation dtype (any row stride).  ``keep`` = (proj, offset, channels, taps):
     the slots also keep, at ``offset`` of their rows, the last ``taps - 1`` rows of the first
     ``channels`` columns of ``proj`` of every sequence (a convolution's inputs, as ``conv_state``
-    does; the kernel before this one has read the old ones)."""
+    does; the kernel before this one has read the old ones).  ``longest`` not 0: sequences with more
+    tokens than that only have their kept rows moved on (``delta_chunks`` / ``decay_chunks`` have
+    walked them)."""
     n = q.shape[0]
     general = z is not None
     delta = g is not None and not general
@@ -147,8 +150,85 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
                              z.stride(0) if general else 0, _ptr(decay), state.data_ptr(),
                              state.stride(0), out.data_ptr(), ctx.seq_slot.data_ptr(),
                              ctx.seq_qstart.data_ptr(), ctx.seq_qlen.data_ptr(), ctx.n_seqs, heads,
-                             heads // qk_heads, key_dim, value_dim, *conv, _stream()),
+                             heads // qk_heads, key_dim, value_dim, *conv,
+                             int(longest) or 0x7fffffff, _stream()),
            "state_scan")
+
+
+CHUNK = 64               # tokens of a chunk of a longer portion
+# portions of at least this many tokens go by chunks (measured on B200, a layer of 16 heads of 128:
+# CHUNK_FIGURES)
+CHUNKED_PORTION = 96
+
+
+def chunks_ok(key_dim: int, value_dim: int) -> bool:
+    """Whether longer portions of these sizes can go by chunks (``csrc/recurrent_chunks.cu``)."""
+    return key_dim in (64, 128) and value_dim % 64 == 0
+
+
+def _chunk_checks(q, k, v, state, out, items, portions, heads, key_dim, value_dim, name) -> None:
+    for t, what in ((q, "q"), (k, "k"), (state, "state"), (out, "out")):
+        _f32(t, what)
+    _i32(items, "items"), _i32(portions, "portions")
+    n = q.shape[0]
+    _need(items.dim() == 2 and items.shape[1] == 4 and portions.dim() == 2
+          and portions.shape[1] == 4, f"{name}: items [m, 4] and portions [.., 4]")
+    _need(v.stride(1) == 1 and v.shape == (n, heads * value_dim) and out.is_contiguous()
+          and tuple(out.shape) == (n, heads * value_dim) and q.shape == k.shape
+          and state.dim() == 2 and state.shape[1] >= heads * key_dim * value_dim,
+          f"{name}: q, k [N, heads dk], v and out [N, H dv], state rows of H dk dv")
+    _need(chunks_ok(key_dim, value_dim), f"{name}: key sizes 64 and 128, value sizes of whole 64")
+
+
+def decay_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor,
+                 out: torch.Tensor, heads: int, key_dim: int, value_dim: int, decay: torch.Tensor,
+                 items: torch.Tensor, portions: torch.Tensor, ctx) -> None:
+    """What ``state_scan`` does with a decay per head, for the portions that ``items`` (int32 [m, 4]:
+    sequence, first token, tokens, 0) and ``portions`` (int32 [.., 4]: sequence, first item, items,
+    0) name, in chunks of ``CHUNK`` tokens.  q, k float32 [N, H dk], v [N, H dv] of any kernel dtype,
+    rows of whole 16-byte pieces."""
+    _chunk_checks(q, k, v, state, out, items, portions, heads, key_dim, value_dim, "decay_chunks")
+    _f32(decay, "decay")
+    _need(decay.shape == (heads,) and decay.is_contiguous() and q.shape[1] == heads * key_dim,
+          "decay_chunks: decay [H], q and k [N, H dk]")
+    m, f32 = items.shape[0], torch.float32
+    xt = ctx.buffer("chunks.xt", (m, heads, key_dim, CHUNK), f32)
+    pt = ctx.buffer("chunks.pt", (m, heads, CHUNK, CHUNK), f32)
+    states = ctx.buffer("chunks.states", (m, heads, key_dim, value_dim), f32)
+    lib = library.load("recurrent_chunks")
+    _check(lib.de_decay_chunks(_tag(v.dtype), q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0),
+                               v.data_ptr(), v.stride(0), decay.data_ptr(), items.data_ptr(), m,
+                               portions.data_ptr(), portions.shape[0], xt.data_ptr(),
+                               pt.data_ptr(), states.data_ptr(), state.data_ptr(),
+                               state.stride(0), ctx.seq_slot.data_ptr(), out.data_ptr(), heads,
+                               key_dim, value_dim, _stream()), "decay_chunks")
+
+
+def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor,
+                 out: torch.Tensor, heads: int, qk_heads: int, key_dim: int, value_dim: int,
+                 g: torch.Tensor, beta: torch.Tensor, items: torch.Tensor, portions: torch.Tensor,
+                 ctx) -> None:
+    """``decay_chunks`` for the delta rule: g [N, H dk] and beta [N, H] as for ``state_scan``, v
+    float32, q and k [N, qk_heads dk]."""
+    _chunk_checks(q, k, v, state, out, items, portions, heads, key_dim, value_dim, "delta_chunks")
+    _f32(g, "g"), _f32(beta, "beta"), _f32(v, "v")
+    n = q.shape[0]
+    _need(q.shape[1] == qk_heads * key_dim and heads % qk_heads == 0
+          and g.shape == (n, heads * key_dim) and beta.shape == (n, heads),
+          "delta_chunks: q, k [N, qk_heads dk], g [N, H dk], beta [N, H]")
+    m, f32 = items.shape[0], torch.float32
+    square, turned = (m, heads, CHUNK, CHUNK), (m, heads, key_dim, CHUNK)
+    work = [ctx.buffer(f"chunks.{name}", shape, f32) for name, shape in (
+        ("at", square), ("pt", square), ("xt", turned), ("kd", turned), ("kh", turned),
+        ("xkt", turned), ("bn", (m, heads, key_dim)), ("xv", (m, heads, CHUNK, value_dim)),
+        ("states", (m, heads, key_dim, value_dim)))]
+    lib = library.load("recurrent_chunks")
+    _check(lib.de_delta_chunks(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(),
+                               v.stride(0), g.data_ptr(), g.stride(0), beta.data_ptr(),
+                               beta.stride(0), items.data_ptr(), m, portions.data_ptr(),
+                               portions.shape[0], *[t.data_ptr() for t in work], state.data_ptr(),
+                               state.stride(0), ctx.seq_slot.data_ptr(), out.data_ptr(), heads,
+                               heads // qk_heads, key_dim, value_dim, _stream()), "delta_chunks")
 
 
 def gdelta_prep(proj: torch.Tensor, r_col: int, k_col: int, a_col: int, wl: torch.Tensor,

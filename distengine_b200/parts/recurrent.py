@@ -43,12 +43,13 @@ projections and what follows the gate are in the activation dtype.
 
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from ..kernels import ops
 from ..kernels import recurrent as rk
 from .base import Mixer, StateSpec, compute_matrix, register_mixer
-from .context import CacheBinding, NormAhead, StepContext, UnscaledRows
+from .context import CacheBinding, NormAhead, StepContext, StepPrep, UnscaledRows
 
 
 def _up8(n: int) -> int:
@@ -140,7 +141,52 @@ class ProjectedMixer(Mixer):
         return out
 
 
-class GatedDeltaRule(ProjectedMixer):
+class ChunkedMixer(ProjectedMixer):
+    """A mixer whose longer portions can go through its state in chunks (``kernels.recurrent``):
+    the step's chunks are the same for layers of all sizes, so one plan serves all of them."""
+
+    prepare_key = "recurrent/chunks"
+
+    def prepare(self, prep: StepPrep) -> None:
+        if "recurrent/chunks" in prep.notes:
+            return
+        qlen, qstart = prep.host.seq_qlen, prep.host.seq_qstart
+        long = np.nonzero(qlen >= rk.CHUNKED_PORTION)[0]
+        # 0: none; else whether there are shorter portions beside them
+        prep.notes["recurrent/chunks"] = 0 if not len(long) else (2 if len(long) < len(qlen) else 1)
+        if not len(long):
+            return
+        count = -(-qlen[long] // rk.CHUNK)
+        first = np.cumsum(count) - count
+        owner = np.repeat(np.arange(len(long)), count)
+        place = (np.arange(int(count.sum())) - first[owner]) * rk.CHUNK
+        items = np.zeros((len(owner), 4), dtype=np.int32)
+        items[:, 0], items[:, 1] = long[owner], qstart[long[owner]] + place
+        items[:, 2] = np.minimum(rk.CHUNK, qlen[long[owner]] - place)
+        portions = np.zeros((len(long), 4), dtype=np.int32)
+        portions[:, 0], portions[:, 1], portions[:, 2] = long, first, count
+        prep.add("recurrent/items", items)
+        prep.add("recurrent/portions", portions)
+
+    def kernel_modules(self):
+        return ("recurrent", "recurrent_chunks")
+
+    def walk(self, q, k, v, state, out, ctx) -> None:
+        """The step's tokens through the states under a fixed decay per head."""
+        chunked = self.chunked(ctx)
+        if chunked:
+            rk.decay_chunks(q, k, v, state, out, self.heads, self.dk, self.dv, self.decay,
+                            ctx.arrays["recurrent/items"], ctx.arrays["recurrent/portions"], ctx)
+        if chunked != 1:
+            rk.state_scan(q, k, v, state, out, self.heads, self.heads, self.dk, self.dv, ctx,
+                          decay=self.decay, longest=rk.CHUNKED_PORTION - 1 if chunked else 0)
+
+    def chunked(self, ctx) -> int:
+        """The step's note: 0 if its portions go token by token."""
+        return ctx.notes.get("recurrent/chunks", 0) if rk.chunks_ok(self.dk, self.dv) else 0
+
+
+class GatedDeltaRule(ChunkedMixer):
     kind = "gated_delta_rule"
 
     def __init__(self, width: int, heads: int, kv_heads: int, key_dim: int, value_dim: int,
@@ -221,15 +267,21 @@ class GatedDeltaRule(ProjectedMixer):
         rk.delta_prep(proj, a, self.conv, self.dt_bias, self.a_log, cache.state, self.state_rows,
                       ctx, qn, kn, vv, beta, gdec, H, G, dk, dv, self.b_col)
         o = ctx.buffer("delta.o", (n, H * dv), f32)
+        chunked = self.chunked(ctx)
+        if chunked:
+            rk.delta_chunks(qn, kn, vv, cache.state, o, H, G, dk, dv, gdec, beta,
+                            ctx.arrays["recurrent/items"], ctx.arrays["recurrent/portions"], ctx)
         # (the scan also moves the slot's kept convolution inputs on: the preparation has read them)
-        rk.state_scan(qn, kn, vv, cache.state, o, H, G, dk, dv, ctx, g=gdec, beta=beta,
-                      keep=(proj, self.state_rows, self.channels, self.taps))
+        if chunked != 1 or self.taps > 1:
+            rk.state_scan(qn, kn, vv, cache.state, o, H, G, dk, dv, ctx, g=gdec, beta=beta,
+                          keep=(proj, self.state_rows, self.channels, self.taps),
+                          longest=rk.CHUNKED_PORTION - 1 if chunked else 0)
         gated = ctx.buffer("delta.gated", (n, H * dv))
         rk.head_gate(o, gate, self.norm, gated, H, dv, self.eps)
         return self.project_out(gated, "delta.out", ctx, ahead, out_dtype=out_dtype)
 
 
-class Retention(ProjectedMixer):
+class Retention(ChunkedMixer):
     kind = "retention"
 
     def __init__(self, width: int, heads: int, key_dim: int, value_dim: int, decay, rotary_dim: int,
@@ -276,8 +328,7 @@ class Retention(ProjectedMixer):
         kr = ctx.buffer("retention.k", (n, H * dk), f32)
         rk.retention_prep(proj, self.inv_freq, self.rotary_dim, H, dk, qr, kr, ctx)
         o = ctx.buffer("retention.o", (n, H * dv), f32)
-        rk.state_scan(qr, kr, proj[:, self.v_col: self.v_col + H * dv], cache.state, o, H, H, dk,
-                      dv, ctx, decay=self.decay)
+        self.walk(qr, kr, proj[:, self.v_col: self.v_col + H * dv], cache.state, o, ctx)
         gated = ctx.buffer("retention.gated", (n, H * dv))
         rk.head_gate(o, proj[:, self.g_col: self.g_col + H * dv], None, gated, H, dv, self.eps)
         return self.project_out(gated, "retention.out", ctx, ahead, out_dtype=out_dtype)
@@ -352,7 +403,7 @@ class GeneralizedDeltaRule(ProjectedMixer):
         return self.project_out(gated, "gdelta.out", ctx, ahead, out_dtype=out_dtype)
 
 
-class LightningAttention(ProjectedMixer):
+class LightningAttention(ChunkedMixer):
     kind = "lightning_attention"
 
     def __init__(self, width: int, heads: int, key_dim: int, value_dim: int, decay, eps: float,
@@ -394,8 +445,8 @@ class LightningAttention(ProjectedMixer):
         qkv = ctx.buffer("lightning.qkv", (n, H * (2 * dk + dv)), f32)
         rk.silu_rows(proj[:, : H * (2 * dk + dv)], qkv)
         o = ctx.buffer("lightning.o", (n, H * dv), f32)
-        rk.state_scan(qkv[:, : H * dk], qkv[:, H * dk: 2 * H * dk], qkv[:, 2 * H * dk:],
-                      cache.state, o, H, H, dk, dv, ctx, decay=self.decay)
+        self.walk(qkv[:, : H * dk], qkv[:, H * dk: 2 * H * dk], qkv[:, 2 * H * dk:], cache.state, o,
+                  ctx)
         gated = ctx.buffer("lightning.gated", (n, H * dv))
         # one root mean square for all heads together: a single "head" as wide as the row
         rk.head_gate(o, proj[:, self.g_col: self.g_col + H * dv], self.norm, gated, 1, H * dv,
