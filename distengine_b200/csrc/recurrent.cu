@@ -99,6 +99,133 @@ __global__ void delta_prep_kernel(const T* __restrict__ proj, int ld, const floa
     pdl_trigger();
 }
 
+// four neighbouring elements
+__device__ __forceinline__ float4 load_four(const float* p) {
+    return *reinterpret_cast<const float4*>(p);
+}
+__device__ __forceinline__ float4 load_four(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
+                       __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void store_four(float* p, const float4& v) {
+    *reinterpret_cast<float4*>(p) = v;
+}
+__device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&a),
+                                              *reinterpret_cast<const unsigned*>(&b));
+}
+
+// The same for steps with portions, in rows of whole groups of four at heads of 64 or 128 channels
+// and up to four taps (KK): a thread has four neighbouring channels and goes through RUN tokens with
+// the last inputs in registers, a head is 16 or 32 lanes of a warp, which form its norm.  The first
+// `conv_blocks` of the blocks do the convolution, 512 channels each, the others the decays (and
+// beta).  grid (runs of tokens, blocks), 128 threads.  2,048 tokens of 6,144 channels and 2,048
+// decays: 55 us (a block a token, a channel at a time: 128).
+constexpr int RUN = 8;
+
+template <typename T, int KK>
+__global__ void __launch_bounds__(128)
+delta_prep_runs_kernel(const T* __restrict__ proj, int ld, const float* __restrict__ a,
+                       const float* __restrict__ taps, const float* __restrict__ dt_bias,
+                       const float* __restrict__ a_log, const float* __restrict__ state,
+                       long long slot_stride, int conv_offset, const int* __restrict__ token_seq,
+                       const int* __restrict__ token_slot, const int* __restrict__ positions,
+                       const int* __restrict__ seq_pos0, float* __restrict__ qn,
+                       float* __restrict__ kn, float* __restrict__ vv, float* __restrict__ beta,
+                       float* __restrict__ gdec, int n_tokens, int H, int G, int dk, int dv,
+                       int b_col, int conv_blocks) {
+    const int n0 = blockIdx.x * RUN, count = min(RUN, n_tokens - n0);
+    const int qk = 2 * G * dk, C = qk + H * dv;
+    pdl_wait();
+    if ((int)blockIdx.y >= conv_blocks) {
+        const int c = ((int)blockIdx.y - conv_blocks) * 512 + (int)threadIdx.x * 4;
+        if (c < H * dk) {
+            const float rate = expf(a_log[c / dk]);
+            const float4 bias = load_four(dt_bias + c);
+#pragma unroll 4
+            for (int i = 0; i < count; ++i) {
+                const size_t at = (size_t)(n0 + i) * (H * dk) + c;
+                float4 x = load_four(a + at);
+                x.x = expf(-rate * softplus_f(x.x + bias.x));
+                x.y = expf(-rate * softplus_f(x.y + bias.y));
+                x.z = expf(-rate * softplus_f(x.z + bias.z));
+                x.w = expf(-rate * softplus_f(x.w + bias.w));
+                store_four(gdec + at, x);
+            }
+        }
+        if ((int)blockIdx.y == conv_blocks)
+            for (int e = threadIdx.x; e < count * H; e += 128) {
+                const size_t n = n0 + e / H;
+                beta[n * H + e % H] = sigmoid_f(to_float(proj[n * ld + b_col + e % H]));
+            }
+        pdl_trigger();
+        return;
+    }
+    const int c = (int)blockIdx.y * 512 + (int)threadIdx.x * 4;
+    if (c >= C) return;                              // (whole warps: C is a multiple of 128)
+    float w[KK][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < KK; ++j) w[j][e] = taps[(c + e) * KK + j];
+    float4 in[RUN];
+#pragma unroll
+    for (int i = 0; i < RUN; ++i)
+        in[i] = i < count ? load_four(proj + (size_t)(n0 + i) * ld + c)
+                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float q_scale = 1.0f / sqrtf((float)dk);
+    float x[KK][4];                                  // the token's input last
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+        if (i >= count) break;
+        const int n = n0 + i;
+        const int off = positions[n] - seq_pos0[token_seq[n]];
+        if (i == 0 || off == 0) {
+            // the inputs before this token: of its portion, or what the slot keeps
+            const float* kept = state + (size_t)token_slot[n] * slot_stride + conv_offset;
+#pragma unroll
+            for (int j = 0; j + 1 < KK; ++j) {
+                const int rel = off - (KK - 1) + j;
+                const float4 v = rel >= 0 ? load_four(proj + (size_t)(n - (KK - 1) + j) * ld + c)
+                                          : load_four(kept + (size_t)(off + j) * C + c);
+                x[j][0] = v.x; x[j][1] = v.y; x[j][2] = v.z; x[j][3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j + 1 < KK; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[j][e] = x[j + 1][e];
+        }
+        x[KK - 1][0] = in[i].x; x[KK - 1][1] = in[i].y;
+        x[KK - 1][2] = in[i].z; x[KK - 1][3] = in[i].w;
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int j = 0; j < KK; ++j) acc = fmaf(w[j][e], x[j][e], acc);
+            y[e] = silu_f(acc);
+        }
+        if (c >= qk) {
+            store_four(vv + (size_t)n * (H * dv) + c - qk, make_float4(y[0], y[1], y[2], y[3]));
+            continue;
+        }
+        float ss = fmaf(y[0], y[0], fmaf(y[1], y[1], fmaf(y[2], y[2], y[3] * y[3])));
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (dk == 128) ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+        const float inv = 1.0f / sqrtf(ss + 1e-6f);
+        const bool is_q = c < G * dk;
+        float* dst = is_q ? qn + (size_t)n * (G * dk) + c : kn + (size_t)n * (G * dk) + c - G * dk;
+        const float more = is_q ? q_scale : 1.0f;
+        store_four(dst, make_float4((y[0] * inv) * more, (y[1] * inv) * more, (y[2] * inv) * more,
+                                    (y[3] * inv) * more));
+    }
+    pdl_trigger();
+}
+
 // After a step: the slot keeps the last K - 1 inputs of the convolution.  One block a sequence.
 template <typename T>
 __global__ void conv_state_kernel(const T* __restrict__ proj, int ld, float* __restrict__ state,
@@ -218,6 +345,32 @@ __global__ void silu_rows_kernel(const T* __restrict__ proj, int ld, float* __re
         const size_t n = idx / cols;
         const int i = (int)(idx - n * cols);
         out[idx] = silu_f(to_float(proj[n * ld + i]));
+    }
+}
+
+// The same in rows of whole groups of four: 2,048 rows of 6,144 columns 25 us (an element a
+// thread: 38).
+template <typename T>
+__global__ void __launch_bounds__(256)
+silu_rows_vec_kernel(const T* __restrict__ proj, int ld, float* __restrict__ out, unsigned quads,
+                     unsigned total) {
+    pdl_wait();
+    pdl_trigger();
+    const unsigned step = gridDim.x * 256;
+    for (unsigned first = blockIdx.x * 256 + threadIdx.x; first < total; first += 4 * step) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const unsigned e = first + u * step;
+            if (e < total) v[u] = load_four(proj + (size_t)(e / quads) * ld + e % quads * 4);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const unsigned e = first + u * step;
+            if (e < total)
+                store_four(out + (size_t)e * 4, make_float4(silu_f(v[u].x), silu_f(v[u].y),
+                                                            silu_f(v[u].z), silu_f(v[u].w)));
+        }
     }
 }
 
@@ -574,6 +727,44 @@ __global__ void row_gate_kernel(const float* __restrict__ o, const T* __restrict
             x[j] * inv * weight[j] * sigmoid_f(to_float(gate[(size_t)n * ld_gate + j])));
 }
 
+// The same for rows of whole groups of four, up to 1,024 NQ elements, kept in registers between the
+// sum and the result: a block a token, 2,048 rows of 2,048 10 us (an element a thread, the row
+// read twice: 20).
+template <typename T, int NQ>
+__global__ void __launch_bounds__(256)
+row_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, int ld_gate,
+                    const float* __restrict__ weight, T* __restrict__ out, int dv, float eps) {
+    __shared__ float scratch[33];
+    const int n = blockIdx.x;
+    const float* x = o + (size_t)n * dv;
+    pdl_wait();
+    float4 v[NQ], g[NQ];
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        const int j = ((int)threadIdx.x + 256 * i) * 4;
+        v[i] = g[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (j < dv) {
+            v[i] = load_four(x + j);
+            g[i] = load_four(gate + (size_t)n * ld_gate + j);
+        }
+        ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
+    }
+    const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)dv + eps);
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        const int j = ((int)threadIdx.x + 256 * i) * 4;
+        if (j >= dv) continue;
+        const float4 w = load_four(weight + j);
+        store_four(out + (size_t)n * dv + j,
+                   make_float4(v[i].x * inv * w.x * sigmoid_f(g[i].x),
+                               v[i].y * inv * w.y * sigmoid_f(g[i].y),
+                               v[i].z * inv * w.z * sigmoid_f(g[i].z),
+                               v[i].w * inv * w.w * sigmoid_f(g[i].w)));
+    }
+}
+
 template <typename VT, int MODE, int COLS, int LANES>
 int launch_scan_cols(int R, dim3 grid, cudaStream_t s, const float* q, int ldq, const float* k,
                      int ldk, const VT* v, int ldv, const float* g, int ldg, const float* beta,
@@ -668,6 +859,32 @@ DE_EXPORT int de_delta_prep(int dtype, const void* proj, int ld, const float* a,
                 : cudaFuncSetAttribute(delta_prep_kernel<float>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
+    }
+    // steps with portions: four channels a thread, eight tokens a block
+    const int esize = dtype == DE_BF16 ? 2 : 4;
+    if (n >= 128 && K <= 4 && (dk == 64 || dk == 128) && (G * dk) % 128 == 0 && (H * dv) % 128 == 0 &&
+        ld % 4 == 0 && (uintptr_t)proj % (4 * esize) == 0 && (uintptr_t)a % 16 == 0 &&
+        (uintptr_t)dt_bias % 16 == 0 && (uintptr_t)state % 16 == 0 && slot_stride % 4 == 0 &&
+        conv_offset % 4 == 0 && (uintptr_t)qn % 16 == 0 && (uintptr_t)kn % 16 == 0 &&
+        (uintptr_t)vv % 16 == 0 && (uintptr_t)gdec % 16 == 0) {
+        const int conv_blocks = (2 * G * dk + H * dv + 511) / 512;
+        const dim3 grid((n + RUN - 1) / RUN, conv_blocks + (H * dk + 511) / 512);
+#define RUNS(T, KK)                                                                             \
+    return de_launch(delta_prep_runs_kernel<T, KK>, grid, dim3(128), 0, s, (const T*)proj, ld, a, \
+                     taps, dt_bias, a_log, state, slot_stride, conv_offset, token_seq,          \
+                     token_slot, positions, seq_pos0, qn, kn, vv, beta, gdec, n, H, G, dk, dv,  \
+                     b_col, conv_blocks)
+#define RUNS_K(T)                                                                               \
+    do {                                                                                        \
+        if (K == 1) RUNS(T, 1);                                                                 \
+        if (K == 2) RUNS(T, 2);                                                                 \
+        if (K == 3) RUNS(T, 3);                                                                 \
+        RUNS(T, 4);                                                                             \
+    } while (0)
+        if (dtype == DE_BF16) RUNS_K(__nv_bfloat16);
+        RUNS_K(float);
+#undef RUNS_K
+#undef RUNS
     }
     // a block a token: many threads, so that a token of a decode step is a few rounds of loads
     // (with few tokens: steps of many tokens fill the GPU with blocks of 256)
@@ -770,6 +987,16 @@ DE_EXPORT int de_silu_rows(int dtype, const void* proj, int ld, float* out, int 
     if (n <= 0 || cols <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t total = (size_t)n * cols;
+    if (cols % 4 == 0 && ld % 4 == 0 && (uintptr_t)proj % (dtype == DE_BF16 ? 8 : 16) == 0 &&
+        (uintptr_t)out % 16 == 0 && total / 4 < (1u << 30)) {
+        const unsigned quads = (unsigned)(total / 4), fours = (quads + 1023) / 1024;
+        const dim3 grid(fours < 148 * 8 ? fours : 148 * 8);
+        if (dtype == DE_BF16)
+            return de_launch(silu_rows_vec_kernel<__nv_bfloat16>, grid, dim3(256), 0, s,
+                             (const __nv_bfloat16*)proj, ld, out, (unsigned)cols / 4, quads);
+        return de_launch(silu_rows_vec_kernel<float>, grid, dim3(256), 0, s, (const float*)proj, ld,
+                         out, (unsigned)cols / 4, quads);
+    }
     size_t blocks = (total + 255) / 256;
     if (blocks > 148 * 32) blocks = 148 * 32;
     if (dtype == DE_BF16)
@@ -786,6 +1013,22 @@ DE_EXPORT int de_head_gate(int dtype, const float* o, const void* gate, int ld_g
     cudaStream_t s = (cudaStream_t)stream;
     if (mode == 2 && H == 1 && dv > 256) {
         const int threads = dv >= 2048 ? 512 : 256;
+        const size_t piece = dtype == DE_BF16 ? 8 : 16;
+        if (dv % 4 == 0 && dv <= 4096 && ld_gate % 4 == 0 && (uintptr_t)o % 16 == 0 &&
+            (uintptr_t)weight % 16 == 0 && (uintptr_t)gate % piece == 0 && (uintptr_t)out % piece == 0) {
+#define GATE(T, NQ)                                                                             \
+    return de_launch(row_gate_vec_kernel<T, NQ>, dim3(n), dim3(256), 0, s, o, (const T*)gate,   \
+                     ld_gate, weight, (T*)out, dv, eps)
+            if (dtype == DE_BF16) {
+                if (dv <= 1024) GATE(__nv_bfloat16, 1);
+                if (dv <= 2048) GATE(__nv_bfloat16, 2);
+                GATE(__nv_bfloat16, 4);
+            }
+            if (dv <= 1024) GATE(float, 1);
+            if (dv <= 2048) GATE(float, 2);
+            GATE(float, 4);
+#undef GATE
+        }
         if (dtype == DE_BF16)
             return de_launch(row_gate_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0, s, o,
                              (const __nv_bfloat16*)gate, ld_gate, weight, (__nv_bfloat16*)out, dv,

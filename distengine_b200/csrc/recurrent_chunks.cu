@@ -56,6 +56,11 @@ __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long
                                      unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
 }
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ unsigned long long pair(float a, float b) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
@@ -251,15 +256,23 @@ decay_pass_kernel(float* __restrict__ states, const float* __restrict__ decay,
     float4 s = four(slot + e);
     float* base = states + (size_t)p.first * H * size + e;
     const size_t step = (size_t)H * size;
-#pragma unroll 8
-    for (int n = 0; n < p.chunks; ++n) {
-        const float f = n == p.chunks - 1 ? part : full;
-        const float4 add = four(base + n * step);
-        *reinterpret_cast<float4*>(base + n * step) = s;
-        s.x = fmaf(f, s.x, add.x);
-        s.y = fmaf(f, s.y, add.y);
-        s.z = fmaf(f, s.z, add.z);
-        s.w = fmaf(f, s.w, add.w);
+    for (int n0 = 0; n0 < p.chunks; n0 += 8) {       // eight chunks' elements asked for at once
+        float4 add[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            add[i] = n0 + i < p.chunks ? four(base + (n0 + i) * step)
+                                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int n = n0 + i;
+            if (n >= p.chunks) break;
+            const float f = n == p.chunks - 1 ? part : full;
+            *reinterpret_cast<float4*>(base + n * step) = s;
+            s.x = fmaf(f, s.x, add[i].x);
+            s.y = fmaf(f, s.y, add[i].y);
+            s.z = fmaf(f, s.z, add[i].z);
+            s.w = fmaf(f, s.w, add[i].w);
+        }
     }
     pdl_trigger();
     *reinterpret_cast<float4*>(slot + e) = s;
@@ -328,9 +341,9 @@ delta_chunk_kernel(const float* __restrict__ q, int ldq, const float* __restrict
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int share = lane >> 3, s0 = warp * 16 + (lane & 7) * 2, s1 = s0 + 1;
-    float w0[4 * R], w1[4 * R];
+    unsigned long long w0[2 * R], w1[2 * R];         // neighbouring channels in pairs
 #pragma unroll
-    for (int i = 0; i < 4 * R; ++i) w0[i] = w1[i] = 0.0f;
+    for (int i = 0; i < 2 * R; ++i) w0[i] = w1[i] = 0ull;
     float* rows = (share < 2 ? at : pt) + (where * CH + (share & 1 ? s1 : s0)) * CH;
     for (int t = 0; t < warp * 16; t += 4)
         *reinterpret_cast<float4*>(rows + t) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -339,39 +352,40 @@ delta_chunk_kernel(const float* __restrict__ q, int ldq, const float* __restrict
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int tt = t + i;
-            float a0 = 0.0f, a1 = 0.0f, p0 = 0.0f, p1 = 0.0f;
-            float c0 = 0.0f, c1 = 0.0f, e0 = 0.0f, e1 = 0.0f;
+            unsigned long long sa0 = 0ull, sa1 = 0ull, sp0 = 0ull, sp1 = 0ull;
             const bool near = tt < warp * 16 + 16;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const int o = tt * W + 16 * r + 4 * share;
                 const float4 gg = four(gs + o), kk = four(ks + o), qq = four(qs + o);
-                const float gv[4] = {gg.x, gg.y, gg.z, gg.w}, kv[4] = {kk.x, kk.y, kk.z, kk.w};
-                const float qv[4] = {qq.x, qq.y, qq.z, qq.w};
+                const unsigned long long gv[2] = {pair(gg.x, gg.y), pair(gg.z, gg.w)};
+                const unsigned long long kv[2] = {pair(kk.x, kk.y), pair(kk.z, kk.w)};
+                const unsigned long long qv[2] = {pair(qq.x, qq.y), pair(qq.z, qq.w)};
 #pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    w0[4 * r + x] *= gv[x];
-                    w1[4 * r + x] *= gv[x];
+                for (int x = 0; x < 2; ++x) {
+                    w0[2 * r + x] = mul2(w0[2 * r + x], gv[x]);
+                    w1[2 * r + x] = mul2(w1[2 * r + x], gv[x]);
                 }
                 if (near) {                          // (a column begins inside its warp's 16 tokens)
 #pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        if (tt == s0) w0[4 * r + x] = kv[x];
-                        if (tt == s1) w1[4 * r + x] = kv[x];
+                    for (int x = 0; x < 2; ++x) {
+                        if (tt == s0) w0[2 * r + x] = kv[x];
+                        if (tt == s1) w1[2 * r + x] = kv[x];
                     }
                 }
 #pragma unroll
-                for (int x = 0; x < 4; x += 2) {
-                    a0 = fmaf(kv[x], w0[4 * r + x], a0);
-                    c0 = fmaf(kv[x + 1], w0[4 * r + x + 1], c0);
-                    a1 = fmaf(kv[x], w1[4 * r + x], a1);
-                    c1 = fmaf(kv[x + 1], w1[4 * r + x + 1], c1);
-                    p0 = fmaf(qv[x], w0[4 * r + x], p0);
-                    e0 = fmaf(qv[x + 1], w0[4 * r + x + 1], e0);
-                    p1 = fmaf(qv[x], w1[4 * r + x], p1);
-                    e1 = fmaf(qv[x + 1], w1[4 * r + x + 1], e1);
+                for (int x = 0; x < 2; ++x) {
+                    fma2(sa0, kv[x], w0[2 * r + x]);
+                    fma2(sa1, kv[x], w1[2 * r + x]);
+                    fma2(sp0, qv[x], w0[2 * r + x]);
+                    fma2(sp1, qv[x], w1[2 * r + x]);
                 }
             }
+            float a0, a1, p0, p1, c0, c1, e0, e1;
+            unpair(sa0, a0, c0);
+            unpair(sa1, a1, c1);
+            unpair(sp0, p0, e0);
+            unpair(sp1, p1, e1);
             a0 += c0; a1 += c1; p0 += e0; p1 += e1;
 #pragma unroll
             for (int m = 8; m < 32; m <<= 1) {
@@ -453,9 +467,12 @@ delta_solve_kernel(const float* __restrict__ at, const float* __restrict__ v, in
             const unsigned long long x = pair(o0[r], o1[r]);
             *reinterpret_cast<unsigned long long*>(mine + (t0 + r) * 128) = x;
 #pragma unroll
-            for (int i = r + 1; i < 16; ++i) {
-                const float a = as[(t0 + r) * LD + t0 + i];
-                fma2(acc[i], pair(a, a), x);
+            for (int i = (r + 1) & ~3; i < 16; i += 4) {       // (acc up to r has been used)
+                const float4 a = four(as + (t0 + r) * LD + t0 + i);
+                fma2(acc[i], pair(a.x, a.x), x);
+                fma2(acc[i + 1], pair(a.y, a.y), x);
+                fma2(acc[i + 2], pair(a.z, a.z), x);
+                fma2(acc[i + 3], pair(a.w, a.w), x);
             }
         }
         if (!live) continue;
@@ -478,25 +495,26 @@ delta_solve_kernel(const float* __restrict__ at, const float* __restrict__ v, in
 }
 
 // The chain from chunk to chunk: states[item] = the state before the chunk, u = X_v - X_k S0 in
-// X_v's place, then the state after it.  grid (portions, H, dv / 16), DK threads: a block has 16
-// columns of a head's state, a warp 32 of its rows in registers.  For u every warp sums over its own
+// X_v's place, then the state after it.  grid (portions, H, dv / 16), 2 DK threads: a block has 16
+// columns of a head's state, a warp 16 of its rows in registers.  For u every warp sums over its own
 // rows; the warps' parts meet in shared memory.  The next chunk's operands arrive meanwhile.
 constexpr int PC = 16, PLD = PC + 4;
 template <int DK> struct Pass {
     static constexpr int W = DK + 4;
     static constexpr int STAGE = DK * LD + CH * W + CH * PLD;  // xkt, kh, xv
-    static constexpr int WARPS = DK / 32;
+    static constexpr int WARPS = DK / 16, THREADS = 2 * DK;
     static constexpr size_t SMEM =
         (size_t)(2 * STAGE + DK * PLD + CH * PLD + WARPS * CH * PLD) * sizeof(float);
 };
 
 template <int DK>
-__global__ void __launch_bounds__(DK)
+__global__ void __launch_bounds__(2 * DK)
 delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
                   const float* __restrict__ bn, float* __restrict__ xv, float* __restrict__ states,
                   const Portion* __restrict__ portions, float* __restrict__ state,
                   long long slot_stride, const int* __restrict__ seq_slot, int H, int dv) {
     constexpr int W = Pass<DK>::W, STAGE = Pass<DK>::STAGE, WARPS = Pass<DK>::WARPS;
+    constexpr int THREADS = Pass<DK>::THREADS;
     extern __shared__ __align__(16) float sh[];
     float* ss = sh + 2 * STAGE;                      // [DK][PLD]: the state before the chunk
     float* us = ss + DK * PLD;                       // [CH][PLD]
@@ -504,10 +522,10 @@ delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
     const Portion p = portions[blockIdx.x];
     const int h = blockIdx.y, j0 = blockIdx.z * PC;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // eight groups of four rows (or of four tokens and four more 32 on) by four of four columns; lanes
-    // l and l ^ 2 share the former, l and l ^ 1 the latter
+    // for u: eight groups of four tokens (and four more 32 on) by four of four columns; for S: four
+    // groups of four rows by eight of two columns.  (Lanes l and l ^ 1, or l ^ 2, share one of the two.)
     const int a4 = ((lane & 1) | ((lane >> 1) & 6)) * 4, j4 = (((lane >> 1) & 1) | ((lane >> 3) & 2)) * 4;
-    const int c0 = warp * 32 + a4;
+    const int j2 = a4 / 2, c0 = warp * 16 + j4;
     pdl_wait();
     float* slot = state + (size_t)seq_slot[p.seq] * slot_stride + (size_t)h * DK * dv + j0;
     auto load = [&](int n) {
@@ -516,26 +534,27 @@ delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
         const float* a = xkt + where * DK * CH;
         const float* b = kh + where * CH * DK;
         const float* x = xv + where * CH * dv + j0;
-        for (int e = threadIdx.x; e < DK * 16; e += DK)
+        for (int e = threadIdx.x; e < DK * 16; e += THREADS)
             cp16(st + (e >> 4) * LD + (e & 15) * 4, a + e * 4, true);
-        for (int e = threadIdx.x; e < CH * DK / 4; e += DK)
+        for (int e = threadIdx.x; e < CH * DK / 4; e += THREADS)
             cp16(st + DK * LD + e / (DK / 4) * W + e % (DK / 4) * 4, b + e * 4, true);
-        for (int e = threadIdx.x; e < CH * 4; e += DK)
+        for (int e = threadIdx.x; e < CH * 4; e += THREADS)
             cp16(st + DK * LD + CH * W + (e >> 2) * PLD + (e & 3) * 4,
                  x + (size_t)(e >> 2) * dv + (e & 3) * 4, true);
         cp_commit();
     };
     load(0);
-    float4 S[4];
+    float2 S[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) S[i] = four(slot + (size_t)(c0 + i) * dv + j4);
+    for (int i = 0; i < 4; ++i)
+        S[i] = *reinterpret_cast<const float2*>(slot + (size_t)(c0 + i) * dv + j2);
     for (int n = 0; n < p.chunks; ++n) {
         const size_t where = (size_t)(p.first + n) * H + h;
         const float4 b = four(bn + where * DK + c0);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            *reinterpret_cast<float4*>(states + (where * DK + c0 + i) * dv + j0 + j4) = S[i];
-            *reinterpret_cast<float4*>(ss + (c0 + i) * PLD + j4) = S[i];
+            *reinterpret_cast<float2*>(states + (where * DK + c0 + i) * dv + j0 + j2) = S[i];
+            *reinterpret_cast<float2*>(ss + (c0 + i) * PLD + j2) = S[i];
         }
         cp_wait<0>();
         __syncthreads();                 // the chunk has landed, the one before it has been used
@@ -546,10 +565,10 @@ delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
             unsigned long long acc[8][2];
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = 0ull;
-            const float* xa = st + warp * 32 * LD + a4;
-            const float* sb = ss + warp * 32 * PLD + j4;
+            const float* xa = st + warp * 16 * LD + a4;
+            const float* sb = ss + warp * 16 * PLD + j4;
 #pragma unroll 8
-            for (int c = 0; c < 32; ++c) {
+            for (int c = 0; c < 16; ++c) {
                 const float4 t0 = four(xa + c * LD), t1 = four(xa + c * LD + 32);
                 const float4 y = four(sb + c * PLD);
                 const float v[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
@@ -571,7 +590,7 @@ delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
             }
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < CH * 4; e += DK) {
+        for (int e = threadIdx.x; e < CH * 4; e += THREADS) {
             const int t = e >> 2, c = (e & 3) * 4;
             float4 u = four(st + DK * LD + CH * W + t * PLD + c);
             float4 sum = four(red + t * PLD + c);
@@ -587,38 +606,33 @@ delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
         __syncthreads();
         {
             // S <- diag(b_n) S + sum over the tokens of kh u
-            unsigned long long acc[4][2];
+            unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
             const float bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
             const float* ka = st + DK * LD + c0;
-#pragma unroll 8
+            const float* ub = us + j2;
+#pragma unroll 16
             for (int s = 0; s < CH; ++s) {
-                const float4 kk = four(ka + s * W), u = four(us + s * PLD + j4);
-                const float v[4] = {kk.x, kk.y, kk.z, kk.w};
-                const unsigned long long u0 = pair(u.x, u.y), u1 = pair(u.z, u.w);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const unsigned long long vv = pair(v[i], v[i]);
-                    fma2(acc[i][0], vv, u0);
-                    fma2(acc[i][1], vv, u1);
-                }
+                const float4 kk = four(ka + s * W);
+                const unsigned long long u =
+                    *reinterpret_cast<const unsigned long long*>(ub + s * PLD);
+                fma2(acc[0], pair(kk.x, kk.x), u);
+                fma2(acc[1], pair(kk.y, kk.y), u);
+                fma2(acc[2], pair(kk.z, kk.z), u);
+                fma2(acc[3], pair(kk.w, kk.w), u);
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                float4 d;
-                unpair(acc[i][0], d.x, d.y);
-                unpair(acc[i][1], d.z, d.w);
-                S[i].x = fmaf(bv[i], S[i].x, d.x);
-                S[i].y = fmaf(bv[i], S[i].y, d.y);
-                S[i].z = fmaf(bv[i], S[i].z, d.z);
-                S[i].w = fmaf(bv[i], S[i].w, d.w);
+                float d0, d1;
+                unpair(acc[i], d0, d1);
+                S[i].x = fmaf(bv[i], S[i].x, d0);
+                S[i].y = fmaf(bv[i], S[i].y, d1);
             }
         }
     }
     pdl_trigger();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(slot + (size_t)(c0 + i) * dv + j4) = S[i];
+    for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float2*>(slot + (size_t)(c0 + i) * dv + j2) = S[i];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -770,7 +784,7 @@ DE_EXPORT int de_delta_chunks(const float* q, int ldq, const float* k, int ldk, 
         RUN(de_launch(delta_solve_kernel<DK>, sgrid, dim3(64), ssmem, s, (const float*)at, v,   \
                       ldv, (const float*)kd, beta, ldb, it, xv, xkt, H, dv));                   \
         RUN(need_smem((const void*)delta_pass_kernel<DK>, Pass<DK>::SMEM));                     \
-        RUN(de_launch(delta_pass_kernel<DK>, pgrid, dim3(DK), Pass<DK>::SMEM, s,                \
+        RUN(de_launch(delta_pass_kernel<DK>, pgrid, dim3(2 * DK), Pass<DK>::SMEM, s,            \
                       (const float*)xkt, (const float*)kh, (const float*)bn, xv, states, po,    \
                       state, slot_stride, seq_slot, H, dv));                                    \
     } while (0)
