@@ -701,16 +701,22 @@ static int need_smem(const void* kernel, size_t bytes) {
 }
 
 // The read-outs and the new states of the portions in `items` / `portions` under a decay per head.
-// Workspaces: xt [m, H, dk, 64], pt [m, H, 64, 64], states [m, H, dk, dv].
+// work: m H (64 dk + 64 64 + dk dv) floats, xt [m, H, dk, 64], pt [m, H, 64, 64] and the states
+// [m, H, dk, dv].
 DE_EXPORT int de_decay_chunks(int v_dtype, const float* q, int ldq, const float* k, int ldk,
                               const void* v, int ldv, const float* decay, const int* items, int m,
-                              const int* portions, int n_portions, float* xt, float* pt,
-                              float* states, float* state, long long slot_stride,
-                              const int* seq_slot, float* out, int H, int dk, int dv, void* stream) {
+                              const int* portions, int n_portions, float* work, float* state,
+                              long long slot_stride, const int* seq_slot, float* out, int H, int dk,
+                              int dv, void* stream) {
     if (m <= 0 || n_portions <= 0) return 0;
     if (!de_chunk_ok(dk, dv) || ldk % 4 || ldv % 4 || (uintptr_t)k % 16 ||
-        (uintptr_t)v % (v_dtype == DE_BF16 ? 8 : 16) || slot_stride % 4 || (uintptr_t)state % 16)
+        (uintptr_t)v % (v_dtype == DE_BF16 ? 8 : 16) || slot_stride % 4 || (uintptr_t)state % 16 ||
+        (uintptr_t)work % 16)
         return -2;
+    const size_t mh = (size_t)m * H;
+    float* xt = work;
+    float* pt = xt + mh * dk * CH;
+    float* states = pt + mh * CH * CH;
     cudaStream_t s = (cudaStream_t)stream;
     const Item* it = (const Item*)items;
     const Portion* po = (const Portion*)portions;
@@ -752,21 +758,30 @@ DE_EXPORT int de_decay_chunks(int v_dtype, const float* q, int ldq, const float*
     return 0;
 }
 
-// The same for the delta rule: g [N, ldg] decays, beta [N, ldb], v float32.  Workspaces: at, pt
-// [m, H, 64, 64], xt, kd, kh, xkt [m, H, dk, 64], bn [m, H, dk], xv [m, H, 64, dv], states
-// [m, H, dk, dv].
+// The same for the delta rule: g [N, ldg] decays, beta [N, ldb], v float32.  work: m H (2 64 64 +
+// 4 64 dk + dk + 64 dv + dk dv) floats, at and pt [m, H, 64, 64], xt, kd, kh, xkt [m, H, dk, 64],
+// the states [m, H, dk, dv], xv [m, H, 64, dv] and bn [m, H, dk].
 DE_EXPORT int de_delta_chunks(const float* q, int ldq, const float* k, int ldk, const float* v,
                               int ldv, const float* g, int ldg, const float* beta, int ldb,
                               const int* items, int m, const int* portions, int n_portions,
-                              float* at, float* pt, float* xt, float* kd, float* kh, float* xkt,
-                              float* bn, float* xv, float* states, float* state,
-                              long long slot_stride, const int* seq_slot, float* out, int H,
-                              int rep, int dk, int dv, void* stream) {
+                              float* work, float* state, long long slot_stride,
+                              const int* seq_slot, float* out, int H, int rep, int dk, int dv,
+                              void* stream) {
     if (m <= 0 || n_portions <= 0) return 0;
     if (!de_chunk_ok(dk, dv) || ldq % 4 || ldk % 4 || ldg % 4 || ldv % 2 || (uintptr_t)q % 16 ||
         (uintptr_t)k % 16 || (uintptr_t)g % 16 || (uintptr_t)v % 8 || slot_stride % 4 ||
-        (uintptr_t)state % 16 || rep <= 0 || H % rep)
+        (uintptr_t)state % 16 || (uintptr_t)work % 16 || rep <= 0 || H % rep)
         return -2;
+    const size_t mh = (size_t)m * H, turned = mh * dk * CH;
+    float* at = work;
+    float* pt = at + mh * CH * CH;
+    float* xt = pt + mh * CH * CH;
+    float* kd = xt + turned;
+    float* kh = kd + turned;
+    float* xkt = kh + turned;
+    float* states = xkt + turned;
+    float* xv = states + mh * dk * dv;
+    float* bn = xv + mh * CH * dv;
     cudaStream_t s = (cudaStream_t)stream;
     const Item* it = (const Item*)items;
     const Portion* po = (const Portion*)portions;

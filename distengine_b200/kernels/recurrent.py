@@ -156,9 +156,11 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
 
 
 CHUNK = 64               # tokens of a chunk of a longer portion
-# portions of at least this many tokens go by chunks (measured on B200, a layer of 16 heads of 128:
-# CHUNK_FIGURES)
-CHUNKED_PORTION = 96
+# Portions of at least this many tokens go by chunks.  (Measured on B200: the delta rule's chunks are
+# five kernels and the host's share of them where its scan is one of 0.37 us a token.  A bfloat16
+# layer with a portion of 100 tokens 151 us by chunks, 122 by the scan, lightning attention 112 and
+# 83; four portions of about 100 tokens 152 and 178; one of 400 tokens in float32 500 and 1,001.)
+CHUNKED_PORTION = 192
 
 
 def chunks_ok(key_dim: int, value_dim: int) -> bool:
@@ -191,16 +193,14 @@ def decay_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch
     _f32(decay, "decay")
     _need(decay.shape == (heads,) and decay.is_contiguous() and q.shape[1] == heads * key_dim,
           "decay_chunks: decay [H], q and k [N, H dk]")
-    m, f32 = items.shape[0], torch.float32
-    xt = ctx.buffer("chunks.xt", (m, heads, key_dim, CHUNK), f32)
-    pt = ctx.buffer("chunks.pt", (m, heads, CHUNK, CHUNK), f32)
-    states = ctx.buffer("chunks.states", (m, heads, key_dim, value_dim), f32)
+    m = items.shape[0]
+    work = ctx.buffer("chunks.work", (m * heads * (key_dim * CHUNK + CHUNK * CHUNK
+                                                   + key_dim * value_dim),), torch.float32)
     lib = library.load("recurrent_chunks")
     _check(lib.de_decay_chunks(_tag(v.dtype), q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0),
                                v.data_ptr(), v.stride(0), decay.data_ptr(), items.data_ptr(), m,
-                               portions.data_ptr(), portions.shape[0], xt.data_ptr(),
-                               pt.data_ptr(), states.data_ptr(), state.data_ptr(),
-                               state.stride(0), ctx.seq_slot.data_ptr(), out.data_ptr(), heads,
+                               portions.data_ptr(), portions.shape[0], work.data_ptr(),
+                               state.data_ptr(), state.stride(0), ctx.seq_slot.data_ptr(), out.data_ptr(), heads,
                                key_dim, value_dim, _stream()), "decay_chunks")
 
 
@@ -216,17 +216,15 @@ def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch
     _need(q.shape[1] == qk_heads * key_dim and heads % qk_heads == 0
           and g.shape == (n, heads * key_dim) and beta.shape == (n, heads),
           "delta_chunks: q, k [N, qk_heads dk], g [N, H dk], beta [N, H]")
-    m, f32 = items.shape[0], torch.float32
-    square, turned = (m, heads, CHUNK, CHUNK), (m, heads, key_dim, CHUNK)
-    work = [ctx.buffer(f"chunks.{name}", shape, f32) for name, shape in (
-        ("at", square), ("pt", square), ("xt", turned), ("kd", turned), ("kh", turned),
-        ("xkt", turned), ("bn", (m, heads, key_dim)), ("xv", (m, heads, CHUNK, value_dim)),
-        ("states", (m, heads, key_dim, value_dim)))]
+    m = items.shape[0]
+    work = ctx.buffer("chunks.work", (m * heads * (2 * CHUNK * CHUNK + 4 * key_dim * CHUNK + key_dim
+                                                   + CHUNK * value_dim + key_dim * value_dim),),
+                      torch.float32)
     lib = library.load("recurrent_chunks")
     _check(lib.de_delta_chunks(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(),
                                v.stride(0), g.data_ptr(), g.stride(0), beta.data_ptr(),
                                beta.stride(0), items.data_ptr(), m, portions.data_ptr(),
-                               portions.shape[0], *[t.data_ptr() for t in work], state.data_ptr(),
+                               portions.shape[0], work.data_ptr(), state.data_ptr(),
                                state.stride(0), ctx.seq_slot.data_ptr(), out.data_ptr(), heads,
                                heads // qk_heads, key_dim, value_dim, _stream()), "delta_chunks")
 
