@@ -1755,6 +1755,142 @@ struct Fuse {
     int ld_gate;
 };
 
+// The token's queries of `g` heads from h0 on into Qs [rw][dk] as float32 (zeros beyond them) and,
+// with fuse.on, what Fuse says of queries, key and value.  Ends with a barrier of the block.
+template <typename T>
+__device__ __forceinline__ void decode_begin(
+    float* Qs, int rw, int g, int h0, int hk, const T* __restrict__ q, int q_stride, int tok,
+    int slot, int pos, T* k_pages, T* v_pages, const int* __restrict__ block_table,
+    int table_stride, int num_pages, int heads, int kv_heads, int dk, int dv, int page,
+    const Fuse& fuse, int* __restrict__ status) {
+    for (int e = threadIdx.x; e < rw * dk; e += (int)blockDim.x) {
+        const int i = e / dk, d = e - i * dk;
+        Qs[e] = i < g ? to_float(q[(size_t)tok * q_stride + (h0 + i) * dk + d]) : 0.0f;
+    }
+    __syncthreads();
+    if (fuse.on) {
+        const float fpos = (float)pos;
+        const int half = fuse.rot / 2;
+        for (int e = threadIdx.x; e < g * half; e += (int)blockDim.x) {
+            const int i = e / half, p = e - i * half;
+            float sn, cs, ra, rb;
+            sincosf(fpos * fuse.fk[p], &sn, &cs);
+            rope_rotate(Qs[i * dk + p], Qs[i * dk + p + half], cs, sn, ra, rb);
+            Qs[i * dk + p] = to_float(from_float<T>(ra));        // rounded as when q goes through memory
+            Qs[i * dk + p + half] = to_float(from_float<T>(rb));
+        }
+        if (fuse.write_kv) {
+            const int page_id = block_table[(size_t)slot * table_stride + pos / page];
+            if (page_id < 0 || page_id >= num_pages) {           // never written outside the pool
+                if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
+            } else {
+                const size_t at = ((size_t)page_id * kv_heads + hk) * page + (size_t)(pos % page);
+                const T* ks = q + (size_t)tok * q_stride + heads * dk + hk * dk;
+                const T* vs = q + (size_t)tok * q_stride + (heads + kv_heads) * dk + hk * dv;
+                T* kd = k_pages + at * dk;
+                T* vd = v_pages + at * dv;
+                for (int i = threadIdx.x; i < dk - half; i += (int)blockDim.x) {
+                    if (i < half) {
+                        float sn, cs, ra, rb;
+                        sincosf(fpos * fuse.fk[i], &sn, &cs);
+                        rope_rotate(to_float(ks[i]), to_float(ks[i + half]), cs, sn, ra, rb);
+                        kd[i] = from_float<T>(ra);
+                        kd[i + half] = from_float<T>(rb);
+                    } else {
+                        kd[i + half] = ks[i + half];
+                    }
+                }
+                if (fuse.fv != nullptr) {
+                    const int vhalf = dv / 2;
+                    for (int i = threadIdx.x; i < dv - vhalf; i += (int)blockDim.x) {
+                        if (i < vhalf) {
+                            float sn, cs, ra, rb;
+                            sincosf(fpos * fuse.fv[i], &sn, &cs);
+                            rope_rotate(to_float(vs[i]), to_float(vs[i + vhalf]), cs, sn, ra, rb);
+                            vd[i] = from_float<T>(ra);
+                            vd[i + vhalf] = from_float<T>(rb);
+                        } else {
+                            vd[i + vhalf] = vs[i + vhalf];
+                        }
+                    }
+                } else {
+                    for (int i = threadIdx.x; i < dv; i += (int)blockDim.x) vd[i] = vs[i];
+                }
+            }
+        }
+        __syncthreads();                             // the block reads what it has just stored
+    }
+}
+
+// The warps' partial results (Pml [warps][rw][2] maximum and sum, Pacc [warps][rw][dv]) merged in
+// ascending order of the warps, a warp a head, and finished.
+template <typename T>
+__device__ __forceinline__ void decode_finish(const float* Pml, float* Pacc, int rw, int warps,
+                                              int g, int h0, int tok, int pos, void* out,
+                                              int out_stride, int dv, const Sight& sight,
+                                              int out_f32, const Fuse& fuse) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = warp; i < g; i += warps) {
+        float top = -INFINITY;
+        for (int w = 0; w < warps; ++w) top = fmaxf(top, Pml[(w * rw + i) * 2]);
+        float sum = 0.0f, res[MAX_D / 32];
+#pragma unroll
+        for (int b = 0; b < MAX_D / 32; ++b) res[b] = 0.0f;
+        for (int w = 0; w < warps; ++w) {
+            const float mw = Pml[(w * rw + i) * 2];
+            if (mw == -INFINITY) continue;
+            const float f = expf(mw - top);
+            sum = fmaf(Pml[(w * rw + i) * 2 + 1], f, sum);
+#pragma unroll
+            for (int b = 0; b < MAX_D / 32; ++b) {
+                const int dd = lane + 32 * b;
+                if (dd < dv) res[b] = fmaf(Pacc[(size_t)(w * rw + i) * dv + dd], f, res[b]);
+            }
+        }
+        const float inv = sight_inverse(sight, h0 + i, top, sum);
+        const size_t o = (size_t)tok * out_stride + (h0 + i) * dv;
+        if (fuse.on) {
+            // the head's result through shared memory (the place of the first warp's share of
+            // this head, which only this warp reads), so that a lane finds its feature's pair
+            float* fin = Pacc + (size_t)i * dv;
+            __syncwarp();
+#pragma unroll
+            for (int b = 0; b < MAX_D / 32; ++b) {
+                const int dd = lane + 32 * b;
+                if (dd < dv) fin[dd] = res[b] * inv;
+            }
+            __syncwarp();
+            const int vhalf = dv / 2;
+            const T* gt = fuse.gate
+                              ? (const T*)fuse.gate + (size_t)tok * fuse.ld_gate + (h0 + i) * dv
+                              : nullptr;
+#pragma unroll
+            for (int b = 0; b < MAX_D / 32; ++b) {
+                const int dd = lane + 32 * b;
+                if (dd >= dv) continue;
+                float x = fin[dd];
+                if (fuse.fv != nullptr && dd < 2 * vhalf) {
+                    const int p = dd < vhalf ? dd : dd - vhalf;
+                    float sn, cs, ra, rb;
+                    sincosf((float)pos * fuse.fv[p], &sn, &cs);
+                    rope_rotate(fin[p], fin[p + vhalf], cs, -sn, ra, rb);
+                    x = dd < vhalf ? ra : rb;
+                }
+                if (gt) x *= 1.0f / (1.0f + expf(-to_float(gt[dd])));
+                ((T*)out)[o + dd] = from_float<T>(x);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int b = 0; b < MAX_D / 32; ++b) {
+            const int dd = lane + 32 * b;
+            if (dd < dv)
+                store_out<T>(out, out_f32, o + dd,
+                             res[b] * inv * sight_gate<T>(sight, (size_t)tok, h0 + i, dv, dd));
+        }
+    }
+}
+
 template <typename T, int RW>
 __global__ void __launch_bounds__(ROWS * 32)
 attn_chunk_decode_kernel(const T* __restrict__ q, int q_stride, void* __restrict__ out,
@@ -1804,63 +1940,8 @@ attn_chunk_decode_kernel(const T* __restrict__ q, int q_stride, void* __restrict
         l[i] = 0.0f;
     }
     pdl_wait();
-    for (int e = threadIdx.x; e < RW * dk; e += ROWS * 32) {
-        const int i = e / dk, d = e - i * dk;
-        Qs[e] = i < g ? to_float(q[(size_t)tok * q_stride + (h0 + i) * dk + d]) : 0.0f;
-    }
-    __syncthreads();
-    if (fuse.on) {
-        const float fpos = (float)pos;
-        const int half = fuse.rot / 2;
-        for (int e = threadIdx.x; e < g * half; e += ROWS * 32) {
-            const int i = e / half, p = e - i * half;
-            float sn, cs, ra, rb;
-            sincosf(fpos * fuse.fk[p], &sn, &cs);
-            rope_rotate(Qs[i * dk + p], Qs[i * dk + p + half], cs, sn, ra, rb);
-            Qs[i * dk + p] = to_float(from_float<T>(ra));        // rounded as when q goes through memory
-            Qs[i * dk + p + half] = to_float(from_float<T>(rb));
-        }
-        if (fuse.write_kv) {
-            const int page_id = block_table[(size_t)slot * table_stride + pos / page];
-            if (page_id < 0 || page_id >= num_pages) {           // never written outside the pool
-                if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
-            } else {
-                const size_t at = ((size_t)page_id * kv_heads + hk) * page + (size_t)(pos % page);
-                const T* ks = q + (size_t)tok * q_stride + heads * dk + hk * dk;
-                const T* vs = q + (size_t)tok * q_stride + (heads + kv_heads) * dk + hk * dv;
-                T* kd = k_pages + at * dk;
-                T* vd = v_pages + at * dv;
-                for (int i = threadIdx.x; i < dk - half; i += ROWS * 32) {
-                    if (i < half) {
-                        float sn, cs, ra, rb;
-                        sincosf(fpos * fuse.fk[i], &sn, &cs);
-                        rope_rotate(to_float(ks[i]), to_float(ks[i + half]), cs, sn, ra, rb);
-                        kd[i] = from_float<T>(ra);
-                        kd[i + half] = from_float<T>(rb);
-                    } else {
-                        kd[i + half] = ks[i + half];
-                    }
-                }
-                if (fuse.fv != nullptr) {
-                    const int vhalf = dv / 2;
-                    for (int i = threadIdx.x; i < dv - vhalf; i += ROWS * 32) {
-                        if (i < vhalf) {
-                            float sn, cs, ra, rb;
-                            sincosf(fpos * fuse.fv[i], &sn, &cs);
-                            rope_rotate(to_float(vs[i]), to_float(vs[i + vhalf]), cs, sn, ra, rb);
-                            vd[i] = from_float<T>(ra);
-                            vd[i + vhalf] = from_float<T>(rb);
-                        } else {
-                            vd[i + vhalf] = vs[i + vhalf];
-                        }
-                    }
-                } else {
-                    for (int i = threadIdx.x; i < dv; i += ROWS * 32) vd[i] = vs[i];
-                }
-            }
-        }
-        __syncthreads();                             // the block reads what it has just stored
-    }
+    decode_begin<T>(Qs, RW, g, h0, hk, q, q_stride, tok, slot, pos, k_pages, v_pages, block_table,
+                    table_stride, num_pages, heads, kv_heads, dk, dv, page, fuse, status);
     float acc[RW][MAX_D / 32];
 #pragma unroll
     for (int i = 0; i < RW; ++i)
@@ -1977,65 +2058,202 @@ attn_chunk_decode_kernel(const T* __restrict__ q, int q_stride, void* __restrict
         }
     }
     __syncthreads();
-    for (int i = warp; i < g; i += ROWS) {
-        float top = -INFINITY;
-        for (int w = 0; w < ROWS; ++w) top = fmaxf(top, Pml[(w * RW + i) * 2]);
-        float sum = 0.0f, res[MAX_D / 32];
-#pragma unroll
-        for (int b = 0; b < MAX_D / 32; ++b) res[b] = 0.0f;
-        for (int w = 0; w < ROWS; ++w) {
-            const float mw = Pml[(w * RW + i) * 2];
-            if (mw == -INFINITY) continue;
-            const float f = expf(mw - top);
-            sum = fmaf(Pml[(w * RW + i) * 2 + 1], f, sum);
-#pragma unroll
-            for (int b = 0; b < MAX_D / 32; ++b) {
-                const int dd = lane + 32 * b;
-                if (dd < dv) res[b] = fmaf(Pacc[(size_t)(w * RW + i) * dv + dd], f, res[b]);
+    decode_finish<T>(Pml, Pacc, RW, ROWS, g, h0, tok, pos, out, out_stride, dv, sight, out_f32, fuse);
+}
+
+// ------------------------------------------------------------------------------------------
+// The same for bfloat16 rows of D = 64 or 128 features (keys and values alike), up to eight query
+// heads a kv head, with both products on the tensor cores as attn_chunk_mma_kernel forms them (a
+// block's heads are the first eight of a product's sixteen rows).  A warp's tiles are 16 keys and
+// come through three stages of its own, so that two are on their way while one is worked on; a
+// block of four warps leaves room for a second on its SM, eight warps serve steps of few sequences.
+// Bound by memory and by the trips to it: 64 sequences of 700 keys, 16 heads on 4 kv heads of 128:
+// 25 us, 3.7 TB/s (the kernel above, which asks for a tile, waits and works: 81).
+// ------------------------------------------------------------------------------------------
+constexpr int DKT = 16, DSTAGES = 3, DRW = 8;
+
+template <int D, int WARPS> constexpr size_t decode_mma_smem() {
+    return (size_t)(DRW * D + WARPS * DRW * 2) * sizeof(float) +
+           (size_t)WARPS * DSTAGES * 2 * DKT * (D + 8) * sizeof(__nv_bfloat16);
+}
+
+template <int D, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+attn_chunk_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
+                             void* __restrict__ out, int out_stride, __nv_bfloat16* k_pages,
+                             __nv_bfloat16* v_pages, const int* __restrict__ block_table,
+                             int table_stride, int num_pages, const int* __restrict__ seq_slot,
+                             const int* __restrict__ seq_qstart, const int* __restrict__ seq_pos0,
+                             const float* __restrict__ r1, const float* __restrict__ r2, int heads,
+                             int kv_heads, int page, float scale, Sight sight, int out_f32,
+                             Fuse fuse, int* __restrict__ status) {
+    using T = __nv_bfloat16;
+    constexpr int LD = D + 8, DT = D / 8, CH = D / 8;
+    extern __shared__ __align__(16) float smem[];
+    float* Qs = smem;                                // [DRW][D]
+    float* Pml = Qs + DRW * D;                       // [WARPS][DRW][2]
+    T* tiles = reinterpret_cast<T*>(Pml + WARPS * DRW * 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gid = lane >> 2, tig = lane & 3;
+    T* mine = tiles + (size_t)warp * DSTAGES * 2 * DKT * LD;   // [stage][K, V][DKT][LD]
+    const int seq = blockIdx.x, hk = blockIdx.y, g = heads / kv_heads, h0 = hk * g;
+    const int pos = seq_pos0[seq], slot = seq_slot[seq], tok = seq_qstart[seq];
+    const int lo = sight_lo(sight, pos), hi = pos + 1, first = sight_first(sight, lo);
+    // the tiles: those of the kept first keys, then from the tile of `lo` on, dealt out in turn
+    const TileWalk walk(lo, first, DKT);
+    const int first_tiles = walk.jump_at > 0 ? walk.jump_at / DKT : 0;
+    const int near0 = walk.jump_at > 0 ? walk.jump_to : walk.start;
+    const int n_tiles = first_tiles + (hi - near0 + DKT - 1) / DKT;
+    auto start_of = [&](int ti) {
+        return ti < first_tiles ? ti * DKT : near0 + (ti - first_tiles) * DKT;
+    };
+    // lane j < 16 finds key j of a tile: its row in the pages, -1 for a key that is not seen
+    auto row_of = [&](int ti) {
+        long long row = -1;
+        if (ti < n_tiles && lane < DKT) {
+            const int kpos = start_of(ti) + lane;
+            if ((kpos >= lo || kpos < first) && kpos < hi) {
+                const int id = block_table[(size_t)slot * table_stride + kpos / page];
+                if (id >= 0 && id < num_pages)
+                    row = ((long long)id * kv_heads + hk) * page + kpos % page;
+                else if (status != nullptr) atomicExch(status, 2);
             }
         }
-        const float inv = sight_inverse(sight, h0 + i, top, sum);
-        const size_t o = (size_t)tok * out_stride + (h0 + i) * dv;
-        if (fuse.on) {
-            // the head's result through shared memory (the place of the first warp's share of
-            // this head, which only this warp reads), so that a lane finds its feature's pair
-            float* fin = Pacc + (size_t)i * dv;
-            __syncwarp();
+        return row;
+    };
+    const bool penalty = r1 != nullptr;
+    const int hq = h0 + min(gid, g - 1);
+    const float pen1 = penalty ? r1[hq] : 0.0f, pen2 = penalty ? r2[hq] : 0.0f;
+    long long next_row = row_of(warp);
+
+    pdl_wait();
+    decode_begin<T>(Qs, DRW, g, h0, hk, q, q_stride, tok, slot, pos, k_pages, v_pages, block_table,
+                    table_stride, num_pages, heads, kv_heads, D, D, page, fuse, status);
+    if (!fuse.on) __syncthreads();
+    unsigned qf[D / 16][4];                          // (rounded already: what q went through)
 #pragma unroll
-            for (int b = 0; b < MAX_D / 32; ++b) {
-                const int dd = lane + 32 * b;
-                if (dd < dv) fin[dd] = res[b] * inv;
-            }
-            __syncwarp();
-            const int vhalf = dv / 2;
-            const T* gt = fuse.gate
-                              ? (const T*)fuse.gate + (size_t)tok * fuse.ld_gate + (h0 + i) * dv
-                              : nullptr;
+    for (int kk = 0; kk < D / 16; ++kk) {
+        const float* p = Qs + gid * D + kk * 16 + 2 * tig;
+        qf[kk][0] = pack2(p[0], p[1]);
+        qf[kk][2] = pack2(p[8], p[9]);
+        qf[kk][1] = qf[kk][3] = 0u;                  // rows 8 to 15
+    }
+    // which of a tile's keys are seen, of the tile worked on and the two behind it
+    unsigned seen[DSTAGES];
+    auto issue = [&](int ti, int stage) {
+        T* kd = mine + (size_t)stage * 2 * DKT * LD;
+        T* vd = kd + DKT * LD;
+        const long long row = next_row;
+        next_row = row_of(ti + WARPS);
 #pragma unroll
-            for (int b = 0; b < MAX_D / 32; ++b) {
-                const int dd = lane + 32 * b;
-                if (dd >= dv) continue;
-                float x = fin[dd];
-                if (fuse.fv != nullptr && dd < 2 * vhalf) {
-                    const int p = dd < vhalf ? dd : dd - vhalf;
-                    float sn, cs, ra, rb;
-                    sincosf((float)pos * fuse.fv[p], &sn, &cs);
-                    rope_rotate(fin[p], fin[p + vhalf], cs, -sn, ra, rb);
-                    x = dd < vhalf ? ra : rb;
-                }
-                if (gt) x *= 1.0f / (1.0f + expf(-to_float(gt[dd])));
-                ((T*)out)[o + dd] = from_float<T>(x);
-            }
-            continue;
+        for (int i = 0; i < DKT * CH / 32; ++i) {
+            const int c = lane + 32 * i, j = c / CH, ch = c % CH;
+            const long long r = __shfl_sync(0xffffffffu, row, j);
+            const size_t at = r >= 0 ? (size_t)r : 0;
+            const int bytes = r >= 0 ? 16 : 0;
+            const unsigned ka = (unsigned)__cvta_generic_to_shared(kd + j * LD + ch * 8);
+            const unsigned va = (unsigned)__cvta_generic_to_shared(vd + j * LD + ch * 8);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(ka),
+                         "l"(k_pages + at * D + ch * 8), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(va),
+                         "l"(v_pages + at * sight.v_stride + ch * 8), "r"(bytes) : "memory");
         }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        return __ballot_sync(0xffffffffu, row >= 0);
+    };
 #pragma unroll
-        for (int b = 0; b < MAX_D / 32; ++b) {
-            const int dd = lane + 32 * b;
-            if (dd < dv)
-                store_out<T>(out, out_f32, o + dd,
-                             res[b] * inv * sight_gate<T>(sight, (size_t)tok, h0 + i, dv, dd));
+    for (int i = 0; i < DSTAGES - 1; ++i) seen[i] = issue(warp + i * WARPS, i);
+
+    float m = -INFINITY, l = 0.0f, acc[DT][2];
+#pragma unroll
+    for (int j = 0; j < DT; ++j) acc[j][0] = acc[j][1] = 0.0f;
+    const int mat = lane >> 3, mr = lane & 7;
+    int stage = 0;
+    for (int ti = warp; ti < n_tiles; ti += WARPS) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(DSTAGES - 2) : "memory");
+        __syncwarp();                // this tile has landed, the one before it has been used
+        const int free = stage == 0 ? DSTAGES - 1 : stage - 1;
+        const unsigned mask = seen[0];
+        seen[0] = seen[1];
+        seen[1] = issue(ti + (DSTAGES - 1) * WARPS, free);
+        const T* kb = mine + (size_t)stage * 2 * DKT * LD;
+        const T* vb = kb + DKT * LD;
+        stage = stage == DSTAGES - 1 ? 0 : stage + 1;
+        float c[2][2][4];            // q . k in two chains of half the features each
+#pragma unroll
+        for (int i = 0; i < 16; ++i) c[i >> 3][(i >> 2) & 1][i & 3] = 0.0f;
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+            unsigned b[4];
+            ldmatrix4(b, kb + ((mat >> 1) * 8 + mr) * LD + kk * 16 + (mat & 1) * 8);
+            mma16816(c[kk & 1][0], qf[kk], b[0], b[1]);
+            mma16816(c[kk & 1][1], qf[kk], b[2], b[3]);
+        }
+        const int kt = start_of(ti);
+        float s[2][2];
+        float top = m;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int key = 8 * j + 2 * tig + x;
+                const float sc = sight_score(sight, c[0][j][x] + c[1][j][x], scale, pen1, pen2,
+                                             penalty, (float)(pos - kt - key));
+                s[j][x] = (mask >> key) & 1u ? sc : -INFINITY;
+                top = fmaxf(top, s[j][x]);
+            }
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        const float use = top == -INFINITY ? 0.0f : top;
+        const float corr = expf(m - use);
+        m = top;
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                s[j][x] = expf(s[j][x] - use);
+                sum += s[j][x];
+            }
+        l = l * corr + sum;
+        unsigned pw[3][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) split3(s[j][0], s[j][1], pw[0][2 * j], pw[1][2 * j], pw[2][2 * j]);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) pw[t][1] = pw[t][3] = 0u;
+#pragma unroll
+        for (int jd = 0; jd < DT; jd += 2) {
+            unsigned b[4];
+            ldmatrix4_trans(b, vb + ((mat & 1) * 8 + mr) * LD + (jd + (mat >> 1)) * 8);
+            float t0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, t1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int term = 2; term >= 0; --term) {
+                mma16816(t0, pw[term], b[0], b[1]);
+                mma16816(t1, pw[term], b[2], b[3]);
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                acc[jd][x] = fmaf(acc[jd][x], corr, t0[x]);
+                acc[jd + 1][x] = fmaf(acc[jd + 1][x], corr, t1[x]);
+            }
         }
     }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    pdl_trigger();
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    __syncthreads();                                 // the tiles' place now holds the partial results
+    float* Pacc = reinterpret_cast<float*>(tiles);   // [WARPS][DRW][D]
+    if (tig == 0) {
+        Pml[(warp * DRW + gid) * 2] = m;
+        Pml[(warp * DRW + gid) * 2 + 1] = l;
+    }
+#pragma unroll
+    for (int j = 0; j < DT; ++j)
+        store_pair(Pacc + (size_t)(warp * DRW + gid) * D + j * 8 + 2 * tig, acc[j][0], acc[j][1]);
+    __syncthreads();
+    decode_finish<T>(Pml, Pacc, DRW, WARPS, g, h0, tok, pos, out, out_stride, D, sight, out_f32,
+                     fuse);
 }
 
 }  // namespace
@@ -2055,6 +2273,16 @@ static bool vec_fits(int dtype, int dk, int dv) {
 static size_t tiled_smem(int dk, int dv) {
     return (size_t)(TILE * (dk + 4) + TILE * dv + TROWS * (dk + 4) + 4 * TILE * 16 + TILE) *
            sizeof(float);
+}
+static int sm_count() {
+    static int count = 0;
+    if (count == 0) {
+        int device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess ||
+            cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+            count = 148;
+    }
+    return count;
 }
 // the tensor-core kernel's sizes: bfloat16, keys and values of 64 or of 128 features
 static bool mma_ok(int dtype, int dk, int dv) {
@@ -2132,6 +2360,30 @@ DE_EXPORT int de_attn_chunk_decode(int dtype, const void* q, int q_stride, void*
     const size_t smem = decode_smem(dtype, rw, dk, dv, v_in_k);
     if ((uintptr_t)v_pages % 16 != 0) return -2;
     if (g > rw && fused) return -2;         // a kv head's blocks would each store the token's key
+    if (mma_ok(dtype, dk, dv) && g <= DRW && sight.v_stride % 8 == 0) {
+        // four warps a block, two blocks an SM; eight where there is at most one block an SM
+        const bool few = (long long)n_seqs * kv_heads <= sm_count();
+#define DECM(D, W)                                                                              \
+    do {                                                                                        \
+        auto kernel = attn_chunk_decode_mma_kernel<D, W>;                                       \
+        const size_t bytes = decode_mma_smem<D, W>();                                           \
+        const cudaError_t me = cudaFuncSetAttribute(                                            \
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);                   \
+        if (me != cudaSuccess) return (int)me;                                                  \
+        return de_launch(kernel, dim3(n_seqs, kv_heads), dim3(W * 32), bytes, s,                \
+                         (const __nv_bfloat16*)q, q_stride, out, out_stride,                    \
+                         (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, block_table,         \
+                         table_stride, num_pages, seq_slot, seq_qstart, seq_pos0, r1, r2,       \
+                         heads, kv_heads, page, scale, sight, out_f32, fuse, status);           \
+    } while (0)
+        if (dk == 64) {
+            if (few) DECM(64, 8);
+            DECM(64, 4);
+        }
+        if (few) DECM(128, 8);
+        DECM(128, 4);
+#undef DECM
+    }
     dim3 grid(n_seqs, kv_heads * ((g + rw - 1) / rw));
 #define DEC(T, RW)                                                                              \
     do {                                                                                        \

@@ -717,3 +717,65 @@ def test_chunk_attention_on_tensor_cores(dim, rows, form):
                 want = want * 1.5 * torch.sigmoid(gate[at, h].double())[:, None]
             err = (got[at, h] - want).abs().max().item()
             assert err <= 4e-6 * max(1.0, want.abs().max().item()), (i, h, err)
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("seqs", [5, 76])            # eight and four warps a block
+@pytest.mark.parametrize("form", ["window", "slopes", "chunk"])
+def test_single_tokens_on_tensor_cores(dim, seqs, form):
+    """Key counts around the tiles of 16 and around what the warps take in a turn, pages that a
+    window has passed, the largest group of heads: float32 results against 64 bits, with the bound
+    of the test above."""
+    from types import SimpleNamespace
+    from distengine_b200.kernels import recurrent as rk
+    heads, kv_heads, page = (16, 2, 16) if form == "slopes" else (6, 2, 16)
+    lens = ([1, 17, 64, 129, 390] * 16)[:seqs]
+    fx = PagedFixture(lens, kv_heads, dim, page, torch.bfloat16, DEV, seed=seqs)
+    g = torch.Generator().manual_seed(dim)
+    group = heads // kv_heads
+    q = (torch.randn(seqs, heads, dim, generator=g) * 3).to(torch.bfloat16)
+    window, keep, chunk, cap = (40, 3, 0, 4.0) if form == "window" else (
+        (0, 0, 50, 0.0) if form == "chunk" else (0, 0, 0, 0.0))
+    r, sink = torch.rand(heads, generator=g) * 0.3, torch.randn(heads, generator=g)
+    gate = torch.randn(seqs, heads, generator=g).to(torch.bfloat16)
+    if form == "window":
+        for i, keys in enumerate(lens):
+            for p in range(1, (keys - window) // page):
+                fx.block_table[fx.slots[i], p] = -1
+    k_pages, v_pages, table = fx.to_device()
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).to(DEV)
+    ctx = SimpleNamespace(n_seqs=seqs, seq_slot=t(np.array(fx.slots)), seq_qstart=t(np.arange(seqs)),
+                          seq_qlen=t(np.ones(seqs)), seq_pos0=t(np.array(lens) - 1),
+                          status=torch.zeros(1, dtype=torch.int32, device=DEV))
+    out = torch.full((seqs, heads * dim), float("nan"), device=DEV)
+    extras = {} if form != "slopes" else dict(slopes=r.to(DEV), sink=sink.to(DEV), gate_per_head=True,
+                                              gate=gate.to(DEV), out_scale=1.5)
+    pen = (r.to(DEV), (4 * r).to(DEV)) if form == "chunk" else (None, None)
+    rk.chunk_attention_decode(q.view(seqs, -1).to(DEV), out, k_pages, v_pages, table, *pen, heads,
+                              kv_heads, dim, dim, dim ** -0.5, chunk, ctx, window=window,
+                              keep_first=keep, softcap=cap, **extras)
+    assert int(ctx.status.item()) == 0
+    got = out.double().cpu().view(seqs, heads, dim)
+    for i, keys in enumerate(lens):
+        j = torch.arange(keys)
+        dist = keys - 1 - j
+        seen = dist >= 0
+        if window:
+            seen = (dist < window) | (j < keep)
+        if chunk:
+            seen = (j // chunk) == ((keys - 1) // chunk)
+        k = fx.k[i].double().repeat_interleave(group, 1)
+        s = torch.einsum("hd,jhd->hj", q[i].double(), k) * dim ** -0.5
+        if form == "slopes":
+            s = s - r.double()[:, None] * dist
+        if form == "chunk":
+            s = s - r.double()[:, None] * torch.log1p(4 * r.double()[:, None] * dist)
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        e = torch.exp(s.masked_fill(~seen, float("-inf")))
+        total = e.sum(1, keepdim=True) + (sink.double().exp()[:, None] if form == "slopes" else 0.0)
+        want = torch.einsum("hj,jhd->hd", e / total, fx.v[i].double().repeat_interleave(group, 1))
+        if form == "slopes":
+            want = want * 1.5 * torch.sigmoid(gate[i].double())[:, None]
+        err = (got[i] - want).abs().max().item()
+        assert err <= 4e-6 * max(1.0, want.abs().max().item()), (i, keys, err)
