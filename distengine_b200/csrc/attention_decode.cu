@@ -158,38 +158,53 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_stride,
     const int hi = empty ? lo : min(it.kv_end, pos + 1);
     const int k_lo = (lo / KT) * KT;
 
-    const size_t slab = (size_t)page * D;
-    // keys and values of a tile from the cache; the token's own row is left out (fill_new)
-    // (two threads take a key's row, one look into the block table each; they alternate over
-    // the row's 16-byte pieces, so that every request of the pair fills a whole 32-byte sector)
-    static_assert(THREADS == 2 * KT && CHUNKS % 2 == 0, "two threads a key row");
-    auto load_tile = [&](int kt, int stage) {
-        __nv_bfloat16* kd = k_s + stage * KT * LDS;
-        __nv_bfloat16* vd = v_s + stage * KT * LDS;
-        const int j = threadIdx.x >> 1, ch0 = threadIdx.x & 1;
-        const int kpos = kt + j;
-        if (new_key && kpos == pos) return;
-        bool ok = kpos >= lo && kpos < hi;
-        size_t off = 0;
-        if (ok) {
+    // A warp fetches the 16 keys of a tile that it works on itself, so the warps' pipelines need no
+    // barrier of the block between them; consecutive lanes take consecutive pieces of a row (two
+    // rows of 128 features a request: whole 128-byte lines).  Lane j looks up key j's row, one tile
+    // ahead of its use.  The token's own row is left out (fill_new).  Measured, 64 sequences of
+    // 4,097 keys, 8 kv heads of 128: 271 -> 175 us (4.0 -> 6.1 TB/s) against two threads a row that
+    // take its pieces by turns (sixteen rows a request, a barrier of the block before and after
+    // each tile); 8 sequences of 520 keys: a layer 0.6 us less.
+    static_assert(NK == 16 && CHUNKS % 2 == 0, "a key a lane of half a warp, whole rounds of pieces");
+    auto row_of = [&](int kt) {                       // -1: not to be read
+        long long row = -1;
+        const int kpos = kt + wn * NK + lane;
+        if (lane < NK && kpos >= lo && kpos < hi && !(new_key && kpos == pos)) {
             const int page_id = block_table[(size_t)slot * table_stride + kpos / page];
-            ok = page_id >= 0 && page_id < num_pages;
-            if (ok) off = ((size_t)page_id * kv_heads + hk) * slab + (size_t)(kpos % page) * D;
-            else if (ch0 == 0) atomicExch(status, 2);                // a visible key has no page
+            if (page_id >= 0 && page_id < num_pages)
+                row = ((long long)page_id * kv_heads + hk) * page + kpos % page;
+            else atomicExch(status, 2);                              // a visible key has no page
         }
+        return row;
+    };
+    long long next_row = row_of(k_lo);
+    // keys and values of this warp's part of tile `kt` (tiles are asked for in ascending order)
+    auto load_tile = [&](int kt, int stage) {
+        __nv_bfloat16* kd = k_s + (stage * KT + wn * NK) * LDS;
+        __nv_bfloat16* vd = v_s + (stage * KT + wn * NK) * LDS;
+        const long long row = next_row;
+        next_row = row_of(kt + KT);
+        const int own = new_key ? pos - kt - wn * NK : -1;
 #pragma unroll
-        for (int ch = ch0; ch < CHUNKS; ch += 2) {
-            cp_async16(kd + j * LDS + ch * 8, k_pages + off + (ok ? ch * 8 : 0), ok);
-            cp_async16(vd + j * LDS + ch * 8, v_pages + off + (ok ? ch * 8 : 0), ok);
+        for (int i = 0; i < NK * CHUNKS / 32; ++i) {
+            const int c = lane + 32 * i, j = c / CHUNKS, ch = c % CHUNKS;
+            const long long r = __shfl_sync(0xffffffffu, row, j);
+            const size_t off = r >= 0 ? (size_t)r * D + ch * 8 : 0;
+            if (j == own) continue;
+            cp_async16(kd + j * LDS + ch * 8, k_pages + off, r >= 0);
+            cp_async16(vd + j * LDS + ch * 8, v_pages + off, r >= 0);
         }
     };
     // the token's own key and value, from this launch and not from the cache, into their row
     auto fill_new = [&](int kt, int stage) {
-        if (!new_key || pos < kt || pos >= kt + KT || threadIdx.x >= 2 * CHUNKS) return;
-        const int ch = threadIdx.x % CHUNKS;
-        __nv_bfloat16* dst = (threadIdx.x < CHUNKS ? k_s : v_s) + (stage * KT + pos - kt) * LDS;
-        const __nv_bfloat16* src = threadIdx.x < CHUNKS ? k_new : v_new;
-        *reinterpret_cast<uint4*>(dst + ch * 8) = *reinterpret_cast<const uint4*>(src + ch * 8);
+        const int own = new_key ? pos - kt - wn * NK : -1;
+        if (own < 0 || own >= NK) return;
+        for (int c = lane; c < 2 * CHUNKS; c += 32) {
+            const int ch = c % CHUNKS;
+            __nv_bfloat16* dst = (c < CHUNKS ? k_s : v_s) + (stage * KT + wn * NK + own) * LDS;
+            const __nv_bfloat16* src = c < CHUNKS ? k_new : v_new;
+            *reinterpret_cast<uint4*>(dst + ch * 8) = *reinterpret_cast<const uint4*>(src + ch * 8);
+        }
     };
 
     // the first tiles are requested before the wait, unless this step's own key is among what
@@ -321,7 +336,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_stride,
         int stage = 0;
         for (int kt = k_lo; kt < hi; kt += KT, stage = stage + 1 == STAGES ? 0 : stage + 1) {
             cp_async_wait<STAGES - 1>();              // this tile has landed; the next may be on their way
-            __syncthreads();
+            __syncwarp();
 
             const __nv_bfloat16* kb = k_s + stage * KT * LDS + wn * NK * LDS;
             const __nv_bfloat16* vb = v_s + stage * KT * LDS + wn * NK * LDS;
@@ -401,7 +416,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_stride,
                     mma_bf16(o_acc[jd + 1], pf[ks], b[2], b[3]);
                 }
             }
-            __syncthreads();                   // this stage is free: the tile after the next goes there
+            __syncwarp();                      // this stage is free: the tile after the next goes there
             if (kt + STAGES * KT < hi) {
                 load_tile(kt + STAGES * KT, stage);
                 fill_new(kt + STAGES * KT, stage);
