@@ -168,6 +168,13 @@ def chunks_ok(key_dim: int, value_dim: int) -> bool:
     return key_dim in (64, 128) and value_dim % 64 == 0
 
 
+def chunks_aligned(v: torch.Tensor, state: torch.Tensor) -> bool:
+    """Whether the rows of the values (four elements at a time) and of the states (16 bytes) lie
+    where the chunks' kernels can take them; the scan takes any."""
+    return (v.stride(0) % 4 == 0 and v.data_ptr() % (4 * v.element_size()) == 0
+            and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0)
+
+
 def _chunk_checks(q, k, v, state, out, items, portions, heads, key_dim, value_dim, name) -> None:
     for t, what in ((q, "q"), (k, "k"), (state, "state"), (out, "out")):
         _f32(t, what)

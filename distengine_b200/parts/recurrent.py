@@ -173,7 +173,7 @@ class ChunkedMixer(ProjectedMixer):
 
     def walk(self, q, k, v, state, out, ctx) -> None:
         """The step's tokens through the states under a fixed decay per head."""
-        chunked = self.chunked(ctx)
+        chunked = self.chunked(ctx, v, state)
         if chunked:
             rk.decay_chunks(q, k, v, state, out, self.heads, self.dk, self.dv, self.decay,
                             ctx.arrays["recurrent/items"], ctx.arrays["recurrent/portions"], ctx)
@@ -181,9 +181,10 @@ class ChunkedMixer(ProjectedMixer):
             rk.state_scan(q, k, v, state, out, self.heads, self.heads, self.dk, self.dv, ctx,
                           decay=self.decay, longest=rk.CHUNKED_PORTION - 1 if chunked else 0)
 
-    def chunked(self, ctx) -> int:
+    def chunked(self, ctx, v, state) -> int:
         """The step's note: 0 if its portions go token by token."""
-        return ctx.notes.get("recurrent/chunks", 0) if rk.chunks_ok(self.dk, self.dv) else 0
+        fits = rk.chunks_ok(self.dk, self.dv) and rk.chunks_aligned(v, state)
+        return ctx.notes.get("recurrent/chunks", 0) if fits else 0
 
 
 class GatedDeltaRule(ChunkedMixer):
@@ -267,7 +268,7 @@ class GatedDeltaRule(ChunkedMixer):
         rk.delta_prep(proj, a, self.conv, self.dt_bias, self.a_log, cache.state, self.state_rows,
                       ctx, qn, kn, vv, beta, gdec, H, G, dk, dv, self.b_col)
         o = ctx.buffer("delta.o", (n, H * dv), f32)
-        chunked = self.chunked(ctx)
+        chunked = self.chunked(ctx, vv, cache.state)
         if chunked:
             rk.delta_chunks(qn, kn, vv, cache.state, o, H, G, dk, dv, gdec, beta,
                             ctx.arrays["recurrent/items"], ctx.arrays["recurrent/portions"], ctx)
