@@ -1,0 +1,161 @@
+"""The recurrences in chunks of 64 tokens, and the kernels around them that take four channels at a
+time, against 64-bit token-by-token loops."""
+
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+import torch
+
+import plain_vomotar as pv
+from test_vomotar_mechanisms_gpu import _ctx, _gen, _scan_inputs
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+EPS = 2.0 ** -24
+
+
+def _step(lens, slots):
+    from distengine_b200.kernels import recurrent as rk
+    from distengine_b200.parts.recurrent import ChunkedMixer
+    ctx = _ctx(lens, [0] * len(lens), slots)
+    arrays, notes = {}, {}
+    prep = SimpleNamespace(host=ctx.host, notes=notes,
+                           add=lambda name, a: arrays.__setitem__(name, torch.from_numpy(a).to(DEV)))
+    ChunkedMixer.prepare(SimpleNamespace(), prep)
+    ctx.buffer = lambda name, shape, dtype: torch.full(shape, float("nan"), dtype=dtype, device=DEV)
+    longest = rk.CHUNKED_PORTION - 1 if notes["recurrent/chunks"] else 0
+    return ctx, arrays.get("recurrent/items"), arrays.get("recurrent/portions"), longest
+
+
+# bound: the sums over a chunk (64 terms, or dk) and over the chunks that a decay leaves, each term
+# of the size of the largest result, in float32: 64 + 128 roundings of 2^-24, doubled
+BOUND = 2 * (64 + 128) * EPS
+
+
+@pytest.mark.parametrize("rule", ["delta", "decay", "decay-bf16"])
+@pytest.mark.parametrize("dk,dv,rep", [(64, 64, 1), (64, 192, 2), (128, 128, 2)])
+@pytest.mark.parametrize("fast", [False, True])
+def test_recurrences_in_chunks(rule, dk, dv, rep, fast):
+    """Portions of whole chunks, of one token and one token less in the last, short ones between
+    them that go token by token; states carried on; decays near 1 and down to 1e-8 a token."""
+    from distengine_b200.kernels import recurrent as rk
+    H, lens, slots = 4, (257, 7, 192, 255), (3, 0, 4, 1)
+    assert rk.CHUNKED_PORTION == 192
+    ctx, items, portions, longest = _step(lens, slots)
+    n, g = sum(lens), _gen(dk + dv)
+    state = torch.randn(6, H * dk * dv + 12, generator=g) * 0.3
+    old = state.clone()
+    state = state.to(DEV)
+    out = torch.full((n, H * dv), float("nan"), device=DEV)
+    flat = lambda t: t.reshape(n, -1).to(DEV).contiguous()
+    if rule == "delta":
+        G = H // rep
+        q, k, v, beta, dec = _scan_inputs(n, H, G, dk, dv, 5)
+        if fast:
+            dec = dec ** torch.logspace(-3, 2, dk)
+        rk.delta_chunks(flat(q), flat(k), flat(v), state, out, H, G, dk, dv, flat(dec), flat(beta),
+                        items, portions, ctx)
+        rk.state_scan(flat(q), flat(k), flat(v), state, out, H, G, dk, dv, ctx, g=flat(dec),
+                      beta=flat(beta), longest=longest)
+        q, k = q.repeat_interleave(rep, 1), k.repeat_interleave(rep, 1)
+        dec = dec.double()
+    else:
+        q, k, v = (torch.randn(n, H, d, generator=g) * s for d, s in ((dk, dk ** -0.5), (dk, 0.3),
+                                                                      (dv, 1.0)))
+        v = v.to(torch.bfloat16 if rule == "decay-bf16" else torch.float32)
+        decay = torch.tensor([1e-8, 0.3, 0.9, 1.0] if fast else [0.99, 0.999, 0.9, 0.97])
+        for walk, extra in ((rk.decay_chunks, (decay.to(DEV), items, portions, ctx)),
+                            (rk.state_scan, (ctx,))):
+            heads = (H, H) if walk is rk.state_scan else (H,)
+            more = dict(decay=decay.to(DEV), longest=longest) if walk is rk.state_scan else {}
+            walk(flat(q), flat(k), flat(v), state, out, *heads, dk, dv, *extra, **more)
+        dec, beta = decay.double()[None, :, None].expand(n, H, dk), None
+    at = 0
+    for i, m in enumerate(lens):
+        S = old[slots[i], : H * dk * dv].double().view(H, dk, dv)
+        want = torch.zeros(m, H, dv, dtype=torch.float64)
+        for t in range(m):
+            j = at + t
+            S = S * dec[j][:, :, None]
+            u = v[j].double()
+            if beta is not None:
+                u = beta[j].double()[:, None] * (u - torch.einsum("hkv,hk->hv", S, k[j].double()))
+            S = S + k[j].double()[:, :, None] * u[:, None, :]
+            want[t] = torch.einsum("hkv,hk->hv", S, q[j].double())
+        got = out[at: at + m].double().cpu().view(m, H, dv)
+        err = (got - want).abs().max().item() / want.abs().max().item()
+        assert err <= BOUND, (rule, i, err)
+        end = state[slots[i], : H * dk * dv].double().cpu().view(H, dk, dv)
+        err = (end - S).abs().max().item() / S.abs().max().item()
+        assert err <= BOUND, (rule, "state", i, err)
+        at += m
+    untouched = [s for s in range(6) if s not in slots]
+    assert torch.equal(state[untouched].cpu(), old[untouched])
+    assert torch.equal(state[:, H * dk * dv:].cpu(), old[:, H * dk * dv:])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K,G,H,dk,dv,lens", [(1, 2, 2, 64, 64, (127, 1)), (2, 1, 3, 128, 128, (3, 130)),
+                                              (3, 4, 4, 64, 96, (9, 2, 140)), (4, 2, 4, 128, 64, (1, 2, 3, 129)),
+                                              (4, 2, 2, 64, 64, (127,))])
+def test_delta_preparation_in_runs(dtype, K, G, H, dk, dv, lens):
+    """Sequences that start within a run of eight tokens, fresh ones beside one whose earlier inputs
+    come from its state, steps around the 128 tokens from which runs are taken."""
+    from distengine_b200.kernels import recurrent as rk
+    g, n, C = _gen(K), sum(lens), 2 * G * dk + H * dv
+    proj = torch.randn(n, C + 4 + H + 4, generator=g)[:, : C + 4 + H + (-H) % 4].to(dtype).contiguous()
+    a = torch.randn(n, H * dk, generator=g)
+    taps, dt_bias = torch.randn(C, K, generator=g), torch.randn(H * dk, generator=g)
+    a_log = torch.randn(H, generator=g) * 0.5
+    rows = H * dk * dv
+    state = torch.randn(len(lens) + 1, rows + (K - 1) * C, generator=g).to(dtype).float()
+    pos0 = [0] * len(lens)
+    pos0[-1] = 50                                         # the last one has gone before
+    slots = list(range(len(lens), 0, -1))
+    state[slots[:-1], rows:] = 0.0                        # as a slot is handed out
+    ctx = _ctx(lens, pos0, slots)
+    bufs = [torch.full((n, w), float("nan"), device=DEV)
+            for w in (G * dk, G * dk, H * dv, H, H * dk)]
+    rk.delta_prep(proj.to(DEV), a.to(DEV), taps.to(DEV), dt_bias.to(DEV), a_log.to(DEV),
+                  state.to(DEV), rows, ctx, *bufs, H, G, dk, dv, C + 4)
+    y, at = [], 0
+    for i, m in enumerate(lens):
+        before = state[slots[i], rows:].double().view(K - 1, C)
+        x = torch.cat((before, proj[at: at + m, :C].double()))
+        y.append(pv.silu(pv.causal_conv(x, taps.double()))[K - 1:])
+        at += m
+    y = torch.cat(y)
+    want = [pv.unit(y[:, : G * dk].view(n, G, dk)) * dk ** -0.5,
+            pv.unit(y[:, G * dk: 2 * G * dk].view(n, G, dk)), y[:, 2 * G * dk:],
+            torch.sigmoid(proj[:, C + 4: C + 4 + H].double()),
+            torch.exp(-torch.exp(a_log.double())[None, :, None]
+                      * pv.softplus(a.double() + dt_bias.double()).view(n, H, dk))]
+    for got, ref, name in zip(bufs, want, ("q", "k", "v", "beta", "decay")):
+        ref = ref.reshape(n, -1)
+        err = (got.double().cpu() - ref).abs().max().item()
+        # float32: up to K products, a sum of dk squares, a few functions of 2 to 4 units each; the
+        # decay's exponent may be a few tens
+        assert err <= 64 * EPS * max(1.0, ref.abs().max().item()), (name, err)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,cols,pad", [(1, 4, 0), (3, 1028, 4), (5, 516, 8), (130, 2048, 0), (7, 258, 2),
+                                        (3, 4096, 4)])
+def test_rows_in_groups_of_four(dtype, n, cols, pad):
+    from distengine_b200.kernels import recurrent as rk
+    g = _gen(cols)
+    x = (torch.randn(n, cols + pad, generator=g) * 4).to(dtype)
+    o, w = torch.randn(n, cols, generator=g), torch.rand(cols, generator=g) + 0.5
+    wide = x.to(DEV)
+    out = torch.full((n, cols), float("nan"), device=DEV)
+    rk.silu_rows(wide[:, pad:], out)
+    want = pv.silu(x[:, pad:].double())
+    assert (out.double().cpu() - want).abs().max().item() <= 8 * EPS * want.abs().max().item()
+    res = torch.empty(n, cols, dtype=dtype, device=DEV)
+    rk.head_gate(o.to(DEV), wide[:, pad:], w.to(DEV), res, 1, cols, 1e-5, spanning=True)
+    o = o.double()
+    want = (o / torch.sqrt((o * o).mean(1, keepdim=True) + 1e-5) * w.double()
+            * torch.sigmoid(x[:, pad:].double()))
+    unit = 16 * EPS if dtype == torch.float32 else 2.0 ** -8 + 16 * EPS
+    assert ((res.double().cpu() - want).abs() <= unit * want.abs() + 1e-7).all()
