@@ -15,7 +15,10 @@
 // registers), so a token costs short chains of multiply-adds and butterfly sums over four lanes,
 // and a block of up to 32 columns walks its sequence's tokens of the step one after the other
 // while the next tokens' vectors arrive through cp.async.  The order of every sum depends on the
-// head's sizes only: a state does not depend, bit for bit, on how its tokens were cut into steps.
+// head's sizes only: a state does not depend, bit for bit, on how its tokens were cut into steps, as
+// long as they come through this scan.  (Portions of 192 tokens and more of the delta rule and of
+// retention, at key sizes 64 and 128, go through recurrent_chunks.cu, whose sums are ordered by
+// chunk; the scan then only moves their kept rows on.)
 //
 // What is token-parallel runs before the scan in a kernel of its own: the short causal
 // convolution over time with its activation (its last taps - 1 inputs are part of the slot's
@@ -122,7 +125,7 @@ __device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
 // the last inputs in registers, a head is 16 or 32 lanes of a warp, which form its norm.  The first
 // `conv_blocks` of the blocks do the convolution, 512 channels each, the others the decays (and
 // beta).  grid (runs of tokens, blocks), 128 threads.  2,048 tokens of 6,144 channels and 2,048
-// decays: 55 us (a block a token, a channel at a time: 128).
+// decays: 48 us (a block a token, a channel at a time: 128).
 constexpr int RUN = 8;
 
 template <typename T, int KK>
@@ -166,10 +169,24 @@ delta_prep_runs_kernel(const T* __restrict__ proj, int ld, const float* __restri
     const int c = (int)blockIdx.y * 512 + (int)threadIdx.x * 4;
     if (c >= C) return;                              // (whole warps: C is a multiple of 128)
     float w[KK][4];
+    if (KK == 4) {                                   // (a channel's taps are 16 bytes)
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+        for (int e = 0; e < 4; ++e) {
+            const float4 v = load_four(taps + (c + e) * KK);
+            const float t[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int j = 0; j < KK; ++j) w[j][e] = taps[(c + e) * KK + j];
+            for (int j = 0; j < KK; ++j) w[j][e] = t[j];
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int j = 0; j < KK; ++j) w[j][e] = taps[(c + e) * KK + j];
+    }
+    // lane i < RUN: token i's place in its sequence's portion
+    const int lane = threadIdx.x & 31;
+    int place = 0;
+    if (lane < count) place = positions[n0 + lane] - seq_pos0[token_seq[n0 + lane]];
     float4 in[RUN];
 #pragma unroll
     for (int i = 0; i < RUN; ++i)
@@ -181,7 +198,7 @@ delta_prep_runs_kernel(const T* __restrict__ proj, int ld, const float* __restri
     for (int i = 0; i < RUN; ++i) {
         if (i >= count) break;
         const int n = n0 + i;
-        const int off = positions[n] - seq_pos0[token_seq[n]];
+        const int off = __shfl_sync(0xffffffffu, place, i);
         if (i == 0 || off == 0) {
             // the inputs before this token: of its portion, or what the slot keeps
             const float* kept = state + (size_t)token_slot[n] * slot_stride + conv_offset;
@@ -865,7 +882,7 @@ DE_EXPORT int de_delta_prep(int dtype, const void* proj, int ld, const float* a,
     if (n >= 128 && K <= 4 && (dk == 64 || dk == 128) && (G * dk) % 128 == 0 && (H * dv) % 128 == 0 &&
         ld % 4 == 0 && (uintptr_t)proj % (4 * esize) == 0 && (uintptr_t)a % 16 == 0 &&
         (uintptr_t)dt_bias % 16 == 0 && (uintptr_t)state % 16 == 0 && slot_stride % 4 == 0 &&
-        conv_offset % 4 == 0 && (uintptr_t)qn % 16 == 0 && (uintptr_t)kn % 16 == 0 &&
+        conv_offset % 4 == 0 && (K != 4 || (uintptr_t)taps % 16 == 0) && (uintptr_t)qn % 16 == 0 && (uintptr_t)kn % 16 == 0 &&
         (uintptr_t)vv % 16 == 0 && (uintptr_t)gdec % 16 == 0) {
         const int conv_blocks = (2 * G * dk + H * dv + 511) / 512;
         const dim3 grid((n + RUN - 1) / RUN, conv_blocks + (H * dk + 511) / 512);
