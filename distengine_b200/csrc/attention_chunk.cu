@@ -1,7 +1,8 @@
 // Softmax attention inside chunks of positions, over the paged cache, with a penalty that grows
 // with the logarithm of the distance, keys and values of different sizes, and values that are
-// cached normalised.  Float32 arithmetic on the CUDA cores for float32 or bfloat16 storage:
-// scores, the penalty, the softmax weights and the weighted sum of the values are all 32-bit.
+// cached normalised.  Scores, the penalty, the softmax weights and the weighted sum of the values are
+// all 32-bit, for float32 or bfloat16 storage: on the CUDA cores, or for bfloat16 rows of 64 and 128
+// features on the tensor cores with the weights as three bfloat16 terms.
 //
 //   score(i, j) = (q_i . k_j) * scale - r1[h] * log(1 + r2[h] * (i - j))
 //   token i sees key j when j <= i and floor(i / chunk) = floor(j / chunk)   (chunks of positions
@@ -149,6 +150,46 @@ __global__ void kv_write_normed_kernel(const T* __restrict__ proj, int ld, int k
         v_pages[at * dv + i] = from_float<T>(to_float(vs[i]) * inv);
 }
 
+// 16 bytes of the projection as floats
+__device__ __forceinline__ void load_piece(const float* p, float* f) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+}
+__device__ __forceinline__ void load_piece(const __nv_bfloat16* p, float* f) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f[2 * i] = __uint_as_float(w[i] << 16);
+        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+}
+
+// two neighbouring features in one store
+__device__ __forceinline__ float4 load_four(const float* p) {
+    return *reinterpret_cast<const float4*>(p);
+}
+__device__ __forceinline__ float4 load_four(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
+                       __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void store_pair(float* p, float a, float b) {
+    *reinterpret_cast<float2*>(p) = make_float2(a, b);
+}
+__device__ __forceinline__ void store_pair(__nv_bfloat16* p, float a, float b) {
+    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
+}
+// and four
+__device__ __forceinline__ void store_four(float* p, const float4& v) {
+    *reinterpret_cast<float4*>(p) = v;
+}
+__device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&a),
+                                              *reinterpret_cast<const unsigned*>(&b));
+}
+
 // Queries and keys turned by position, values turned by position over all their features, keys
 // and values into the pages.  proj row = [q (H dk) | k (G dk) | v (G dv) | ...] (a run that reads
 // another run's cache has q only: write_kv 0).  Pairs are (i, i + n/2) of the first n features:
@@ -226,6 +267,76 @@ __global__ void kv_write_rotated_kernel(T* __restrict__ proj, int ld, const int*
     pdl_trigger();
 }
 
+// a token's cosines and sines of one list of frequencies, [half] each (as every head would form them)
+__device__ __forceinline__ void angles(float* tab, const float* __restrict__ freq, int half, float pos) {
+    for (int i = threadIdx.x; i < half; i += blockDim.x)
+        sincosf(pos * freq[i], tab + half + i, tab + i);
+}
+// four neighbouring pairs (i, i + half) of src turned into dst
+template <typename T>
+__device__ __forceinline__ void turn_four(const T* src, T* dst, const float* tab, int half, int i) {
+    const float4 a = load_four(src + i), b = load_four(src + i + half);
+    const float4 c = load_four(tab + i), s = load_four(tab + half + i);
+    float4 x, y;
+    rope_rotate(a.x, b.x, c.x, s.x, x.x, y.x);
+    rope_rotate(a.y, b.y, c.y, s.y, x.y, y.y);
+    rope_rotate(a.z, b.z, c.z, s.z, x.z, y.z);
+    rope_rotate(a.w, b.w, c.w, s.w, x.w, y.w);
+    store_four(dst + i, x);
+    store_four(dst + i + half, y);
+}
+
+// The same in groups of four features, the token's angles formed once for all heads: where half the
+// turned part, the plain part and the values' (half) rows are whole groups, and everything lies at
+// such addresses.  2,048 tokens, 16 + 4 heads of 128: 13 us (23, each head forming its angles).
+template <typename T>
+__global__ void kv_write_rotated_vec_kernel(
+    T* __restrict__ proj, int ld, const int* __restrict__ positions,
+    const int* __restrict__ token_slot, const float* __restrict__ fk, int rot,
+    const float* __restrict__ fv, int H, int G, int dk, int dv, T* __restrict__ k_pages,
+    T* __restrict__ v_pages, const int* __restrict__ block_table, int table_stride, int page,
+    int num_pages, int write_kv, int* __restrict__ status) {
+    __shared__ __align__(16) float ktab[MAX_D], vtab[MAX_D];
+    const int n = blockIdx.x;
+    const int pos = positions[n];
+    T* row = proj + (size_t)n * ld;
+    const int half = rot / 2, vhalf = dv / 2;
+    size_t at = 0;
+    bool can_write = write_kv != 0;
+    if (can_write) {
+        const int page_id = block_table[(size_t)token_slot[n] * table_stride + pos / page];
+        if (page_id < 0 || page_id >= num_pages) {   // never written outside the pool
+            if (threadIdx.x == 0) atomicExch(status, 1);
+            can_write = false;
+        }
+        at = ((size_t)page_id * G) * page + (size_t)(pos % page);
+    }
+    angles(ktab, fk, half, (float)pos);
+    if (can_write && fv != nullptr) angles(vtab, fv, vhalf, (float)pos);
+    __syncthreads();
+    pdl_wait();
+    const int per = (dk - half) / 4;                 // groups of pairs, then plain groups
+    const int qk_heads = H + (can_write ? G : 0);
+    for (int idx = threadIdx.x; idx < qk_heads * per; idx += blockDim.x) {
+        const int h = idx / per, i = (idx - h * per) * 4;
+        T* src = row + h * dk;
+        T* dst = h < H ? src : k_pages + (at + (size_t)(h - H) * page) * dk;   // q in place
+        if (i < half) turn_four(src, dst, ktab, half, i);
+        else if (h >= H) store_four(dst + i + half, load_four(src + i + half));
+    }
+    if (can_write) {
+        const T* vs = row + (H + G) * dk;
+        const int vper = (fv != nullptr ? vhalf : dv) / 4;
+        for (int idx = threadIdx.x; idx < G * vper; idx += blockDim.x) {
+            const int h = idx / vper, i = (idx - h * vper) * 4;
+            T* dst = v_pages + (at + (size_t)h * page) * dv;
+            if (fv != nullptr) turn_four(vs + h * dv, dst, vtab, vhalf, i);
+            else store_four(dst + i, load_four(vs + h * dv + i));
+        }
+    }
+    pdl_trigger();
+}
+
 // What lies between a mixer's stacked projection and its attention, for mixers that do more to
 // q, k and v than turn them: proj row = [q (H dk) | k (G dk) | v (G dv) | ...], C = (H + G) dk +
 // G dv channels.  In this order, each step optional:
@@ -253,6 +364,7 @@ __global__ void kv_write_rotated_kernel(T* __restrict__ proj, int ld, const int*
 struct Prepare {
     const float* bias;
     const float* taps;
+    int by_tap;                      // taps lie [K][C] at 16-byte addresses, as does the bias; else [C][K]
     int K;
     float* state;
     long long slot_stride;
@@ -274,37 +386,6 @@ struct Prepare {
     int v_from_k;
 };
 
-// 16 bytes of the projection as floats
-__device__ __forceinline__ void load_piece(const float* p, float* f) {
-    const float4 v = *reinterpret_cast<const float4*>(p);
-    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
-}
-__device__ __forceinline__ void load_piece(const __nv_bfloat16* p, float* f) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const unsigned w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
-}
-
-// two neighbouring features in one store
-__device__ __forceinline__ void store_pair(float* p, float a, float b) {
-    *reinterpret_cast<float2*>(p) = make_float2(a, b);
-}
-__device__ __forceinline__ void store_pair(__nv_bfloat16* p, float a, float b) {
-    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
-}
-// and four
-__device__ __forceinline__ void store_four(float* p, const float4& v) {
-    *reinterpret_cast<float4*>(p) = v;
-}
-__device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&a),
-                                              *reinterpret_cast<const unsigned*>(&b));
-}
 // Two sums over a block at once; every thread gets both.  The order of the additions depends on
 // the block's size only.
 __device__ __forceinline__ void block_sum2(float& a, float& b, float* scratch /* 66 floats */) {
@@ -327,9 +408,21 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float* scratch /*
     b = scratch[65];
 }
 
+template <int PN> __device__ __forceinline__ void load_run(const float* p, int wide, float* f) {
+    if (wide) {
+#pragma unroll
+        for (int e = 0; e < PN; e += 4) load_piece(p + e, f + e);
+    } else {
+#pragma unroll
+        for (int e = 0; e < PN; ++e) f[e] = p[e];
+    }
+}
+
 // VEC: the rows of proj are whole 16-byte pieces at 16-byte addresses and C is a whole number of
 // pieces; a thread then takes the convolution of a piece's channels at once.  The sums are the
 // same chains of multiply-adds either way.
+// The taps come tap by tap (a lane's channels side by side): 2,402 tokens of 3,072 channels with
+// four taps 44 us, 60 where a channel's taps lay together (32 lines a request).
 template <typename T, bool VEC>
 __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __restrict__ q_out,
                                    const int* __restrict__ positions,
@@ -369,10 +462,8 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __rest
         for (int c0 = threadIdx.x * PN; c0 < C; c0 += blockDim.x * PN) {
             float acc[PN], b[PN];
 #pragma unroll
-            for (int e = 0; e < PN; ++e) {
-                acc[e] = 0.0f;
-                b[e] = pp.bias ? pp.bias[c0 + e] : 0.0f;
-            }
+            for (int e = 0; e < PN; ++e) acc[e] = b[e] = 0.0f;
+            if (pp.bias) load_run<PN>(pp.bias + c0, pp.by_tap, b);
             for (int j = 0; j < K; ++j) {
                 const int rel = off - (K - 1) + j;
                 if (pos - (K - 1) + j < 0) continue;             // before the sequence's start
@@ -383,12 +474,19 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __rest
 #pragma unroll
                     for (int e = 0; e < PN; ++e) x[e] = kept[(size_t)(off + j) * C + c0 + e];
                 }
+                float w[PN];
+                if (pp.by_tap) {
+                    load_run<PN>(pp.taps + (size_t)j * C + c0, 1, w);
+                } else {
 #pragma unroll
-                for (int e = 0; e < PN; ++e)
-                    acc[e] = fmaf(pp.taps[(c0 + e) * K + j], x[e] + b[e], acc[e]);
+                    for (int e = 0; e < PN; ++e) w[e] = pp.taps[(c0 + e) * K + j];
+                }
+#pragma unroll
+                for (int e = 0; e < PN; ++e) acc[e] = fmaf(w[e], x[e] + b[e], acc[e]);
             }
 #pragma unroll
-            for (int e = 0; e < PN; ++e) sh[c0 + e] = acc[e];
+            for (int e = 0; e < PN; e += 4)
+                store_four(sh + c0 + e, make_float4(acc[e], acc[e + 1], acc[e + 2], acc[e + 3]));
         }
     } else if (pp.taps != nullptr && pp.K > 1) {
         const int K = pp.K;
@@ -401,7 +499,7 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __rest
                 if (pos - (K - 1) + j < 0) continue;             // before the sequence's start
                 const float x = rel >= 0 ? to_float(proj[(size_t)(n - (K - 1) + j) * ld + c])
                                          : kept[(size_t)(off + j) * C + c];
-                acc = fmaf(pp.taps[c * K + j], x + b, acc);
+                acc = fmaf(pp.taps[pp.by_tap ? j * C + c : c * K + j], x + b, acc);
             }
             sh[c] = acc;
         }
@@ -679,6 +777,53 @@ __global__ void attn_finish_kernel(const float* __restrict__ o, const int* __res
             if (gt) x *= 1.0f / (1.0f + expf(-to_float(gt[gate_per_head ? idx / dv : idx])));
             dst[idx] = from_float<T>(x);
         }
+    }
+}
+
+// The same in groups of four features (with `fv`: of four pairs, the angles formed once a token), for
+// heads of whole groups at such addresses.  2,048 tokens, 16 heads of 128, turned: 10 us (14).
+template <typename T>
+__global__ void attn_finish_vec_kernel(const float* __restrict__ o, const int* __restrict__ positions,
+                                       const float* __restrict__ fv, const T* __restrict__ gate,
+                                       int ld_gate, T* __restrict__ out, int H, int dv,
+                                       int gate_per_head) {
+    __shared__ __align__(16) float tab[MAX_D];
+    const int n = blockIdx.x, half = dv / 2;
+    const float* src = o + (size_t)n * H * dv;
+    T* dst = out + (size_t)n * H * dv;
+    const T* gt = gate ? gate + (size_t)n * ld_gate : nullptr;
+    if (fv != nullptr) angles(tab, fv, half, (float)positions[n]);
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    auto finish = [&](float4 v, int h, int at) {
+        if (gt) {
+            float4 g;
+            if (gate_per_head) g.x = g.y = g.z = g.w = to_float(gt[h]);
+            else g = load_four(gt + at);
+            v.x *= 1.0f / (1.0f + expf(-g.x));
+            v.y *= 1.0f / (1.0f + expf(-g.y));
+            v.z *= 1.0f / (1.0f + expf(-g.z));
+            v.w *= 1.0f / (1.0f + expf(-g.w));
+        }
+        store_four(dst + at, v);
+    };
+    if (fv == nullptr) {
+        for (int i = threadIdx.x * 4; i < H * dv; i += blockDim.x * 4)
+            finish(load_four(src + i), i / dv, i);
+        return;
+    }
+    for (int idx = threadIdx.x; idx < H * half / 4; idx += blockDim.x) {
+        const int h = idx / (half / 4), i = (idx - h * (half / 4)) * 4, at = h * dv + i;
+        const float4 a = load_four(src + at), b = load_four(src + at + half);
+        const float4 c = load_four(tab + i), s = load_four(tab + half + i);
+        float4 x, y;
+        rope_rotate(a.x, b.x, c.x, -s.x, x.x, y.x);
+        rope_rotate(a.y, b.y, c.y, -s.y, x.y, y.y);
+        rope_rotate(a.z, b.z, c.z, -s.z, x.z, y.z);
+        rope_rotate(a.w, b.w, c.w, -s.w, x.w, y.w);
+        finish(x, h, at);
+        finish(y, h, at + half);
     }
 }
 
@@ -2441,6 +2586,18 @@ DE_EXPORT int de_kv_write_rotated(int dtype, void* proj, int ld, const int* posi
     cudaStream_t s = (cudaStream_t)stream;
     const int work = (H + G) * dk + G * dv;
     const int threads = n >= 512 ? 128 : (work >= 2048 ? 512 : 256);
+    const size_t four = dtype == DE_BF16 ? 8 : 16;   // bytes of a group of four
+    if (rot % 8 == 0 && (dk - rot) % 4 == 0 && dv % (fv != nullptr ? 8 : 4) == 0 && ld % 4 == 0 &&
+        dk <= MAX_D && dv <= MAX_D && (uintptr_t)proj % four == 0 && (uintptr_t)k_pages % four == 0 &&
+        (uintptr_t)v_pages % four == 0) {
+#define ROT(T)                                                                                  \
+    return de_launch(kv_write_rotated_vec_kernel<T>, dim3(n), dim3(work >= 1024 ? 256 : 128), 0, s, \
+                     (T*)proj, ld, positions, token_slot, fk, rot, fv, H, G, dk, dv, (T*)k_pages, \
+                     (T*)v_pages, block_table, table_stride, page, num_pages, write_kv, status)
+        if (dtype == DE_BF16) ROT(__nv_bfloat16);
+        ROT(float);
+#undef ROT
+    }
     if (dtype == DE_BF16)
         return de_launch(kv_write_rotated_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0, s,
                          (__nv_bfloat16*)proj, ld, positions, token_slot, fk, rot, fv, H, G, dk, dv,
@@ -2453,7 +2610,7 @@ DE_EXPORT int de_kv_write_rotated(int dtype, void* proj, int ld, const int* posi
 
 DE_EXPORT int de_qkv_prepare(int dtype, const void* proj, int ld, void* q_out,
                              const int* positions, const int* token_seq, const int* token_slot,
-                             const int* seq_pos0, const float* bias, const float* taps, int K,
+                             const int* seq_pos0, const float* bias, const float* taps, int by_tap, int K,
                              float* state, long long slot_stride, int conv_offset, int norm,
                              const float* q_weight, const float* k_weight, float eps,
                              const float* freq, int rot, float magnitude, int adjacent,
@@ -2469,7 +2626,8 @@ DE_EXPORT int de_qkv_prepare(int dtype, const void* proj, int ld, void* q_out,
         (mix != 0 && v_first == nullptr) || (mix == 2 && lambda == nullptr) ||
         (taps != nullptr && (K < 1 || (K > 1 && state == nullptr))))
         return -2;
-    const Prepare pp = {bias, taps, K, state, slot_stride, conv_offset, norm, q_weight, k_weight,
+    if (by_tap && ((uintptr_t)taps % 16 || (uintptr_t)bias % 16)) return -2;
+    const Prepare pp = {bias, taps, by_tap, K, state, slot_stride, conv_offset, norm, q_weight, k_weight,
                         eps, freq, rot, magnitude, adjacent, temp_coef, temp_every, mix, lambda,
                         v_first, keep_here, v_from_k};
     cudaStream_t s = (cudaStream_t)stream;
@@ -2521,6 +2679,17 @@ DE_EXPORT int de_attn_finish(int dtype, const float* o, const int* positions, co
     if (fv != nullptr && dv % 2) return -2;
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = n >= 512 ? 128 : (H * dv >= 2048 ? 512 : 256);
+    const size_t four = dtype == DE_BF16 ? 8 : 16;   // bytes of a group of four
+    if (dv % (fv != nullptr ? 8 : 4) == 0 && dv <= MAX_D && (uintptr_t)o % 16 == 0 &&
+        (uintptr_t)out % four == 0 &&
+        (gate == nullptr || gate_per_head || (ld_gate % 4 == 0 && (uintptr_t)gate % four == 0))) {
+#define FIN(T)                                                                                  \
+    return de_launch(attn_finish_vec_kernel<T>, dim3(n), dim3(H * dv >= 1024 ? 256 : 128), 0, s, o, \
+                     positions, fv, (const T*)gate, ld_gate, (T*)out, H, dv, gate_per_head)
+        if (dtype == DE_BF16) FIN(__nv_bfloat16);
+        FIN(float);
+#undef FIN
+    }
     if (dtype == DE_BF16)
         return de_launch(attn_finish_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0, s, o,
                          positions, fv, (const __nv_bfloat16*)gate, ld_gate, (__nv_bfloat16*)out, H,

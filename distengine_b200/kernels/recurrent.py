@@ -352,7 +352,8 @@ def chunk_rows_per_tile(dtype: torch.dtype, key_dim: int, value_dim: int, wide: 
                         longest_rows: int = 0) -> int:
     """Rows of a tile of the chunk attention: 8, or 32 for steps with prompt portions (``wide``)
     at sizes whose rows are whole 16-byte pieces, or 64 where the longest portion has at least 48
-    rows (``longest_rows``: its tokens times the query heads a kv head)."""
+    rows (``longest_rows``: its tokens times the query heads a kv head).  bfloat16 rows of 64 and
+    128 features go to the tensor cores in tiles of 32 or 64 by the same rule."""
     hint = max(int(wide), int(longest_rows)) if wide else 0
     return int(library.load("attention_chunk").de_attn_chunk_rows(_tag(dtype), key_dim, value_dim,
                                                                   hint))
@@ -364,9 +365,9 @@ _sm_count: dict[int, int] = {}
 def long_portion_rows(seq_qlen, heads: int, kv_heads: int) -> int:
     """The rows of a step's longest portion (tokens times query heads a kv head) if tiles of 64
     rows would still give every SM two blocks, else 0: what ``chunk_rows_per_tile`` takes as
-    ``longest_rows``.  (Measured on B200, 16 heads on 4 kv heads of 128: a prompt of 512 tokens
-    takes 274 us in 128 blocks of 64 rows against 221 us in 256 blocks of 32; one of 2,048 tokens
-    739 against 1,362 us.)"""
+    ``longest_rows``.  (Measured on B200 with the kernels of the CUDA cores, 16 heads on 4 kv heads
+    of 128: a prompt of 512 tokens takes 274 us in 128 blocks of 64 rows against 221 us in 256 blocks
+    of 32; one of 2,048 tokens 739 against 1,362 us.)"""
     group = heads // kv_heads
     device = torch.cuda.current_device()
     if device not in _sm_count:
@@ -583,7 +584,8 @@ def qkv_prepare(proj: torch.Tensor, q_out: torch.Tensor, heads: int, kv_heads: i
                 taps: "torch.Tensor | None" = None, kept: "tuple | None" = None,
                 norm: "tuple | None" = None, rotation: "tuple | None" = None,
                 temperature: "tuple | None" = None, mix: "tuple | None" = None,
-                keep_here: bool = False, values_from_keys: bool = False) -> None:
+                keep_here: bool = False, values_from_keys: bool = False,
+                by_tap: bool = False) -> None:
     """From the stacked projection ``proj`` = [q (H dk) | k (G dk) | v (G dv) | ...] to the
     queries ``q_out`` [N, H dk] and the keys and values in the pages, through (each optional, in
     this order): ``bias`` float32 [C] (C = (H + G) dk + G dv); ``taps`` float32 [C, K], a causal
@@ -594,7 +596,8 @@ def qkv_prepare(proj: torch.Tensor, q_out: torch.Tensor, heads: int, kv_heads: i
     v_first) or ("take", v_first, lambda [1]) with v_first float32 [N, G dv].  ``keep_here``:
     only for a step in which every sequence brings one token - the kernel then also moves the
     slots' kept rows on, and no ``conv_keep`` follows.  ``values_from_keys``: there is no v in
-    ``proj`` (C = (H + G) dk, dv = dk): the values are the keys before norm and rotation."""
+    ``proj`` (C = (H + G) dk, dv = dk): the values are the keys before norm and rotation.
+    ``by_tap``: the taps lie [K, C] (faster: neighbouring channels side by side)."""
     n = proj.shape[0]
     channels = (heads + kv_heads) * key_dim + (0 if values_from_keys else kv_heads * value_dim)
     _need(not values_from_keys or key_dim == value_dim,
@@ -610,19 +613,19 @@ def qkv_prepare(proj: torch.Tensor, q_out: torch.Tensor, heads: int, kv_heads: i
     if bias is not None:
         _f32(bias, "bias")
         _need(bias.shape == (channels,) and bias.is_contiguous(), "qkv_prepare: bias [C]")
-    conv = (None, 0, None, 0, 0)
+    conv = (None, 0, 0, None, 0, 0)
     if taps is not None:
         _f32(taps, "taps")
-        _need(taps.dim() == 2 and taps.shape[0] == channels and taps.is_contiguous(),
-              "qkv_prepare: taps [C, K]")
-        k = taps.shape[1]
-        conv = (taps.data_ptr(), k, None, 0, 0)
+        _need(taps.dim() == 2 and taps.shape[int(by_tap)] == channels and taps.is_contiguous(),
+              "qkv_prepare: taps [C, K], or [K, C] by tap")
+        k = taps.shape[1 - int(by_tap)]
+        conv = (taps.data_ptr(), int(by_tap), k, None, 0, 0)
         if k > 1:
             state, offset = kept
             _f32(state, "state")
             _need(state.dim() == 2 and offset + (k - 1) * channels <= state.shape[1],
                   "qkv_prepare: the state rows are too short for the convolution's inputs")
-            conv = (taps.data_ptr(), k, state.data_ptr(), state.stride(0), offset)
+            conv = (taps.data_ptr(), int(by_tap), k, state.data_ptr(), state.stride(0), offset)
     normed = (0, None, None, 0.0)
     if norm is not None:
         mode, qw, kw, eps = norm

@@ -175,8 +175,8 @@ class SinkAttention(ProjectedMixer):
             self.sink = torch.zeros(self.heads, dtype=torch.float32, device=dev)
         self.bias = vector32(torch.cat([tensors[n + ".b"].reshape(-1) for n in names]), dev) \
             if self.biased else None
-        self.conv = vector32(torch.cat([tensors[n + ".conv"] for n in names], dim=0), dev) \
-            if self.taps else None
+        self.conv = vector32(torch.cat([tensors[n + ".conv"] for n in names], dim=0).t()
+                             .contiguous(), dev) if self.taps else None       # [taps, channels]
         weighted = self.norm is not None and self.norm_weighted
         self.q_norm = vector32(tensors["q.norm"], dev) if weighted else None
         self.k_norm = vector32(tensors["k.norm"], dev) if weighted else None
@@ -271,7 +271,7 @@ class SinkAttention(ProjectedMixer):
         keep_here = state is not None and bool(ctx.notes.get("sink_attention/single_tokens"))
         rk.qkv_prepare(
             proj, q, H, G, dk, dv, pages.k_pages, pages.v_pages, pages.block_table, ctx,
-            bias=self.bias, taps=self.conv, kept=(state.state, 0) if state is not None else None,
+            bias=self.bias, taps=self.conv, by_tap=True, kept=(state.state, 0) if state is not None else None,
             norm=(self.norm, self.q_norm, self.k_norm, self.eps) if self.norm else None,
             rotation=(self.freq, self.magnitude, self.adjacent), temperature=self.temperature,
             mix=mix, keep_here=keep_here, values_from_keys=self.values_from_keys)

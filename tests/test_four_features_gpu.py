@@ -1,0 +1,79 @@
+"""The kernels before and after the window and sink attention that take four features at a time
+against their general forms, which rows at other addresses reach: the same bits."""
+
+import pytest
+import torch
+
+from test_vomotar_mechanisms_gpu import _ctx, _gen
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rows(t, pad):
+    """The same rows, `pad` elements apart beyond their own."""
+    wide = torch.zeros(t.shape[0], t.shape[1] + pad, dtype=t.dtype, device=DEV)
+    wide[:, : t.shape[1]] = t.to(DEV)
+    return wide[:, : t.shape[1]]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,dk,dv,rot,turned", [(3, 1, 64, 64, 64, True), (4, 2, 128, 40, 32, True),
+                                                   (2, 2, 12, 4, 8, False), (8, 4, 256, 256, 256, True),
+                                                   (1, 1, 20, 12, 0, False)])
+@pytest.mark.parametrize("write", [True, False])
+def test_rotation_and_cache_write(dtype, H, G, dk, dv, rot, turned, write):
+    from distengine_b200.kernels import recurrent as rk
+    lens, page, g = (5, 1, 9), 8, _gen(dk)
+    ctx = _ctx(lens, (3, 900, 0), (1, 0, 2))
+    n = sum(lens)
+    proj = torch.randn(n, H * dk + G * (dk + dv), generator=g).to(dtype)
+    fk, fv = torch.rand(rot // 2, generator=g), torch.rand(dv // 2, generator=g)
+    table = torch.full((3, 120), -1, dtype=torch.int32)
+    table[1, 0], table[0, 112], table[2, 0], table[2, 1] = 2, 0, 3, 1
+    results = []
+    for pad in (4 - proj.shape[1] % 4, 5 - proj.shape[1] % 4):      # whole groups of four, or not
+        p = _rows(proj, pad)
+        kp = torch.zeros(4, G, page, dk, dtype=dtype, device=DEV)
+        vp = torch.zeros(4, G, page, dv, dtype=dtype, device=DEV)
+        rk.kv_write_rotated(p, fk.to(DEV), rot, fv.to(DEV) if turned else None, H, G, dk, dv, kp, vp,
+                            table.to(DEV), write, ctx)
+        # (the second sequence's position 900 has its page; one of the first's does not matter)
+        o = torch.randn(n, H * dv, generator=_gen(1)).to(DEV)
+        gate = torch.randn(n, H * dv, generator=_gen(2)).to(dtype)
+        out = torch.empty(n, H * dv, dtype=dtype, device=DEV)
+        rk.attention_finish(o, fv.to(DEV) if turned else None, _rows(gate, 4 if pad % 2 == 0 else 5),
+                            out, H, dv, ctx)
+        results.append((p.clone(), kp, vp, out))
+    assert int(ctx.status.item()) == 0
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K", [1, 2, 4, 5])
+@pytest.mark.parametrize("biased", [True, False])
+def test_taps_by_tap(dtype, K, biased):
+    from distengine_b200.kernels import recurrent as rk
+    H, G, dk, dv, page, g = 4, 2, 64, 64, 16, _gen(K)
+    lens, C = (7, 1, 3), (H + G) * dk + G * dv
+    ctx = _ctx(lens, (0, 20, 2), (1, 0, 2))
+    n = sum(lens)
+    taps, bias = torch.randn(C, K, generator=g), torch.randn(C, generator=g)
+    state = torch.randn(3, max(K - 1, 1) * C, generator=g).to(DEV)
+    table = torch.tensor([[-1, 3], [0, -1], [2, -1]], dtype=torch.int32, device=DEV)
+    proj = torch.randn(n, C, generator=g).to(dtype)
+    results = []
+    for by_tap, pad in ((False, 8), (True, 8), (True, 3)):
+        q = torch.empty(n, H * dk, dtype=dtype, device=DEV)
+        kp = torch.zeros(4, G, page, dk, dtype=dtype, device=DEV)
+        vp = torch.zeros(4, G, page, dv, dtype=dtype, device=DEV)
+        rk.qkv_prepare(_rows(proj, pad), q, H, G, dk, dv, kp, vp, table, ctx,
+                       bias=bias.to(DEV) if biased else None,
+                       taps=(taps.t().contiguous() if by_tap else taps).to(DEV), by_tap=by_tap,
+                       kept=(state, 0) if K > 1 else None)
+        results.append((q, kp, vp))
+    assert int(ctx.status.item()) == 0
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            assert torch.equal(a, b)
