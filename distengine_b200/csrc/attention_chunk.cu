@@ -1457,7 +1457,9 @@ attn_chunk_tiled_kernel(const T* __restrict__ q, int q_stride, void* __restrict_
 // its product with the values as three bfloat16 terms whose sum is the float32 weight.  What the
 // tensor cores add up is a tile's share only, the small terms first; the running sums of a row are
 // float32 multiply-adds (acc <- acc * correction + tile's share).  Scores, cap, penalty, maximum and
-// exponentials are those of the kernels above.  A row's tiles lie at absolute multiples of 32, so its result does not depend on what shares its block or its step.
+// exponentials are those of the kernels above.  A row's tiles lie at
+// absolute multiples of 32, so its result does not depend on what shares its block or its step (but
+// on whether the step's tiles are of 32 or 64 rows).
 // The kernel above runs the same work on the CUDA cores, where a prompt of 2,048 tokens of 16 heads
 // of 128 on 4 kv heads takes 734 us with a window of 1,024 and a cap, 147 us here, 39 us of
 // 512 tokens against 221 (its distance from 64 bits 2.5e-7 of the result against 4.7e-7); without
@@ -1487,6 +1489,7 @@ __device__ __forceinline__ unsigned pack2(float lo, float hi) {
     return *reinterpret_cast<const unsigned*>(&v);
 }
 // x and y as sums of three bfloat16 numbers each: all 24 bits of a float32 mantissa
+// (an infinite value of v meets lower terms that are zero: its rows become NaN, not infinite)
 __device__ __forceinline__ void split3(float x, float y, unsigned& a, unsigned& b, unsigned& c) {
     a = pack2(x, y);
     const float rx = x - __uint_as_float(a << 16), ry = y - __uint_as_float(a & 0xffff0000u);
