@@ -1489,12 +1489,72 @@ __device__ __forceinline__ unsigned pack2(float lo, float hi) {
     return *reinterpret_cast<const unsigned*>(&v);
 }
 // x and y as sums of three bfloat16 numbers each: all 24 bits of a float32 mantissa
-// (an infinite value of v meets lower terms that are zero: its rows become NaN, not infinite)
 __device__ __forceinline__ void split3(float x, float y, unsigned& a, unsigned& b, unsigned& c) {
     a = pack2(x, y);
     const float rx = x - __uint_as_float(a << 16), ry = y - __uint_as_float(a & 0xffff0000u);
     b = pack2(rx, ry);
     c = pack2(rx - __uint_as_float(b << 16), ry - __uint_as_float(b & 0xffff0000u));
+}
+
+// A row formed again, as attn_chunk_kernel forms it (features and keys in ascending order, keys of
+// weight 0 skipped), by one warp straight from the pages: for rows in which the products on the
+// tensor cores met an infinity or NaN.  A weight of 0 times such a value is NaN there, so that a
+// value that the row does not see would spoil it, and an infinite value meets lower terms of a
+// weight that are 0.  q: the row's D query features; a lane returns features lane, lane + 32, ...
+// Rows without such values pay for the look at their results: 0 to 0.25 us a launch, up to 3 %.
+template <int D, typename Q>
+__device__ __forceinline__ void row_again(
+    const Q* q, const __nv_bfloat16* k_pages, const __nv_bfloat16* v_pages, const int* table,
+    int num_pages, int hk, int kv_heads, int page, int pos, int kv_begin, int kv_end, float scale,
+    float pen1, float pen2, bool penalty, const Sight& sight, float& m_out, float& l_out,
+    float (&acc)[D / 32]) {
+    const int lane = threadIdx.x & 31;
+    const int lo = max(kv_begin, sight_lo(sight, pos)), hi = min(kv_end, pos + 1);
+    const int first = kv_begin > 0 ? 0 : sight_first(sight, lo);
+    const TileWalk walk(lo, first, TILE);
+    float m = -INFINITY, l = 0.0f;
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) acc[i] = 0.0f;
+    for (int kt = walk.start; kt < hi; kt = walk.next(kt, TILE)) {
+        const int kpos = kt + lane;
+        bool valid = (kpos >= lo || kpos < first) && kpos < hi;
+        long long at = 0;
+        if (valid) {
+            const int id = table[kpos / page];
+            valid = id >= 0 && id < num_pages;
+            if (valid) at = ((long long)id * kv_heads + hk) * page + kpos % page;
+        }
+        float s = 0.0f;
+        if (valid) {
+            for (int i = 0; i < D; i += 8) {
+                float k[8];
+                load_piece(k_pages + at * D + i, k);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) s = fmaf(to_float(q[i + e]), k[e], s);
+            }
+            s = sight_score(sight, s, scale, pen1, pen2, penalty, (float)(pos - kpos));
+        } else {
+            s = -INFINITY;
+        }
+        const float m_new = fmaxf(m, warp_max(s));
+        if (m_new == -INFINITY) continue;
+        const float p = valid ? expf(s - m_new) : 0.0f;
+        const float corr = expf(m - m_new);
+        l = l * corr + warp_sum(p);
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) acc[i] *= corr;
+        for (int j = 0; j < TILE; ++j) {
+            const float pj = __shfl_sync(0xffffffffu, p, j);
+            const long long row = __shfl_sync(0xffffffffu, at, j);
+            if (pj == 0.0f) continue;
+#pragma unroll
+            for (int i = 0; i < D / 32; ++i)
+                acc[i] = fmaf(pj, to_float(v_pages[row * sight.v_stride + lane + 32 * i]), acc[i]);
+        }
+        m = m_new;
+    }
+    m_out = m;
+    l_out = l;
 }
 
 // tanh(x) for |x| <= TANH_NEAR to 7e-8 of its value (as good as tanhf and a third of its
@@ -1846,6 +1906,7 @@ attn_chunk_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, void* _
                                  joint[(4 * j + x) * 64] * other_f[x >> 1]);
     }
     const bool pairs = out_stride % 2 == 0 && (uintptr_t)out % (out_f32 ? 8 : 4) == 0;
+    unsigned spoilt = 0;                             // rows that met an infinity or NaN
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         l[e] += __shfl_xor_sync(0xffffffffu, l[e], 1);
@@ -1854,12 +1915,14 @@ attn_chunk_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, void* _
         const float inv = sight_inverse(sight, hq[e], m[e], l[e]);
         const size_t token = (size_t)(tok0 + tok[e]);
         const size_t o = token * out_stride + hq[e] * D;
+        float zero = 0.0f;
 #pragma unroll
         for (int j = 0; j < DT; ++j) {
             const int col = j * 8 + 2 * tig;
             const float a = acc[j][2 * e] * inv * sight_gate<T>(sight, token, hq[e], D, col);
             const float b = acc[j][2 * e + 1] * inv *
                             sight_gate<T>(sight, token, hq[e], D, col + 1);
+            zero = fmaf(a, 0.0f, fmaf(b, 0.0f, zero));
             if (!pairs) {
                 store_out<T>(out, out_f32, o + col, a);
                 store_out<T>(out, out_f32, o + col + 1, b);
@@ -1868,6 +1931,27 @@ attn_chunk_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, void* _
             } else {
                 store_pair((T*)out + o + col, a, b);
             }
+        }
+        if (!(zero == 0.0f)) spoilt |= 1u << (gid + 8 * e);
+    }
+    spoilt = __reduce_or_sync(0xffffffffu, spoilt);
+    if (spoilt == 0) return;
+    __syncwarp();
+    for (int row = 0; row < 16; ++row) {
+        if (!((spoilt >> row) & 1u)) continue;
+        const int r = it.row0 + warp % WARPS * 16 + row, t = r / g, h = hk * g + r % g;
+        float mr, lr, res[D / 32];
+        row_again<D>(q + (size_t)(tok0 + t) * q_stride + h * D, k_pages, v_pages,
+                     block_table + (size_t)slot * table_stride, num_pages, hk, kv_heads, page,
+                     pos0 + t, it.kv_begin, it.kv_end, scale, penalty ? r1[h] : 0.0f,
+                     penalty ? r2[h] : 0.0f, penalty, sight, mr, lr, res);
+        const float inv = sight_inverse(sight, h, mr, lr);
+        const size_t o = (size_t)(tok0 + t) * out_stride + h * D;
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) {
+            const int col = lane + 32 * i;
+            store_out<T>(out, out_f32, o + col,
+                         res[i] * inv * sight_gate<T>(sight, (size_t)(tok0 + t), h, D, col));
         }
     }
 }
@@ -2396,10 +2480,34 @@ attn_chunk_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         Pml[(warp * DRW + gid) * 2] = m;
         Pml[(warp * DRW + gid) * 2 + 1] = l;
     }
+    float zero = 0.0f;
 #pragma unroll
-    for (int j = 0; j < DT; ++j)
+    for (int j = 0; j < DT; ++j) {
         store_pair(Pacc + (size_t)(warp * DRW + gid) * D + j * 8 + 2 * tig, acc[j][0], acc[j][1]);
-    __syncthreads();
+        zero = fmaf(acc[j][1], 0.0f, fmaf(acc[j][0], 0.0f, zero));
+    }
+    // heads that met an infinity or NaN: their result in the first warp's place
+    if (__syncthreads_or(gid < g && !(zero == 0.0f))) {
+        for (int i = warp; i < g; i += WARPS) {
+            bool spoilt = false;
+            for (int w = 0; w < WARPS; ++w)
+                for (int c = lane; c < D; c += 32)
+                    spoilt |= !(Pacc[(size_t)(w * DRW + i) * D + c] * 0.0f == 0.0f);
+            if (!__any_sync(0xffffffffu, spoilt)) continue;
+            float mr, lr, res[D / 32];
+            row_again<D>(Qs + i * D, (const T*)k_pages, (const T*)v_pages,
+                         block_table + (size_t)slot * table_stride, num_pages, hk, kv_heads, page,
+                         pos, 0, hi, scale, penalty ? r1[h0 + i] : 0.0f,
+                         penalty ? r2[h0 + i] : 0.0f, penalty, sight, mr, lr, res);
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) Pacc[(size_t)i * D + lane + 32 * c] = res[c];
+            if (lane < WARPS) {
+                Pml[(lane * DRW + i) * 2] = lane == 0 ? mr : -INFINITY;
+                Pml[(lane * DRW + i) * 2 + 1] = lr;
+            }
+        }
+        __syncthreads();
+    }
     decode_finish<T>(Pml, Pacc, DRW, WARPS, g, h0, tok, pos, out, out_stride, D, sight, out_f32,
                      fuse);
 }
