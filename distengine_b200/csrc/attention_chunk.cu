@@ -1559,7 +1559,8 @@ __device__ __forceinline__ void row_again(
 
 // tanh(x) for |x| <= TANH_NEAR to 7e-8 of its value (as good as tanhf and a third of its
 // instructions): x + x^3 P(x^2), P of degree 4 fitted to tanh at Chebyshev nodes by reweighted
-// least squares (3e-9 but for float32's rounding).  Scores under a cap mostly lie here.
+// least squares (3e-9 but for float32's rounding).  Scores under a cap mostly lie here; the others
+// take tanhf of the quotient, as in the kernels above.
 constexpr float TANH_NEAR = 0.6f;
 __device__ __forceinline__ float tanh_near(float x) {
     const float u = x * x;
@@ -1778,26 +1779,22 @@ attn_chunk_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, void* _
 #pragma unroll
                 for (int j = 0; j < NT; ++j)
 #pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        s[j][x] *= inv_cap;
-                        far = fmaxf(far, fabsf(s[j][x]));
-                    }
-                if (__any_sync(0xffffffffu, far > TANH_NEAR)) {
+                    for (int x = 0; x < 4; ++x) far = fmaxf(far, fabsf(s[j][x]));
+                if (__any_sync(0xffffffffu, far * inv_cap > TANH_NEAR)) {
 #pragma unroll
                     for (int j = 0; j < NT; ++j)
 #pragma unroll
-                        for (int x = 0; x < 4; ++x) {
-                            const float y = s[j][x], a = fabsf(y);
-                            const float t = 1.0f - __fdividef(2.0f, 1.0f + expf(2.0f * a));
+                        for (int x = 0; x < 4; ++x)
                             s[j][x] = sight.softcap *
-                                      (a > TANH_NEAR ? copysignf(t, y) : tanh_near(y));
-                        }
+                                      (fabsf(s[j][x]) * inv_cap > TANH_NEAR
+                                           ? tanhf(s[j][x] / sight.softcap)
+                                           : tanh_near(s[j][x] * inv_cap));
                 } else {
 #pragma unroll
                     for (int j = 0; j < NT; ++j)
 #pragma unroll
                         for (int x = 0; x < 4; ++x)
-                            s[j][x] = sight.softcap * tanh_near(s[j][x]);
+                            s[j][x] = sight.softcap * tanh_near(s[j][x] * inv_cap);
                 }
             }
             if (!inside) {

@@ -779,3 +779,44 @@ def test_single_tokens_on_tensor_cores(dim, seqs, form):
             want = want * 1.5 * torch.sigmoid(gate[i].double())[:, None]
         err = (got[i] - want).abs().max().item()
         assert err <= 4e-6 * max(1.0, want.abs().max().item()), (i, keys, err)
+
+
+@pytest.mark.parametrize("cap,low,high", [(1000.0, 0.05, 0.59), (1000.0, 0.61, 1.2), (300.0, 1.2, 3.0)])
+@pytest.mark.parametrize("rows", [32, 64])
+def test_soft_cap_on_tensor_cores(cap, low, high, rows):
+    """Scores below and above the line between the two forms of tanh, two keys a token whose values are
+    1 and 0: the weights' logarithms give the difference of the two capped scores, in units of
+    cap 2^-24.  Bound: a score's quotient or product with the cap's inverse, tanh to two units of
+    its last place, the product with the cap, each time two, and the weights' own roundings.  Above
+    the line the results are the bits of the kernel for float32 storage, which takes tanhf."""
+    from types import SimpleNamespace
+    from distengine_b200.kernels import recurrent as rk
+    from distengine_b200.kernels.attention_plan import build_plan
+    n, dim, page = 600, 64, 16
+    g = torch.Generator().manual_seed(3)
+    x = ((torch.rand(n, generator=g) * (high - low) + low) * cap).to(torch.bfloat16).float()
+    y = (x * (1 + 1 / 128)).to(torch.bfloat16).float()
+    k, v, q = torch.zeros(n, 1, page, dim), torch.zeros(n, 1, page, dim), torch.zeros(n, dim)
+    k[:, 0, 0, 0] = k[:, 0, 1, 1] = 1.0
+    v[:, 0, 0] = 1.0
+    q[:, 0], q[:, 1] = x, y
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).to(DEV)
+    one = np.ones(n, dtype=np.int32)
+    ctx = SimpleNamespace(seq_slot=t(np.arange(n)), seq_qstart=t(np.arange(n)), seq_qlen=t(one),
+                          seq_pos0=t(one), status=torch.zeros(1, dtype=torch.int32, device=DEV))
+    items = t(build_plan(one, one, 1, 1, rows, 0, chunk=0).items)
+    results = []
+    for dtype in (torch.bfloat16, torch.float32):
+        out = torch.empty(n, dim, device=DEV)
+        rk.chunk_attention(*(a.to(dtype).to(DEV) if a is not out else out for a in (q, out, k, v)),
+                           t(np.arange(n).reshape(n, 1)), items, None, None, 1, 1, dim, dim, 1.0, 0, ctx,
+                           tile_rows=rows, softcap=cap)
+        results.append(out[:, 0].cpu())
+    if low > 0.6:
+        assert torch.equal(*results)
+    p = results[0].double()
+    clear = (p > 0.02) & (p < 0.98)             # (where the weights tell the difference)
+    assert int(clear.sum()) > 100
+    want = cap * (torch.tanh(x.double() / cap) - torch.tanh(y.double() / cap))
+    units = (torch.log(p) - torch.log1p(-p) - want).abs() / (cap * 2.0 ** -24)
+    assert units[clear].max().item() <= 2 * (0.5 + 2 + 0.5) + 1
