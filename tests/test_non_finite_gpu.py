@@ -1,6 +1,6 @@
 """Infinities and NaN among the values: they reach the tokens that see them and no others, and an
 infinity stays one.  Attention with 32-bit weights on the tensor cores, whose products take a whole
-tile's values for a whole tile's tokens."""
+tile's values for a whole tile's tokens, and the read-outs of the chunked recurrences."""
 
 from types import SimpleNamespace
 
@@ -9,7 +9,8 @@ import pytest
 import torch
 
 from gpu_helpers import PagedFixture
-from test_vomotar_mechanisms_gpu import _gen
+from test_chunked_recurrences_gpu import _step
+from test_vomotar_mechanisms_gpu import _gen, _scan_inputs
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -81,3 +82,41 @@ def test_values_that_are_not_finite(dim, window, keep, rows, copies):
             assert ((got[at + t] - want)[fine].abs() <= 4e-6 * want[fine].abs().max()).all(), (i, pos)
         at += qlen[i]
     assert met
+
+
+@pytest.mark.parametrize("rule", ["delta", "decay", "decay-bf16"])
+@pytest.mark.parametrize("value", [INF, NAN])
+def test_chunks_with_a_value_that_is_not_finite(rule, value):
+    """One head's value at one token of a portion: the same bits as without it but for that head's
+    column from that token on, and that column not finite there."""
+    from distengine_b200.kernels import recurrent as rk
+    H, dk, dv, lens, slots = 2, 64, 128, (200, 193), (1, 0)
+    ctx, items, portions, _ = _step(lens, slots)
+    n, bad, head, col = sum(lens), 100, 1, 37
+    flat = lambda t: t.reshape(n, -1).to(DEV).contiguous()
+    q, k, v, beta, dec = _scan_inputs(n, H, H, dk, dv, 3)
+    results = []
+    for dirty in (False, True):
+        vv = v.clone()
+        if dirty:
+            vv[bad, head, col] = value
+        if rule == "decay-bf16":
+            vv = vv.to(torch.bfloat16)
+        state = torch.randn(2, H * dk * dv, generator=_gen(1)).to(DEV)
+        out = torch.full((n, H * dv), 77.0, device=DEV)
+        if rule == "delta":
+            rk.delta_chunks(flat(q), flat(k), flat(vv), state, out, H, H, dk, dv, flat(dec),
+                            flat(beta), items, portions, ctx)
+        else:
+            rk.decay_chunks(flat(q), flat(k), flat(vv), state, out, H, dk, dv,
+                            torch.tensor([0.99, 0.9]).to(DEV), items, portions, ctx)
+        results.append((out.cpu().view(n, H, dv), state.cpu().view(2, H, dk, dv)))
+    (clean, clean_state), (got, got_state) = results
+    reached = torch.zeros_like(clean, dtype=torch.bool)
+    reached[bad: lens[0], head, col] = True
+    assert torch.equal(got[~reached], clean[~reached])
+    assert not got[reached].isfinite().any()
+    kept = torch.ones_like(clean_state, dtype=torch.bool)
+    kept[slots[0], head, :, col] = False
+    assert torch.equal(got_state[kept], clean_state[kept])
+    assert not got_state[~kept].isfinite().any()
