@@ -128,6 +128,38 @@ __device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
 // decays: 48 us (a block a token, a channel at a time: 128).
 constexpr int RUN = 8;
 
+// The sum of a head's squares, four neighbouring channels a lane, the head on 16 or 32 lanes.  In
+// float32 in the order of the kernel above (channels 32 apart in a chain, then 16, 8 .. 1 apart), so
+// that a token has the same bits in a step of any size; in bfloat16, where the products before
+// this kernel depend on the step's size themselves, in the fewest steps.
+template <typename T> __device__ __forceinline__ float head_squares(const float (&y)[4], int dk);
+template <>
+__device__ __forceinline__ float head_squares<__nv_bfloat16>(const float (&y)[4], int dk) {
+    float ss = fmaf(y[0], y[0], fmaf(y[1], y[1], fmaf(y[2], y[2], y[3] * y[3])));
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (dk == 128) ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+    return ss;
+}
+template <> __device__ __forceinline__ float head_squares<float>(const float (&y)[4], int dk) {
+    const int lane = threadIdx.x & 31, eighth = (lane >> 3) & (dk / 32 - 1);     // of 32 channels
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = fmaf(y[e], y[e], 0.0f);
+    for (int r = 1; r < dk / 32; ++r)                // the chain ends in the last eight lanes of a head
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float before = __shfl_up_sync(0xffffffffu, v[e], 8);
+            if (eighth == r) v[e] = fmaf(y[e], y[e], before);
+        }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] += __shfl_xor_sync(0xffffffffu, v[e], o);
+    const float ss = (v[0] + v[2]) + (v[1] + v[3]);
+    return __shfl_sync(0xffffffffu, ss, lane | (dk / 4 - 1));       // the head's last lane
+}
+
 template <typename T, int KK>
 __global__ void __launch_bounds__(128)
 delta_prep_runs_kernel(const T* __restrict__ proj, int ld, const float* __restrict__ a,
@@ -229,11 +261,7 @@ delta_prep_runs_kernel(const T* __restrict__ proj, int ld, const float* __restri
             store_four(vv + (size_t)n * (H * dv) + c - qk, make_float4(y[0], y[1], y[2], y[3]));
             continue;
         }
-        float ss = fmaf(y[0], y[0], fmaf(y[1], y[1], fmaf(y[2], y[2], y[3] * y[3])));
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (dk == 128) ss += __shfl_xor_sync(0xffffffffu, ss, 16);
-        const float inv = 1.0f / sqrtf(ss + 1e-6f);
+        const float inv = 1.0f / sqrtf(head_squares<T>(y, dk) + 1e-6f);
         const bool is_q = c < G * dk;
         float* dst = is_q ? qn + (size_t)n * (G * dk) + c : kn + (size_t)n * (G * dk) + c - G * dk;
         const float more = is_q ? q_scale : 1.0f;
