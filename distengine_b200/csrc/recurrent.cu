@@ -16,9 +16,9 @@
 // and a block of up to 32 columns walks its sequence's tokens of the step one after the other
 // while the next tokens' vectors arrive through cp.async.  The order of every sum depends on the
 // head's sizes only: a state does not depend, bit for bit, on how its tokens were cut into steps, as
-// long as they come through this scan.  (Portions of 192 tokens and more of the delta rule and of
-// retention, at key sizes 64 and 128, go through recurrent_chunks.cu, whose sums are ordered by
-// chunk; the scan then only moves their kept rows on.)
+// long as they come through this scan.  (In bfloat16 longer portions of the delta rule, of retention
+// and of lightning attention, at key sizes 64 and 128, can go through recurrent_chunks.cu, whose sums
+// are ordered by chunk; the scan then only moves their kept rows on.  Float32 always comes here.)
 //
 // What is token-parallel runs before the scan in a kernel of its own: the short causal
 // convolution over time with its activation (its last taps - 1 inputs are part of the slot's

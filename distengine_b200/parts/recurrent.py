@@ -182,9 +182,16 @@ class ChunkedMixer(ProjectedMixer):
                           decay=self.decay, longest=rk.CHUNKED_PORTION - 1 if chunked else 0)
 
     def chunked(self, ctx, v, state) -> int:
-        """The step's note: 0 if its portions go token by token."""
-        fits = rk.chunks_ok(self.dk, self.dv) and rk.chunks_aligned(v, state)
-        return ctx.notes.get("recurrent/chunks", 0) if fits else 0
+        """0: the step goes token by token; 1: by chunks; 2: its longer portions by chunks.
+
+        In float32 always token by token: there every product gives a row the same bits beside any
+        others, so that with the scan a request's states and tokens do not depend on how its prompt
+        was cut (a preempted one is cut anew).  The chunks sum in another order than the scan.  In
+        bfloat16 the products of the step themselves depend on its number of rows."""
+        note = ctx.notes.get("recurrent/chunks", 0)
+        if not note or self.dtype == torch.float32:
+            return 0
+        return note if rk.chunks_ok(self.dk, self.dv) and rk.chunks_aligned(v, state) else 0
 
 
 class GatedDeltaRule(ChunkedMixer):

@@ -186,3 +186,89 @@ def test_delta_preparation_of_any_number_of_tokens(K, G, H, dk, dv):
         results.append([torch.cat(x) for x in zip(*parts)])
     for got, want, name in zip(*results, ("q", "k", "v", "beta", "decay")):
         assert torch.equal(got, want), name
+
+
+def _walk(rule, lens, inputs, state, H, dk, dv, begin=0):
+    """The tokens from ``begin`` on of one sequence, in steps of ``lens``: portions of 192 tokens and
+    more by chunks, others by the scan.  Returns the read-outs."""
+    from distengine_b200.kernels import recurrent as rk
+    q, k, v, beta, dec = inputs
+    outs = []
+    for n in lens:
+        ctx, items, portions, longest = _step([n], [0])
+        flat = lambda t: t[begin: begin + n].reshape(n, -1).to(DEV).contiguous()
+        out = torch.full((n, H * dv), float("nan"), device=DEV)
+        if rule == "delta" and longest:
+            rk.delta_chunks(flat(q), flat(k), flat(v), state, out, H, H, dk, dv, flat(dec), flat(beta),
+                            items, portions, ctx)
+        elif rule == "delta":
+            rk.state_scan(flat(q), flat(k), flat(v), state, out, H, H, dk, dv, ctx, g=flat(dec),
+                          beta=flat(beta))
+        elif longest:
+            rk.decay_chunks(flat(q), flat(k), flat(v), state, out, H, dk, dv, dec, items, portions, ctx)
+        else:
+            rk.state_scan(flat(q), flat(k), flat(v), state, out, H, H, dk, dv, ctx, decay=dec)
+        outs.append(out)
+        begin += n
+    return torch.cat(outs)
+
+
+@pytest.mark.parametrize("rule", ["delta", "decay"])
+@pytest.mark.parametrize("dim", [64, 128])
+def test_cuts_on_both_sides_of_the_line(rule, dim):
+    """One prompt whole, in portions that the scan takes and in portions of both kinds: the same but
+    for the order of float32 sums, each within the bound of the test above."""
+    H, n = 2, 460
+    inputs = list(_scan_inputs(n, H, H, dim, dim, 9))
+    if rule == "decay":
+        inputs[4] = torch.tensor([0.99, 0.97]).to(DEV)
+    results = []
+    for lens in ((460,), (150, 150, 160), (200, 60, 200), (191, 192, 77)):
+        state = torch.zeros(1, H * dim * dim, device=DEV)
+        out = _walk(rule, lens, inputs, state, H, dim, dim)
+        results.append((out.double(), state.double()))
+    for out, state in results[1:]:
+        for got, want in ((out, results[0][0]), (state, results[0][1])):
+            assert (got - want).abs().max().item() <= 2 * BOUND * want.abs().max().item()
+
+
+def _layer(kind, dtype, taps=3):
+    from distengine_b200.config.model import PartSpec
+    from distengine_b200.parts import build_mixer
+    width, heads, dim = 64, 2, 64
+    params = dict(width=width, heads=heads, key_dim=dim, value_dim=dim, eps=1e-5)
+    if kind == "gated_delta_rule":
+        params.update(kv_heads=heads, taps=taps, rank=8)
+    else:
+        params.update(decay=(0.99, 0.97))
+        if kind == "retention":
+            params.update(rotary_dim=dim, theta=1e4)
+    mixer = build_mixer(PartSpec.of(kind, **params), dtype, torch.device(DEV))
+    g = _gen(4)
+    mixer.load({name: (torch.randn(*shape, generator=g) * (0.1 if role == "matrix" else 0.3)).to(
+        dtype if role == "matrix" else torch.float32) for name, (shape, role) in mixer.tensors().items()})
+    return mixer, width
+
+
+def _feed(mixer, x, dtype, lens):
+    """One sequence through a layer in steps of ``lens``; its outputs and the state it leaves."""
+    from gpu_helpers import PartHarness
+    harness = PartHarness([mixer], [mixer.cache_spec()], dtype, max_seqs=2)
+    outs, at = [], 0
+    for n in lens:
+        outs.append(harness.run([("a", n)], lambda ctx, bindings: mixer.forward(
+            x[at: at + n], ctx, bindings[0]).clone()))
+        at += n
+    return torch.cat(outs), harness.cache.bindings()[0].state[harness.cache.slot("a")].clone()
+
+
+@pytest.mark.parametrize("kind", ["gated_delta_rule", "retention", "lightning_attention"])
+def test_a_float32_layer_does_not_depend_on_the_cut(kind):
+    """In float32 a prompt's results and the state it leaves are the same bits however it was cut,
+    portions of 192 tokens and more among them."""
+    mixer, width = _layer(kind, torch.float32)
+    x = torch.randn(900, width, generator=_gen(8)).to(DEV)
+    out, state = _feed(mixer, x, torch.float32, (900,))
+    for lens in ((191, 192, 517), (1, 640, 259), (100,) * 9):
+        other, end = _feed(mixer, x, torch.float32, lens)
+        assert torch.equal(other, out) and torch.equal(end, state), lens
