@@ -156,11 +156,33 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
 
 
 CHUNK = 64               # tokens of a chunk of a longer portion
-# Portions of at least this many tokens go by chunks.  (Measured on B200: the delta rule's chunks are
-# five kernels and the host's share of them where its scan is one of 0.37 us a token.  A bfloat16
-# layer with a portion of 100 tokens 151 us by chunks, 122 by the scan, lightning attention 112 and
-# 83; four portions of about 100 tokens 152 and 178; one of 400 tokens in float32 500 and 1,001.)
+# Portions of at least this many tokens can go by chunks (of shorter ones the last chunk is mostly
+# padding); whether a step's do is for chunks_pay.
 CHUNKED_PORTION = 192
+
+
+def chunks_pay(delta: bool, heads: int, key_dim: int, value_dim: int, longest: int, tokens: int,
+               chunks: int) -> bool:
+    """Whether a layer's step goes through its states by chunks sooner than by the scan: ``longest``,
+    ``tokens`` and ``chunks`` of the portions of ``CHUNKED_PORTION`` tokens and more.
+
+    The scan costs the longest portion's chain and every (token, head)'s work, the chunks mostly a
+    fixed time a (chunk, head).  In us, from layers of 1 to 32 portions of 192 to 4,096 tokens with 8,
+    16 and 64 heads on B200 (a bfloat16 layer by the scan / by chunks): delta rule 128 x 128, 16
+    heads, one portion of 512 tokens 234 / 132, ten of 200 517 / 436, 32 of 200 1,307 / 1,382; delta
+    rule 64 x 64, 16 heads, one of 512 149 / 86, ten of 200 181 / 207, 32 of 200 496 / 538, 64 heads,
+    ten of 400 1,044 / 1,110, four of 500 699 / 554; a decay per head gains at all of these.  The
+    chunks are four or five launches instead of one, and a step that runs launch by launch waits for
+    the host: what the scan does in less than that stays with it (delta 64 x 64, 8 heads, one
+    portion of 256: 122 against 147; a decay per head 64 x 64, 16 heads, the same 77 against 83)."""
+    wide = key_dim == 128
+    by = value_dim / key_dim
+    if not delta:
+        return (0.43 if wide else 0.27) * longest \
+            + (0.0075 if wide else 0.004) * by * tokens * heads >= 100.0
+    scan = (0.37 if wide else 0.24) * longest + (0.0118 if wide else 0.0037) * by * tokens * heads
+    walk = 30.0 + longest / CHUNK + (0.62 if wide else 0.25) * by * chunks * heads
+    return scan >= 145.0 and walk < scan
 
 
 def chunks_ok(key_dim: int, value_dim: int) -> bool:

@@ -152,11 +152,13 @@ class ChunkedMixer(ProjectedMixer):
             return
         qlen, qstart = prep.host.seq_qlen, prep.host.seq_qstart
         long = np.nonzero(qlen >= rk.CHUNKED_PORTION)[0]
-        # 0: none; else whether there are shorter portions beside them
-        prep.notes["recurrent/chunks"] = 0 if not len(long) else (2 if len(long) < len(qlen) else 1)
         if not len(long):
+            prep.notes["recurrent/chunks"] = 0
             return
         count = -(-qlen[long] // rk.CHUNK)
+        # whether there are shorter portions beside them (1: no, 2: yes); longest, tokens, chunks
+        prep.notes["recurrent/chunks"] = (2 if len(long) < len(qlen) else 1, int(qlen[long].max()),
+                                          int(qlen[long].sum()), int(count.sum()))
         first = np.cumsum(count) - count
         owner = np.repeat(np.arange(len(long)), count)
         place = (np.arange(int(count.sum())) - first[owner]) * rk.CHUNK
@@ -181,7 +183,7 @@ class ChunkedMixer(ProjectedMixer):
             rk.state_scan(q, k, v, state, out, self.heads, self.heads, self.dk, self.dv, ctx,
                           decay=self.decay, longest=rk.CHUNKED_PORTION - 1 if chunked else 0)
 
-    def chunked(self, ctx, v, state) -> int:
+    def chunked(self, ctx, v, state, delta: bool = False) -> int:
         """0: the step goes token by token; 1: by chunks; 2: its longer portions by chunks.
 
         In float32 always token by token: there every product gives a row the same bits beside any
@@ -191,7 +193,10 @@ class ChunkedMixer(ProjectedMixer):
         note = ctx.notes.get("recurrent/chunks", 0)
         if not note or self.dtype == torch.float32:
             return 0
-        return note if rk.chunks_ok(self.dk, self.dv) and rk.chunks_aligned(v, state) else 0
+        kind, longest, tokens, chunks = note
+        fits = (rk.chunks_ok(self.dk, self.dv) and rk.chunks_aligned(v, state)
+                and rk.chunks_pay(delta, self.heads, self.dk, self.dv, longest, tokens, chunks))
+        return kind if fits else 0
 
 
 class GatedDeltaRule(ChunkedMixer):
@@ -275,7 +280,7 @@ class GatedDeltaRule(ChunkedMixer):
         rk.delta_prep(proj, a, self.conv, self.dt_bias, self.a_log, cache.state, self.state_rows,
                       ctx, qn, kn, vv, beta, gdec, H, G, dk, dv, self.b_col)
         o = ctx.buffer("delta.o", (n, H * dv), f32)
-        chunked = self.chunked(ctx, vv, cache.state)
+        chunked = self.chunked(ctx, vv, cache.state, delta=True)
         if chunked:
             rk.delta_chunks(qn, kn, vv, cache.state, o, H, G, dk, dv, gdec, beta,
                             ctx.arrays["recurrent/items"], ctx.arrays["recurrent/portions"], ctx)
