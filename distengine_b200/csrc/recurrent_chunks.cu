@@ -38,6 +38,14 @@ struct Item {                      // a chunk
 struct Portion {
     int seq, first, chunks, pad;   // its first item and how many
 };
+// What of a portion lies among the items [begin, begin + m) of a launch: from which item of the launch
+// on, and how many.
+__device__ __forceinline__ Portion part_of(Portion p, int begin, int m) {
+    const int lo = max(p.first, begin), hi = min(p.first + p.chunks, begin + m);
+    p.first = lo - begin;
+    p.chunks = max(hi - lo, 0);
+    return p;
+}
 
 __device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -243,17 +251,17 @@ decay_states_kernel(const float* __restrict__ k, int ldk, const VT* __restrict__
 // Eight states are asked for before any is used: 9 us, memory's rate.
 __global__ void __launch_bounds__(256)
 decay_pass_kernel(float* __restrict__ states, const float* __restrict__ decay,
-                  const Item* __restrict__ items, const Portion* __restrict__ portions,
-                  float* __restrict__ state, long long slot_stride,
+                  const Item* __restrict__ items, const Portion* __restrict__ portions, int begin,
+                  int m, float* __restrict__ state, long long slot_stride,
                   const int* __restrict__ seq_slot, int H, int size) {
-    const Portion p = portions[blockIdx.x];
+    const Portion p = part_of(portions[blockIdx.x], begin, m);
     const int e = ((int)blockIdx.y * 256 + (int)threadIdx.x) * 4;
-    const int last = items[p.first + p.chunks - 1].count;
-    float* slot = state + (size_t)seq_slot[p.seq] * slot_stride;
-    if (e >= H * size) {
+    if (e >= H * size || p.chunks == 0) {
         pdl_wait();
         return;
     }
+    const int last = items[p.first + p.chunks - 1].count;
+    float* slot = state + (size_t)seq_slot[p.seq] * slot_stride;
     const double d = (double)decay[e / size];
     double f64 = 1.0, flast = 1.0;
     for (int i = 0; i < CH; ++i) f64 *= d;
@@ -522,16 +530,21 @@ template <int DK>
 __global__ void __launch_bounds__(2 * DK)
 delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
                   const float* __restrict__ bn, float* __restrict__ xv, float* __restrict__ states,
-                  const Portion* __restrict__ portions, float* __restrict__ state,
-                  long long slot_stride, const int* __restrict__ seq_slot, int H, int dv) {
+                  const Portion* __restrict__ portions, int begin, int m,
+                  float* __restrict__ state, long long slot_stride,
+                  const int* __restrict__ seq_slot, int H, int dv) {
     constexpr int W = Pass<DK>::W, STAGE = Pass<DK>::STAGE, WARPS = Pass<DK>::WARPS;
     constexpr int THREADS = Pass<DK>::THREADS;
     extern __shared__ __align__(16) float sh[];
     float* ss = sh + 2 * STAGE;                      // [DK][PLD]: the state before the chunk
     float* us = ss + DK * PLD;                       // [CH][PLD]
     float* red = us + CH * PLD;                      // [WARPS][CH][PLD]
-    const Portion p = portions[blockIdx.x];
+    const Portion p = part_of(portions[blockIdx.x], begin, m);
     const int h = blockIdx.y, j0 = blockIdx.z * PC;
+    if (p.chunks == 0) {
+        pdl_wait();
+        return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // for u: eight groups of four tokens (and four more 32 on) by four of four columns; for S: four
     // groups of four rows by eight of two columns.  (Lanes l and l ^ 1, or l ^ 2, share one of the two.)
@@ -730,114 +743,122 @@ static int need_smem(const void* kernel, size_t bytes) {
                : 0;
 }
 
-// The read-outs and the new states of the portions in `items` / `portions` under a decay per head.
-// work: m H (64 dk + 64 64 + dk dv) floats, xt [m, H, dk, 64], pt [m, H, 64, 64] and the states
-// [m, H, dk, dv].
+// The read-outs and the new states of the portions in `items` / `portions` under a decay per head,
+// `group` items at a time (a portion that is cut goes on from the state that the group before it left:
+// the same bits).  work, for a group of m: m H (64 dk + 64 64 + dk dv) floats, xt [m, H, dk, 64], pt
+// [m, H, 64, 64] and the states [m, H, dk, dv].
 DE_EXPORT int de_decay_chunks(int v_dtype, const float* q, int ldq, const float* k, int ldk,
-                              const void* v, int ldv, const float* decay, const int* items, int m,
-                              const int* portions, int n_portions, float* work, float* state,
-                              long long slot_stride, const int* seq_slot, float* out, int H, int dk,
-                              int dv, void* stream) {
-    if (m <= 0 || n_portions <= 0) return 0;
+                              const void* v, int ldv, const float* decay, const int* items,
+                              int n_items, const int* portions, int n_portions, float* work,
+                              int group, float* state, long long slot_stride, const int* seq_slot,
+                              float* out, int H, int dk, int dv, void* stream) {
+    if (n_items <= 0 || n_portions <= 0) return 0;
     if (!de_chunk_ok(dk, dv) || ldk % 4 || ldv % 4 || (uintptr_t)k % 16 ||
         (uintptr_t)v % (v_dtype == DE_BF16 ? 8 : 16) || slot_stride % 4 || (uintptr_t)state % 16 ||
-        (uintptr_t)work % 16)
+        (uintptr_t)work % 16 || group <= 0)
         return -2;
-    const size_t mh = (size_t)m * H;
-    float* xt = work;
-    float* pt = xt + mh * dk * CH;
-    float* states = pt + mh * CH * CH;
     cudaStream_t s = (cudaStream_t)stream;
-    const Item* it = (const Item*)items;
     const Portion* po = (const Portion*)portions;
     const size_t psmem = (size_t)2 * dk * LD * sizeof(float);
+    const size_t osmem = (size_t)4 * CH * LD * sizeof(float);
+    const dim3 pgrid(n_portions, (H * dk * dv / 4 + 255) / 256);
     int e;
 #define RUN(...)                                                                                \
     do {                                                                                        \
         if ((e = (__VA_ARGS__)) != 0) return e;                                                 \
     } while (0)
-    if (dk == 64) {
-        RUN(need_smem((const void*)decay_products_kernel<64>, psmem));
-        RUN(de_launch(decay_products_kernel<64>, dim3(m, H), dim3(128), psmem, s, q, ldq, k, ldk,
-                      decay, it, xt, pt, H));
-    } else {
-        RUN(need_smem((const void*)decay_products_kernel<128>, psmem));
-        RUN(de_launch(decay_products_kernel<128>, dim3(m, H), dim3(128), psmem, s, q, ldq, k, ldk,
-                      decay, it, xt, pt, H));
-    }
-    const dim3 grid(m, H, dk / 64 * (dv / 64)), ogrid(m, H, dv / 64);
-    const size_t osmem = (size_t)4 * CH * LD * sizeof(float);
-    const dim3 pgrid(n_portions, (H * dk * dv / 4 + 255) / 256);
-    if (v_dtype == DE_BF16)
-        RUN(de_launch(decay_states_kernel<__nv_bfloat16>, grid, dim3(128), 0, s, k, ldk,
-                      (const __nv_bfloat16*)v, ldv, decay, it, states, H, dk, dv));
-    else
-        RUN(de_launch(decay_states_kernel<float>, grid, dim3(128), 0, s, k, ldk, (const float*)v,
-                      ldv, decay, it, states, H, dk, dv));
-    RUN(de_launch(decay_pass_kernel, pgrid, dim3(256), 0, s, states, decay, it, po, state,
-                  slot_stride, seq_slot, H, dk * dv));
-    if (v_dtype == DE_BF16) {
-        RUN(need_smem((const void*)chunk_out_kernel<__nv_bfloat16>, osmem));
-        RUN(de_launch(chunk_out_kernel<__nv_bfloat16>, ogrid, dim3(128), osmem, s, xt, states, pt,
-                      (const __nv_bfloat16*)v, ldv, 0, it, out, H, dk, dv));
-    } else {
-        RUN(need_smem((const void*)chunk_out_kernel<float>, osmem));
-        RUN(de_launch(chunk_out_kernel<float>, ogrid, dim3(128), osmem, s, xt, states, pt,
-                      (const float*)v, ldv, 0, it, out, H, dk, dv));
+    for (int begin = 0; begin < n_items; begin += group) {
+        const int m = n_items - begin < group ? n_items - begin : group;
+        const Item* it = (const Item*)items + begin;
+        const size_t mh = (size_t)m * H;
+        float* xt = work;
+        float* pt = xt + mh * dk * CH;
+        float* states = pt + mh * CH * CH;
+        if (dk == 64) {
+            RUN(need_smem((const void*)decay_products_kernel<64>, psmem));
+            RUN(de_launch(decay_products_kernel<64>, dim3(m, H), dim3(128), psmem, s, q, ldq, k, ldk,
+                          decay, it, xt, pt, H));
+        } else {
+            RUN(need_smem((const void*)decay_products_kernel<128>, psmem));
+            RUN(de_launch(decay_products_kernel<128>, dim3(m, H), dim3(128), psmem, s, q, ldq, k,
+                          ldk, decay, it, xt, pt, H));
+        }
+        const dim3 grid(m, H, dk / 64 * (dv / 64)), ogrid(m, H, dv / 64);
+        if (v_dtype == DE_BF16)
+            RUN(de_launch(decay_states_kernel<__nv_bfloat16>, grid, dim3(128), 0, s, k, ldk,
+                          (const __nv_bfloat16*)v, ldv, decay, it, states, H, dk, dv));
+        else
+            RUN(de_launch(decay_states_kernel<float>, grid, dim3(128), 0, s, k, ldk,
+                          (const float*)v, ldv, decay, it, states, H, dk, dv));
+        RUN(de_launch(decay_pass_kernel, pgrid, dim3(256), 0, s, states, decay, it, po, begin, m,
+                      state, slot_stride, seq_slot, H, dk * dv));
+        if (v_dtype == DE_BF16) {
+            RUN(need_smem((const void*)chunk_out_kernel<__nv_bfloat16>, osmem));
+            RUN(de_launch(chunk_out_kernel<__nv_bfloat16>, ogrid, dim3(128), osmem, s, xt, states, pt,
+                          (const __nv_bfloat16*)v, ldv, 0, it, out, H, dk, dv));
+        } else {
+            RUN(need_smem((const void*)chunk_out_kernel<float>, osmem));
+            RUN(de_launch(chunk_out_kernel<float>, ogrid, dim3(128), osmem, s, xt, states, pt,
+                          (const float*)v, ldv, 0, it, out, H, dk, dv));
+        }
     }
     return 0;
 }
 
-// The same for the delta rule: g [N, ldg] decays, beta [N, ldb], v float32.  work: m H (2 64 64 +
-// 4 64 dk + dk + 64 dv + dk dv) floats, at and pt [m, H, 64, 64], xt, kd, kh, xkt [m, H, dk, 64],
-// the states [m, H, dk, dv], xv [m, H, 64, dv] and bn [m, H, dk].
+// The same for the delta rule: g [N, ldg] decays, beta [N, ldb], v float32.  work, for a group of m:
+// m H (2 64 64 + 4 64 dk + dk + 64 dv + dk dv) floats, at and pt [m, H, 64, 64], xt, kd, kh, xkt
+// [m, H, dk, 64], the states [m, H, dk, dv], xv [m, H, 64, dv] and bn [m, H, dk].
 DE_EXPORT int de_delta_chunks(const float* q, int ldq, const float* k, int ldk, const float* v,
                               int ldv, const float* g, int ldg, const float* beta, int ldb,
-                              const int* items, int m, const int* portions, int n_portions,
-                              float* work, float* state, long long slot_stride,
+                              const int* items, int n_items, const int* portions, int n_portions,
+                              float* work, int group, float* state, long long slot_stride,
                               const int* seq_slot, float* out, int H, int rep, int dk, int dv,
                               void* stream) {
-    if (m <= 0 || n_portions <= 0) return 0;
+    if (n_items <= 0 || n_portions <= 0) return 0;
     if (!de_chunk_ok(dk, dv) || ldq % 4 || ldk % 4 || ldg % 4 || ldv % 2 || (uintptr_t)q % 16 ||
         (uintptr_t)k % 16 || (uintptr_t)g % 16 || (uintptr_t)v % 8 || slot_stride % 4 ||
-        (uintptr_t)state % 16 || (uintptr_t)work % 16 || rep <= 0 || H % rep)
+        (uintptr_t)state % 16 || (uintptr_t)work % 16 || rep <= 0 || H % rep || group <= 0)
         return -2;
-    const size_t mh = (size_t)m * H, turned = mh * dk * CH;
-    float* at = work;
-    float* pt = at + mh * CH * CH;
-    float* xt = pt + mh * CH * CH;
-    float* kd = xt + turned;
-    float* kh = kd + turned;
-    float* xkt = kh + turned;
-    float* states = xkt + turned;
-    float* xv = states + mh * dk * dv;
-    float* bn = xv + mh * CH * dv;
     cudaStream_t s = (cudaStream_t)stream;
-    const Item* it = (const Item*)items;
     const Portion* po = (const Portion*)portions;
     const size_t csmem = (size_t)3 * CH * (dk + 4) * sizeof(float);
     const size_t ssmem = (size_t)(CH * LD + CH * 128) * sizeof(float);
     const size_t osmem = (size_t)4 * CH * LD * sizeof(float);
-    const dim3 sgrid(m, H, (dv + dk + 127) / 128), pgrid(n_portions, H, dv / PC);
+    const dim3 pgrid(n_portions, H, dv / PC);
     int e;
 #define DELTA(DK)                                                                               \
     do {                                                                                        \
-        RUN(need_smem((const void*)delta_chunk_kernel<DK>, csmem));                             \
+        RUN(need_smem((const void*)delta_chunk_kernel<DK>, csmem));                     \
         RUN(de_launch(delta_chunk_kernel<DK>, dim3(m, H), dim3(128), csmem, s, q, ldq, k, ldk,  \
                       g, ldg, it, at, pt, xt, kd, kh, bn, H, rep));                             \
-        RUN(need_smem((const void*)delta_solve_kernel<DK>, ssmem));                             \
+        RUN(need_smem((const void*)delta_solve_kernel<DK>, ssmem));                     \
         RUN(de_launch(delta_solve_kernel<DK>, sgrid, dim3(64), ssmem, s, (const float*)at, v,   \
                       ldv, (const float*)kd, beta, ldb, it, xv, xkt, H, dv));                   \
-        RUN(need_smem((const void*)delta_pass_kernel<DK>, Pass<DK>::SMEM));                     \
+        RUN(need_smem((const void*)delta_pass_kernel<DK>, Pass<DK>::SMEM));             \
         RUN(de_launch(delta_pass_kernel<DK>, pgrid, dim3(2 * DK), Pass<DK>::SMEM, s,            \
                       (const float*)xkt, (const float*)kh, (const float*)bn, xv, states, po,    \
-                      state, slot_stride, seq_slot, H, dv));                                    \
+                      begin, m, state, slot_stride, seq_slot, H, dv));                          \
     } while (0)
-    if (dk == 64) DELTA(64);
-    else DELTA(128);
-    RUN(need_smem((const void*)chunk_out_kernel<float>, osmem));
-    RUN(de_launch(chunk_out_kernel<float>, dim3(m, H, dv / 64), dim3(128), osmem, s,
-                  (const float*)xt, (const float*)states, (const float*)pt, (const float*)xv, 0, 1,
-                  it, out, H, dk, dv));
+    for (int begin = 0; begin < n_items; begin += group) {
+        const int m = n_items - begin < group ? n_items - begin : group;
+        const Item* it = (const Item*)items + begin;
+        const size_t mh = (size_t)m * H, turned = mh * dk * CH;
+        float* at = work;
+        float* pt = at + mh * CH * CH;
+        float* xt = pt + mh * CH * CH;
+        float* kd = xt + turned;
+        float* kh = kd + turned;
+        float* xkt = kh + turned;
+        float* states = xkt + turned;
+        float* xv = states + mh * dk * dv;
+        float* bn = xv + mh * CH * dv;
+        const dim3 sgrid(m, H, (dv + dk + 127) / 128);
+        if (dk == 64) DELTA(64);
+        else DELTA(128);
+        RUN(need_smem((const void*)chunk_out_kernel<float>, osmem));
+        RUN(de_launch(chunk_out_kernel<float>, dim3(m, H, dv / 64), dim3(128), osmem, s,
+                      (const float*)xt, (const float*)states, (const float*)pt, (const float*)xv, 0,
+                      1, it, out, H, dk, dv));
+    }
     return 0;
 }

@@ -101,8 +101,9 @@ SIGNATURES: dict[str, dict[str, list]] = {
     },
     "recurrent_chunks": {
         "de_chunk_tokens": [], "de_chunk_ok": [I, I],
-        "de_decay_chunks": [I, P, I, P, I, P, I, P, P, I, P, I, P, P, L, P, P, I, I, I, P],
-        "de_delta_chunks": [P, I, P, I, P, I, P, I, P, I, P, I, P, I, P, P, L, P, P, I, I, I, I, P],
+        "de_decay_chunks": [I, P, I, P, I, P, I, P, P, I, P, I, P, I, P, L, P, P, I, I, I, P],
+        "de_delta_chunks": [P, I, P, I, P, I, P, I, P, I, P, I, P, I, P, I, P, L, P, P, I, I, I, I,
+                            P],
     },
     "ssm": {
         "de_ssm_max_state": [], "de_ssm_chunk": [],

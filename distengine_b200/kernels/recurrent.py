@@ -159,6 +159,9 @@ CHUNK = 64               # tokens of a chunk of a longer portion
 # Portions of at least this many tokens can go by chunks (of shorter ones the last chunk is mostly
 # padding); whether a step's do is for chunks_pay.
 CHUNKED_PORTION = 192
+# Floats of the chunks' workspace (256 MB): a step's chunks are walked in groups that fit it.  (2,048
+# tokens of 16 heads of 128 x 128 are one group of the delta rule's and take half of it.)
+CHUNK_WORK = 1 << 26
 
 
 def chunks_pay(delta: bool, heads: int, key_dim: int, value_dim: int, longest: int, tokens: int,
@@ -211,6 +214,15 @@ def _chunk_checks(q, k, v, state, out, items, portions, heads, key_dim, value_di
     _need(chunks_ok(key_dim, value_dim), f"{name}: key sizes 64 and 128, value sizes of whole 64")
 
 
+def _chunk_work(count: int, floats: int, ctx) -> "tuple[torch.Tensor, int]":
+    """The workspace of ``count`` chunks of ``floats`` each, and how many are walked at a time."""
+    group = min(count, max(1, CHUNK_WORK // floats))
+    size = group * floats
+    if size > CHUNK_WORK // 2:      # (a buffer that grows doubles: never beyond the bound)
+        size = max(size, CHUNK_WORK)
+    return ctx.buffer("chunks.work", (size,), torch.float32), group
+
+
 def decay_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor,
                  out: torch.Tensor, heads: int, key_dim: int, value_dim: int, decay: torch.Tensor,
                  items: torch.Tensor, portions: torch.Tensor, ctx) -> None:
@@ -222,15 +234,15 @@ def decay_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch
     _f32(decay, "decay")
     _need(decay.shape == (heads,) and decay.is_contiguous() and q.shape[1] == heads * key_dim,
           "decay_chunks: decay [H], q and k [N, H dk]")
-    m = items.shape[0]
-    work = ctx.buffer("chunks.work", (m * heads * (key_dim * CHUNK + CHUNK * CHUNK
-                                                   + key_dim * value_dim),), torch.float32)
+    work, group = _chunk_work(items.shape[0], heads * (key_dim * CHUNK + CHUNK * CHUNK
+                                                       + key_dim * value_dim), ctx)
     lib = library.load("recurrent_chunks")
     _check(lib.de_decay_chunks(_tag(v.dtype), q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0),
-                               v.data_ptr(), v.stride(0), decay.data_ptr(), items.data_ptr(), m,
-                               portions.data_ptr(), portions.shape[0], work.data_ptr(),
-                               state.data_ptr(), state.stride(0), ctx.seq_slot.data_ptr(), out.data_ptr(), heads,
-                               key_dim, value_dim, _stream()), "decay_chunks")
+                               v.data_ptr(), v.stride(0), decay.data_ptr(), items.data_ptr(),
+                               items.shape[0], portions.data_ptr(), portions.shape[0],
+                               work.data_ptr(), group, state.data_ptr(), state.stride(0),
+                               ctx.seq_slot.data_ptr(), out.data_ptr(), heads, key_dim, value_dim,
+                               _stream()), "decay_chunks")
 
 
 def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor,
@@ -245,17 +257,16 @@ def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch
     _need(q.shape[1] == qk_heads * key_dim and heads % qk_heads == 0
           and g.shape == (n, heads * key_dim) and beta.shape == (n, heads),
           "delta_chunks: q, k [N, qk_heads dk], g [N, H dk], beta [N, H]")
-    m = items.shape[0]
-    work = ctx.buffer("chunks.work", (m * heads * (2 * CHUNK * CHUNK + 4 * key_dim * CHUNK + key_dim
-                                                   + CHUNK * value_dim + key_dim * value_dim),),
-                      torch.float32)
+    work, group = _chunk_work(items.shape[0], heads * (2 * CHUNK * CHUNK + 4 * key_dim * CHUNK + key_dim
+                                                       + CHUNK * value_dim + key_dim * value_dim), ctx)
     lib = library.load("recurrent_chunks")
     _check(lib.de_delta_chunks(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(),
                                v.stride(0), g.data_ptr(), g.stride(0), beta.data_ptr(),
-                               beta.stride(0), items.data_ptr(), m, portions.data_ptr(),
-                               portions.shape[0], work.data_ptr(), state.data_ptr(),
-                               state.stride(0), ctx.seq_slot.data_ptr(), out.data_ptr(), heads,
-                               heads // qk_heads, key_dim, value_dim, _stream()), "delta_chunks")
+                               beta.stride(0), items.data_ptr(), items.shape[0],
+                               portions.data_ptr(), portions.shape[0], work.data_ptr(), group,
+                               state.data_ptr(), state.stride(0), ctx.seq_slot.data_ptr(),
+                               out.data_ptr(), heads, heads // qk_heads, key_dim, value_dim,
+                               _stream()), "delta_chunks")
 
 
 def gdelta_prep(proj: torch.Tensor, r_col: int, k_col: int, a_col: int, wl: torch.Tensor,

@@ -272,3 +272,35 @@ def test_a_float32_layer_does_not_depend_on_the_cut(kind):
     for lens in ((191, 192, 517), (1, 640, 259), (100,) * 9):
         other, end = _feed(mixer, x, torch.float32, lens)
         assert torch.equal(other, out) and torch.equal(end, state), lens
+
+
+@pytest.mark.parametrize("rule", ["delta", "decay"])
+@pytest.mark.parametrize("group", [1, 2, 5])
+def test_chunks_a_few_at_a_time(rule, group, monkeypatch):
+    """A workspace of a few chunks, smaller than the step and cutting its portions: the same bits as
+    all at once, and no buffer is larger."""
+    from distengine_b200.kernels import recurrent as rk
+    H, dk, dv, lens, slots = 2, 64, 128, (257, 193, 320), (2, 0, 1)
+    n, g = sum(lens), _gen(group)
+    q, k, v, beta, dec = _scan_inputs(n, H, H, dk, dv, 5)
+    flat = lambda t: t.reshape(n, -1).to(DEV).contiguous()
+    start = torch.randn(3, H * dk * dv, generator=g).to(DEV)
+    a_chunk = H * (2 * 64 * 64 + 4 * dk * 64 + dk + 64 * dv + dk * dv if rule == "delta"
+                   else dk * 64 + 64 * 64 + dk * dv)
+    results = []
+    for work in (1 << 26, group * a_chunk + a_chunk // 2):
+        monkeypatch.setattr(rk, "CHUNK_WORK", work)
+        ctx, items, portions, _ = _step(lens, slots)
+        assert items.shape[0] == 14
+        make, sizes = ctx.buffer, []
+        ctx.buffer = lambda name, shape, dtype: (sizes.append(shape[0]), make(name, shape, dtype))[1]
+        state, out = start.clone(), torch.full((n, H * dv), float("nan"), device=DEV)
+        if rule == "delta":
+            rk.delta_chunks(flat(q), flat(k), flat(v), state, out, H, H, dk, dv, flat(dec), flat(beta),
+                            items, portions, ctx)
+        else:
+            rk.decay_chunks(flat(q), flat(k), flat(v), state, out, H, dk, dv,
+                            torch.tensor([0.99, 0.9]).to(DEV), items, portions, ctx)
+        assert len(sizes) == 1 and min(14, work // a_chunk) * a_chunk <= sizes[0] <= work
+        results.append((out, state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
