@@ -110,7 +110,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     const int l_k = tid & 7, l_row = tid >> 3;
 
     const int segments = (k_dim + SEG - 1) / SEG;
-    // the next step of 8 k to bring, of this group's segments; past the last: zeros
+    // the next step of 16 k to bring, of this group's segments; past the last: zeros
     int n_k = group * SEG, n_slot = 0;
     const float* wp = w + (size_t)(col0 + l_row) * ldw + l_k;
     const float* xp = x + (size_t)(row0 + l_row) * ldx + l_k;
@@ -394,6 +394,161 @@ gemm_f32_small_kernel(const float* __restrict__ x, const float* __restrict__ w,
     cp_async_wait<0>();
 }
 
+// ------------------------------------------------------------------------------------------
+// Short sums (k of one or two segments), where the kernels above leave most of their warps without a
+// segment: a thread forms its outputs over all of k, a segment at a time.  Bound by the trip to
+// memory and, with many tiles, by the reads of shared memory (four and two multiply-adds a read).
+// By tiles of 64 x 64: 4 x 4 outputs a thread on 16 x 16 threads, operands of any stride and address.
+// 130 rows of 64 against 2,048 columns: 5.1 us (the few-row kernel 22).
+// ------------------------------------------------------------------------------------------
+constexpr int WT = 64, WK = 16;
+
+template <bool VEC4>
+__global__ void __launch_bounds__(256)
+gemm_f32_wide_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                     float* __restrict__ out, int n_rows, int m_cols, int k_dim, int ldx, int ldw,
+                     int ldo) {
+    __shared__ float xs[WK][WT + 4];
+    __shared__ float ws[WK][WT + 4];
+    const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
+    const int row0 = blockIdx.y * WT, col0 = blockIdx.x * WT;
+    const int l_row = tid / 4, l_k = (tid % 4) * 4;  // a thread stages 4 k of a row of each operand
+    float acc[4][4], sum[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = sum[i][j] = 0.0f;
+
+    pdl_wait();
+    for (int k0 = 0; k0 < k_dim; k0 += WK) {
+        float xv[4] = {0.f, 0.f, 0.f, 0.f}, wv[4] = {0.f, 0.f, 0.f, 0.f};
+        const int gr = row0 + l_row, gc = col0 + l_row, gk = k0 + l_k;
+        if (gr < n_rows) {
+            const float* p = x + (size_t)gr * ldx + gk;
+            if (VEC4 && gk + 3 < k_dim) {
+                const float4 t = *reinterpret_cast<const float4*>(p);
+                xv[0] = t.x; xv[1] = t.y; xv[2] = t.z; xv[3] = t.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) if (gk + i < k_dim) xv[i] = p[i];
+            }
+        }
+        if (gc < m_cols) {
+            const float* p = w + (size_t)gc * ldw + gk;
+            if (VEC4 && gk + 3 < k_dim) {
+                const float4 t = *reinterpret_cast<const float4*>(p);
+                wv[0] = t.x; wv[1] = t.y; wv[2] = t.z; wv[3] = t.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) if (gk + i < k_dim) wv[i] = p[i];
+            }
+        }
+        __syncthreads();                             // the step before this one has been used
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            xs[l_k + i][l_row] = xv[i];
+            ws[l_k + i][l_row] = wv[i];
+        }
+        __syncthreads();
+        if (k0 > 0 && k0 % SEG == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    sum[i][j] += acc[i][j];
+                    acc[i][j] = 0.0f;
+                }
+        }
+#pragma unroll
+        for (int k = 0; k < WK; ++k) {
+            const float4 a = *reinterpret_cast<const float4*>(&xs[k][ty * 4]);
+            const float4 b = *reinterpret_cast<const float4*>(&ws[k][tx * 4]);
+            const float av[4] = {a.x, a.y, a.z, a.w};
+            const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = row0 + ty * 4 + i;
+        if (r >= n_rows) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int c = col0 + tx * 4 + j;
+            if (c < m_cols) out[(size_t)r * ldo + c] = sum[i][j] + acc[i][j];
+        }
+    }
+}
+
+// By tiles of 16 x 16, an output a thread, k = 64 a stage of 16-byte cp.async, four stages.  24 rows of
+// 64 against 2,048 columns: 3.0 us (the few-row kernel 5.7).
+constexpr int NT = 16, NK = 64, NSTAGES = 4, NLD = NK + 4;
+
+__global__ void __launch_bounds__(NT * NT)
+gemm_f32_narrow_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                       float* __restrict__ out, int n_rows, int m_cols, int k_dim, int ldx,
+                       int ldw, int ldo) {
+    extern __shared__ __align__(16) float smem[];
+    float* xs = smem;                                // [STAGES][16][LD]
+    float* ws = smem + NSTAGES * NT * NLD;
+    const int tid = threadIdx.x, ty = tid / NT, tx = tid % NT;
+    const int row0 = blockIdx.y * NT, col0 = blockIdx.x * NT;
+    const int l_row = tid / 16, l_k = (tid % 16) * 4;
+    const int steps = (k_dim + NK - 1) / NK;         // k_dim is a multiple of 4 here
+    auto stage_w = [&](int step) {
+        const int gk = step * NK + l_k, gc = col0 + l_row;
+        const bool ok = step < steps && gc < m_cols && gk < k_dim;
+        cp_async16_f32(ws + (step % NSTAGES * NT + l_row) * NLD + l_k,
+                       ok ? w + (size_t)gc * ldw + gk : w, ok);
+    };
+    auto stage_x = [&](int step) {
+        const int gk = step * NK + l_k, gr = row0 + l_row;
+        const bool ok = step < steps && gr < n_rows && gk < k_dim;
+        cp_async16_f32(xs + (step % NSTAGES * NT + l_row) * NLD + l_k,
+                       ok ? x + (size_t)gr * ldx + gk : x, ok);
+    };
+    // (as above: the weights' first stages before the wait)
+#pragma unroll
+    for (int t = 0; t < NSTAGES - 1; ++t) stage_w(t);
+    pdl_wait();
+#pragma unroll
+    for (int t = 0; t < NSTAGES - 1; ++t) {
+        stage_x(t);
+        cp_async_commit();
+    }
+    float acc = 0.0f, sum = 0.0f;
+    for (int step = 0; step < steps; ++step) {
+        cp_async_wait<NSTAGES - 2>();
+        __syncthreads();                     // this step has landed; the stage refilled below is free
+        stage_w(step + NSTAGES - 1);
+        stage_x(step + NSTAGES - 1);
+        cp_async_commit();
+        if (step > 0 && step % (SEG / NK) == 0) {
+            sum += acc;
+            acc = 0.0f;
+        }
+        const float* xr = xs + (step % NSTAGES * NT + ty) * NLD;
+        const float* wr = ws + (step % NSTAGES * NT + tx) * NLD;
+#pragma unroll
+        for (int k = 0; k < NK; k += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(xr + k);
+            const float4 b = *reinterpret_cast<const float4*>(wr + k);
+            acc = fmaf(a.x, b.x, acc);
+            acc = fmaf(a.y, b.y, acc);
+            acc = fmaf(a.z, b.z, acc);
+            acc = fmaf(a.w, b.w, acc);
+        }
+    }
+    cp_async_wait<0>();
+    pdl_trigger();
+    const int r = row0 + ty, c = col0 + tx;
+    if (r < n_rows && c < m_cols) out[(size_t)r * ldo + c] = sum + acc;
+}
+
 int sm_count() {
     static int count = 0;
     if (count == 0) {
@@ -448,39 +603,108 @@ int launch_small(const float* x, const float* w, float* out, int n_rows, int m_c
                      ldx, ldw, ldo, tiles);
 }
 
+int launch_wide(const float* x, const float* w, float* out, int n_rows, int m_cols, int k_dim,
+                int ldx, int ldw, int ldo, bool vec, cudaStream_t s) {
+    dim3 grid((m_cols + WT - 1) / WT, (n_rows + WT - 1) / WT);
+    if (grid.y > 65535) return -3;
+    return de_launch(vec ? gemm_f32_wide_kernel<true> : gemm_f32_wide_kernel<false>, grid, dim3(256),
+                     0, s, x, w, out, n_rows, m_cols, k_dim, ldx, ldw, ldo);
+}
+
+int launch_narrow(const float* x, const float* w, float* out, int n_rows, int m_cols, int k_dim,
+                  int ldx, int ldw, int ldo, cudaStream_t s) {
+    static bool configured = false;
+    const size_t smem = (size_t)NSTAGES * 2 * NT * NLD * sizeof(float);
+    if (int e = allow_smem(gemm_f32_narrow_kernel, smem, configured)) return e;
+    dim3 grid((m_cols + NT - 1) / NT, (n_rows + NT - 1) / NT);
+    if (grid.y > 65535) return -3;
+    return de_launch(gemm_f32_narrow_kernel, grid, dim3(NT * NT), smem, s, x, w, out, n_rows, m_cols,
+                     k_dim, ldx, ldw, ldo);
+}
+
 }  // namespace
 
 DE_EXPORT int de_gemm_f32_small_rows() { return 32; }
 
-DE_EXPORT int de_gemm_f32(const float* x, const float* w, float* out, int n_rows, int m_cols,
-                          int k_dim, int ldx, int ldw, int ldo, void* stream) {
-    if (n_rows <= 0 || m_cols <= 0) return 0;
-    if (k_dim <= 0) return -2;
-    cudaStream_t s = (cudaStream_t)stream;
-#define ARGS x, w, out, n_rows, m_cols, k_dim, ldx, ldw, ldo, s
+namespace {
+enum Form { NARROW, WIDE, FEW8, FEW16_WIDE, FEW16, FEW32_WIDE, FEW32, TILES64, TILES128 };
+
+// `vec`: rows of whole 16-byte pieces at such addresses (NARROW and the FEW forms need them).
+Form choose(int n_rows, int m_cols, int k_dim, bool vec) {
     auto tiles = [&](int rows, int cols) {
         return (long long)((n_rows + rows - 1) / rows) * ((m_cols + cols - 1) / cols);
     };
     const int sms = sm_count();
-    const bool vec = (ldx % 4 == 0) && (ldw % 4 == 0) && (((uintptr_t)x) % 16 == 0) &&
-                     (((uintptr_t)w) % 16 == 0) && k_dim % 4 == 0;
+    // Short sums, few tiles: an output a thread (us at k = 64 / 256, against 2,048 columns: 1 row 2.1 /
+    // 3.6, by FEW8 3.7 / 4.6; 24 rows 3.0 / 5.9, by FEW32 5.7 / 9.2; 64 rows 4.1 / 9.9, 9.8 / 16.8;
+    // 130 rows, 1,152 tiles, go to WIDE, 5.1 / 14.7, by FEW32_WIDE 22 / 44.7).  From two segments on
+    // FEW8 is faster for eight rows (k = 320: 4.5 and 4.8; 512: 6.1 and 4.7), and from three the others
+    // (24 rows against 512 columns, k = 512: 5.5 and 9.0; 1,024: 9.3 and 6.4).  At k = 16 WIDE is as
+    // fast from 128 tiles on and faster with many.
+    if (vec && k_dim <= 512 && !(k_dim > 320 && n_rows <= 8) && tiles(16, 16) <= 704 &&
+        (k_dim > 32 || tiles(16, 16) <= 128))
+        return NARROW;
+    // Short sums, more tiles: WIDE, or tiles of 128 with one of their two groups at work where these
+    // are nearly whole rounds of one block an SM (us, 3.2 + 0.105 k a round; 2 + (8 + 0.058 a tile) k /
+    // 256; measured at k = 64 / 256: 704 tiles of 64 14.9 / 50.0 and, two rounds, 19.0 / 57.7; 1,024
+    // tiles 20.4 / 68.2 and, two rounds, 19.0 / 56.9).
+    if (k_dim <= 320) {
+        const float rounds = (float)((tiles(128, 128) + sms - 1) / sms);
+        return rounds * (3.2f + 0.105f * k_dim) <
+                       2.0f + (8.0f + 0.058f * tiles(64, 64)) * k_dim * (1.0f / 256)
+                   ? TILES128 : WIDE;
+    }
     // few rows, and somewhat more where tiles of 64 x 64 would leave a third of the SMs without one
     // (64 rows against 2,048 x 5,632: 74 against 152 us; 40 against 2,560 x 2,048: 40 against 61; 130
-    // against 2,560 x 2,048, 120 tiles: 77 against 61).  (Zeros beyond k_dim add nothing to a
-    // chain, so the kernels' results are the same bits.)
-    if (vec && (n_rows <= 32 || (n_rows <= 256 && tiles(64, 64) * 3 < 2LL * sms))) {
+    // against 2,560 x 2,048, 120 tiles: 77 against 61; with k = 512 not: 24 rows against 11,264 45
+    // against 34, 100 against 2,048 32 against 21).  (Zeros beyond k_dim add nothing to a chain, so
+    // the kernels' results are the same bits.)
+    if (vec && (n_rows <= (k_dim > 512 ? 32 : 16) ||
+                (k_dim > 512 && n_rows <= 256 && tiles(64, 64) * 3 < 2LL * sms))) {
         // 32 columns a block where that still gives every SM two blocks' worth
-        if (n_rows <= 8) return launch_small<8, 16, 2, 64>(ARGS);
-        if (n_rows <= 16)
-            return tiles(16, 32) >= 2LL * sms ? launch_small<16, 32, 3, 32>(ARGS)
-                                              : launch_small<16, 16, 4, 32>(ARGS);
-        return tiles(32, 32) >= 2LL * sms ? launch_small<32, 32, 2, 32>(ARGS)
-                                          : launch_small<32, 16, 3, 32>(ARGS);
+        if (n_rows <= 8) return FEW8;
+        if (n_rows <= 16) return tiles(16, 32) >= 2LL * sms ? FEW16_WIDE : FEW16;
+        // (few columns: blocks of 16 rows are more blocks; 24 rows against 512 columns, k = 1,024: 6.4
+        // against 10.0)
+        if (tiles(16, 16) <= 128 && n_rows <= 64) return FEW16;
+        return tiles(32, 32) >= 2LL * sms ? FEW32_WIDE : FEW32;
     }
     // tiles of 128: one block an SM; of 64: two, which take 0.54 of the time together.  The fewer
     // rounds of blocks decide.
     const long long wide = (tiles(128, 128) + sms - 1) / sms;
     const long long narrow = (tiles(64, 64) + 2 * sms - 1) / (2 * sms);
-    return wide * 100 <= narrow * 54 ? launch_tiles<128, 2>(ARGS) : launch_tiles<64, 4>(ARGS);
+    return wide * 100 <= narrow * 54 ? TILES128 : TILES64;
+}
+
+int launch(Form form, const float* x, const float* w, float* out, int n_rows, int m_cols, int k_dim,
+           int ldx, int ldw, int ldo, bool vec, cudaStream_t s) {
+#define ARGS x, w, out, n_rows, m_cols, k_dim, ldx, ldw, ldo
+    switch (form) {
+        case NARROW: return launch_narrow(ARGS, s);
+        case WIDE: return launch_wide(ARGS, vec, s);
+        case FEW8: return launch_small<8, 16, 2, 64>(ARGS, s);
+        case FEW16_WIDE: return launch_small<16, 32, 3, 32>(ARGS, s);
+        case FEW16: return launch_small<16, 16, 4, 32>(ARGS, s);
+        case FEW32_WIDE: return launch_small<32, 32, 2, 32>(ARGS, s);
+        case FEW32: return launch_small<32, 16, 3, 32>(ARGS, s);
+        case TILES64: return launch_tiles<64, 4>(ARGS, s);
+        default: return launch_tiles<128, 2>(ARGS, s);
+    }
 #undef ARGS
+}
+}  // namespace
+
+// Which kernel a product takes (a Form): operands of whole 16-byte pieces (`vec`) or not.
+DE_EXPORT int de_gemm_f32_form(int n_rows, int m_cols, int k_dim, int vec) {
+    return (int)choose(n_rows, m_cols, k_dim, vec != 0);
+}
+
+DE_EXPORT int de_gemm_f32(const float* x, const float* w, float* out, int n_rows, int m_cols,
+                          int k_dim, int ldx, int ldw, int ldo, void* stream) {
+    if (n_rows <= 0 || m_cols <= 0) return 0;
+    if (k_dim <= 0) return -2;
+    const bool vec4 = ldx % 4 == 0 && ldw % 4 == 0 && (uintptr_t)x % 16 == 0 &&
+                      (uintptr_t)w % 16 == 0;
+    return launch(choose(n_rows, m_cols, k_dim, vec4 && k_dim % 4 == 0), x, w, out, n_rows, m_cols,
+                  k_dim, ldx, ldw, ldo, vec4, (cudaStream_t)stream);
 }

@@ -41,6 +41,7 @@ SIGNATURES: dict[str, dict[str, list]] = {
     },
     "gemm_f32": {
         "de_gemm_f32": [P, P, P, I, I, I, I, I, I, P], "de_gemm_f32_small_rows": [],
+        "de_gemm_f32_form": [I, I, I, I],
     },
     "attention_simt": {
         "de_attn_simt_rows_per_tile": [],

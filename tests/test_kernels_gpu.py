@@ -186,9 +186,9 @@ def test_attention_f32_tiles_of_8_and_32_rows_agree_bit_for_bit(head_dim, heads,
 @pytest.mark.parametrize("k,m", [(256, 64), (260, 65), (512, 15), (2304, 129), (4100, 33), (52, 4800)])
 def test_gemm_f32_rows_of_every_batch_size(k, m):
     """Segments that end in the middle, more segments than warps, columns around the tiles' edges:
-    a row has the same bits among 1, 8, 9, 16, 17, 32, 33, 64, 129 and 700 rows (all kernels and
-    tile sizes).  Bound: a chain of 256 roundings and one a segment, each of half a unit of the sum
-    of absolute terms."""
+    a row has the same bits among 1, 8, 9, 16, 17, 32, 33, 64, 129 and 700 rows
+    (test_gemm_f32_forms names the kernels).  Bound: a chain of 256 roundings and one a segment, each
+    of half a unit of the sum of absolute terms."""
     ops = _ops()
     g = torch.Generator(device=DEV).manual_seed(k + m)
     x = torch.randn(700, k, generator=g, device=DEV)
@@ -820,3 +820,36 @@ def test_soft_cap_on_tensor_cores(cap, low, high, rows):
     want = cap * (torch.tanh(x.double() / cap) - torch.tanh(y.double() / cap))
     units = (torch.log(p) - torch.log1p(-p) - want).abs() / (cap * 2.0 ** -24)
     assert units[clear].max().item() <= 2 * (0.5 + 2 + 0.5) + 1
+
+
+# the kernels of a float32 product, by number (``de_gemm_f32_form``)
+FORMS = ("narrow", "wide", "few8", "few16 wide", "few16", "few32 wide", "few32", "tiles64", "tiles128")
+
+
+@pytest.mark.parametrize("n,m,k,form", [
+    (1, 130, 260, "narrow"), (100, 100, 508, "narrow"), (130, 2050, 52, "wide"), (40, 70, 51, "wide"),
+    (300, 130, 258, "wide"), (8, 131, 600, "few8"), (5, 9700, 2308, "few8"),
+    (11, 9700, 2308, "few16 wide"), (16, 130, 2308, "few16"), (40, 300, 772, "few16"),
+    (17, 9700, 2308, "few32 wide"), (31, 1100, 2308, "few32"), (130, 2000, 772, "few32 wide"),
+    (70, 515, 1028, "few32"), (33, 2051, 2305, "tiles64"), (300, 2052, 1028, "tiles64"),
+    (700, 2310, 1029, "tiles128"), (1000, 2051, 772, "tiles128"), (2040, 2300, 124, "tiles128")])
+def test_gemm_f32_forms(n, m, k, form):
+    """Every kernel of the float32 product at sizes that are whole tiles of nothing, several segments
+    with a ragged one last: a row's bits are those of the row alone, and of the rows that other
+    kernels take.  Bound: as the test of every batch size."""
+    from distengine_b200.kernels import library
+    ops = _ops()
+    choose = library.load("gemm_f32").de_gemm_f32_form
+    assert FORMS[choose(n, m, k, int(k % 4 == 0))] == form
+    g = torch.Generator(device=DEV).manual_seed(n + m)
+    x, w = torch.randn(n, k, generator=g, device=DEV), torch.randn(m, k, generator=g, device=DEV)
+    out = torch.full((n, m), float("nan"), device=DEV)
+    ops.gemm_f32(x, w, out)
+    terms = x.double().abs() @ w.double().abs().t()
+    bound = (min(k, 256) + (k + 255) // 256) * 2.0 ** -24 * terms
+    assert ((out.double() - x.double() @ w.double().t()).abs() <= bound).all()
+    for first, count in ((0, 1), (n - 1, 1), (n // 3, min(n - n // 3, 13)), (0, min(n, 29)),
+                         (n // 2, min(n - n // 2, 150))):
+        part = torch.full((count, m), float("nan"), device=DEV)
+        ops.gemm_f32(x[first: first + count], w, part)
+        assert torch.equal(part, out[first: first + count]), (first, count)
