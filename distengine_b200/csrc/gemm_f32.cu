@@ -9,6 +9,8 @@
 // It stands where the reference calls F.linear in float32 with TF32 switched off
 // (src/layers/linear.py:19-20, src/distengine/worker.py:427-428).
 
+#include <atomic>
+
 #include "common.cuh"
 
 DE_DEFINE_PDL_SWITCH
@@ -148,17 +150,10 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
         if (n_k % SEG == 0) n_k += (GROUPS - 1) * SEG;
     };
 
-    // the weights do not depend on the kernel before this one
+    pdl_wait();
 #pragma unroll
     for (int t = 0; t < STAGES - 1; ++t) {
         load_w();
-        advance();
-    }
-    pdl_wait();
-    n_k = group * SEG;
-    n_slot = 0;
-#pragma unroll
-    for (int t = 0; t < STAGES - 1; ++t) {
         load_x();
         advance();
         cp_async_commit();
@@ -255,7 +250,7 @@ template <int T, int COLS, int SM_STAGES, int SM_K>
 __global__ void __launch_bounds__(SM_WARPS * 32)
 gemm_f32_small_kernel(const float* __restrict__ x, const float* __restrict__ w,
                       float* __restrict__ out, int n_rows, int m_cols, int k_dim, int ldx, int ldw,
-                      int ldo, int col_tiles) {
+                      int ldo, int col_tiles, int early) {
     constexpr int SM_LD = SM_K + 4;
     constexpr int PAIRS = COLS / 2;                          // lanes along the columns
     constexpr int TG = 32 / PAIRS;                           // groups of tokens
@@ -311,15 +306,17 @@ gemm_f32_small_kernel(const float* __restrict__ x, const float* __restrict__ w,
         n_round = 0;
         ++n_tile;
     };
-    // the weights do not depend on the kernel before this one: their first stages are requested
-    // before the wait
+    auto first_w = [&]() {
 #pragma unroll
-    for (int t = 0; t < SM_STAGES - 1; ++t) {
-        stage_w();
-        advance();
-    }
+        for (int t = 0; t < SM_STAGES - 1; ++t) {
+            stage_w();
+            advance();
+        }
+        n_step = n_round = n_tile = n_slot = 0;
+    };
+    if (early) first_w();
     pdl_wait();
-    n_step = n_round = n_tile = n_slot = 0;
+    if (!early) first_w();
 #pragma unroll
     for (int t = 0; t < SM_STAGES - 1; ++t) {
         stage_x();
@@ -491,7 +488,7 @@ constexpr int NT = 16, NK = 64, NSTAGES = 4, NLD = NK + 4;
 __global__ void __launch_bounds__(NT * NT)
 gemm_f32_narrow_kernel(const float* __restrict__ x, const float* __restrict__ w,
                        float* __restrict__ out, int n_rows, int m_cols, int k_dim, int ldx,
-                       int ldw, int ldo) {
+                       int ldw, int ldo, int early) {
     extern __shared__ __align__(16) float smem[];
     float* xs = smem;                                // [STAGES][16][LD]
     float* ws = smem + NSTAGES * NT * NLD;
@@ -511,10 +508,13 @@ gemm_f32_narrow_kernel(const float* __restrict__ x, const float* __restrict__ w,
         cp_async16_f32(xs + (step % NSTAGES * NT + l_row) * NLD + l_k,
                        ok ? x + (size_t)gr * ldx + gk : x, ok);
     };
-    // (as above: the weights' first stages before the wait)
+    auto first_w = [&]() {
 #pragma unroll
-    for (int t = 0; t < NSTAGES - 1; ++t) stage_w(t);
+        for (int t = 0; t < NSTAGES - 1; ++t) stage_w(t);
+    };
+    if (early) first_w();
     pdl_wait();
+    if (!early) first_w();
 #pragma unroll
     for (int t = 0; t < NSTAGES - 1; ++t) {
         stage_x(t);
@@ -560,22 +560,32 @@ int sm_count() {
     return count;
 }
 
-template <typename F> int allow_smem(F kernel, size_t smem, bool& configured) {
-    if (configured) return 0;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+// Lets a kernel's blocks have `smem` bytes of dynamic shared memory, once a device: `devices` (one a
+// kernel) notes which.
+template <typename F>
+int allow_smem(F kernel, size_t smem, std::atomic<unsigned long long>& devices) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return (int)e;
-    configured = true;
+    const unsigned long long bit = device < 64 ? 1ull << device : 0ull;
+    if (devices.load() & bit) return 0;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    devices |= bit;
     return 0;
 }
+
+// Up to 32 rows (decode steps) the kernels ask for their first weights before the wait for the kernel
+// before them, which must not have formed them; with more rows, they wait first.
+int early_weights(int n_rows) { return n_rows <= 32; }
 
 template <int TILE, int GROUPS>
 int launch_tiles(const float* x, const float* w, float* out, int n_rows, int m_cols, int k_dim,
                  int ldx, int ldw, int ldo, cudaStream_t s) {
     using Shape = Tiles<TILE, GROUPS>;
-    static bool configured = false;
+    static std::atomic<unsigned long long> allowed{0};
     auto kernel = gemm_f32_kernel<TILE, GROUPS>;
-    if (int e = allow_smem(kernel, Shape::SMEM, configured)) return e;
+    if (int e = allow_smem(kernel, Shape::SMEM, allowed)) return e;
     dim3 grid((m_cols + TILE - 1) / TILE, (n_rows + TILE - 1) / TILE);
     if (grid.y > 65535) return -3;
     const int vec_out = ldo % 4 == 0 && (uintptr_t)out % 16 == 0;
@@ -588,19 +598,21 @@ int launch_small(const float* x, const float* w, float* out, int n_rows, int m_c
                  int ldx, int ldw, int ldo, cudaStream_t s) {
     const size_t smem = ((size_t)2 * SM_WARPS * T * COLS +
                          (size_t)SM_WARPS * SM_STAGES * (COLS + T) * (SM_K + 4)) * sizeof(float);
-    static bool configured = false;
-    static int per_sm = 1;
+    static std::atomic<unsigned long long> allowed{0};
+    static std::atomic<int> blocks{0};               // of an SM
     auto kernel = gemm_f32_small_kernel<T, COLS, SM_STAGES, SM_K>;
-    if (!configured) {
-        if (int e = allow_smem(kernel, smem, configured)) return e;
+    if (int e = allow_smem(kernel, smem, allowed)) return e;
+    int per_sm = blocks.load();
+    if (per_sm == 0) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, SM_WARPS * 32, smem) !=
                 cudaSuccess || per_sm < 1) per_sm = 1;
+        blocks = per_sm;
     }
     const int tiles = (m_cols + COLS - 1) / COLS, row_tiles = (n_rows + T - 1) / T;
     const int places = sm_count() * per_sm / row_tiles;
     dim3 grid(tiles < places ? tiles : (places < 1 ? 1 : places), row_tiles);
     return de_launch(kernel, grid, dim3(SM_WARPS * 32), smem, s, x, w, out, n_rows, m_cols, k_dim,
-                     ldx, ldw, ldo, tiles);
+                     ldx, ldw, ldo, tiles, early_weights(n_rows));
 }
 
 int launch_wide(const float* x, const float* w, float* out, int n_rows, int m_cols, int k_dim,
@@ -613,13 +625,13 @@ int launch_wide(const float* x, const float* w, float* out, int n_rows, int m_co
 
 int launch_narrow(const float* x, const float* w, float* out, int n_rows, int m_cols, int k_dim,
                   int ldx, int ldw, int ldo, cudaStream_t s) {
-    static bool configured = false;
+    static std::atomic<unsigned long long> allowed{0};
     const size_t smem = (size_t)NSTAGES * 2 * NT * NLD * sizeof(float);
-    if (int e = allow_smem(gemm_f32_narrow_kernel, smem, configured)) return e;
+    if (int e = allow_smem(gemm_f32_narrow_kernel, smem, allowed)) return e;
     dim3 grid((m_cols + NT - 1) / NT, (n_rows + NT - 1) / NT);
     if (grid.y > 65535) return -3;
     return de_launch(gemm_f32_narrow_kernel, grid, dim3(NT * NT), smem, s, x, w, out, n_rows, m_cols,
-                     k_dim, ldx, ldw, ldo);
+                     k_dim, ldx, ldw, ldo, early_weights(n_rows));
 }
 
 }  // namespace

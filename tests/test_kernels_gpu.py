@@ -853,3 +853,23 @@ def test_gemm_f32_forms(n, m, k, form):
         part = torch.full((count, m), float("nan"), device=DEV)
         ops.gemm_f32(x[first: first + count], w, part)
         assert torch.equal(part, out[first: first + count]), (first, count)
+
+
+@pytest.mark.parametrize("n", [33, 64, 130, 700])
+def test_gemm_f32_by_rows_that_were_just_formed(n):
+    """The second operand comes from the kernel before, as the first may: with more than 32 rows a
+    product reads neither before that kernel has finished."""
+    ops = _ops()
+    g = torch.Generator(device=DEV).manual_seed(n)
+    a, b = torch.randn(2000, 1500, generator=g, device=DEV), torch.randn(2052, 1500, generator=g, device=DEV)
+    x = torch.randn(n, 2052, generator=g, device=DEV)
+    w, out = torch.empty(2000, 2052, device=DEV), torch.empty(n, 2000, device=DEV)
+    ops.gemm_f32(a, b, w)
+    torch.cuda.synchronize()
+    ops.gemm_f32(x, w, out)
+    want = out.clone()
+    for _ in range(5):
+        w.fill_(float("nan")), out.fill_(float("nan"))
+        ops.gemm_f32(a, b, w)
+        ops.gemm_f32(x, w, out)
+        assert torch.equal(out, want)
