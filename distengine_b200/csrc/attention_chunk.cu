@@ -423,7 +423,10 @@ template <int PN> __device__ __forceinline__ void load_run(const float* p, int w
 // same chains of multiply-adds either way.
 // The taps come tap by tap (a lane's channels side by side): 2,402 tokens of 3,072 channels with
 // four taps 44 us, 60 where a channel's taps lay together (32 lines a request).
-template <typename T, bool VEC>
+// CONV: there are taps, more than one.  (A kernel of its own: without the convolution it needs 48
+// registers, five blocks an SM, with it 54; 2,048 tokens of 16 + 4 heads of 128 without taps 26 us in
+// one kernel for both, 23 so.)
+template <typename T, bool VEC, bool CONV>
 __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __restrict__ q_out,
                                    const int* __restrict__ positions,
                                    const int* __restrict__ token_seq,
@@ -455,7 +458,7 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __rest
     }
     pdl_wait();
     const T* row = proj + (size_t)n * ld;
-    if (VEC && pp.taps != nullptr && pp.K > 1) {
+    if (VEC && CONV) {
         constexpr int PN = 16 / (int)sizeof(T);
         const int K = pp.K;
         const float* kept = pp.state + (size_t)slot * pp.slot_stride + pp.conv_offset;
@@ -488,7 +491,7 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __rest
             for (int e = 0; e < PN; e += 4)
                 store_four(sh + c0 + e, make_float4(acc[e], acc[e + 1], acc[e + 2], acc[e + 3]));
         }
-    } else if (pp.taps != nullptr && pp.K > 1) {
+    } else if (CONV) {
         const int K = pp.K;
         const float* kept = pp.state + (size_t)slot * pp.slot_stride + pp.conv_offset;
         for (int c = threadIdx.x; c < C; c += blockDim.x) {
@@ -528,7 +531,7 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __rest
         }
     }
     __syncthreads();
-    if (pp.keep_here && pp.taps != nullptr && pp.K > 1) {
+    if (CONV && pp.keep_here) {
         // every thread has read what it needs of the kept rows; a thread moves its channels on
         float* kept = pp.state + (size_t)slot * pp.slot_stride + pp.conv_offset;
         for (int c = threadIdx.x; c < C; c += blockDim.x) {
@@ -2747,18 +2750,24 @@ DE_EXPORT int de_qkv_prepare(int dtype, const void* proj, int ld, void* q_out,
     const int threads = C >= 2048 && n < 512 ? 512 : 256;
     const int pn = dtype == DE_BF16 ? 8 : 4;
     const bool vec = C % pn == 0 && ld % pn == 0 && (uintptr_t)proj % 16 == 0;
-#define PREP(T, V)                                                                              \
+    const bool conv = taps != nullptr && K > 1;
+#define PREP_C(T, V, CONV)                                                                      \
     do {                                                                                        \
         if (smem > 48 * 1024) {                                                                 \
-            cudaError_t e = cudaFuncSetAttribute(qkv_prepare_kernel<T, V>,                      \
+            cudaError_t e = cudaFuncSetAttribute(qkv_prepare_kernel<T, V, CONV>,                \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                                                  (int)smem);                                    \
             if (e != cudaSuccess) return (int)e;                                                \
         }                                                                                       \
-        return de_launch(qkv_prepare_kernel<T, V>, dim3(n), dim3(threads), smem, s,             \
+        return de_launch(qkv_prepare_kernel<T, V, CONV>, dim3(n), dim3(threads), smem, s,       \
                          (const T*)proj, ld, (T*)q_out, positions, token_seq, token_slot,       \
                          seq_pos0, pp, H, G, dk, dv, (T*)k_pages, (T*)v_pages, block_table,     \
                          table_stride, page, num_pages, status);                                \
+    } while (0)
+#define PREP(T, V)                                                                              \
+    do {                                                                                        \
+        if (conv) PREP_C(T, V, true);                                                           \
+        PREP_C(T, V, false);                                                                    \
     } while (0)
     if (dtype == DE_BF16) {
         if (vec) PREP(__nv_bfloat16, true);
@@ -2767,6 +2776,7 @@ DE_EXPORT int de_qkv_prepare(int dtype, const void* proj, int ld, void* q_out,
     if (vec) PREP(float, true);
     PREP(float, false);
 #undef PREP
+#undef PREP_C
 }
 
 DE_EXPORT int de_conv_keep(int dtype, const void* proj, int ld, float* state, long long slot_stride,
