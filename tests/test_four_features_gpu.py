@@ -77,3 +77,25 @@ def test_taps_by_tap(dtype, K, biased):
     for other in results[1:]:
         for a, b in zip(results[0], other):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,dv,turned", [(16, 40, True), (10, 64, False), (5, 128, True), (4, 160, True),
+                                         (159, 4, False)])
+@pytest.mark.parametrize("gate", [None, "feature", "head"])
+def test_finish_of_rows_of_640_features(dtype, H, dv, turned, gate):
+    """Rows around the 640 features from which four are taken at a time."""
+    from distengine_b200.kernels import recurrent as rk
+    n, g = 9, _gen(dv)
+    ctx = _ctx((5, 4), (3, 900), (1, 0))
+    o = torch.randn(n, H * dv, generator=g).to(DEV)
+    fv = torch.rand(dv // 2, generator=g).to(DEV) if turned else None
+    gt = None if gate is None else torch.randn(n, H * dv if gate == "feature" else H, generator=g).to(dtype)
+    results = []
+    for shift in (0, 1):                                  # results at 16-byte addresses, or not
+        out = torch.zeros(n * H * dv + 8, dtype=dtype, device=DEV)[shift: shift + n * H * dv].view(n, -1)
+        rk.attention_finish(o, fv, None if gt is None else gt.to(DEV), out, H, dv, ctx,
+                            **({"gate_per_head": True} if gate == "head" else {}))
+        results.append(out.clone())
+    assert torch.equal(*results)
+
