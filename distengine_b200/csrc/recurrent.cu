@@ -1032,8 +1032,12 @@ DE_EXPORT int de_silu_rows(int dtype, const void* proj, int ld, float* out, int 
     if (n <= 0 || cols <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t total = (size_t)n * cols;
-    if (cols % 4 == 0 && ld % 4 == 0 && (uintptr_t)proj % (dtype == DE_BF16 ? 8 : 16) == 0 &&
-        (uintptr_t)out % 16 == 0 && total / 4 < (1u << 30)) {
+    // groups of four from 600,000 elements on (us, an element a thread and so: 8 rows of 6,144 1.5 and
+    // 3.1, 300 of 1,536 2.7 and 3.2, 100 of 6,144 3.4 and 3.4, 2,048 of 6,144 31 and 20): with few
+    // elements four loads a thread one after the other are a longer chain on fewer blocks
+    if (total >= 600000 && cols % 4 == 0 && ld % 4 == 0 &&
+        (uintptr_t)proj % (dtype == DE_BF16 ? 8 : 16) == 0 && (uintptr_t)out % 16 == 0 &&
+        total / 4 < (1u << 30)) {
         const unsigned quads = (unsigned)(total / 4), fours = (quads + 1023) / 1024;
         const dim3 grid(fours < 148 * 8 ? fours : 148 * 8);
         if (dtype == DE_BF16)

@@ -188,6 +188,19 @@ def test_delta_preparation_of_any_number_of_tokens(K, G, H, dk, dv):
         assert torch.equal(got, want), name
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,cols", [(157, 4100), (300, 2000), (1201, 516), (300, 1996)])
+def test_silu_of_many_rows(dtype, n, cols):
+    """Around the 600,000 elements from which a thread takes four groups of four, remainders of a grid's
+    last round among them."""
+    from distengine_b200.kernels import recurrent as rk
+    x = (torch.randn(n, cols + 4, generator=_gen(n)) * 4).to(dtype)
+    out = torch.full((n, cols), float("nan"), device=DEV)
+    rk.silu_rows(x.to(DEV)[:, 4:], out)
+    want = pv.silu(x[:, 4:].double())
+    assert (out.double().cpu() - want).abs().max().item() <= 8 * EPS * want.abs().max().item()
+
+
 def _walk(rule, lens, inputs, state, H, dk, dv, begin=0):
     """The tokens from ``begin`` on of one sequence, in steps of ``lens``: portions of 192 tokens and
     more by chunks, others by the scan.  Returns the read-outs."""
