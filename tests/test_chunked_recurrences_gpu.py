@@ -161,30 +161,40 @@ def test_rows_in_groups_of_four(dtype, n, cols, pad):
     assert ((res.double().cpu() - want).abs() <= unit * want.abs() + 1e-7).all()
 
 
-@pytest.mark.parametrize("K,G,H,dk,dv", [(4, 2, 4, 64, 64), (2, 1, 2, 128, 192), (3, 4, 4, 128, 64)])
+@pytest.mark.parametrize("K,G,H,dk,dv", [(4, 2, 4, 64, 64), (2, 1, 2, 128, 192), (3, 4, 4, 128, 64),
+                                         (1, 2, 2, 64, 320)])
 def test_delta_preparation_of_any_number_of_tokens(K, G, H, dk, dv):
-    """In float32 a token's vectors are the same bits in a step of 300 tokens, which is prepared in
-    runs, and in steps of fewer than 128 tokens, which are not."""
+    """In float32 a token's vectors are the same bits in a step of 840 tokens of three sequences, which
+    is prepared in runs, and in steps of fewer than 128 tokens of one, which are not."""
     from distengine_b200.kernels import recurrent as rk
-    n, C, g = 300, 2 * G * dk + H * dv, _gen(dk)
-    inputs = [torch.randn(n, C + H, generator=g), torch.randn(n, H * dk, generator=g)]
-    rest = [torch.randn(C, K, generator=g), torch.randn(H * dk, generator=g),
-            torch.randn(H, generator=g) * 0.5]
-    rows = H * dk * dv
-    results = []
-    for lens in ((300,), (127, 100, 73)):
-        state, at, parts = torch.zeros(1, rows + (K - 1) * C, device=DEV), 0, []
-        for m in lens:
-            proj, a = (x[at: at + m].to(DEV) for x in inputs)
-            ctx = _ctx([m], [at], [0])
-            bufs = [torch.full((m, w), float("nan"), device=DEV)
-                    for w in (G * dk, G * dk, H * dv, H, H * dk)]
-            rk.delta_prep(proj, a, *(t.to(DEV) for t in rest), state, rows, ctx, *bufs, H, G, dk, dv, C)
-            state[0, rows:] = proj[m - (K - 1):, :C].reshape(-1)
-            parts.append(bufs)
-            at += m
-        results.append([torch.cat(x) for x in zip(*parts)])
-    for got, want, name in zip(*results, ("q", "k", "v", "beta", "decay")):
+    lens, pos0, C, g = (501, 3, 336), (0, 50, 7), 2 * G * dk + H * dv, _gen(dk)
+    n, rows = sum(lens), H * dk * dv
+    proj, a = torch.randn(n, C + H, generator=g).to(DEV), torch.randn(n, H * dk, generator=g).to(DEV)
+    rest = [t.to(DEV) for t in (torch.randn(C, K, generator=g), torch.randn(H * dk, generator=g),
+                                torch.randn(H, generator=g) * 0.5)]
+    kept = torch.randn(3, rows + (K - 1) * C, generator=g).to(DEV)
+
+    def prepare(lens, pos0, slots, first, state):
+        m = sum(lens)
+        bufs = [torch.full((m, w), float("nan"), device=DEV)
+                for w in (G * dk, G * dk, H * dv, H, H * dk)]
+        rk.delta_prep(proj[first: first + m], a[first: first + m], *rest, state, rows,
+                      _ctx(lens, pos0, slots), *bufs, H, G, dk, dv, C)
+        return bufs
+
+    together = prepare(lens, pos0, (0, 1, 2), 0, kept)
+    parts, first = [], 0
+    for slot, length in enumerate(lens):
+        state, at = kept.clone(), 0
+        while at < length:
+            m = min(127, length - at)
+            parts.append(prepare([m], [pos0[slot] + at], [slot], first, state))
+            if K > 1:
+                state[slot, rows:] = torch.cat((state[slot, rows:].view(K - 1, C), proj[
+                    first: first + m, :C]))[-(K - 1):].reshape(-1)
+            at, first = at + m, first + m
+    for got, want, name in zip(together, (torch.cat(x) for x in zip(*parts)),
+                               ("q", "k", "v", "beta", "decay")):
         assert torch.equal(got, want), name
 
 
