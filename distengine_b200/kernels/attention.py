@@ -93,8 +93,8 @@ class AttentionLauncher:
         else:
             self.shapes = [_Shape("rows8", 8, -1)]
             if dtype == torch.float32 and head_dim % 4 == 0:
-                # rows of whole 16-byte pieces: sequences with many rows take tiles of 32 (a row's
-                # result is the same bits in either)
+                # rows of whole 16-byte pieces: steps with many rows take tiles of 32 (a row's result is
+                # the same bits in either)
                 self.shapes.insert(0, _Shape("rows32", 32, -1))
             self.module = ("attention_simt", ())
         self.fixed_chunk = F32_CHUNK if dtype == torch.float32 else None
@@ -139,6 +139,22 @@ class AttentionLauncher:
         narrow |= seq_qlen == 1
         return [np.where(narrow, 0, seq_qlen).astype(np.int32),
                 np.where(narrow, seq_qlen, 0).astype(np.int32)]
+
+    def _few_blocks(self, host, graph_shape) -> bool:
+        """Whether a float32 step is so small that tiles of 8 rows, which are four times as many blocks
+        with a shorter chain each, are done sooner than tiles of 32 (us, heads of 64, 32 query heads on
+        4: one portion of 5 tokens 5.2 and 8.4, four of 17 6.2 and 9.2, one of 100, 400 blocks, 18.2
+        and 25.5; of 200, 1,088 blocks, 42.7 and 34.9; 8 heads on 8: one of 400, 832 blocks, 43.6 and
+        35.4).  Above 128 features an SM holds one block: the line is lower (heads of 256, 256 and
+        240 blocks 26.3 and 25.2, 56 and 53)."""
+        spans = host.seq_pos0.astype(np.int64) + host.seq_qlen
+        if graph_shape is not None:              # (of the batch's shape only)
+            spans = np.full_like(spans, int(graph_shape["context_cap"]))
+        if self.window:
+            spans = np.minimum(spans, self.window + host.seq_qlen.astype(np.int64))
+        tiles = (host.seq_qlen.astype(np.int64) * self.group + 7) // 8
+        blocks = int((tiles * ((spans + F32_CHUNK - 1) // F32_CHUNK)).sum()) * self.kv_heads
+        return blocks <= (512 if self.head_dim <= 128 else 200)
 
     def _prepare_decode(self, prep, force_split: "tuple[int, int, int] | None") -> None:
         """A step in which every sequence brings one token: the work list of the one-launch
@@ -201,6 +217,8 @@ class AttentionLauncher:
         prep.notes[self.key + "/decode"] = None
         notes = {}
         parts = self._split(host.seq_qlen)
+        if self.shapes[0].name == "rows32" and self._few_blocks(host, prep.graph_shape):
+            parts = [np.zeros_like(host.seq_qlen), host.seq_qlen]
         if force_shape is not None:
             parts = [host.seq_qlen if s.name == force_shape else np.zeros_like(host.seq_qlen)
                      for s in self.shapes]

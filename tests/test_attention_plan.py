@@ -100,3 +100,33 @@ def test_chunk_choice_fills_the_gpu_or_leaves_ranges_whole():
     assert choose_chunk(1000, 4, 4096, sm_count=SMS) == 0                  # enough tiles: no split
     c = choose_chunk(8, 4, 4096, sm_count=SMS)
     assert c in (2048, 1024, 512, 256, 128, 64) and 8 * 4 * -(-4096 // c) >= 2 * SMS
+
+
+@pytest.mark.parametrize("qlen,pos0,heads,kv_heads,dim,shape", [
+    ([5], [0], 32, 4, 64, "rows8"), ([17] * 4, [0] * 4, 32, 4, 60, "rows8"), ([100], [0], 32, 4, 64, "rows8"),
+    ([200], [0], 32, 4, 64, "rows32"), ([400], [0], 8, 8, 64, "rows32"), ([100], [1000], 8, 8, 128, "rows32"),
+    ([17] * 4, [0] * 4, 32, 4, 256, "rows32"), ([17], [0], 8, 8, 256, "rows8")])
+def test_float32_tiles_by_the_blocks_of_a_step(qlen, pos0, heads, kv_heads, dim, shape):
+    """Small float32 steps take tiles of 8 rows, larger ones tiles of 32; single tokens beside a portion
+    tiles of 8 either way; a step shaped for replay decides by its shape alone."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from distengine_b200.kernels.attention import AttentionLauncher
+    from distengine_b200.parts.context import StepPrep
+    launcher = AttentionLauncher(torch.float32, heads, kv_heads, dim, 1.0, None)
+    for more in ([], [1]):
+        arrays = []
+        for graph_shape, start in ((None, 0), ({"context_cap": 1536}, 0), ({"context_cap": 1536}, 100)):
+            host = SimpleNamespace(seq_qlen=np.array(qlen + more, dtype=np.int32),
+                                   seq_pos0=np.array(pos0 + more, dtype=np.int32) + start)
+            prep = StepPrep(host, graph_shape)
+            launcher.prepare(prep)
+            count = {s.name: prep.extra[f"{launcher.key}/{s.name}/items"] for s in launcher.shapes}
+            arrays.append({name: a.shape for name, a in count.items()})
+            if graph_shape is None:
+                assert len(count[shape]) and (shape == "rows8" or bool(len(count["rows8"])) == bool(more))
+                assert shape == "rows32" or not len(count["rows32"])
+        assert arrays[1] == arrays[2]
+
