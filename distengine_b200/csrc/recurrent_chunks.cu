@@ -701,30 +701,32 @@ chunk_out_kernel(const float* __restrict__ xt, const float* __restrict__ states,
         __syncthreads();
     }
     pdl_trigger();
+    unsigned spoilt = 0;
+    float* o = out + (size_t)it.token * (H * dv) + h * dv + j0 + tile.col;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int t = tile.row_of(i);
+        const float4 v = tile.get(i);
         if (t >= it.count) continue;
-        float4 v = tile.get(i);
-        // an infinity or NaN: its sums again, without the products of pt's zeros with the u of later
-        // tokens, which would spoil this one too
-        if (!(fmaf(v.x, 0.0f, fmaf(v.y, 0.0f, fmaf(v.z, 0.0f, v.w * 0.0f))) == 0.0f)) {
-            float r[4];
-            for (int e = 0; e < 4; ++e) {
-                const int j = j0 + tile.col + e;
-                r[e] = 0.0f;
-                for (int c = 0; c < dk; ++c)
-                    r[e] = fmaf(xt[(at * dk + c) * CH + t], states[(at * dk + c) * dv + j], r[e]);
-                for (int s = 0; s <= t; ++s)
-                    r[e] = fmaf(pt[(at * CH + s) * CH + t],
-                                to_float(u_by_item ? u[(at * CH + s) * dv + j]
-                                                   : u[(size_t)(it.token + s) * ldu + h * dv + j]),
-                                r[e]);
-            }
-            v = make_float4(r[0], r[1], r[2], r[3]);
+        *reinterpret_cast<float4*>(o + (size_t)t * (H * dv)) = v;
+        if (!(fmaf(v.x, 0.0f, fmaf(v.y, 0.0f, fmaf(v.z, 0.0f, v.w * 0.0f))) == 0.0f)) spoilt |= 1u << i;
+    }
+    // an infinity or NaN: a token's sums again, without the products of pt's zeros with the u of later
+    // tokens, which would spoil this one too
+    for (int i = 0; spoilt != 0; ++i, spoilt >>= 1) {
+        if (!(spoilt & 1u)) continue;
+        const int t = tile.row_of(i);
+        for (int e = 0; e < 4; ++e) {
+            const int j = j0 + tile.col + e;
+            float r = 0.0f;
+            for (int c = 0; c < dk; ++c)
+                r = fmaf(xt[(at * dk + c) * CH + t], states[(at * dk + c) * dv + j], r);
+            for (int s = 0; s <= t; ++s)
+                r = fmaf(pt[(at * CH + s) * CH + t],
+                         to_float(u_by_item ? u[(at * CH + s) * dv + j]
+                                            : u[(size_t)(it.token + s) * ldu + h * dv + j]), r);
+            o[(size_t)t * (H * dv) + e] = r;
         }
-        *reinterpret_cast<float4*>(out + (size_t)(it.token + t) * (H * dv) + h * dv + j0 + tile.col) =
-            v;
     }
 }
 
