@@ -106,9 +106,21 @@ SEBI_WIDE = {
     ],
 }
 
-ALL = {"sebi_a": SEBI_A, "sebi_b": SEBI_B, "sebi_c": SEBI_C, "sebi_wide": SEBI_WIDE}
-SEEDS = {"sebi_a": 15, "sebi_b": 16, "sebi_c": 17, "sebi_wide": 18}
-PAGES = {"sebi_a": 16, "sebi_b": 8, "sebi_c": 16, "sebi_wide": 16}
+# heads of 64 features, which bfloat16 takes to the tensor cores and to the chunks
+SEBI_64 = {
+    "architecture": "Sebilorn", "vocab": 200, "width": 256, "norm": {"eps": 1e-6},
+    "embedding": {"scale": 4.0}, "logit_softcap": 30.0,
+    "layers": [
+        _attention(8, 2, 64, 64, 0.125, 300, 5, _rot(32, 250000.0, (4.0, 1.0, 4.0, 256)), 20.0,
+                   ff=256),
+        _lightning(4, 64, 64, [0.9, 0.99, 0.999, 0.97], 256),
+        _attention(8, 2, 64, 64, 0.125, 1000, 0, _rot(64, 10000.0)),
+    ],
+}
+
+ALL = {"sebi_64": SEBI_64, "sebi_a": SEBI_A, "sebi_b": SEBI_B, "sebi_c": SEBI_C, "sebi_wide": SEBI_WIDE}
+SEEDS = {"sebi_64": 19, "sebi_a": 15, "sebi_b": 16, "sebi_c": 17, "sebi_wide": 18}
+PAGES = {"sebi_64": 16, "sebi_a": 16, "sebi_b": 8, "sebi_c": 16, "sebi_wide": 16}
 
 
 def write_folder(config: dict, folder: str, weights: dict) -> str:

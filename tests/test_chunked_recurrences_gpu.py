@@ -327,3 +327,50 @@ def test_chunks_a_few_at_a_time(rule, group, monkeypatch):
         assert len(sizes) == 1 and min(14, work // a_chunk) * a_chunk <= sizes[0] <= work
         results.append((out, state))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("kind,taps", [("gated_delta_rule", 3), ("gated_delta_rule", 1),
+                                       ("retention", 0), ("lightning_attention", 0)])
+def test_steps_by_chunks_as_graphs(kind, taps):
+    """A bfloat16 step of a long portion beside a short one, or alone (with one tap the scan then has
+    nothing to do), replayed as a CUDA graph: the bits of the step launch by launch."""
+    from gpu_helpers import PartHarness
+    from distengine_b200.kernels import recurrent as rk
+    mixer, width = _layer(kind, torch.bfloat16, taps or 3)
+    for lens in ((900, 37), (900,)):
+        assert rk.chunks_pay(kind == "gated_delta_rule", 2, 64, 64, 900, 900, 15)
+        harness = PartHarness([mixer], [mixer.cache_spec()], torch.bfloat16, num_pages=80, max_seqs=2,
+                              max_len=2048)
+        harness.runner.use_graphs = True
+        x = torch.randn(sum(lens), width, generator=_gen(8)).to(torch.bfloat16).to(DEV)
+        names, results = [f"r{i}" for i in range(len(lens))], []
+        for _ in range(7):
+            out = harness.run(list(zip(names, lens)),
+                              lambda ctx, bindings: mixer.forward(x, ctx, bindings[0]))
+            states = [harness.cache.bindings()[0].state[harness.cache.slot(n)].clone() for n in names]
+            results.append((out.clone(), torch.stack(states)))
+            for name in names:
+                harness.cache.release(name)
+        assert harness.runner.graph_replays >= 2
+        for out, state in results[1:]:
+            assert torch.equal(out, results[0][0]) and torch.equal(state, results[0][1])
+
+
+@pytest.mark.parametrize("kind,taps", [("gated_delta_rule", 3), ("gated_delta_rule", 1),
+                                       ("lightning_attention", 0)])
+def test_a_bfloat16_layer_by_chunks_and_by_the_scan(kind, taps, monkeypatch):
+    """The same step both ways: the states within the bound of float32 sums, the outputs within two
+    roundings of bfloat16; and portions that are not in whole 16-byte pieces go by the scan."""
+    from distengine_b200.kernels import recurrent as rk
+    mixer, width = _layer(kind, torch.bfloat16, taps or 3)
+    x = torch.randn(900, width, generator=_gen(8)).to(torch.bfloat16).to(DEV)
+    out, state = _feed(mixer, x, torch.bfloat16, (900,))
+    monkeypatch.setattr(rk, "chunks_pay", lambda *a: False)
+    other, end = _feed(mixer, x, torch.bfloat16, (900,))
+    assert not torch.equal(end, state)                       # (two ways)
+    assert (end - state).abs().max().item() <= 2 * BOUND * state.abs().max().item()
+    assert (other.float() - out.float()).abs().max().item() <= 2 ** -6 * out.float().abs().max().item()
+    monkeypatch.undo()
+    monkeypatch.setattr(rk, "chunks_aligned", lambda v, state: False)
+    last, end_too = _feed(mixer, x, torch.bfloat16, (900,))
+    assert torch.equal(last, other) and torch.equal(end_too, end)

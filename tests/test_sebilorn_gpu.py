@@ -154,6 +154,32 @@ def test_a_long_prompt_at_wide_sizes(dtype_name, model_root):
     _compare(rows, {"w": want, "c": want}, DTYPES[dtype_name], f"wide {dtype_name}")
 
 
+def test_a_long_prompt_with_heads_of_64(model_root):
+    """The kernels for heads of 64 features in bfloat16 through a whole model: attention on the tensor
+    cores, its single tokens, and lightning attention by chunks, for a prompt of 1,100 tokens, then
+    tokens one by one, then the prompt in two portions, the second too short for chunks."""
+    from distengine_b200.engine.replay import build_runner
+    from distengine_b200.kernels import recurrent as rk
+    name = "sebi_64"
+    folder, weights = sc.make_folder(name, model_root)
+    ids = sc.tokens(name, 1108, 3)
+    assert rk.chunks_pay(False, 4, 64, 64, 1100, 1100, 18)
+    want = ps.forward(sc.ALL[name], weights, ids, act=torch.bfloat16).to(torch.float32).numpy()
+    picked = [0, 1, 63, 64, 299, 300, 305, 700, 1099]
+    head = {"step": 0, "end": [], "entries": [{"id": "w", "tokens": ids[:1100], "want": picked}]}
+    tail = [{"step": 1 + i, "end": ["w"] if i == 7 else [],
+             "entries": [{"id": "w", "tokens": [ids[1100 + i]], "want": [0]}]} for i in range(8)]
+    cut = [{"step": 9, "end": [], "entries": [{"id": "c", "tokens": ids[:950], "want": [949]}]},
+           {"step": 10, "end": ["c"], "entries": [{"id": "c", "tokens": ids[950:], "want": [0, 157]}]}]
+    runner = build_runner(folder, "bfloat16", 1152, page_size=16, poison_freed_pages=True)
+    steps = [head] + tail + cut
+    with tempfile.TemporaryDirectory() as out:
+        th.replay_in_process(runner, steps, out)
+        rows = th.collect(steps, out, sc.ALL[name]["vocab"])
+    assert len(rows) == len(picked) + 8 + 3
+    _compare(rows, {"w": want, "c": want}, torch.bfloat16, "heads of 64")
+
+
 def test_pages_behind_a_window_come_back_but_the_first_stay(model_root):
     """After 200 tokens the windowed groups hold the pages of their kept first tokens and of the
     window only; the group that sees everything holds all."""
