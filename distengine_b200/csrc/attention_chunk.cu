@@ -11,7 +11,10 @@
 // A row is (token, query head within its kv head's group); a block takes a tile of 8 rows of one
 // sequence and one kv head, a warp a row, a lane a key of the current tile of 32 keys.  Tiles of
 // keys lie at absolute multiples of 32 and a row walks the tiles of its chunk in ascending order,
-// so a row's result does not depend, bit for bit, on what shares its tile, its step or its batch.
+// so a row's result does not depend, bit for bit, on what shares its tile.  The kernels below for other
+// sizes, longer portions, single tokens and the tensor cores each sum in an order of their own; which
+// one takes a row depends on its step (on how many rows the step's portions have and, for bfloat16
+// rows of 64 and 128 features, how many single tokens there are).
 // The host's work items are those of the other attention kernels (kernels/attention_plan.py),
 // unsplit: a chunk bounds every key range.
 //
@@ -165,7 +168,7 @@ __device__ __forceinline__ void load_piece(const __nv_bfloat16* p, float* f) {
     }
 }
 
-// two neighbouring features in one store
+// four neighbouring features in one load
 __device__ __forceinline__ float4 load_four(const float* p) {
     return *reinterpret_cast<const float4*>(p);
 }
@@ -174,6 +177,7 @@ __device__ __forceinline__ float4 load_four(const __nv_bfloat16* p) {
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
                        __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
 }
+// two in one store
 __device__ __forceinline__ void store_pair(float* p, float a, float b) {
     *reinterpret_cast<float2*>(p) = make_float2(a, b);
 }
@@ -1455,7 +1459,7 @@ attn_chunk_tiled_kernel(const T* __restrict__ q, int q_stride, void* __restrict_
 // ------------------------------------------------------------------------------------------
 // The same attention on the tensor cores, for bfloat16 rows of D = 64 or 128 features (keys and
 // values alike): mma.sync m16n8k16, a block of four warps takes 64 rows, a warp 16 of them against
-// tiles of 64 keys that come through two stages of cp.async.  Nothing loses precision against the
+// tiles of 32 keys that come through two stages of cp.async.  Nothing loses precision against the
 // kernels above: the products of bfloat16 queries and keys are exact, and a softmax weight enters
 // its product with the values as three bfloat16 terms whose sum is the float32 weight.  What the
 // tensor cores add up is a tile's share only, the small terms first; the running sums of a row are
@@ -2298,7 +2302,10 @@ attn_chunk_decode_kernel(const T* __restrict__ q, int q_stride, void* __restrict
 // heads a kv head, with both products on the tensor cores as attn_chunk_mma_kernel forms them (a
 // block's heads are the first eight of a product's sixteen rows).  A warp's tiles are 16 keys and
 // come through three stages of its own, so that two are on their way while one is worked on; a
-// block of four warps leaves room for a second on its SM, eight warps serve steps of few sequences.
+// block of four warps leaves room for a second on its SM, eight warps serve steps of few sequences
+// (four or eight partial results are merged: a row's bits depend on which, so on the step's size.  Four
+// warps with two shares of the tiles each would give one order, and were slower: 64 sequences of 700
+// keys of 64 features 15.8 -> 19.9 us, of one key on 16 kv heads 11.0 -> 14.7).
 // Bound by memory and by the trips to it: 64 sequences of 700 keys, 16 heads on 4 kv heads of 128:
 // 25 us, 3.7 TB/s (the kernel above, which asks for a tile, waits and works: 81).
 // ------------------------------------------------------------------------------------------
@@ -2361,7 +2368,6 @@ attn_chunk_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     pdl_wait();
     decode_begin<T>(Qs, DRW, g, h0, hk, q, q_stride, tok, slot, pos, k_pages, v_pages, block_table,
                     table_stride, num_pages, heads, kv_heads, D, D, page, fuse, status);
-    if (!fuse.on) __syncthreads();
     unsigned qf[D / 16][4];                          // (rounded already: what q went through)
 #pragma unroll
     for (int kk = 0; kk < D / 16; ++kk) {

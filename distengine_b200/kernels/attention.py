@@ -7,7 +7,7 @@ items on the host and launches them.
   its narrow tile (16 rows, the keys of a tile split over the warps).
 * float32, or any other even head size up to 256: the CUDA-core kernels in float32 arithmetic
   (``csrc/attention_simt.cu``), 8 rows a tile; in float32 with head sizes that are a multiple of 4
-  32 rows a tile for sequences with many query rows.
+  32 rows a tile for portions in steps with enough rows.
 
 Long key ranges of a step with few tiles are cut into chunks; ``de_attn_combine`` merges the
 partial results (``attention_plan``).  In float32 the chunk length is fixed (``F32_CHUNK`` keys,

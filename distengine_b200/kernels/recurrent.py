@@ -398,9 +398,10 @@ _sm_count: dict[int, int] = {}
 def long_portion_rows(seq_qlen, heads: int, kv_heads: int) -> int:
     """The rows of a step's longest portion (tokens times query heads a kv head) if tiles of 64
     rows would still give every SM two blocks, else 0: what ``chunk_rows_per_tile`` takes as
-    ``longest_rows``.  (Measured on B200 with the kernels of the CUDA cores, 16 heads on 4 kv heads
-    of 128: a prompt of 512 tokens takes 274 us in 128 blocks of 64 rows against 221 us in 256 blocks
-    of 32; one of 2,048 tokens 739 against 1,362 us.)"""
+    ``longest_rows``.  (Measured on B200, tiles of 64 and of 32 rows, heads of 128: on the tensor cores
+    1,024 tokens of 8 heads on 2, 128 and 256 blocks, 100 and 79 us, 2,048 tokens of 16 heads, 512 and
+    1,024 blocks, 199 and 231; with the kernels of the CUDA cores, 16 heads on 4, 512 tokens 274 and
+    221, 2,048 tokens 739 and 1,362.)"""
     group = heads // kv_heads
     device = torch.cuda.current_device()
     if device not in _sm_count:

@@ -140,8 +140,8 @@ def test_silu_mul(dtype):
                                    (64, 2048, 2560), (3, 5632, 2048), (20, 2048, 300),
                                    (33, 72, 40), (32, 200, 17)])
 def test_gemm_f32(n, k, m):
-    """(up to 32 rows take the kernel of narrow tiles, more the wide one; a row alone and the same
-    row in a batch of more than 32 go through both and must agree bit for bit)"""
+    """(a row alone and the same row in its batch, which go through different kernels at most of these
+    sizes, must agree bit for bit; test_gemm_f32_forms names the kernels)"""
     ops = _ops()
     g = torch.Generator().manual_seed(n + k + m)
     x = torch.randn(n, k, generator=g)
