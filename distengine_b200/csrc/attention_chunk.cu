@@ -2306,8 +2306,9 @@ attn_chunk_decode_kernel(const T* __restrict__ q, int q_stride, void* __restrict
 // (four or eight partial results are merged: a row's bits depend on which, so on the step's size.  Four
 // warps with two shares of the tiles each would give one order, and were slower: 64 sequences of 700
 // keys of 64 features 15.8 -> 19.9 us, of one key on 16 kv heads 11.0 -> 14.7).
-// Bound by memory and by the trips to it: 64 sequences of 700 keys, 16 heads on 4 kv heads of 128:
-// 25 us, 3.7 TB/s (the kernel above, which asks for a tile, waits and works: 81).
+// Bound by memory and by the trips to it: 64 sequences of up to 700 keys (614 on average, 80 MB), 16
+// heads on 4 kv heads of 128: 26 us, 3.0 TB/s (the kernel above, which asks for a tile, waits and works:
+// 81).
 // ------------------------------------------------------------------------------------------
 constexpr int DKT = 16, DSTAGES = 3, DRW = 8;
 
