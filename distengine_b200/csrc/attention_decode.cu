@@ -163,8 +163,8 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_stride,
     // rows of 128 features a request: whole 128-byte lines).  Lane j looks up key j's row, one tile
     // ahead of its use.  The token's own row is left out (fill_new).  Measured, 64 sequences of
     // up to 4,097 keys (3,636 on average, 0.95 GB), 8 kv heads of 128: 271 -> 174 us (3.5 -> 5.5 TB/s)
-    // against two threads a row that take its pieces by turns (sixteen rows a request, a barrier of the block before and after
-    // each tile); 8 sequences of 520 keys: a layer 0.6 us less.
+    // against two threads a row that take its pieces by turns (sixteen rows a request, a barrier of the
+    // block before and after each tile); 8 sequences of 520 keys: a layer 0.6 us less.
     static_assert(NK == 16 && CHUNKS % 2 == 0, "a key a lane of half a warp, whole rounds of pieces");
     auto row_of = [&](int kt) {                       // -1: not to be read
         long long row = -1;
