@@ -39,6 +39,7 @@ MODULES: dict[str, tuple[str, tuple[str, ...]]] = {
     "linear_mid": ("linear_mid.cu", ("cuda",)),
     "attention_tcgen05": ("attention_tcgen05.cu", ()),  # built per head size: HEAD_DIM=64|128
     "attention_chunk": ("attention_chunk.cu", ()),
+    "attention_chunk_tcgen05": ("attention_chunk_tcgen05.cu", ("cuda",)),
     "recurrent": ("recurrent.cu", ()),
     "recurrent_chunks": ("recurrent_chunks.cu", ()),
     "ssm": ("ssm.cu", ()),

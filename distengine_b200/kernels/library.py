@@ -87,6 +87,11 @@ SIGNATURES: dict[str, dict[str, list]] = {
         "de_attn_chunk": [I, P, I, P, I, P, P, P, I, I, P, P, P, P, P, I, P, P, I, I, I, I, I, F,
                           I, I, I, F, I, I, I, I, P, P, I, I, F, P, P],
     },
+    "attention_chunk_tcgen05": {
+        "de_attn_chunk_tcgen05_rows": [], "de_attn_chunk_tcgen05_ok": [I, I, I],
+        "de_attn_chunk_tcgen05": [P, I, P, I, P, P, P, I, I, P, P, P, P, P, I, P, P, I, I, I, I, I,
+                                  F, I, I, I, F, I, I, P, P, I, I, F, P, P],
+    },
     "recurrent": {
         "de_recurrent_max_key_dim": [],
         "de_delta_prep": [I, P, I, P, P, P, P, P, L, I, P, P, P, P, P, P, P, P, P, I, I, I, I, I,

@@ -395,6 +395,14 @@ def chunk_rows_per_tile(dtype: torch.dtype, key_dim: int, value_dim: int, wide: 
 _sm_count: dict[int, int] = {}
 
 
+def _sms() -> int:
+    """SMs of the current device."""
+    device = torch.cuda.current_device()
+    if device not in _sm_count:
+        _sm_count[device] = torch.cuda.get_device_properties(device).multi_processor_count
+    return _sm_count[device]
+
+
 def long_portion_rows(seq_qlen, heads: int, kv_heads: int) -> int:
     """The rows of a step's longest portion (tokens times query heads a kv head) if tiles of 64
     rows would still give every SM two blocks, else 0: what ``chunk_rows_per_tile`` takes as
@@ -403,11 +411,51 @@ def long_portion_rows(seq_qlen, heads: int, kv_heads: int) -> int:
     1,024 blocks, 199 and 231; with the kernels of the CUDA cores, 16 heads on 4, 512 tokens 274 and
     221, 2,048 tokens 739 and 1,362.)"""
     group = heads // kv_heads
-    device = torch.cuda.current_device()
-    if device not in _sm_count:
-        _sm_count[device] = torch.cuda.get_device_properties(device).multi_processor_count
     blocks = int(((seq_qlen.astype("int64") * group + 63) // 64).sum()) * kv_heads
-    return int(seq_qlen.max()) * group if blocks >= 2 * _sm_count[device] else 0
+    return int(seq_qlen.max()) * group if blocks >= 2 * _sms() else 0
+
+
+WIDE_ROWS = 128         # of a tile of csrc/attention_chunk_tcgen05.cu
+
+
+def _wide_ok(key_dim: int, value_dim: int, page: int) -> bool:
+    return bool(library.load("attention_chunk_tcgen05").de_attn_chunk_tcgen05_ok(key_dim, value_dim,
+                                                                                 page))
+
+
+def portion_kernels(dtype: torch.dtype, key_dim: int, value_dim: int) -> "tuple[str, ...]":
+    """The kernel libraries that ``chunk_attention`` calls for such rows."""
+    wide = dtype == torch.bfloat16 and key_dim == value_dim and key_dim in (64, 128)
+    return ("attention_chunk",) + (("attention_chunk_tcgen05",) if wide else ())
+
+
+def portion_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int, prep, heads: int,
+                      kv_heads: int) -> int:
+    """Rows of a tile of the chunk attention for a step with prompt portions: 128 (the tcgen05
+    kernel) or what ``chunk_rows_per_tile`` says.
+
+    A tile of 128 rows is two blocks of the tcgen05 kernel, two of which an SM holds.  It is the sooner
+    one (us, heads of 128, 16 on 4, tiles of 32 / 64 / 128 rows) for one portion of 9 tokens behind
+    1,900 keys 113 / 152 / 77, of 500 tokens 43 / 51 / 33, of 2,048 238 / 213 / 88, four of 30 behind
+    500 43 / 53 / 39; with as many blocks as places also for 20 single tokens behind 600 keys beside a
+    portion of 300 (46 / 59 / 43).  Not where tiles are mostly empty and take several rounds - 60
+    single tokens beside it 54 / 62 / 77, 64 portions of 2 tokens 41 / 51 / 69 - or where many of
+    them have few keys each (16 portions of 40 tokens from position 0: 21 / 21 / 26)."""
+    host = prep.host
+    seq_qlen = host.seq_qlen
+    wide = int(seq_qlen.max()) > 1
+    if wide and len(portion_kernels(dtype, key_dim, value_dim)) > 1:
+        rows = seq_qlen.astype("int64") * (heads // kv_heads)
+        tiles = int(((rows + WIDE_ROWS - 1) // WIDE_ROWS).sum())
+        blocks, sms = 2 * tiles * kv_heads, _sms()
+        # (in a step whose graph is replayed: by the batch's shape only)
+        longest = (int((host.seq_pos0 + seq_qlen).max()) if prep.graph_shape is None
+                   else int(prep.graph_shape["context_cap"]))
+        if blocks <= sms or (longest > 128 and (blocks <= 2 * sms
+                                                or 2 * int(rows.sum()) >= tiles * WIDE_ROWS)):
+            return WIDE_ROWS
+    return chunk_rows_per_tile(dtype, key_dim, value_dim, wide,
+                               long_portion_rows(seq_qlen, heads, kv_heads))
 
 
 def chunk_decode_ok(dtype: torch.dtype, heads: int, kv_heads: int, key_dim: int,
@@ -522,6 +570,18 @@ def chunk_attention(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor,
     _i32(block_table, "block_table"), _i32(items, "items")
     r1, r2, last = _penalty(r1, r2, heads, slopes, sink, gate, gate_per_head, q.dtype, value_dim,
                             out_scale)
+    if (tile_rows == WIDE_ROWS and q.dtype == torch.bfloat16 and v_stride == 0
+            and _wide_ok(key_dim, value_dim, k_pages.shape[2])):
+        lib = library.load("attention_chunk_tcgen05")
+        _check(lib.de_attn_chunk_tcgen05(
+            q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), k_pages.data_ptr(),
+            v_pages.data_ptr(), block_table.data_ptr(), block_table.stride(0), k_pages.shape[0],
+            ctx.seq_slot.data_ptr(), ctx.seq_qstart.data_ptr(), ctx.seq_qlen.data_ptr(),
+            ctx.seq_pos0.data_ptr(), items.data_ptr(), items.shape[0], _ptr(r1), _ptr(r2), heads,
+            kv_heads, key_dim, value_dim, k_pages.shape[2], float(scale), int(chunk), int(window),
+            int(keep_first), float(softcap), int(out.dtype == torch.float32), *last,
+            ctx.status.data_ptr(), _stream()), "chunk_attention (tcgen05)")
+        return
     lib = library.load("attention_chunk")
     _check(lib.de_attn_chunk(_tag(q.dtype), q.data_ptr(), q.stride(0), out.data_ptr(),
                              out.stride(0), k_pages.data_ptr(), v_pages.data_ptr(),

@@ -61,7 +61,7 @@ class ChunkAttention(ProjectedMixer):
         return self._host_in
 
     def kernel_modules(self):
-        return ("attention_chunk",)
+        return rk.portion_kernels(self.dtype, self.dk, self.dv)
 
     def cache_spec(self):
         return PagedKVSpec(self.kv_heads, self.dk, None, value_dim=self.dv, chunk=self.chunk)
@@ -84,9 +84,7 @@ class ChunkAttention(ProjectedMixer):
             prep.notes[self.key] = 0
             return
         # tiles of 32 rows when the step brings prompt portions, of 8 for single tokens
-        rows = rk.chunk_rows_per_tile(self.dtype, self.dk, self.dv,
-                                      int(host.seq_qlen.max()) > 1,
-                                      rk.long_portion_rows(host.seq_qlen, self.heads, self.kv_heads))
+        rows = rk.portion_tile_rows(self.dtype, self.dk, self.dv, prep, self.heads, self.kv_heads)
         plan = build_plan(host.seq_qlen, host.seq_pos0, self.heads // self.kv_heads,
                           self.kv_heads, rows, 0, chunk=0)
         prep.add(name, plan.items)

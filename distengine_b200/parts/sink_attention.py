@@ -187,7 +187,7 @@ class SinkAttention(ProjectedMixer):
 
     def kernel_modules(self):
         if self.launcher is None:
-            return ("attention_chunk",)
+            return rk.portion_kernels(self.dtype, self.dk, self.dv)
         return ("attention_chunk", self.launcher.module, ("attention_simt", ()))
 
     # the norms of a block that reads the stream itself never ride on this mixer's products
@@ -227,9 +227,7 @@ class SinkAttention(ProjectedMixer):
             prep.add(name, np.zeros((0, 8), dtype=np.int32))
             prep.notes[self.key] = 0
             return
-        rows = rk.chunk_rows_per_tile(self.dtype, self.dk, self.dv,
-                                      int(host.seq_qlen.max()) > 1,
-                                      rk.long_portion_rows(host.seq_qlen, self.heads, self.kv_heads))
+        rows = rk.portion_tile_rows(self.dtype, self.dk, self.dv, prep, self.heads, self.kv_heads)
         plan = build_plan(host.seq_qlen, host.seq_pos0, self.heads // self.kv_heads,
                           self.kv_heads, rows, 0, chunk=0)
         prep.add(name, plan.items)

@@ -113,7 +113,7 @@ class WindowAttention(ProjectedMixer):
         return self._host_in
 
     def kernel_modules(self):
-        return ("attention_chunk",)
+        return rk.portion_kernels(self.dtype, self.dk, self.dv)
 
     def cache_spec(self):
         return PagedKVSpec(self.kv_heads, self.dk, self.cache_window, value_dim=self.dv,
@@ -136,9 +136,7 @@ class WindowAttention(ProjectedMixer):
             prep.add(name, np.zeros((0, 8), dtype=np.int32))
             prep.notes[self.key] = 0
             return
-        rows = rk.chunk_rows_per_tile(self.dtype, self.dk, self.dv,
-                                      int(host.seq_qlen.max()) > 1,
-                                      rk.long_portion_rows(host.seq_qlen, self.heads, self.kv_heads))
+        rows = rk.portion_tile_rows(self.dtype, self.dk, self.dv, prep, self.heads, self.kv_heads)
         plan = build_plan(host.seq_qlen, host.seq_pos0, self.heads // self.kv_heads,
                           self.kv_heads, rows, 0, chunk=0)
         prep.add(name, plan.items)
