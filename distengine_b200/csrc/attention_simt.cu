@@ -176,6 +176,45 @@ attn_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
     }
 }
 
+// Row w of a tile: its partial results `first` .. `first + count - 1`, in ascending order, into o.  A warp.
+template <typename T, int BLOCKS>                  // BLOCKS: of 32 features
+__device__ __forceinline__ void merge_row(T* o, const float* partial_acc, const float* partial_ml,
+                                          int first, int count, int kv_heads, int hk,
+                                          int rows_per_tile, int w, int d) {
+    const int lane = threadIdx.x & 31;
+    float m = -INFINITY;
+    for (int c = 0; c < count; ++c) {
+        const size_t idx = ((size_t)(first + c) * kv_heads + hk) * rows_per_tile + w;
+        m = fmaxf(m, __ldcg(partial_ml + idx * 2));
+    }
+    float l = 0.0f;
+    float acc[BLOCKS];
+#pragma unroll
+    for (int i = 0; i < BLOCKS; ++i) acc[i] = 0.0f;
+    // (everything is loaded without a branch on what was loaded before it)
+#pragma unroll 4
+    for (int c = 0; c < count; ++c) {
+        const size_t idx = ((size_t)(first + c) * kv_heads + hk) * rows_per_tile + w;
+        const float mc = __ldcg(partial_ml + idx * 2), lc = __ldcg(partial_ml + idx * 2 + 1);
+        const bool any = mc != -INFINITY;         // else the chunk held no visible key
+        const float f = any ? expf(mc - m) : 0.0f;
+        if (any) l += lc * f;
+        const float* pa = partial_acc + idx * d;
+#pragma unroll
+        for (int i = 0; i < BLOCKS; ++i) {
+            const int dd = lane + 32 * i;
+            const float v = dd < d ? __ldcg(pa + dd) : 0.0f;
+            if (any) acc[i] = fmaf(v, f, acc[i]);
+        }
+    }
+    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+#pragma unroll
+    for (int i = 0; i < BLOCKS; ++i) {
+        const int dd = lane + 32 * i;
+        if (dd < d) o[dd] = from_float<T>(acc[i] * inv);
+    }
+}
+
 // The same attention for float32 pages whose rows are whole 16-byte pieces: tiles of keys and values
 // come through three stages of 16-byte cp.async (eight threads a key, which look its page up once
 // and a tile ahead), a warp takes RW rows and reads a key or a value from shared memory once for
@@ -410,22 +449,72 @@ attn_simt_vec_kernel(const float* __restrict__ q, int q_stride, float* __restric
 // keys before values: a thread forms the scores of one key with RPT rows, a warp takes a row's maxima,
 // weights and sums over the tiles of 32 keys, and then two rows' weighted sums over half of the
 // features.  All sums in the order of the kernels above, so the same bits.
-// Bound by the trips to memory and a barrier between its three phases.  A decode step of 8 sequences of
-// 520 keys (22 layers): 2,151 -> 2,000 us against one warp a row through tiles of 32 keys (19 us a
-// layer, of which a row's chain of 64 multiply-adds a tile and a branch a key were most).
+// Bound by the trips to memory that follow one another and by barriers.  A decode step of 8 sequences of
+// 520 keys through 22 layers: 2,151 us with a warp a row through tiles of 32 keys, 2,000 so, 1,829 in one
+// kernel with rotation, cache write and merge (`Fuse`; 16 us a layer instead of 28 for the three).
+//
+// With `fuse.on` (a step of single tokens, one tile of rows a sequence; an item's row0 and pad2 are then
+// the token's position and its slot) a block also does what rope_kv_write and attn_combine do around it,
+// in their arithmetic: it turns its queries, the block whose range ends with the token's own position
+// turns that key and stores it and its value, and the block that finishes a tile last merges the
+// tile's partial results.  No block waits for another.
+// The code is kept small (a step streams all weights between two launches: instructions come from far)
+// and so is the number of loads that wait for one another.
+struct Fuse {
+    int on;
+    const float* inv_freq;     // or null: nothing is turned
+    int rot, writes;           // writes 0: the cache is another run's
+    int* counters;             // [sequences][kv heads], zero before and after
+};
+
+// `KEYS` rows of keys (`hide` given) or values of one kv head into `to`, eight threads a row; `skip`: a
+// position that does not come from the pages.
+template <int KEYS>
+__device__ __noinline__ void copy_rows(const float* pages, float* to, int stride, float* hide,
+                                       const int* table, int kt, int lo, int hi, int skip, int num_pages,
+                                       int hk, int kv_heads, int page, int d, int aligned, int* status) {
+    const int j0 = threadIdx.x >> 3, part = threadIdx.x & 7;
+    int ids[KEYS / 32];
+#pragma unroll
+    for (int i = 0; i < KEYS / 32; ++i) {
+        const int kpos = kt + j0 + 32 * i;
+        ids[i] = kpos < lo || kpos >= hi ? -2 : table[kpos / page];      // -2: outside the range
+    }
+#pragma unroll
+    for (int i = 0; i < KEYS / 32; ++i) {
+        const int j = j0 + 32 * i;
+        const bool read = ids[i] >= 0 && ids[i] < num_pages;
+        const float* from = pages + (read ? (((size_t)ids[i] * kv_heads + hk) * page +
+                                             (size_t)((kt + j) % page)) * d : 0);
+        if (hide != nullptr && part == 0) {
+            const bool gone = ids[i] != -2 && !read;
+            hide[j] = gone ? -INFINITY : 0.0f;
+            if (gone && status != nullptr) atomicExch(status, 2);
+        }
+        if (kt + j == skip && read) continue;
+        if (aligned) {
+            const unsigned at = (unsigned)__cvta_generic_to_shared(to + j * stride);
+            for (int c = 4 * part; c < d; c += 32)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(at + 4 * c),
+                             "l"(from + c), "r"(read ? 16 : 0) : "memory");
+        } else {                                     // pages that do not start at 16 bytes
+            for (int c = part; c < d; c += 8) to[j * stride + c] = read ? from[c] : 0.0f;
+        }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
 template <int VW, int KEYS>
 __global__ void __launch_bounds__(ROWS * 32, 3)
 attn_simt_rows_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out,
-                      int out_stride, const float* __restrict__ k_pages,
-                      const float* __restrict__ v_pages, const int* __restrict__ block_table,
-                      int table_stride, int num_pages, const int* __restrict__ seq_slot,
-                      const int* __restrict__ seq_qstart, const int* __restrict__ seq_qlen,
-                      const int* __restrict__ seq_pos0, const WorkItem* __restrict__ items,
-                      float* __restrict__ partial_acc, float* __restrict__ partial_ml,
+                      int out_stride, const float* k_pages, const float* v_pages,
+                      const int* __restrict__ block_table, int table_stride, int num_pages,
+                      const int* __restrict__ seq_slot, const int* __restrict__ seq_qstart,
+                      const int* __restrict__ seq_qlen, const int* __restrict__ seq_pos0,
+                      const WorkItem* __restrict__ items, float* partial_acc, float* partial_ml,
                       int partial_limit, int heads, int kv_heads, int d, int page, float scale,
-                      int window, int aligned, int* __restrict__ status) {
+                      int window, int aligned, Fuse fuse, int* __restrict__ status) {
     constexpr int RPT = ROWS * KEYS / 256, NT = KEYS / TILE;   // rows of a thread's scores; tiles
-    constexpr int PASSES = KEYS / 32;                // keys a copying thread takes part in
     extern __shared__ __align__(16) float smem[];
     const int ks = d + 4;                            // a key's stride: 16-byte reads without conflicts
     float* Ks = smem;                                // [KEYS][ks]
@@ -435,82 +524,87 @@ attn_simt_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
     float* hide = Ps + ROWS * KEYS;                  // [KEYS]: 0, or -inf without a page
     float* corr_s = hide + KEYS;                     // [ROWS][NT]
     float* l_s = corr_s + ROWS * NT;                 // [ROWS]
+    float* turn_s = l_s + ROWS;                      // [d]: cosines, then sines (with fuse.on)
 
     const WorkItem it = items[blockIdx.x];
     if (it.kv_begin >= it.kv_end || it.partial >= partial_limit) {
         pdl_wait();
         return;
     }
-    const int hk = blockIdx.y;
-    const int g = heads / kv_heads;
-    const int qlen = seq_qlen[it.seq], pos0 = seq_pos0[it.seq];
-    const int slot = seq_slot[it.seq], tok0 = seq_qstart[it.seq];
-    const int rows_total = qlen * g;
+    const int hk = blockIdx.y, g = heads / kv_heads;
+    const int row0 = fuse.on ? 0 : it.row0, rows_total = fuse.on ? g : seq_qlen[it.seq] * g;
+    const int pos0 = fuse.on ? it.row0 : seq_pos0[it.seq];
+    const int slot = fuse.on ? it.pad2 : seq_slot[it.seq], tok0 = seq_qstart[it.seq];
+    const int* table = block_table + (size_t)slot * table_stride;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int last_row = min(it.row0 + ROWS, rows_total) - 1;
-    const int max_pos = pos0 + last_row / g, min_pos = pos0 + it.row0 / g;
-    const int k_hi = min(it.kv_end, max_pos + 1);
+    const int last_row = min(row0 + ROWS, rows_total) - 1;
+    const int k_hi = min(it.kv_end, pos0 + last_row / g + 1);
     int k_lo_true = it.kv_begin;
-    if (window > 0) k_lo_true = max(k_lo_true, min_pos - window + 1);
+    if (window > 0) k_lo_true = max(k_lo_true, pos0 + row0 / g - window + 1);
     const int k_lo = (k_lo_true / TILE) * TILE;      // tiles sit at absolute positions
+    // the token's own key, if it is this block's to store; among the first keys it does not come from the
+    // pages but from here, later ones are read back
+    const int own = fuse.on && fuse.writes && pos0 >= k_lo_true && pos0 < k_hi ? pos0 : -1;
+    const int skip = own < k_lo + KEYS ? own : -1;
+    auto copy = [&](int kt, bool keys) {
+        copy_rows<KEYS>(keys ? k_pages : v_pages, keys ? Ks : Vs, keys ? ks : d, keys ? hide : nullptr,
+                        table, kt, k_lo_true, k_hi, skip, num_pages, hk, kv_heads, page, d, aligned,
+                        status);
+    };
 
-    // copies: eight threads a key
-    const int j0 = threadIdx.x >> 3, part = threadIdx.x & 7;
-    int ids[PASSES];                                 // pages of this thread's keys; -2: outside the range
-    auto look_up = [&](int kt) {
-#pragma unroll
-        for (int i = 0; i < PASSES; ++i) {
-            const int kpos = kt + j0 + 32 * i;
-            ids[i] = kpos < k_lo_true || kpos >= k_hi
-                         ? -2 : block_table[(size_t)slot * table_stride + kpos / page];
+    // Older keys, the only ones that a step's own cache holds here, are from kernels long before the last:
+    // they are asked for before the wait.  Another run's cache got its newest key in this step, and
+    // portions' keys were stored by the kernel before this one.
+    const bool early = fuse.on && fuse.writes;
+    if (!early) pdl_wait();
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) copy(k_lo, i == 0);
+    const int half = fuse.on ? fuse.rot / 2 : 0;
+    if ((int)threadIdx.x < half) {                   // (half <= MAX_D / 2)
+        float sn = 0.0f, cs = 1.0f;
+        if (fuse.inv_freq) sincosf((float)pos0 * fuse.inv_freq[threadIdx.x], &sn, &cs);
+        turn_s[threadIdx.x] = cs;
+        turn_s[half + threadIdx.x] = sn;
+    }
+    if (early) pdl_wait();
+    if (fuse.on) __syncthreads();
+    // queries, a warp a row; with fuse.on the warps go on with the token's own key and value
+    const int qkv_rows = ROWS + (own >= 0 ? 2 : 0);
+#pragma unroll 1
+    for (int w = warp; w < qkv_rows; w += ROWS) {
+        const int r = row0 + w;
+        const bool active = w >= ROWS || r < rows_total;
+        const int head = w == ROWS ? heads + hk : w > ROWS ? heads + kv_heads + hk : hk * g + r % g;
+        const float* src = q + (size_t)(tok0 + (active && w < ROWS ? r / g : 0)) * q_stride +
+                           (size_t)(active ? head : 0) * d;
+        float *to = Qs + w * d, *to_page = nullptr;
+        if (w >= ROWS) {
+            // (its page is missing: the key is hidden, and the status says so)
+            const int id = table[own / page];
+            if (id < 0 || id >= num_pages) continue;
+            const size_t at = (((size_t)id * kv_heads + hk) * page + (size_t)(own % page)) * d;
+            to_page = const_cast<float*>(w == ROWS ? k_pages : v_pages) + at;
+            to = skip < 0 ? nullptr : w == ROWS ? Ks + (own - k_lo) * ks : Vs + (own - k_lo) * d;
         }
-    };
-    auto issue = [&](int kt, const float* pages, float* to, int stride, bool keys) {
-#pragma unroll
-        for (int i = 0; i < PASSES; ++i) {
-            const int j = j0 + 32 * i;
-            const bool read = ids[i] >= 0 && ids[i] < num_pages;
-            const size_t off = read ? (((size_t)ids[i] * kv_heads + hk) * page +
-                                       (size_t)((kt + j) % page)) * d : 0;
-            if (aligned) {
-                const int bytes = read ? 16 : 0;
-                for (int c = 4 * part; c < d; c += 32) {
-                    const unsigned at = (unsigned)__cvta_generic_to_shared(to + j * stride + c);
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(at),
-                                 "l"(pages + off + c), "r"(bytes) : "memory");
-                }
-            } else {                                 // pages that do not start at 16 bytes
-                for (int c = part; c < d; c += 8) to[j * stride + c] = read ? pages[off + c] : 0.0f;
+        const int turned = w > ROWS ? 0 : half;      // pairs
+#pragma unroll 1
+        for (int i = lane; i < d - turned; i += 32) {
+            const int c = i < turned ? i : i + turned;
+            float a = active ? src[c] : 0.0f, b = 0.0f;
+            if (i < turned) {
+                b = active ? src[i + half] : 0.0f;
+                rope_rotate(a, b, turn_s[i], turn_s[half + i], a, b);
+                if (to != nullptr) to[i + half] = b;
             }
-            if (keys && part == 0) {
-                const bool gone = ids[i] != -2 && !read;
-                hide[j] = gone ? -INFINITY : 0.0f;
-                if (gone && status != nullptr) atomicExch(status, 2);
+            if (to != nullptr) to[c] = a;
+            if (to_page != nullptr) {
+                to_page[c] = a;
+                if (i < turned) to_page[i + half] = b;
             }
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    look_up(k_lo);
-    pdl_wait();            // q, and the keys and values of this step's tokens, are just written
-    issue(k_lo, k_pages, Ks, ks, true);
-    issue(k_lo, v_pages, Vs, d, false);
-    {
-        const int r = it.row0 + warp;                // a warp a row of q
-        const bool active = r < rows_total;
-        const float* src = q + (size_t)(tok0 + (active ? r / g : 0)) * q_stride +
-                           (hk * g + (active ? r % g : 0)) * d;
-        for (int i = lane; i < d; i += 32) Qs[warp * d + i] = active ? src[i] : 0.0f;
     }
     // scores: key `key` with rows srow .. srow + RPT - 1
     const int key = threadIdx.x % KEYS, srow = threadIdx.x / KEYS * RPT;
-    int row_lo[RPT], row_hi[RPT];
-#pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-        const int r = it.row0 + srow + i, pos = pos0 + (r < rows_total ? r / g : 0);
-        row_lo[i] = it.kv_begin;
-        if (window > 0) row_lo[i] = max(row_lo[i], pos - window + 1);
-        row_hi[i] = r < rows_total ? min(it.kv_end, pos + 1) : 0;
-    }
     float m = -INFINITY, l = 0.0f;                   // of row `warp`
     // weighted sums: rows arow, arow + 1, features f .. f + VW - 1
     const int arow = 2 * (warp & 3), f = (warp >> 2) * 32 * VW + VW * lane;
@@ -518,7 +612,9 @@ attn_simt_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
 #pragma unroll
     for (int e = 0; e < VW; ++e) acc[0][e] = acc[1][e] = 0.0f;
 
+#pragma unroll 1
     for (int kt = k_lo; kt < k_hi; kt += KEYS) {
+        const bool more = kt + KEYS < k_hi;
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();                             // the keys have landed
         {
@@ -540,45 +636,36 @@ attn_simt_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
                 }
             }
             const int kpos = kt + key;
-            const bool held = hide[key] == 0.0f;
+            const bool held = hide[key] == 0.0f && kpos < it.kv_end;
 #pragma unroll
-            for (int i = 0; i < RPT; ++i)
-                Ps[(srow + i) * KEYS + key] =
-                    kpos >= row_lo[i] && kpos < row_hi[i] && held ? s[i] * scale : -INFINITY;
+            for (int i = 0; i < RPT; ++i) {
+                const int r = row0 + srow + i, pos = pos0 + r / g;
+                const bool valid = held && r < rows_total && kpos >= it.kv_begin && kpos <= pos &&
+                                   (window <= 0 || kpos > pos - window);
+                Ps[(srow + i) * KEYS + key] = valid ? s[i] * scale : -INFINITY;
+            }
         }
         __syncthreads();                             // the scores are written, the keys have been used
-        const bool more = kt + KEYS < k_hi;
-        if (more) {
-            // (the pages of this group are still needed: its values are on their way, not its ids)
-            look_up(kt + KEYS);
-            issue(kt + KEYS, k_pages, Ks, ks, true);
-        } else {
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-        }
+        if (more) copy(kt + KEYS, true);
+        else asm volatile("cp.async.commit_group;\n" ::: "memory");
         {
-            float sc[NT], top[NT];
+            float sc[NT], top[NT], corr[NT];
 #pragma unroll
             for (int t = 0; t < NT; ++t) sc[t] = Ps[warp * KEYS + t * TILE + lane];
 #pragma unroll
             for (int t = 0; t < NT; ++t) top[t] = warp_max(sc[t]);
-            float corr[NT], sum[NT];
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 const float m_new = fmaxf(m, top[t]);
-                corr[t] = 1.0f;
-                if (m_new == -INFINITY) {            // nothing of this tile is visible to the row
-                    sc[t] = 0.0f;
-                    continue;
-                }
-                sc[t] = sc[t] == -INFINITY ? 0.0f : expf(sc[t] - m_new);
-                corr[t] = expf(m - m_new);           // 0 when m was -inf
+                // (nothing of this tile is visible to the row, nor of those before: all weights are 0)
+                const float use = m_new == -INFINITY ? 0.0f : m_new;
+                corr[t] = m_new == -INFINITY ? 1.0f : expf(m - use);     // 0 when m was -inf
+                sc[t] = sc[t] == -INFINITY ? 0.0f : expf(sc[t] - use);
                 m = m_new;
             }
 #pragma unroll
-            for (int t = 0; t < NT; ++t) sum[t] = warp_sum(sc[t]);
-#pragma unroll
             for (int t = 0; t < NT; ++t) {
-                l = l * corr[t] + sum[t];
+                l = l * corr[t] + warp_sum(sc[t]);
                 Ps[warp * KEYS + t * TILE + lane] = sc[t];
                 if (lane == 0) corr_s[warp * NT + t] = corr[t];
             }
@@ -586,49 +673,42 @@ attn_simt_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();                             // the weights are written, the values have landed
         if (f < d) {
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                if (kt + t * TILE >= k_hi) break;
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const float c = corr_s[(arow + i) * NT + t];
-#pragma unroll
-                    for (int e = 0; e < VW; ++e) acc[i][e] *= c;
-                }
-#pragma unroll 2
-                for (int k0 = t * TILE; k0 < (t + 1) * TILE; k0 += 4) {
-                    float p[2][4], v[4][VW];
+#pragma unroll 1
+            for (int k0 = 0; k0 < KEYS && kt + k0 < k_hi; k0 += 4) {
+                if (k0 % TILE == 0) {
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
-                        *reinterpret_cast<float4*>(p[i]) =
-                            *reinterpret_cast<const float4*>(Ps + (arow + i) * KEYS + k0);
 #pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        const float* vr = Vs + (k0 + x) * d + f;
-                        if (VW == 4) *reinterpret_cast<float4*>(v[x]) = *reinterpret_cast<const float4*>(vr);
-                        else if (VW == 2) *reinterpret_cast<float2*>(v[x]) = *reinterpret_cast<const float2*>(vr);
-                        else v[x][0] = vr[0];
-                    }
-#pragma unroll
-                    for (int x = 0; x < 4; ++x)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            if (p[i][x] != 0.0f)     // (keys of weight 0 add nothing, whatever their values)
-#pragma unroll
-                                for (int e = 0; e < VW; ++e)
-                                    acc[i][e] = fmaf(p[i][x], v[x][e], acc[i][e]);
+                        for (int e = 0; e < VW; ++e) acc[i][e] *= corr_s[(arow + i) * NT + k0 / TILE];
                 }
+                const float4 p0 = *reinterpret_cast<const float4*>(Ps + arow * KEYS + k0);
+                const float4 p1 = *reinterpret_cast<const float4*>(Ps + (arow + 1) * KEYS + k0);
+                const float p[2][4] = {{p0.x, p0.y, p0.z, p0.w}, {p1.x, p1.y, p1.z, p1.w}};
+                float v[4][VW];
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int e = 0; e < VW; ++e) v[x][e] = Vs[(k0 + x) * d + f + e];
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int e = 0; e < VW; ++e) {
+                            // (keys of weight 0 add nothing, whatever their values)
+                            const float with = fmaf(p[i][x], v[x][e], acc[i][e]);
+                            acc[i][e] = p[i][x] != 0.0f ? with : acc[i][e];
+                        }
             }
         }
         __syncthreads();                             // the values have been used
-        if (more) issue(kt + KEYS, v_pages, Vs, d, false);
+        if (more) copy(kt + KEYS, false);
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     pdl_trigger();
     if (lane == 0) {
         l_s[warp] = l;
-        const int r = it.row0 + warp;
-        if (it.partial >= 0 && r < rows_total) {
+        if (it.partial >= 0 && row0 + warp < rows_total) {
             const size_t idx = ((size_t)it.partial * kv_heads + hk) * ROWS + warp;
             partial_ml[idx * 2] = m;
             partial_ml[idx * 2 + 1] = l;
@@ -637,19 +717,33 @@ attn_simt_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const int r = it.row0 + arow + i;
+        const int r = row0 + arow + i;
         if (r >= rows_total || f >= d) continue;
+        float factor = 1.0f;
+        float* o = partial_acc + (((size_t)max(it.partial, 0) * kv_heads + hk) * ROWS + arow + i) * d + f;
         if (it.partial < 0) {
-            const float sum = l_s[arow + i], factor = sum > 0.0f ? 1.0f / sum : 0.0f;
-            float* o = out + (size_t)(tok0 + r / g) * out_stride + (hk * g + r % g) * d + f;
-#pragma unroll
-            for (int e = 0; e < VW; ++e) o[e] = acc[i][e] * factor;
-        } else {
-            float* o = partial_acc + (((size_t)it.partial * kv_heads + hk) * ROWS + arow + i) * d + f;
-#pragma unroll
-            for (int e = 0; e < VW; ++e) o[e] = acc[i][e];
+            factor = l_s[arow + i] > 0.0f ? 1.0f / l_s[arow + i] : 0.0f;
+            o = out + (size_t)(tok0 + r / g) * out_stride + (hk * g + r % g) * d + f;
         }
+#pragma unroll
+        for (int e = 0; e < VW; ++e) o[e] = it.partial < 0 ? acc[i][e] * factor : acc[i][e];
     }
+    if (!fuse.on || it.partial < 0) return;
+    // the block that finishes the tile last merges its live partial results
+    __shared__ int last_s;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int* counter = fuse.counters + (size_t)it.seq * kv_heads + hk;
+        last_s = atomicAdd(counter, 1) == it.pad1 - 1;
+        if (last_s) *counter = 0;
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    if (warp < rows_total)
+        merge_row<float, 2 * VW>(out + (size_t)tok0 * out_stride + (hk * g + warp) * d, partial_acc,
+                                 partial_ml, it.pad0, it.pad1, kv_heads, hk, ROWS, warp, d);
 }
 
 // Merge the chunks of each row, in ascending order of the chunks.
@@ -668,44 +762,13 @@ attn_combine_kernel(T* __restrict__ out, int out_stride, const int* __restrict__
     const int hk = blockIdx.y;
     const int g = heads / kv_heads;
     const int rows_total = seq_qlen[it.seq] * g;
-    const int lane = threadIdx.x & 31;
     // a warp a row, the rows of a tile over blockIdx.z
     for (int w = blockIdx.z * ROWS + (threadIdx.x >> 5); w < rows_per_tile; w += ROWS * gridDim.z) {
         const int r = it.row0 + w;
         if (r >= rows_total) continue;
         const int t = r / g, hq = hk * g + r % g;
-        float m = -INFINITY;
-        for (int c = 0; c < it.num_partials; ++c) {
-            const size_t idx = ((size_t)(it.first_partial + c) * kv_heads + hk) * rows_per_tile + w;
-            m = fmaxf(m, partial_ml[idx * 2]);
-        }
-        float l = 0.0f;
-        float acc[MAX_D / 32];
-#pragma unroll
-        for (int i = 0; i < MAX_D / 32; ++i) acc[i] = 0.0f;
-        // (everything is loaded without a branch on what was loaded before it)
-#pragma unroll 4
-        for (int c = 0; c < it.num_partials; ++c) {
-            const size_t idx = ((size_t)(it.first_partial + c) * kv_heads + hk) * rows_per_tile + w;
-            const float mc = partial_ml[idx * 2], lc = partial_ml[idx * 2 + 1];
-            const bool any = mc != -INFINITY;         // else the chunk held no visible key
-            const float f = any ? expf(mc - m) : 0.0f;
-            if (any) l += lc * f;
-            const float* pa = partial_acc + idx * d;
-#pragma unroll
-            for (int i = 0; i < MAX_D / 32; ++i) {
-                const int dd = lane + 32 * i;
-                const float v = dd < d ? pa[dd] : 0.0f;
-                if (any) acc[i] = fmaf(v, f, acc[i]);
-            }
-        }
-        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-        T* o = out + (size_t)(seq_qstart[it.seq] + t) * out_stride + hq * d;
-#pragma unroll
-        for (int i = 0; i < MAX_D / 32; ++i) {
-            const int dd = lane + 32 * i;
-            if (dd < d) o[dd] = from_float<T>(acc[i] * inv);
-        }
+        merge_row<T, MAX_D / 32>(out + (size_t)(seq_qstart[it.seq] + t) * out_stride + hq * d, partial_acc,
+                     partial_ml, it.first_partial, it.num_partials, kv_heads, hk, rows_per_tile, w, d);
     }
 }
 
@@ -719,7 +782,8 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
                        const int* seq_qstart, const int* seq_qlen, const int* seq_pos0,
                        const int* items, int num_items, float* partial_acc, float* partial_ml,
                        int partial_limit, int heads, int kv_heads, int d, int page, float scale,
-                       int window, int* status, void* stream, int tile_rows = ROWS);
+                       int window, int* status, void* stream, int tile_rows = ROWS,
+                       Fuse fuse = Fuse{0, nullptr, 0, 0, nullptr});
 static int launch_combine(int dtype, void* out, int out_stride, const int* seq_qstart,
                           const int* seq_qlen, const int* items, int num_items,
                           const float* partial_acc, const float* partial_ml, int partial_limit,
@@ -746,7 +810,7 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
                        const int* seq_qstart, const int* seq_qlen, const int* seq_pos0,
                        const int* items, int num_items, float* partial_acc, float* partial_ml,
                        int partial_limit, int heads, int kv_heads, int d, int page, float scale,
-                       int window, int* status, void* stream, int tile_rows) {
+                       int window, int* status, void* stream, int tile_rows, Fuse fuse) {
     if (num_items <= 0) return 0;
     if (d <= 0 || d > MAX_D || heads % kv_heads != 0) return -2;
     cudaStream_t s = (cudaStream_t)stream;
@@ -776,7 +840,7 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
     do {                                                                                        \
         auto kernel = attn_simt_rows_kernel<VW, KEYS>;                                          \
         const size_t need = (size_t)(KEYS * (2 * d + 4) + ROWS * d + ROWS * KEYS + KEYS +       \
-                                     ROWS * (KEYS / TILE) + ROWS) * sizeof(float);              \
+                                     ROWS * (KEYS / TILE) + ROWS + d) * sizeof(float);          \
         if (need > 48 * 1024) {                                                                 \
             const cudaError_t e = cudaFuncSetAttribute(                                         \
                 kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);                \
@@ -787,7 +851,7 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
                          (const float*)k_pages, (const float*)v_pages, block_table,             \
                          table_stride, num_pages, seq_slot, seq_qstart, seq_qlen, seq_pos0,     \
                          (const WorkItem*)items, partial_acc, partial_ml, partial_limit, heads, \
-                         kv_heads, d, page, scale, window, aligned, status);                    \
+                         kv_heads, d, page, scale, window, aligned, fuse, status);              \
     } while (0)
             if (d <= 64) LAUNCH_ROWS(1, 128);
             if (d <= 128) LAUNCH_ROWS(2, 64);
@@ -822,6 +886,24 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
 
 // `rows_per_tile`: rows of a tile in the partial layout (8 for the kernel above; the tensor-core
 // kernel writes the same layout with its own tile height).
+// A step of single tokens in float32 in one launch: qkv rows [q heads | k heads | v heads] as the product
+// left them (`Fuse`); `items` as de_attn_simt takes them for tiles of 8 rows, up to 8 query heads a kv
+// head; `counters`: int32 [tiles * kv_heads], zero before and after.
+DE_EXPORT int de_attn_simt_decode(const void* qkv, int qkv_stride, void* out, int out_stride,
+                                  void* k_pages, void* v_pages, const int* block_table,
+                                  int table_stride, int num_pages, const int* seq_slot,
+                                  const int* seq_qstart, const int* seq_qlen, const int* seq_pos0,
+                                  const int* items, int num_items, float* partial_acc,
+                                  float* partial_ml, int* counters, const float* inv_freq, int rot,
+                                  int writes, int heads, int kv_heads, int d, int page, float scale,
+                                  int window, int* status, void* stream) {
+    if (d % 4 != 0 || kv_heads <= 0 || heads > ROWS * kv_heads || rot < 0 || rot % 2 || rot > d) return -2;
+    return launch_simt(DE_F32, qkv, qkv_stride, out, out_stride, k_pages, v_pages, block_table,
+                       table_stride, num_pages, seq_slot, seq_qstart, seq_qlen, seq_pos0, items,
+                       num_items, partial_acc, partial_ml, 0x7fffffff, heads, kv_heads, d, page,
+                       scale, window, status, stream, ROWS, Fuse{1, inv_freq, rot, writes, counters});
+}
+
 DE_EXPORT int de_attn_combine(int dtype, void* out, int out_stride, const int* seq_qstart,
                               const int* seq_qlen, const int* items, int num_items,
                               const float* partial_acc, const float* partial_ml, int heads,

@@ -102,6 +102,10 @@ class AttentionLauncher:
         # DISTENGINE_B200_DECODE_ATTENTION=split keeps them apart
         self.fused_decode = (self.tensor_cores and not exact_weights and os.environ.get(
             "DISTENGINE_B200_DECODE_ATTENTION", "fused") != "split")
+        # the same in float32: the kernel for tiles of 8 rows, whose last block of a tile merges
+        self.fused_rows = (dtype == torch.float32 and head_dim % 4 == 0 and self.group <= 8
+                           and os.environ.get("DISTENGINE_B200_DECODE_ATTENTION",
+                                              "fused") != "split")
         self._decode_blocks_per_sm: "int | None" = None     # asked of the kernel at first use
         self._device = device
         self._sm_count: "int | None" = None                 # asked of the device at first use
@@ -214,7 +218,9 @@ class AttentionLauncher:
         if self.fused_decode and one_each and force_shape is None and allow_decode:
             self._prepare_decode(prep, force_split)
             return
-        prep.notes[self.key + "/decode"] = None
+        prep.notes[self.key + "/decode"] = (
+            (len(host.seq_qlen),) if self.fused_rows and one_each and force_shape is None
+            and allow_decode else None)
         notes = {}
         parts = self._split(host.seq_qlen)
         if self.shapes[0].name == "rows32" and self._few_blocks(host, prep.graph_shape):
@@ -256,6 +262,11 @@ class AttentionLauncher:
                                      sm_count=self.sm_count())
             plan = build_plan(qlen, host.seq_pos0, self.group, self.kv_heads, shape.rows,
                               self.window, chunk, chunks_cap)
+            if prep.notes[self.key + "/decode"] is not None:
+                # (a tile a sequence: the items carry the token's position and slot instead of their
+                # rows and their tile)
+                seq = plan.items[:, 0]
+                plan.items[:, 1], plan.items[:, 7] = host.seq_pos0[seq], host.seq_slot[seq]
             prep.add(f"{self.key}/{shape.name}/items", plan.items)
             prep.add(f"{self.key}/{shape.name}/combine", plan.combine)
             notes[shape.name] = plan.num_partials
@@ -320,6 +331,9 @@ class AttentionLauncher:
               and v_pages.shape == k_pages.shape,
               "decode attention: pages must be [pages, kv_heads, page, head_dim]")
         _i32(block_table, "block_table")
+        if self.fused_rows:
+            self._run_rows(qkv, out, k_pages, v_pages, block_table, inv_freq, rotary_dim, writes, ctx)
+            return
         items = ctx.arrays[f"{self.key}/decode/items"]
         for name, t in (("seq_slot", ctx.seq_slot), ("seq_qstart", ctx.seq_qstart),
                         ("seq_pos0", ctx.seq_pos0), ("items", items)):
@@ -346,6 +360,37 @@ class AttentionLauncher:
             counters.data_ptr(), _ptr(inv_freq), int(rotary_dim) if inv_freq is not None else 0,
             1 if writes else 0, self.heads, self.kv_heads, d, k_pages.shape[2],
             float(self.scale), self.window, ctx.status.data_ptr(), _stream()), "decode attention")
+
+
+    def _run_rows(self, qkv, out, k_pages, v_pages, block_table, inv_freq, rotary_dim, writes,
+                  ctx) -> None:
+        """``run_decode`` in float32."""
+        d, items = self.head_dim, ctx.arrays[f"{self.key}/rows8/items"]
+        for name, t in (("seq_slot", ctx.seq_slot), ("seq_qstart", ctx.seq_qstart),
+                        ("seq_qlen", ctx.seq_qlen), ("seq_pos0", ctx.seq_pos0), ("items", items)):
+            _i32(t, name)
+        (tiles,) = ctx.notes[self.key + "/decode"]
+        num_partials = dict(ctx.notes[self.key])["rows8"]
+        acc = ml = None
+        if num_partials:
+            rows = num_partials * self.kv_heads * 8
+            acc = ctx.buffer("attention.partial_acc.rows8", (rows * d,), torch.float32)
+            ml = ctx.buffer("attention.partial_ml.rows8", (rows * 2,), torch.float32)
+        counters = ctx.buffer("attention.counters", (max(tiles, 1) * self.kv_heads,), torch.int32,
+                              zero=True)
+        if inv_freq is not None:
+            _need(inv_freq.dtype == torch.float32 and inv_freq.is_contiguous()
+                  and inv_freq.shape[0] * 2 == rotary_dim, "decode attention: inv_freq must be "
+                  "float32 [rotary_dim / 2]")
+        lib = library.load("attention_simt")
+        _check(lib.de_attn_simt_decode(
+            qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), k_pages.data_ptr(),
+            v_pages.data_ptr(), block_table.data_ptr(), block_table.stride(0), k_pages.shape[0],
+            ctx.seq_slot.data_ptr(), ctx.seq_qstart.data_ptr(), ctx.seq_qlen.data_ptr(),
+            ctx.seq_pos0.data_ptr(), items.data_ptr(), items.shape[0], _ptr(acc), _ptr(ml),
+            counters.data_ptr(), _ptr(inv_freq), int(rotary_dim) if inv_freq is not None else 0,
+            1 if writes else 0, self.heads, self.kv_heads, d, k_pages.shape[2], float(self.scale),
+            self.window, ctx.status.data_ptr(), _stream()), "decode attention (float32)")
 
 
 def launch_items(code: int, module, q, out, k_pages, v_pages, block_table, seq_slot, seq_qstart,

@@ -44,6 +44,8 @@ SIGNATURES: dict[str, dict[str, list]] = {
         "de_gemm_f32_form": [I, I, I, I],
     },
     "attention_simt": {
+        "de_attn_simt_decode": [P, I, P, I, P, P, P, I, I, P, P, P, P, P, I, P, P, P, P, I, I, I, I, I,
+                                I, F, I, P, P],
         "de_attn_simt_rows_per_tile": [],
         "de_attn_simt": [I, P, I, P, I, P, P, P, I, I, P, P, P, P, P, I, P, P, I, I, I, I, F, I, I,
                          P, P],
