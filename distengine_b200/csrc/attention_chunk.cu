@@ -630,6 +630,186 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ proj, int ld, T* __rest
     }
 }
 
+// The same for steps with portions, heads of D = 64 or 128 features (keys and values alike), norm over a
+// head or none, values as they are: runs of RUN tokens, a lane four neighbouring channels of a head
+// (32 or 16 lanes a head), which hold their taps, bias and weights for the run, read every row of
+// proj once and keep the last K - 1 inputs in registers; a head's squares and the partners of a turn
+// go from lane to lane.  The sums are those of the kernel above, bit for bit.  grid (runs, heads in
+// blocks of 8 warps).  Bound by instructions and the latency of a token after the other (some 200 a head
+// and token; the kernel above reads taps and bias, 48 KB, for every token).  Prompts of 1,201 and 1,172
+// tokens of 16 + 4 + 4 heads of 128 with three taps 31 us against 45; runs of 8 tokens 29, of 16 27,
+// but portions of 400 17 and 24 instead of 13.
+constexpr int RUN = 4;            // at most 32: a lane a token
+
+template <typename T, int D, int KK>              // KK: taps, 1 for none
+__global__ void __launch_bounds__(256, 3)
+qkv_prepare_runs_kernel(const T* __restrict__ proj, int ld, T* __restrict__ q_out,
+                        const int* __restrict__ positions, const int* __restrict__ token_seq,
+                        const int* __restrict__ token_slot, const int* __restrict__ seq_pos0,
+                        Prepare pp, int H, int G, T* __restrict__ k_pages, T* __restrict__ v_pages,
+                        const int* __restrict__ block_table, int table_stride, int page,
+                        int num_pages, int n_tokens, int* __restrict__ status) {
+    constexpr int LANES = D / 4, PER = 32 / LANES;   // lanes of a head, heads of a warp
+    __shared__ __align__(16) float tab[RUN][D];      // a token's cosines, then its sines
+    const int n0 = blockIdx.x * RUN, count = min(RUN, n_tokens - n0);
+    const int heads = H + (pp.v_from_k ? G : 2 * G), C = heads * D, half = pp.rot / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int h = ((int)blockIdx.y * 8 + warp) * PER + lane / LANES;
+    const int i0 = lane % LANES * 4, c = h * D + i0;
+    const bool live = h < heads, is_q = h < H, is_k = !is_q && h < H + G;
+    const int g = is_q ? 0 : is_k ? h - H : h - H - G;         // kv head
+    // lane i < RUN: token i
+    int pos = 0, off = 0, slot = 0, page_id = -1, in_page = 0;
+    float temp = 1.0f;
+    if (lane < count) {
+        pos = positions[n0 + lane];
+        slot = token_slot[n0 + lane];
+        off = pos - seq_pos0[token_seq[n0 + lane]];
+        page_id = block_table[(size_t)slot * table_stride + pos / page];
+        in_page = pos % page;
+        if (page_id < 0 || page_id >= num_pages) {   // never written outside the pool
+            page_id = -1;
+            if (warp == 0) atomicExch(status, 1);
+        }
+        if (pp.temp_every > 0)
+            temp = 1.0f + pp.temp_coef * logf((float)((pos + 1) / pp.temp_every) + 1.0f);
+    }
+    for (int e = threadIdx.x; e < count * half; e += 256) {
+        const int i = e / half, f = e - i * half;
+        // the angle as in the kernel above
+        const double turns = (double)positions[n0 + i] * ((double)pp.freq[f] * 0.15915494309189535);
+        float sn, cs;
+        sincospif((float)(2.0 * (turns - rint(turns))), &sn, &cs);
+        tab[i][f] = cs * pp.magnitude;
+        tab[i][half + f] = sn * pp.magnitude;
+    }
+    float w[KK][4], b[4] = {0.0f, 0.0f, 0.0f, 0.0f}, wt[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+    const float* weight = pp.norm == 0 ? nullptr : is_q ? pp.q_weight : is_k ? pp.k_weight : nullptr;
+    if (live) {
+        if (pp.bias) load_run<4>(pp.bias + c, pp.by_tap, b);
+        if (KK > 1) {
+#pragma unroll
+            for (int j = 0; j < KK; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    w[j][e] = pp.taps[pp.by_tap ? (size_t)j * C + c + e : (size_t)(c + e) * KK + j];
+        }
+        if (weight)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) wt[e] = weight[i0 + e];
+    }
+    __syncthreads();
+    pdl_wait();
+    auto fetch = [&](int i) {
+        return live && i < count ? load_four(proj + (size_t)(n0 + i) * ld + c)
+                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    auto take = [&](float (&to)[4], const float4& v) {           // an input, with its bias
+        to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
+        if (pp.bias)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) to[e] += b[e];
+    };
+    float4 in = fetch(0), in_next = fetch(1);        // two tokens ahead
+    float x[KK][4];                                  // the token's input last
+#pragma unroll 1
+    for (int i = 0; i < count; ++i) {
+        const float4 now = in;
+        in = in_next;
+        in_next = fetch(i + 2);
+        const int n = n0 + i, tpos = __shfl_sync(0xffffffffu, pos, i);
+        const int toff = __shfl_sync(0xffffffffu, off, i), id = __shfl_sync(0xffffffffu, page_id, i);
+        const int row = __shfl_sync(0xffffffffu, in_page, i);
+        const float mul = __shfl_sync(0xffffffffu, temp, i);
+        if (KK > 1 && (i == 0 || toff == 0)) {
+            // the inputs before this token: of its portion, or what the slot keeps
+            const int tslot = __shfl_sync(0xffffffffu, slot, i);
+            const float* kept = pp.state + (size_t)tslot * pp.slot_stride + pp.conv_offset;
+#pragma unroll
+            for (int j = 0; j + 1 < KK; ++j) {
+                const int rel = toff - (KK - 1) + j;
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (live && rel >= 0) {
+                    v = load_four(proj + (size_t)(n - (KK - 1) + j) * ld + c);
+                } else if (live && tpos - (KK - 1) + j >= 0) {
+                    const float* k = kept + (size_t)(toff + j) * C + c;
+                    v = make_float4(k[0], k[1], k[2], k[3]);
+                }
+                take(x[j], v);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j + 1 < KK; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[j][e] = x[j + 1][e];
+        }
+        take(x[KK - 1], now);
+        float y[4];
+        if (KK == 1) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] = x[0][e];
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] = 0.0f;
+#pragma unroll
+            for (int j = 0; j < KK; ++j) {
+                if (tpos - (KK - 1) + j < 0) continue;           // before the sequence's start
+#pragma unroll
+                for (int e = 0; e < 4; ++e) y[e] = fmaf(w[j][e], x[j][e], y[e]);
+            }
+        }
+        const size_t at = ((size_t)max(id, 0) * G + g) * page + (size_t)row;
+        const float4 plain = make_float4(y[0], y[1], y[2], y[3]);
+        const bool has_v = live && id >= 0 && (pp.v_from_k ? is_k : !is_q && !is_k);
+        if (has_v)
+            store_four(v_pages + at * D + i0, plain);
+        float4 v = plain;
+        if (pp.norm == 1) {
+            float ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, 0.0f))));
+#pragma unroll
+            for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            const float inv = 1.0f / sqrtf(ss / (float)D + pp.eps);
+            v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+            if (weight) { v.x *= wt[0]; v.y *= wt[1]; v.z *= wt[2]; v.w *= wt[3]; }
+        }
+        if (!pp.adjacent && half > 0) {              // partners half a turned part apart
+            const bool first = i0 < half;
+            const int from = i0 < pp.rot ? lane + (first ? half / 4 : -(half / 4)) : lane;
+            const float4 o = make_float4(
+                __shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from),
+                __shfl_sync(0xffffffffu, v.z, from), __shfl_sync(0xffffffffu, v.w, from));
+            if (i0 < pp.rot) {
+                const int p = first ? i0 : i0 - half;
+                const float4 cs = *reinterpret_cast<const float4*>(&tab[i][p]);
+                const float4 sn = *reinterpret_cast<const float4*>(&tab[i][half + p]);
+                float other;
+                if (first) {
+                    rope_rotate(v.x, o.x, cs.x, sn.x, v.x, other);
+                    rope_rotate(v.y, o.y, cs.y, sn.y, v.y, other);
+                    rope_rotate(v.z, o.z, cs.z, sn.z, v.z, other);
+                    rope_rotate(v.w, o.w, cs.w, sn.w, v.w, other);
+                } else {
+                    rope_rotate(o.x, v.x, cs.x, sn.x, other, v.x);
+                    rope_rotate(o.y, v.y, cs.y, sn.y, other, v.y);
+                    rope_rotate(o.z, v.z, cs.z, sn.z, other, v.z);
+                    rope_rotate(o.w, v.w, cs.w, sn.w, other, v.w);
+                }
+            }
+        } else if (i0 < pp.rot) {
+            const float* cs = &tab[i][i0 / 2];
+            rope_rotate(v.x, v.y, cs[0], cs[half], v.x, v.y);
+            rope_rotate(v.z, v.w, cs[1], cs[half + 1], v.z, v.w);
+        }
+        if (live && is_q) {
+            v.x *= mul; v.y *= mul; v.z *= mul; v.w *= mul;
+            store_four(q_out + (size_t)n * (H * D) + h * D + i0, v);
+        } else if (live && is_k && id >= 0) {
+            store_four(k_pages + at * D + i0, v);
+        }
+    }
+    pdl_trigger();
+}
+
 // After qkv_prepare: every sequence's slot keeps the last K - 1 rows of the first C columns of
 // proj (the convolution's inputs of the next step), kept[i] = the row at position
 // pos0 + qlen - (K - 1) + i; a portion shorter than K - 1 moves the older rows up.  The layout is
@@ -2591,6 +2771,37 @@ DE_EXPORT int de_qkv_prepare(int dtype, const void* proj, int ld, void* q_out,
                         v_first, keep_here, v_from_k};
     cudaStream_t s = (cudaStream_t)stream;
     const int C = (H + G) * dk + (v_from_k ? 0 : G * dv);
+    const size_t four = dtype == DE_BF16 ? 8 : 16;   // bytes of a group of four
+    // (us a call, a token a block and in runs, 16 + 4 + 4 heads of 128, bfloat16: with three taps 128
+    // tokens 13.3 and 12.2, 400 19.5 and 13.3, 1,000 25.6 and 20.4; without taps 400 16.4 and 12.3, 700
+    // 13.3 and 16.4 - one round of blocks of 256 threads against two - 1,000 18.6 and 16.4)
+    if (n >= 128 && (taps != nullptr || n < 512 || n >= 800) && dk == dv && (dk == 64 || dk == 128) && norm != 2 && mix == 0 && !keep_here &&
+        (taps == nullptr || (K >= 2 && K <= 4)) && rot % (adjacent ? 4 : 8) == 0 && ld % 4 == 0 &&
+        (uintptr_t)proj % four == 0 && (uintptr_t)q_out % four == 0 &&
+        (uintptr_t)k_pages % four == 0 && (uintptr_t)v_pages % four == 0) {
+        const int heads = C / dk, per_block = dk == 64 ? 16 : 8;
+        const dim3 grid((n + RUN - 1) / RUN, (heads + per_block - 1) / per_block);
+#define PREP_RUNS(T, D, KK)                                                                     \
+    return de_launch(qkv_prepare_runs_kernel<T, D, KK>, grid, dim3(256), 0, s, (const T*)proj,  \
+                     ld, (T*)q_out, positions, token_seq, token_slot, seq_pos0, pp, H, G,       \
+                     (T*)k_pages, (T*)v_pages, block_table, table_stride, page, num_pages, n,   \
+                     status)
+#define PREP_RUNS_K(T, D)                                                                       \
+    do {                                                                                        \
+        if (taps == nullptr) PREP_RUNS(T, D, 1);                                                \
+        if (K == 2) PREP_RUNS(T, D, 2);                                                         \
+        if (K == 3) PREP_RUNS(T, D, 3);                                                         \
+        PREP_RUNS(T, D, 4);                                                                     \
+    } while (0)
+        if (dtype == DE_BF16) {
+            if (dk == 64) PREP_RUNS_K(__nv_bfloat16, 64);
+            PREP_RUNS_K(__nv_bfloat16, 128);
+        }
+        if (dk == 64) PREP_RUNS_K(float, 64);
+        PREP_RUNS_K(float, 128);
+#undef PREP_RUNS_K
+#undef PREP_RUNS
+    }
     const size_t smem = (size_t)(C + rot + H + G) * sizeof(float);
     if (smem > 200 * 1024) return -2;
     const int threads = C >= 2048 && n < 512 ? 512 : 256;

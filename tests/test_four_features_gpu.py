@@ -99,3 +99,48 @@ def test_finish_of_rows_of_640_features(dtype, H, dv, turned, gate):
         results.append(out.clone())
     assert torch.equal(*results)
 
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D,H,G,rot,adjacent,K,norm,magnitude,temp,from_keys", [
+    (128, 5, 1, 128, True, 3, True, 1.0, None, False), (128, 3, 3, 128, False, 4, True, 1.25, (0.3, 64), False),
+    (64, 6, 2, 64, False, 2, False, 1.0, None, False), (64, 5, 1, 32, False, 3, True, 1.0, (0.3, 16), True),
+    (128, 16, 4, 24, False, None, True, 1.0, None, False), (64, 1, 1, 12, True, 4, "plain", 1.0, None, False),
+    (128, 4, 2, 0, False, None, False, 1.0, (0.1, 8), True),
+])
+@pytest.mark.parametrize("lens,starts", [((128,), (0,)), ((61, 1, 2, 3, 70), (0, 40, 1, 2, 9)),
+                                         ((801,), (5,))])
+def test_preparation_in_runs_of_tokens(dtype, D, H, G, rot, adjacent, K, norm, magnitude, temp,
+                                             from_keys, lens, starts):
+    """128 tokens and more: against the kernel with a token a block, which rows at other addresses
+    reach.  Portions that begin inside a run, and behind 0 to 3 kept rows."""
+    from distengine_b200.kernels import recurrent as rk
+    page, g = 16, _gen(D + H)
+    slots = tuple(range(len(lens)))
+    ctx = _ctx(lens, starts, slots)
+    n, C = sum(lens), (H + (G if from_keys else 2 * G)) * D
+    need = [(s + l + page - 1) // page for s, l in zip(starts, lens)]
+    table = torch.full((len(lens), max(need)), -1, dtype=torch.int32)
+    order, at = torch.randperm(sum(need), generator=g).int(), 0
+    for i, m in enumerate(need):
+        table[i, :m] = order[at: at + m]
+        at += m
+    proj = torch.randn(n, C, generator=g).to(dtype)
+    bias = torch.randn(C, generator=g).to(DEV) if K else None
+    taps = torch.randn(K, C, generator=g).to(DEV) if K else None
+    state = torch.randn(len(lens), 4 * C, generator=g).to(DEV)
+    weights = [torch.rand(D, generator=g).to(DEV) + 0.5 for _ in range(2)] if norm is True else [None, None]
+    freq = (torch.rand(rot // 2, generator=g) * 2).to(DEV)
+    results = []
+    for pad in (8, 7):
+        q = torch.zeros(n, H * D, dtype=dtype, device=DEV)
+        kp = torch.zeros(sum(need), G, page, D, dtype=dtype, device=DEV)
+        vp = torch.zeros(sum(need), G, page, D, dtype=dtype, device=DEV)
+        rk.qkv_prepare(_rows(proj, pad), q, H, G, D, D, kp, vp, table.to(DEV), ctx, bias=bias, taps=taps,
+                       by_tap=True, kept=(state, 0) if K else None,
+                       norm=("head", *weights, 1e-5) if norm else None,
+                       rotation=(freq, magnitude, adjacent), temperature=temp, values_from_keys=from_keys)
+        results.append((q, kp, vp))
+    assert int(ctx.status.item()) == 0
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
