@@ -152,7 +152,28 @@ def build(module: str, defines: tuple[str, ...] = (), verbose: bool = True) -> s
     return build_many([(module, defines)], verbose)[0]
 
 
+def build_bindings(text: str) -> str:
+    """Compile the generated source ``text`` of ``bindings`` for this interpreter; the path."""
+    from . import bindings
+    folder = _build_dir()
+    path = bindings.library_path(text, folder)
+    if os.path.isfile(path):
+        return path
+    tmp = f"{path}.{os.getpid()}.tmp"
+    with open(tmp + ".cpp", "w") as handle:
+        handle.write(text)
+    done = subprocess.run([find_nvcc(), "-O2", "-std=c++17", "--shared", "-Xcompiler", "-fPIC",
+                           "-cudart", "none", "-I", bindings.include_dir(), tmp + ".cpp", "-o", tmp],
+                          stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    os.remove(tmp + ".cpp")
+    if done.returncode != 0 or not os.path.isfile(tmp):
+        raise BuildError(f"the bindings' source does not compile (exit {done.returncode}):\n"
+                         f"{done.stdout}")
+    os.replace(tmp, path)
+    return path
+
+
 def build_all(verbose: bool = True) -> list[str]:
-    """Every module in its default form (the build check)."""
-    from .library import default_build_requests
-    return build_many(default_build_requests(), verbose)
+    """Every module in its default form, and the bindings (the build check)."""
+    from .library import bindings_source, default_build_requests
+    return build_many(default_build_requests(), verbose) + [build_bindings(bindings_source())]

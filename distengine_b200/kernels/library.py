@@ -1,4 +1,4 @@
-"""Loads the compiled kernel libraries and declares their C signatures.
+"""Loads the compiled kernel libraries and declares their C signatures (``bindings`` calls them).
 
 There is no fallback: if a library cannot be compiled or loaded, or no CUDA device is present, the
 first kernel call raises ``KernelsUnavailable`` with the reason.
@@ -10,6 +10,7 @@ import ctypes
 import os
 from ctypes import c_float, c_int, c_void_p
 
+from . import bindings as _bindings
 from . import build as _build
 
 
@@ -158,7 +159,7 @@ SIGNATURES: dict[str, dict[str, list]] = {
     },
 }
 
-_loaded: dict[tuple[str, tuple[str, ...]], ctypes.CDLL] = {}
+_loaded: dict[tuple[str, tuple[str, ...]], "Library"] = {}
 
 # percent of an SM's memory that the decode step's kernels ask for as shared memory (-1: each
 # kernel's default)
@@ -180,22 +181,55 @@ def default_build_requests() -> list[tuple[str, tuple[str, ...]]]:
             + [("attention_decode", (f"HEAD_DIM={d}",)) for d in (16, 64, 128)])
 
 
-def load(module: str, defines: tuple[str, ...] = ()) -> ctypes.CDLL:
+_LETTERS = {P: "P", I: "I", F: "F", L: "L"}
+
+
+def _letters(argtypes: list) -> str:
+    return "".join(_LETTERS[t] for t in argtypes)
+
+
+def _all_letters() -> list[str]:
+    return sorted({_letters(args) for functions in SIGNATURES.values()
+                   for args in functions.values()})
+
+
+def bindings_source() -> str:
+    return _bindings.source(_all_letters())
+
+
+_bind = None
+
+
+class Library:
+    """A kernel library: the functions of ``SIGNATURES`` as ``bindings`` calls them; anything else
+    that it exports through ctypes."""
+
+    def __init__(self, cdll: ctypes.CDLL, functions: dict[str, list]) -> None:
+        global _bind
+        letters = _all_letters()
+        if _bind is None:
+            _bind = _bindings.load(_build.build_bindings(bindings_source())).bind
+        self._cdll = cdll
+        for name, argtypes in functions.items():
+            address = ctypes.cast(getattr(cdll, name), c_void_p).value
+            setattr(self, name, _bind(letters.index(_letters(argtypes)), address))
+
+    def __getattr__(self, name: str):
+        return getattr(self._cdll, name)
+
+
+def load(module: str, defines: tuple[str, ...] = ()) -> Library:
     key = (module, defines)
     lib = _loaded.get(key)
     if lib is not None:
         return lib
     try:
         path = _build.build(module, defines)
-        lib = ctypes.CDLL(path)
-    except (_build.BuildError, OSError) as error:
+        lib = Library(ctypes.CDLL(path), SIGNATURES[module])
+    except (_build.BuildError, OSError, ImportError) as error:
         raise KernelsUnavailable(
             f"the CUDA kernel library '{module}' of distengine_b200 could not be built or "
             f"loaded: {error}") from error
-    for name, argtypes in SIGNATURES[module].items():
-        fn = getattr(lib, name)
-        fn.argtypes = argtypes
-        fn.restype = c_int
     # programmatic dependent launch (a kernel may start while the one before it finishes) is on
     # unless DISTENGINE_B200_PDL=0
     lib.de_set_pdl.argtypes = [c_int]
