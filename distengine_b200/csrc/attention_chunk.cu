@@ -814,7 +814,8 @@ qkv_prepare_runs_kernel(const T* __restrict__ proj, int ld, T* __restrict__ q_ou
 // proj (the convolution's inputs of the next step), kept[i] = the row at position
 // pos0 + qlen - (K - 1) + i; a portion shorter than K - 1 moves the older rows up.  The layout is
 // the one that the state mixers' convolution keeps (recurrent.cu); a model whose only
-// convolution is this mixer's needs no other library for it.  One block a sequence.
+// convolution is this mixer's needs no other library for it.  grid (sequences, channels / 256): a
+// thread a channel, 2.9 us for two sequences of 3,072 channels (6.5 with a block a sequence).
 template <typename T>
 __global__ void conv_keep_kernel(const T* __restrict__ proj, int ld, float* __restrict__ state,
                                  long long slot_stride, int conv_offset,
@@ -826,7 +827,7 @@ __global__ void conv_keep_kernel(const T* __restrict__ proj, int ld, float* __re
     pdl_wait();
     pdl_trigger();
     float* kept = state + (size_t)seq_slot[s] * slot_stride + conv_offset;
-    for (int c = threadIdx.x; c < C; c += blockDim.x)
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x)
         for (int i = 0; i < K - 1; ++i) {            // ascending: what is read lies ahead
             const int rel = qlen - (K - 1) + i;
             kept[(size_t)i * C + c] = rel >= 0 ? to_float(proj[(size_t)(tok0 + rel) * ld + c])
@@ -2841,11 +2842,12 @@ DE_EXPORT int de_conv_keep(int dtype, const void* proj, int ld, float* state, lo
                            const int* seq_qlen, int n_seqs, int C, int K, void* stream) {
     if (n_seqs <= 0 || K <= 1) return 0;
     cudaStream_t s = (cudaStream_t)stream;
+    const dim3 grid(n_seqs, (C + 255) / 256);
     if (dtype == DE_BF16)
-        return de_launch(conv_keep_kernel<__nv_bfloat16>, dim3(n_seqs), dim3(256), 0, s,
+        return de_launch(conv_keep_kernel<__nv_bfloat16>, grid, dim3(256), 0, s,
                          (const __nv_bfloat16*)proj, ld, state, slot_stride, conv_offset, seq_slot,
                          seq_qstart, seq_qlen, C, K);
-    return de_launch(conv_keep_kernel<float>, dim3(n_seqs), dim3(256), 0, s, (const float*)proj,
+    return de_launch(conv_keep_kernel<float>, grid, dim3(256), 0, s, (const float*)proj,
                      ld, state, slot_stride, conv_offset, seq_slot, seq_qstart, seq_qlen, C, K);
 }
 
