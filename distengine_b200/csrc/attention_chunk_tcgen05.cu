@@ -175,7 +175,8 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
                           const int* __restrict__ seq_qlen, const int* __restrict__ seq_pos0,
                           const WorkItem* __restrict__ items, const float* __restrict__ r1,
                           const float* __restrict__ r2, int heads, int kv_heads, int page, int box,
-                          float scale, Sight sight, int out_f32, int* __restrict__ status) {
+                          float scale, Sight sight, const float* __restrict__ fv, int out_f32,
+                          int* __restrict__ status) {
     using U = Umma<D>;
     constexpr int KS = U::KS, STAGES = U::STAGES, HD = D / 2;   // HD: output features of a thread
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -357,6 +358,9 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
                                      : 1.0f;
     const unsigned lanes = (unsigned)((warp & 3) * 32) << 16;
     float M = -INFINITY, top = -INFINITY, l = 0.0f;
+    // a thread's features: two runs, D / 2 apart, so that it holds both features of a turned pair
+    constexpr int RUN = HD / 2;
+    auto feature = [&](int i) { return (i < RUN ? 0 : D / 2 - RUN) + RUN * half + i; };
     Two acc[HD / 2];
 #pragma unroll
     for (int i = 0; i < HD / 2; ++i) acc[i] = 0ull;
@@ -493,14 +497,16 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
         after_sync();
         if (warp == FETCHER && fetched < n_tiles && __all_sync(0xffffffffu, ok)) fetch(fetched++);
 #pragma unroll
-        for (int c = 0; c < HD; c += 32) {
-            unsigned o[32];
-            tmem_load_32cols(tmem + lanes + O_COL + HD * half + c, o);
+        for (int run = 0; run < 2; ++run) {          // (see feature)
+            unsigned o[RUN];
+            if constexpr (RUN == 32) tmem_load_32cols(tmem + lanes + O_COL + feature(run * RUN), o);
+            else tmem_load_16cols(tmem + lanes + O_COL + feature(run * RUN), o);
             tmem_wait_loads();
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                acc[c / 2 + i] = fma_two(acc[c / 2 + i], two(corr, corr),
-                                         two(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1])));
+            for (int i = 0; i < RUN / 2; ++i)
+                acc[run * RUN / 2 + i] =
+                    fma_two(acc[run * RUN / 2 + i], two(corr, corr),
+                            two(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1])));
         }
         before_sync();
     }
@@ -509,6 +515,18 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
             mbar_wait(&kv_full[t % STAGES], (t / STAGES) & 1, status);
     pdl_trigger();
 
+    // back by position: cosines and sines of the block's tokens and this rank's pairs, where q was (all
+    // products with it are over); pair p of token k at p xor k
+    float2* turn_s = reinterpret_cast<float2*>(q_s);           // [128][RUN]
+    if (fv != nullptr) {
+        const int first = it.row0 / g, count = last_row / g - first + 1;
+        for (int e = tid; e < count * RUN; e += UTHREADS) {
+            const int k = e / RUN, p = e % RUN;
+            float sn, cs;
+            sincosf((float)(pos0 + first + k) * fv[RUN * rank + p], &sn, &cs);
+            turn_s[k * RUN + (p ^ (k & (RUN - 1)))] = make_float2(cs, -sn);
+        }
+    }
     share_s[half * UROWS + rowi] = l;
     asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (warp & 3)) : "memory");
     // (the same sum in both halves)
@@ -552,7 +570,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
                             fmaf(sight.sink[hq], LOG2E, M == -INFINITY ? 0.0f : -M)));
     const float inv = l > 0.0f ? sight.out_scale / l : 0.0f;
     const size_t token = (size_t)(tok0 + tok);
-    const size_t o = token * out_stride + hq * D + HD * half;
+    const size_t o = token * out_stride + hq * D;
     const bool pieces = out_f32 ? out_stride % 4 == 0 && (uintptr_t)out % 16 == 0
                                 : out_stride % 8 == 0 && (uintptr_t)out % 16 == 0;
     const __nv_bfloat16* gate = (const __nv_bfloat16*)sight.gate;
@@ -563,16 +581,32 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
     float zero = 0.0f;
     if (live && ok && half == rank) {
 #pragma unroll
+        for (int i = 0; i < HD / 2; ++i) acc[i] = mul_two(acc[i], two(inv, inv));
+        if (fv != nullptr) {
+            const int k = tok - it.row0 / g;
+            const float2* turn = turn_s + k * RUN;
+#pragma unroll
+            for (int p = 0; p < RUN; p += 2) {
+                float a[2], b[2];
+                untwo(acc[p / 2], a[0], a[1]);
+                untwo(acc[(RUN + p) / 2], b[0], b[1]);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float2 cs = turn[(p + e) ^ (k & (RUN - 1))];
+                    rope_rotate(a[e], b[e], cs.x, cs.y, a[e], b[e]);
+                }
+                acc[p / 2] = two(a[0], a[1]);
+                acc[(RUN + p) / 2] = two(b[0], b[1]);
+            }
+        }
+#pragma unroll
         for (int c = 0; c < HD; c += 8) {
             float x[8];
+            const int at = feature(c);
 #pragma unroll
-            for (int i = 0; i < 8; i += 2) {
-                untwo(acc[(c + i) / 2], x[i], x[i + 1]);
-                x[i] *= inv;
-                x[i + 1] *= inv;
-            }
+            for (int i = 0; i < 8; i += 2) untwo(acc[(c + i) / 2], x[i], x[i + 1]);
             if (per_feature) {
-                const __nv_bfloat16* gp = gate + token * sight.ld_gate + hq * D + HD * half + c;
+                const __nv_bfloat16* gp = gate + token * sight.ld_gate + hq * D + at;
                 float f[8];
                 if (gate_pieces) {
                     load_piece(gp, f);
@@ -589,13 +623,13 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
 #pragma unroll
             for (int i = 0; i < 8; ++i) zero = fmaf(x[i], 0.0f, zero);
             if (pieces && out_f32) {
-                store8((float*)out + o + c, x);
+                store8((float*)out + o + at, x);
             } else if (pieces) {
-                store8((__nv_bfloat16*)out + o + c, x);
+                store8((__nv_bfloat16*)out + o + at, x);
             } else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    store_out<__nv_bfloat16>(out, out_f32, o + c + i, x[i]);
+                    store_out<__nv_bfloat16>(out, out_f32, o + at + i, x[i]);
             }
         }
     }
@@ -620,10 +654,20 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
         const float inv = sight_inverse(sight, h, mr, lr);
         const size_t o = (size_t)(tok0 + tk) * out_stride + h * D;
 #pragma unroll
-        for (int i = 0; i < D / 64; ++i) {                     // this block's half of the features
-            const int col = lane + 32 * i + HD * rank;
-            store_out<__nv_bfloat16>(out, out_f32, o + col, (rank == 0 ? res[i] : res[i + D / 64]) * inv *
-                sight_gate<__nv_bfloat16>(sight, (size_t)(tok0 + tk), h, D, col));
+        for (int i = 0; i < D / 32; ++i) res[i] *= inv;
+#pragma unroll
+        for (int i = 0; i < D / 64; ++i) {                     // pairs (i, i + D / 2)
+            const int col = lane + 32 * i;
+            if (fv != nullptr) {
+                float sn, cs;
+                sincosf((float)(pos0 + tk) * fv[col], &sn, &cs);
+                rope_rotate(res[i], res[i + D / 64], cs, -sn, res[i], res[i + D / 64]);
+            }
+            if (col / RUN != rank) continue;                   // the other block's
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                store_out<__nv_bfloat16>(out, out_f32, o + col + e * (D / 2), res[i + e * (D / 64)] *
+                    sight_gate<__nv_bfloat16>(sight, (size_t)(tok0 + tk), h, D, col + e * (D / 2)));
         }
     }
 }
@@ -633,8 +677,8 @@ int launch(const void* q, int q_stride, void* out, int out_stride, const void* k
            const void* v_pages, const int* block_table, int table_stride, int num_pages,
            const int* seq_slot, const int* seq_qstart, const int* seq_qlen, const int* seq_pos0,
            const int* items, int num_items, const float* r1, const float* r2, int heads, int kv_heads,
-           int page, int box, float scale, const Sight& sight, int out_f32, int* status,
-           cudaStream_t s) {
+           int page, int box, float scale, const Sight& sight, const float* fv, int out_f32,
+           int* status, cudaStream_t s) {
     CUtensorMap map_k, map_v;
     const long long rows = (long long)num_pages * kv_heads * page;
     int code = tensor_maps::get(&map_k, k_pages, rows, D, D, box, 64);
@@ -670,7 +714,7 @@ int launch(const void* q, int q_stride, void* out, int out_stride, const void* k
         &cfg, kernel, (const __nv_bfloat16*)q, q_stride, out, out_stride, map_k, map_v,
         (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_table, table_stride,
         num_pages, seq_slot, seq_qstart, seq_qlen, seq_pos0, (const WorkItem*)items, r1, r2, heads,
-        kv_heads, page, box, scale, sight, out_f32, status));
+        kv_heads, page, box, scale, sight, fv, out_f32, status));
 }
 
 }  // namespace
@@ -682,7 +726,9 @@ DE_EXPORT int de_attn_chunk_tcgen05_ok(int dk, int dv, int page) {
     return dk == dv && (dk == 64 || dk == 128) && page > 0 && page % 8 == 0;
 }
 
-// As de_attn_chunk for bfloat16, with items of 128 rows; keys and values in pages of their own.
+// As de_attn_chunk for bfloat16, with items of 128 rows; keys and values in pages of their own.  fv
+// [dv / 2] or null: every result is turned back by its token's position, pairs (i, i + dv / 2), before the
+// gate (as attn_finish turns them).
 DE_EXPORT int de_attn_chunk_tcgen05(const void* q, int q_stride, void* out, int out_stride,
                                     const void* k_pages, const void* v_pages,
                                     const int* block_table, int table_stride, int num_pages,
@@ -692,7 +738,8 @@ DE_EXPORT int de_attn_chunk_tcgen05(const void* q, int q_stride, void* out, int 
                                     int dk, int dv, int page, float scale, int chunk, int window,
                                     int keep_first, float softcap, int out_f32, int linear,
                                     const float* sink, const void* out_gate, int ld_out_gate,
-                                    int gate_per_head, float out_scale, int* status, void* stream) {
+                                    int gate_per_head, float out_scale, const float* fv, int* status,
+                                    void* stream) {
     if (num_items <= 0) return 0;
     if (!de_attn_chunk_tcgen05_ok(dk, dv, page) || kv_heads <= 0 || heads % kv_heads != 0) return -2;
     if ((uintptr_t)k_pages % 16 != 0 || (uintptr_t)v_pages % 16 != 0) return -5;
@@ -705,7 +752,7 @@ DE_EXPORT int de_attn_chunk_tcgen05(const void* q, int q_stride, void* out, int 
     return launch<D, FORM>(q, q_stride, out, out_stride, k_pages, v_pages, block_table,         \
                            table_stride, num_pages, seq_slot, seq_qstart, seq_qlen, seq_pos0,   \
                            items, num_items, r1, r2, heads, kv_heads, page, box, scale, sight,  \
-                           out_f32, status, (cudaStream_t)stream)
+                           fv, out_f32, status, (cudaStream_t)stream)
     if (dk == 64) {
         if (form == 0) GO(64, 0);
         if (form == 1) GO(64, 1);

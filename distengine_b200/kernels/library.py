@@ -93,7 +93,7 @@ SIGNATURES: dict[str, dict[str, list]] = {
     "attention_chunk_tcgen05": {
         "de_attn_chunk_tcgen05_rows": [], "de_attn_chunk_tcgen05_ok": [I, I, I],
         "de_attn_chunk_tcgen05": [P, I, P, I, P, P, P, I, I, P, P, P, P, P, I, P, P, I, I, I, I, I,
-                                  F, I, I, I, F, I, I, P, P, I, I, F, P, P],
+                                  F, I, I, I, F, I, I, P, P, I, I, F, P, P, P],
     },
     "recurrent": {
         "de_recurrent_max_key_dim": [],

@@ -423,6 +423,14 @@ def _wide_ok(key_dim: int, value_dim: int, page: int) -> bool:
                                                                                  page))
 
 
+def finishes_portions(tile_rows: int, dtype: torch.dtype, key_dim: int, value_dim: int,
+                      page: int) -> bool:
+    """Whether ``chunk_attention`` takes items of this height to the kernel that also turns its
+    results back and gates them (any kernel gates)."""
+    return (tile_rows == WIDE_ROWS and dtype == torch.bfloat16
+            and _wide_ok(key_dim, value_dim, page))
+
+
 def portion_kernels(dtype: torch.dtype, key_dim: int, value_dim: int) -> "tuple[str, ...]":
     """The kernel libraries that ``chunk_attention`` calls for such rows."""
     wide = dtype == torch.bfloat16 and key_dim == value_dim and key_dim in (64, 128)
@@ -559,19 +567,25 @@ def chunk_attention(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor,
                     window: int = 0, keep_first: int = 0, softcap: float = 0.0,
                     v_stride: int = 0, slopes: "torch.Tensor | None" = None,
                     sink: "torch.Tensor | None" = None, gate: "torch.Tensor | None" = None,
-                    gate_per_head: bool = False, out_scale: float = 1.0) -> None:
+                    gate_per_head: bool = False, out_scale: float = 1.0,
+                    turned_back: "torch.Tensor | None" = None) -> None:
     """Attention of the step's rows over the pages: q rows of [heads dk] at the front of ``q``
     (row stride free), out [N, heads dv]; ``tile_rows``: the rows of a tile that ``items`` were
-    cut for (``chunk_rows_per_tile``); ``v_stride`` as in ``chunk_attention_decode``; see
-    ``csrc/attention_chunk.cu``."""
+    cut for (``chunk_rows_per_tile``); ``v_stride`` as in ``chunk_attention_decode``;
+    ``turned_back`` (where ``finishes_portions``): the results turned back as ``attention_finish``
+    does with its ``fv``; see ``csrc/attention_chunk.cu``."""
     _need(q.stride(1) == 1 and out.stride(1) == 1 and q.dtype == k_pages.dtype
           and out.dtype in (q.dtype, torch.float32)
           and out.shape[1] == heads * value_dim, "chunk_attention: q, out and pages")
     _i32(block_table, "block_table"), _i32(items, "items")
     r1, r2, last = _penalty(r1, r2, heads, slopes, sink, gate, gate_per_head, q.dtype, value_dim,
                             out_scale)
-    if (tile_rows == WIDE_ROWS and q.dtype == torch.bfloat16 and v_stride == 0
-            and _wide_ok(key_dim, value_dim, k_pages.shape[2])):
+    if turned_back is not None:
+        _f32(turned_back, "turned_back")
+        _need(finishes_portions(tile_rows, q.dtype, key_dim, value_dim, k_pages.shape[2])
+              and turned_back.shape == (value_dim // 2,) and turned_back.is_contiguous(),
+              "chunk_attention: turned_back [dv / 2], by the kernel that finishes its results")
+    if v_stride == 0 and finishes_portions(tile_rows, q.dtype, key_dim, value_dim, k_pages.shape[2]):
         lib = library.load("attention_chunk_tcgen05")
         _check(lib.de_attn_chunk_tcgen05(
             q.data_ptr(), q.stride(0), out.data_ptr(), out.stride(0), k_pages.data_ptr(),
@@ -580,7 +594,7 @@ def chunk_attention(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor,
             ctx.seq_pos0.data_ptr(), items.data_ptr(), items.shape[0], _ptr(r1), _ptr(r2), heads,
             kv_heads, key_dim, value_dim, k_pages.shape[2], float(scale), int(chunk), int(window),
             int(keep_first), float(softcap), int(out.dtype == torch.float32), *last,
-            ctx.status.data_ptr(), _stream()), "chunk_attention (tcgen05)")
+            _ptr(turned_back), ctx.status.data_ptr(), _stream()), "chunk_attention (tcgen05)")
         return
     lib = library.load("attention_chunk")
     _check(lib.de_attn_chunk(_tag(q.dtype), q.data_ptr(), q.stride(0), out.data_ptr(),

@@ -164,17 +164,20 @@ class WindowAttention(ProjectedMixer):
                                     out_dtype=out_dtype)
         rk.kv_write_rotated(proj, self.fk, self.rotary_dim, self.fv, H, self.kv_heads, self.dk,
                             dv, cache.k_pages, cache.v_pages, cache.block_table, cache.writes, ctx)
-        finish = self.fv is not None or self.gated
+        rows = ctx.notes[self.key]
+        gate = proj[:, self.g_col: self.g_col + H * dv] if self.gated else None
+        # the kernel for 128 rows a tile turns its results back and gates them itself
+        inside = rk.finishes_portions(rows, self.dtype, self.dk, dv, cache.k_pages.shape[2])
+        finish = (self.fv is not None or self.gated) and not inside
         raw = (ctx.buffer("window_attention.raw", (n, H * dv), torch.float32) if finish
                else context)
         sight = dict(window=self.window or 0, keep_first=self.keep_first if self.window else 0,
                      softcap=self.softcap or 0.0)
         rk.chunk_attention(proj, raw, cache.k_pages, cache.v_pages, cache.block_table,
                            ctx.arrays[self.key + "/items"], None, None, H, self.kv_heads,
-                           self.dk, dv, self.scale, 0, ctx, tile_rows=ctx.notes[self.key],
-                           **sight)
+                           self.dk, dv, self.scale, 0, ctx, tile_rows=rows, **sight,
+                           **(dict(gate=gate, turned_back=self.fv) if inside else {}))
         if finish:
-            gate = proj[:, self.g_col: self.g_col + H * dv] if self.gated else None
             rk.attention_finish(raw, self.fv, gate, context, H, dv, ctx)
         return self.project_out(context, "window_attention.out", ctx, ahead, out_dtype=out_dtype)
 

@@ -146,3 +146,32 @@ def test_soft_cap(cap, low, high):
     want = cap * (torch.tanh(x.double() / cap) - torch.tanh(y.double() / cap))
     units = (torch.log(p) - torch.log1p(-p) - want).abs() / (cap * 2.0 ** -24)
     assert units[clear].max().item() <= 2 * (0.5 + 2 + 0.5) + 1
+
+
+@pytest.mark.parametrize("dim,heads,kv_heads", [(64, 4, 4), (128, 8, 2), (128, 3, 3), (64, 16, 1), (128, 5, 1)])
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("spoilt", [False, True])
+def test_results_turned_back(dim, heads, kv_heads, gated, spoilt):
+    """In the attention's own epilogue: the bits of float32 results that attention_finish then turns and
+    gates, for one to 128 tokens a block, and in rows that are formed again."""
+    from distengine_b200.kernels import recurrent as rk
+    lens, qlen = [500, 131, 70], [300, 131, 1]
+    fx = PagedFixture(lens, kv_heads, dim, 16, torch.bfloat16, DEV, seed=dim + heads)
+    if spoilt:
+        fx.v[0][450, 0, 5] = float("inf")
+        fx.v[1][100, kv_heads - 1, dim - 1] = float("nan")
+        fx.rewrite()
+    g = torch.Generator().manual_seed(heads)
+    n = sum(qlen)
+    q = torch.randn(n, heads * dim, generator=g).to(torch.bfloat16).to(DEV)
+    gate = torch.randn(n, heads * dim, generator=g).to(torch.bfloat16).to(DEV) if gated else None
+    fv = torch.rand(dim // 2, generator=g).to(DEV)
+    raw, want = torch.empty(n, heads * dim, device=DEV), torch.empty_like(q)
+    pos0 = _run(fx, qlen, heads, kv_heads, q, raw, dim ** -0.5, window=200, keep_first=3)
+    positions = _t(np.concatenate([np.arange(p, p + l) for p, l in zip(pos0, qlen)]))
+    rk.attention_finish(raw, fv, gate, want, heads, dim, SimpleNamespace(positions=positions))
+    out = torch.full_like(q, 9.0)
+    _run(fx, qlen, heads, kv_heads, q, out, dim ** -0.5, window=200, keep_first=3, turned_back=fv, gate=gate)
+    assert torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out.nan_to_num(1.0), want.nan_to_num(1.0))
+    assert bool(want.isnan().any()) == spoilt
