@@ -283,10 +283,10 @@ int sm_count() {
     return count;
 }
 
-// The tile width: the candidate whose rounds of tiles over the SMs take least, a round of tiles
-// bn wide taking about bn + 16 units.  Tiles narrower than 128 read too much of x and w per flop;
-// they are candidates only when wider ones would leave SMs without a tile.
-int choose_bn(int m_rows, int n_out, bool gated) {
+// The tile width: the candidate whose rounds of tiles over the SMs take least, a round of tiles bn wide
+// taking about bn + `fixed` units.  Tiles narrower than 128 read too much of x and w per flop; they are
+// candidates only when wider ones would leave SMs without a tile.
+int best_width(int m_rows, int n_out, bool gated, int fixed) {
     const int tiles_m = (m_rows + BM - 1) / BM;
     const long sms = sm_count();
     auto tiles = [&](int bn) {
@@ -298,7 +298,7 @@ int choose_bn(int m_rows, int n_out, bool gated) {
     const bool small = tiles(128) < sms;
     const int step = gated ? 64 : 32;
     for (int bn = MAX_BN; bn >= (small ? step : 128); bn -= step) {
-        const long cost = ((tiles(bn) + sms - 1) / sms) * (bn + 16);
+        const long cost = ((tiles(bn) + sms - 1) / sms) * (bn + fixed);
         if (best == 0 || cost < best_cost) {
             best = bn;
             best_cost = cost;
@@ -306,6 +306,12 @@ int choose_bn(int m_rows, int n_out, bool gated) {
     }
     return best;
 }
+
+// A round hardly depends on the tiles' width: at k = 2,048 11.4 us for 128 columns, 12.2 for 192, 13.4 for
+// 256, at k = 4,096 23, 24.5 and 26.8, so the number of rounds decides and, among equals, the narrowest.
+// (By width + 16, as it was chosen: 1,300 rows against 2 x 5,632 gated 79 us in seven rounds of 128, 53
+// in four of 256; 2,048 against 2 x 11,008 with k = 4,096 336 and 268; 1,024 against 2 x 5,632 64 and 43.)
+int choose_bn(int m_rows, int n_out, bool gated) { return best_width(m_rows, n_out, gated, 600); }
 
 template <bool GATED, typename OutT>
 int launch(const void* x, int ldx, const void* w, int ldw, void* out, int ldo, int m_rows, int n_out,
@@ -341,10 +347,11 @@ int launch(const void* x, int ldx, const void* w, int ldw, void* out, int ldo, i
 
 }  // namespace
 
-// The tile width the kernel would take for this shape (the host decides with it whether the
-// shape suits the kernel).
+// How wide the tiles would have to be if a tile took as long as its columns: the host decides with it
+// whether the shape suits the kernel better than the library's (by the width that the kernel really takes,
+// 2,048 rows against 4,096 x 4,096 would come here, 53 us against the library's 50).
 DE_EXPORT int de_gemm_tcgen05_tile(int m_rows, int n_out, int gated) {
-    return choose_bn(m_rows, n_out, gated != 0);
+    return best_width(m_rows, n_out, gated != 0, 16);
 }
 DE_EXPORT int de_gemm_tcgen05_sms() { return sm_count(); }
 
@@ -380,7 +387,8 @@ DE_EXPORT int de_gemm_tcgen05_grouped(const void* x, int ldx, const void* w, voi
     if (k_dim <= 0 || k_dim % 8 != 0 || ldx % 8 != 0 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15))
         return -3;
     const int m_rows = tiles * BM;
-    const int bn = choose_bn(m_rows, n_out, false);
+    // most reserved tiles may be without tokens: their rounds cost nothing, wider tiles would
+    const int bn = best_width(m_rows, n_out, false, 16);
     CUtensorMap map_x, map_w;
     int code = make_map(&map_x, x, m_rows, k_dim, ldx, BM);
     if (code) return code;

@@ -622,6 +622,26 @@ def test_gemm_tcgen05_gated(m, inner, k):
     assert_close(out, plain.plain_swiglu(gate, up, torch.bfloat16), torch.bfloat16, "gated tcgen05")
 
 
+@pytest.mark.parametrize("m,n,gated", [(1025, 5632, True), (1300, 5601, True), (1300, 5120, False),
+                                       (1900, 4100, False), (2048, 11008, True)])
+def test_gemm_tcgen05_in_few_rounds(m, n, gated):
+    """Shapes at which the wide tiles win by their number of rounds, with ragged last tiles."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(m + n)
+    k = 72
+    x = torch.randn(m, k, generator=g).to(torch.bfloat16)
+    w = (torch.randn((2 if gated else 1) * n, k, generator=g) * 0.1).to(torch.bfloat16)
+    out = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.gemm_tcgen05(x.to(DEV), w.to(DEV), out, gated=gated, status=status)
+    assert status.item() == 0
+    want = plain.plain_linear(x.float(), w[:n].float(), torch.bfloat16)
+    if gated:
+        up = plain.plain_linear(x.float(), w[n:].float(), torch.bfloat16)
+        want = plain.plain_swiglu(want, up, torch.bfloat16)
+    assert_close(out, want, torch.bfloat16, "tcgen05 in few rounds")
+
+
 def test_products_of_many_rows_take_the_tcgen05_kernel():
     """From a thousand rows on, ``linear`` (in a shape that suits it) and ``linear_gated`` run this
     package's tcgen05 kernel: the results agree with the plain product, and the kernel library is
