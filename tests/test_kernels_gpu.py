@@ -642,6 +642,25 @@ def test_gemm_tcgen05_in_few_rounds(m, n, gated):
     assert_close(out, want, torch.bfloat16, "tcgen05 in few rounds")
 
 
+@pytest.mark.parametrize("m,n,pitch,first", [(300, 96, 104, 8), (300, 96, 104, 0), (129, 63, 64, 0),
+                                             (129, 64, 71, 3), (33, 40, 48, 8), (256, 256, 256, 0)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32"])
+def test_gemm_tcgen05_output_rows(m, n, pitch, first, out_dtype):
+    """Output rows at any pitch and address, whole groups of 32 columns and not: every element where it
+    belongs and nothing beside it."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(m + n + pitch)
+    x = torch.randn(m, 136, generator=g).to(torch.bfloat16)
+    w = (torch.randn(n, 136, generator=g) * 0.1).to(torch.bfloat16)
+    whole = torch.full((m, pitch), 7.0, dtype=out_dtype, device=DEV)
+    out = whole[:, first: first + n]
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.gemm_tcgen05(x.to(DEV), w.to(DEV), out, status=status)
+    assert status.item() == 0
+    assert_close(out, plain.plain_linear(x.float(), w.float(), out_dtype), out_dtype, "output rows")
+    assert bool((whole[:, :first] == 7).all()) and bool((whole[:, first + n:] == 7).all())
+
+
 def test_products_of_many_rows_take_the_tcgen05_kernel():
     """From a thousand rows on, ``linear`` (in a shape that suits it) and ``linear_gated`` run this
     package's tcgen05 kernel: the results agree with the plain product, and the kernel library is
