@@ -20,8 +20,8 @@
 // A cut of a portion changes the order of float32 sums only.
 //
 // Figures below: 2,048 tokens of 16 heads of 128 x 128 on B200.  The scan takes 0.37 us a
-// token for the delta rule, 760 us in all, by chunks 270 us; under a decay per head a layer with its
-// products took 1,861 us by the scan, 202 us by chunks (107 of them here).
+// token for the delta rule, 760 us in all, by chunks 221 us; under a decay per head a layer with its
+// products took 1,861 us by the scan, 200 us by chunks (105 of them here).
 
 #include "common.cuh"
 
@@ -130,18 +130,20 @@ __device__ __forceinline__ void powers(float d, float* pw) {
     }
 }
 
-// 64 rows of 64 columns (rows beyond `rows` are zeros) into tile [64][LD]; 128 threads
+// N rows of 64 columns (rows beyond `rows` are zeros) into tile [N][LD]; 128 threads
+template <int N = 64>
 __device__ __forceinline__ void load_tile(float* tile, const float* src, size_t ld, int rows) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < N / 8; ++i) {
         const int e = threadIdx.x + 128 * i, r = e >> 4, c = (e & 15) * 4;
         cp16(tile + r * LD + c, r < rows ? src + (size_t)r * ld + c : src, r < rows);
     }
 }
+template <int N = 64>
 __device__ __forceinline__ void load_tile(float* tile, const __nv_bfloat16* src, size_t ld,
                                           int rows) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < N / 8; ++i) {
         const int e = threadIdx.x + 128 * i, r = e >> 4, c = (e & 15) * 4;
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (r < rows) {
@@ -155,40 +157,51 @@ __device__ __forceinline__ void load_tile(float* tile, const __nv_bfloat16* src,
 
 // ------------------------------------------------------------------------------------------
 // A decay per head.  products: pt[item][h][s][t] = d^(t-s) q_t . k_s (0 for s > t) and
-// xt[item][h][c][t] = d^(t+1) q_t[c].  grid (items, H), 128 threads.  28 us, bound by shared memory
-// (both operands of 64 x 64 outputs pass through it once a block).
+// xt[item][h][c][t] = d^(t+1) q_t[c].  grid (items, H), 128 threads.  64 channels at a time, so that 512
+// blocks are one round: 25 us, the way in of operands that are used once a block (all 128 at once, three
+// blocks an SM: 28).
 // ------------------------------------------------------------------------------------------
 template <int DK>
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, 4)
 decay_products_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
                       const float* __restrict__ decay, const Item* __restrict__ items,
                       float* __restrict__ xt, float* __restrict__ pt, int H) {
     extern __shared__ __align__(16) float sh[];
-    float* qs = sh;                                  // [DK][LD]
-    float* ks = qs + DK * LD;                        // [DK][LD]
+    float* qs = sh;                                  // [64][LD]: 64 channels at a time
+    float* ks = qs + 64 * LD;
     __shared__ float pw[CH + 1];
     const Item it = items[blockIdx.x];
     const int h = blockIdx.y;
     powers(decay[h], pw);
     pdl_wait();
-    // turned on the way in: a warp copies 8 channels of 4 tokens at a time
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c0 = 0; c0 < DK; c0 += 8)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = (i * 4 + warp) * 4 + (lane >> 3), c = c0 + (lane & 7);
-            const bool ok = t < it.count;
-            const size_t tok = (size_t)(it.token + (ok ? t : 0));
-            cp4(qs + c * LD + t, q + tok * ldq + h * DK + c, ok);
-            cp4(ks + c * LD + t, k + tok * ldk + h * DK + c, ok);
-        }
-    cp_commit();
-    cp_wait<0>();
-    __syncthreads();
-    Tile tile;
-    tile.add<DK>(ks, qs);
-    pdl_trigger();
     const size_t at = (size_t)blockIdx.x * H + h;
+    float* x = xt + at * DK * CH;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Tile tile;
+    for (int half = 0; half < DK; half += 64) {
+        // turned on the way in: a warp copies 8 channels of 4 tokens at a time
+        for (int c0 = 0; c0 < 64; c0 += 8)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int t = (i * 4 + warp) * 4 + (lane >> 3), c = c0 + (lane & 7);
+                const bool ok = t < it.count;
+                const size_t tok = (size_t)(it.token + (ok ? t : 0));
+                cp4(qs + c * LD + t, q + tok * ldq + h * DK + half + c, ok);
+                cp4(ks + c * LD + t, k + tok * ldk + h * DK + half + c, ok);
+            }
+        cp_commit();
+        cp_wait<0>();
+        __syncthreads();
+        tile.add<64>(ks, qs);
+        for (int e = threadIdx.x; e < 64 * CH / 4; e += 128) {
+            const int c = e >> 4, t = (e & 15) * 4;
+            const float4 v = four(qs + c * LD + t);
+            *reinterpret_cast<float4*>(x + (half + c) * CH + t) = make_float4(
+                v.x * pw[t + 1], v.y * pw[t + 2], v.z * pw[t + 3], v.w * pw[t + 4]);
+        }
+        __syncthreads();
+    }
+    pdl_trigger();
     float* p = pt + at * CH * CH;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -200,13 +213,6 @@ decay_products_kernel(const float* __restrict__ q, int ldq, const float* __restr
         v.z = d >= -2 ? v.z * pw[d + 2] : 0.0f;
         v.w = d >= -3 ? v.w * pw[d + 3] : 0.0f;
         *reinterpret_cast<float4*>(p + s * CH + tile.col) = v;
-    }
-    float* x = xt + at * DK * CH;
-    for (int e = threadIdx.x; e < DK * CH / 4; e += 128) {
-        const int c = e >> 4, t = (e & 15) * 4;
-        const float4 v = four(qs + c * LD + t);
-        *reinterpret_cast<float4*>(x + c * CH + t) = make_float4(
-            v.x * pw[t + 1], v.y * pw[t + 2], v.z * pw[t + 3], v.w * pw[t + 4]);
     }
 }
 
@@ -296,20 +302,20 @@ decay_pass_kernel(float* __restrict__ states, const float* __restrict__ decay,
 // ------------------------------------------------------------------------------------------
 // The delta rule.  What a chunk's tokens give by themselves: at[item][h][s][t] = A_ts,
 // pt[item][h][s][t] = P_ts (0 for s > t), xt[item][h][c][t] = b_t q_t, kd[item][h][t][c] = b_t k_t,
-// kh[item][h][s][c] = (b_n / b_s) k_s and bn[item][h][c] = b_n.  grid (items, H), 128 threads.
-// A thread walks w of two columns s over the tokens, a quarter of the channels each (lanes 8 apart
-// share a column), as the scan walks the state; bound by the reads of a token's three vectors
-// from shared memory, which two columns share.  73 us, an
-// instruction issued in a third of the cycles on two blocks an SM.
+// kh[item][h][s][c] = (b_n / b_s) k_s and bn[item][h][c] = b_n.  grid (items, H), 256 threads.
+// A thread walks w of two columns s over the tokens, an eighth of the channels each (lanes 4 apart
+// share a column), as the scan walks the state; the eight sums of a column meet four tokens at a time,
+// each lane left with two of the 16 results.  Two blocks an SM (a chunk's vectors are 99 KB): 55 us, an
+// instruction issued in 40 % of the cycles; four warps with a quarter of the channels a lane took 76.
 // ------------------------------------------------------------------------------------------
 template <int DK>
-__global__ void __launch_bounds__(128, 2)
+__global__ void __launch_bounds__(256, 2)
 delta_chunk_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
                    const float* __restrict__ g, int ldg, const Item* __restrict__ items,
                    float* __restrict__ at, float* __restrict__ pt, float* __restrict__ xt,
                    float* __restrict__ kd, float* __restrict__ kh, float* __restrict__ bn, int H,
                    int rep) {
-    constexpr int W = DK + 4, R = DK / 16;           // a row in shared memory; quads of a lane
+    constexpr int W = DK + 4, R = DK / 32;           // a row in shared memory; quads of a lane
     extern __shared__ __align__(16) float sh[];
     float* qs = sh;                                  // [CH][W]
     float* ks = qs + CH * W;
@@ -318,7 +324,7 @@ delta_chunk_kernel(const float* __restrict__ q, int ldq, const float* __restrict
     const int h = blockIdx.y, hk = h / rep;
     const size_t where = (size_t)blockIdx.x * H + h;
     pdl_wait();
-    for (int e = threadIdx.x; e < CH * DK / 4; e += 128) {
+    for (int e = threadIdx.x; e < CH * DK / 4; e += 256) {
         const int t = e / (DK / 4), c = e % (DK / 4) * 4;
         const bool ok = t < it.count;
         const size_t tok = (size_t)(it.token + (ok ? t : 0));
@@ -330,49 +336,54 @@ delta_chunk_kernel(const float* __restrict__ q, int ldq, const float* __restrict
     cp_commit();
     cp_wait<0>();
     __syncthreads();
-    if (threadIdx.x < DK) {
-        const int c = threadIdx.x;
-        float b = 1.0f;
-        float* x = xt + (where * DK + c) * CH;
-        float* d = kd + where * CH * DK + c;
+    if (threadIdx.x < 2 * DK) {                      // (whole warps)
+        const int c = threadIdx.x % DK;
+        if (threadIdx.x < DK) {
+            float b = 1.0f;
+            float* x = xt + (where * DK + c) * CH;
+            float* d = kd + where * CH * DK + c;
 #pragma unroll 2
-        for (int t = 0; t < CH; t += 4) {
-            float v[4];
+            for (int t = 0; t < CH; t += 4) {
+                float v[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                b *= gs[(t + i) * W + c];
-                v[i] = b * qs[(t + i) * W + c];
-                d[(size_t)(t + i) * DK] = b * ks[(t + i) * W + c];
+                for (int i = 0; i < 4; ++i) {
+                    b *= gs[(t + i) * W + c];
+                    v[i] = b * qs[(t + i) * W + c];
+                    d[(size_t)(t + i) * DK] = b * ks[(t + i) * W + c];
+                }
+                *reinterpret_cast<float4*>(x + t) = make_float4(v[0], v[1], v[2], v[3]);
             }
-            *reinterpret_cast<float4*>(x + t) = make_float4(v[0], v[1], v[2], v[3]);
-        }
-        bn[where * DK + c] = b;
-        float* o = kh + where * CH * DK + c;
-        float r = 1.0f;
+            bn[where * DK + c] = b;
+        } else {
+            float* o = kh + where * CH * DK + c;
+            float r = 1.0f;
 #pragma unroll 4
-        for (int t = CH - 1; t >= 0; --t) {
-            o[(size_t)t * DK] = r * ks[t * W + c];
-            r *= gs[t * W + c];
+            for (int t = CH - 1; t >= 0; --t) {
+                o[(size_t)t * DK] = r * ks[t * W + c];
+                r *= gs[t * W + c];
+            }
         }
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int share = lane >> 3, s0 = warp * 16 + (lane & 7) * 2, s1 = s0 + 1;
+    const int share = lane >> 2, s0 = warp * 8 + (lane & 3) * 2, s1 = s0 + 1;
     unsigned long long w0[2 * R], w1[2 * R];         // neighbouring channels in pairs
 #pragma unroll
     for (int i = 0; i < 2 * R; ++i) w0[i] = w1[i] = 0ull;
-    float* rows = (share < 2 ? at : pt) + (where * CH + (share & 1 ? s1 : s0)) * CH;
-    for (int t = 0; t < warp * 16; t += 4)
+    // what a lane writes: A or P, of column s0 or s1, two of four tokens
+    const bool is_p = share & 4, second = share & 2, later = share & 1;
+    float* rows = (is_p ? pt : at) + (where * CH + (second ? s1 : s0)) * CH;
+    for (int t = later * 4; t < warp * 8; t += 8)
         *reinterpret_cast<float4*>(rows + t) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int t = warp * 16; t < CH; t += 4) {
-        float keep[4];
+    for (int t = warp * 8; t < CH; t += 4) {
+        float va[2][4], vp[2][4];                    // by column and token
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int tt = t + i;
             unsigned long long sa0 = 0ull, sa1 = 0ull, sp0 = 0ull, sp1 = 0ull;
-            const bool near = tt < warp * 16 + 16;
+            const bool near = tt < warp * 8 + 8;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const int o = tt * W + 16 * r + 4 * share;
+                const int o = tt * W + 32 * r + 4 * share;
                 const float4 gg = four(gs + o), kk = four(ks + o), qq = four(qs + o);
                 const unsigned long long gv[2] = {pair(gg.x, gg.y), pair(gg.z, gg.w)};
                 const unsigned long long kv[2] = {pair(kk.x, kk.y), pair(kk.z, kk.w)};
@@ -382,7 +393,7 @@ delta_chunk_kernel(const float* __restrict__ q, int ldq, const float* __restrict
                     w0[2 * r + x] = mul2(w0[2 * r + x], gv[x]);
                     w1[2 * r + x] = mul2(w1[2 * r + x], gv[x]);
                 }
-                if (near) {                          // (a column begins inside its warp's 16 tokens)
+                if (near) {                          // (a column begins inside its warp's 8 tokens)
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
                         if (tt == s0) w0[2 * r + x] = kv[x];
@@ -397,32 +408,42 @@ delta_chunk_kernel(const float* __restrict__ q, int ldq, const float* __restrict
                     fma2(sp1, qv[x], w1[2 * r + x]);
                 }
             }
-            float a0, a1, p0, p1, c0, c1, e0, e1;
-            unpair(sa0, a0, c0);
-            unpair(sa1, a1, c1);
-            unpair(sp0, p0, e0);
-            unpair(sp1, p1, e1);
-            a0 += c0; a1 += c1; p0 += e0; p1 += e1;
-#pragma unroll
-            for (int m = 8; m < 32; m <<= 1) {
-                a0 += __shfl_xor_sync(0xffffffffu, a0, m);
-                a1 += __shfl_xor_sync(0xffffffffu, a1, m);
-                p0 += __shfl_xor_sync(0xffffffffu, p0, m);
-                p1 += __shfl_xor_sync(0xffffffffu, p1, m);
-            }
-            if (tt <= s0) a0 = 0.0f;                 // A is strictly below the diagonal
-            if (tt <= s1) a1 = 0.0f;
-            keep[i] = share == 0 ? a0 : share == 1 ? a1 : share == 2 ? p0 : p1;
+            float lo, hi;
+            unpair(sa0, lo, hi);
+            va[0][i] = tt <= s0 ? 0.0f : lo + hi;    // A is strictly below the diagonal
+            unpair(sa1, lo, hi);
+            va[1][i] = tt <= s1 ? 0.0f : lo + hi;
+            unpair(sp0, lo, hi);
+            vp[0][i] = lo + hi;
+            unpair(sp1, lo, hi);
+            vp[1][i] = lo + hi;
         }
-        *reinterpret_cast<float4*>(rows + t) = make_float4(keep[0], keep[1], keep[2], keep[3]);
+        // the shares' sums: at each step a lane keeps half of what it has and gives the other half
+        float one[2][4], two[4], out[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                one[c][i] = (is_p ? vp[c][i] : va[c][i]) +
+                            __shfl_xor_sync(0xffffffffu, is_p ? va[c][i] : vp[c][i], 16);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            two[i] = (second ? one[1][i] : one[0][i]) +
+                     __shfl_xor_sync(0xffffffffu, second ? one[0][i] : one[1][i], 8);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            out[i] = (later ? two[2 + i] : two[i]) +
+                     __shfl_xor_sync(0xffffffffu, later ? two[i] : two[2 + i], 4);
+        *reinterpret_cast<float2*>(rows + t + 2 * later) = make_float2(out[0], out[1]);
     }
     pdl_trigger();
 }
 
 // X of (1 + diag(beta) A) X = diag(beta) [v | b k]: xv[item][h][t][j] and, turned, xkt[item][h][c][t].
 // grid (items, H, ceil((dv + DK) / 128)), 64 threads with two columns each: forward substitution by
-// blocks of 16 tokens, a thread's earlier rows in shared memory of its own.  48 us: a chain of 64
-// rows, an instruction issued in a third of the cycles.
+// blocks of 16 tokens, a thread's earlier rows in shared memory of its own.  35 us: a chain of 64
+// rows, an instruction issued in a third of the cycles.  (A column a thread, twice the warps: 42, the
+// reads of A, which all lanes share, are what fills shared memory's pipe.)
 template <int DK>
 __global__ void __launch_bounds__(64)
 delta_solve_kernel(const float* __restrict__ at, const float* __restrict__ v, int ldv,
@@ -482,7 +503,6 @@ delta_solve_kernel(const float* __restrict__ at, const float* __restrict__ v, in
             o0[r] = b * (rhs[r].x - s0);
             o1[r] = b * (rhs[r].y - s1);
             const unsigned long long x = pair(o0[r], o1[r]);
-            *reinterpret_cast<unsigned long long*>(mine + (t0 + r) * 128) = x;
 #pragma unroll
             for (int i = (r + 1) & ~3; i < 16; i += 4) {       // (acc up to r has been used)
                 const float4 a = four(as + (t0 + r) * LD + t0 + i);
@@ -492,6 +512,10 @@ delta_solve_kernel(const float* __restrict__ at, const float* __restrict__ v, in
                 fma2(acc[i + 3], pair(a.w, a.w), x);
             }
         }
+        // (not sooner: a store would hold back the reads of A after it)
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+            *reinterpret_cast<float2*>(mine + (t0 + r) * 128) = make_float2(o0[r], o1[r]);
         if (!live) continue;
         if (is_v) {
 #pragma unroll
@@ -661,31 +685,32 @@ delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
 
 // ------------------------------------------------------------------------------------------
 // The read-outs, both rules: out[t][j] = sum_c xt[c][t] S0[c][j] + sum_s pt[s][t] u_s[j].
-// grid (items, H, dv / 64), 128 threads; steps of 64 through two stages.  u: rows of the step
-// (u_by_item 0) or of the chunks' own rows [item][h][64][dv].  36 to 38 us, bound like the others by
-// shared memory at one read a two multiply-adds.
+// grid (items, H, dv / 64), 128 threads; steps of 32 through two stages.  u: rows of the step
+// (u_by_item 0) or of the chunks' own rows [item][h][64][dv].  40 us on four blocks an SM, whose 1,024
+// blocks are two rounds (steps of 64, three blocks: 43); the multiply-adds alone are 26.
 // ------------------------------------------------------------------------------------------
 template <typename VT>
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, 4)
 chunk_out_kernel(const float* __restrict__ xt, const float* __restrict__ states,
                  const float* __restrict__ pt, const VT* __restrict__ u, int ldu, int u_by_item,
                  const Item* __restrict__ items, float* __restrict__ out, int H, int dk, int dv) {
-    extern __shared__ __align__(16) float sh[];      // [2][2][64][LD]
+    extern __shared__ __align__(16) float sh[];      // [2][2][32][LD]
     const Item it = items[blockIdx.x];
     const int h = blockIdx.y, j0 = blockIdx.z * 64;
     const size_t at = (size_t)blockIdx.x * H + h;
-    const int steps = dk / 64 + 1;
+    const int of_state = dk / 32, steps = of_state + 2;
     pdl_wait();
     auto load = [&](int step) {
-        float* a = sh + (step & 1) * 2 * CH * LD;
-        float* b = a + CH * LD;
-        if (step + 1 < steps) {
-            load_tile(a, xt + (at * dk + step * 64) * CH, CH, 64);
-            load_tile(b, states + (at * dk + step * 64) * dv + j0, dv, 64);
+        float* a = sh + (step & 1) * 2 * 32 * LD;
+        float* b = a + 32 * LD;
+        if (step < of_state) {
+            load_tile<32>(a, xt + (at * dk + step * 32) * CH, CH, 32);
+            load_tile<32>(b, states + (at * dk + step * 32) * dv + j0, dv, 32);
         } else {
-            load_tile(a, pt + at * CH * CH, CH, 64);
-            if (u_by_item) load_tile(b, u + at * CH * dv + j0, dv, it.count);
-            else load_tile(b, u + (size_t)it.token * ldu + h * dv + j0, ldu, it.count);
+            const int s0 = (step - of_state) * 32;
+            load_tile<32>(a, pt + (at * CH + s0) * CH, CH, 32);
+            if (u_by_item) load_tile<32>(b, u + (at * CH + s0) * dv + j0, dv, it.count - s0);
+            else load_tile<32>(b, u + (size_t)(it.token + s0) * ldu + h * dv + j0, ldu, it.count - s0);
         }
         cp_commit();
     };
@@ -696,8 +721,8 @@ chunk_out_kernel(const float* __restrict__ xt, const float* __restrict__ states,
         else cp_commit();
         cp_wait<1>();
         __syncthreads();
-        const float* a = sh + (step & 1) * 2 * CH * LD;
-        tile.add<CH>(a, a + CH * LD);
+        const float* a = sh + (step & 1) * 2 * 32 * LD;
+        tile.add<32>(a, a + 32 * LD);
         __syncthreads();
     }
     pdl_trigger();
@@ -761,8 +786,8 @@ DE_EXPORT int de_decay_chunks(int v_dtype, const float* q, int ldq, const float*
         return -2;
     cudaStream_t s = (cudaStream_t)stream;
     const Portion* po = (const Portion*)portions;
-    const size_t psmem = (size_t)2 * dk * LD * sizeof(float);
-    const size_t osmem = (size_t)4 * CH * LD * sizeof(float);
+    const size_t psmem = (size_t)2 * 64 * LD * sizeof(float);
+    const size_t osmem = (size_t)4 * 32 * LD * sizeof(float);
     const dim3 pgrid(n_portions, (H * dk * dv / 4 + 255) / 256);
     int e;
 #define RUN(...)                                                                                \
@@ -825,13 +850,13 @@ DE_EXPORT int de_delta_chunks(const float* q, int ldq, const float* k, int ldk, 
     const Portion* po = (const Portion*)portions;
     const size_t csmem = (size_t)3 * CH * (dk + 4) * sizeof(float);
     const size_t ssmem = (size_t)(CH * LD + CH * 128) * sizeof(float);
-    const size_t osmem = (size_t)4 * CH * LD * sizeof(float);
+    const size_t osmem = (size_t)4 * 32 * LD * sizeof(float);
     const dim3 pgrid(n_portions, H, dv / PC);
     int e;
 #define DELTA(DK)                                                                               \
     do {                                                                                        \
         RUN(need_smem((const void*)delta_chunk_kernel<DK>, csmem));                     \
-        RUN(de_launch(delta_chunk_kernel<DK>, dim3(m, H), dim3(128), csmem, s, q, ldq, k, ldk,  \
+        RUN(de_launch(delta_chunk_kernel<DK>, dim3(m, H), dim3(256), csmem, s, q, ldq, k, ldk,  \
                       g, ldg, it, at, pt, xt, kd, kh, bn, H, rep));                             \
         RUN(need_smem((const void*)delta_solve_kernel<DK>, ssmem));                     \
         RUN(de_launch(delta_solve_kernel<DK>, sgrid, dim3(64), ssmem, s, (const float*)at, v,   \
