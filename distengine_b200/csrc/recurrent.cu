@@ -124,9 +124,10 @@ __device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
 // and up to four taps (KK): a thread has four neighbouring channels and goes through RUN tokens with
 // the last inputs in registers, a head is 16 or 32 lanes of a warp, which form its norm.  The first
 // `conv_blocks` of the blocks do the convolution, 512 channels each, the others the decays (and
-// beta).  grid (runs of tokens, blocks), 128 threads.  2,048 tokens of 6,144 channels and 2,048
-// decays: 48 us (a block a token, a channel at a time: 128).
-constexpr int RUN = 8;
+// beta).  grid (runs of tokens, blocks), 128 threads.  Bound by the instructions of the exponentials and
+// quotients (one in 72 % of the cycles): 2,048 tokens of 6,144 channels and 2,048 decays 40 us; runs of
+// eight, whose registers leave half as many warps, 45; a block a token, a channel at a time 128.
+constexpr int RUN = 4;
 
 // The sum of a head's squares, four neighbouring channels a lane, the head on 16 or 32 lanes.  In
 // float32 in the order of the kernel above (channels 32 apart in a chain, then 16, 8 .. 1 apart), so
@@ -729,6 +730,51 @@ __global__ void head_gate_kernel(const float* __restrict__ o, const void* __rest
     }
 }
 
+// The same for heads of up to 32 QUADS groups of four values, a lane QUADS groups of the head: 2,048
+// tokens of 16 heads of 128, mode 0: 13 us (an element a lane at a time: 19).
+template <typename T, int QUADS>
+__global__ void __launch_bounds__(128)
+head_gate_vec_kernel(const float* __restrict__ o, const void* __restrict__ gate, int ld_gate,
+                     const float* __restrict__ weight, T* __restrict__ out, int n_tokens, int H, int dv,
+                     float eps, int mode) {
+    const int lane = threadIdx.x & 31;
+    const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_trigger();
+    if (item >= n_tokens * H) return;
+    const int n = item / H, h = item - n * H;
+    const size_t at = (size_t)item * dv, gate_at = (size_t)n * ld_gate + h * dv;
+    float4 x[QUADS], g[QUADS], w[QUADS];
+    float ss = 0.0f;
+#pragma unroll
+    for (int q = 0; q < QUADS; ++q) {
+        const int j = (q * 32 + lane) * 4;
+        x[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        w[q] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        if (j >= dv) continue;
+        x[q] = load_four(o + at + j);
+        g[q] = mode == 0 ? load_four((const float*)gate + gate_at + j)
+                         : load_four((const T*)gate + gate_at + j);
+        if (mode != 1) w[q] = load_four(weight + (mode == 2 ? h * dv : 0) + j);
+    }
+#pragma unroll
+    for (int q = 0; q < QUADS; ++q)
+        ss = fmaf(x[q].x, x[q].x, fmaf(x[q].y, x[q].y, fmaf(x[q].z, x[q].z, fmaf(x[q].w, x[q].w, ss))));
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)dv + eps);
+#pragma unroll
+    for (int q = 0; q < QUADS; ++q) {
+        const int j = (q * 32 + lane) * 4;
+        if (j >= dv) continue;
+        const float4 s = mode == 1 ? make_float4(silu_f(g[q].x), silu_f(g[q].y), silu_f(g[q].z),
+                                                 silu_f(g[q].w))
+                                   : make_float4(sigmoid_f(g[q].x), sigmoid_f(g[q].y),
+                                                 sigmoid_f(g[q].z), sigmoid_f(g[q].w));
+        store_four(out + at + j,
+                   make_float4((x[q].x * inv) * w[q].x * s.x, (x[q].y * inv) * w[q].y * s.y,
+                               (x[q].z * inv) * w[q].z * s.z, (x[q].w * inv) * w[q].w * s.w));
+    }
+}
+
 // out = (a / rms(a) * wa + b / rms(b) * wb) / 2 over the model width.  One block a token.
 template <typename T>
 __global__ void mean_of_normed_kernel(const T* __restrict__ a, const T* __restrict__ b,
@@ -1090,6 +1136,21 @@ DE_EXPORT int de_head_gate(int dtype, const float* o, const void* gate, int ld_g
     }
     const int warps = 4;
     dim3 grid((n * H + warps - 1) / warps);
+    const size_t out_piece = dtype == DE_BF16 ? 8 : 16, gate_piece = mode == 0 ? 16 : out_piece;
+    if (dv % 4 == 0 && dv <= 256 && ld_gate % 4 == 0 && (uintptr_t)o % 16 == 0 &&
+        (mode == 1 || (uintptr_t)weight % 16 == 0) && (uintptr_t)gate % gate_piece == 0 &&
+        (uintptr_t)out % out_piece == 0) {
+#define GATE(T, Q)                                                                              \
+    return de_launch(head_gate_vec_kernel<T, Q>, grid, dim3(32 * warps), 0, s, o, gate, ld_gate, \
+                     weight, (T*)out, n, H, dv, eps, mode)
+        if (dtype == DE_BF16) {
+            if (dv <= 128) GATE(__nv_bfloat16, 1);
+            GATE(__nv_bfloat16, 2);
+        }
+        if (dv <= 128) GATE(float, 1);
+        GATE(float, 2);
+#undef GATE
+    }
     if (dtype == DE_BF16)
         return de_launch(head_gate_kernel<__nv_bfloat16>, grid, dim3(warps * 32), 0, s, o, gate,
                          ld_gate, weight, (__nv_bfloat16*)out, n, H, dv, eps, mode);

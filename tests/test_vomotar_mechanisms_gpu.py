@@ -307,6 +307,32 @@ def test_values_are_cached_normalised(dtype):
     assert float(kp.float().abs().sum(dim=(1, 3))[1].sum()) == 0.0       # page 1 untouched
 
 
+@pytest.mark.parametrize("dv,pad", [(4, 4), (64, 0), (128, 8), (128, 2), (132, 4), (256, 0), (260, 4)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_head_gates_by_fours(dtype, dv, pad):
+    """Heads of whole groups of four values, up to 256 and beyond, gates at aligned and odd addresses."""
+    from distengine_b200.kernels import recurrent as rk
+    n, H = 5, 3
+    g = _gen(dv + pad)
+    o = torch.randn(n, H * dv, generator=g) * 5
+    gate32 = torch.randn(n, H * dv + pad, generator=g)
+    weight = torch.rand(dv, generator=g) + 0.5
+    out = torch.full((n, H * dv), float("nan"), dtype=dtype, device=DEV)
+    normed = pv.rms(o.double().view(n, H, dv), 1e-5)
+    rk.head_gate(o.to(DEV), gate32.to(DEV)[:, pad:], weight.to(DEV), out, H, dv, 1e-5)
+    want = normed * weight.double() * torch.sigmoid(gate32[:, pad:].double()).view(n, H, dv)
+    assert_close(out.view(n, H, dv), want, dtype, "sigmoid gate")
+    gate = gate32.to(dtype)
+    rk.head_gate(o.to(DEV), gate.to(DEV)[:, pad:], None, out, H, dv, 1e-5)
+    assert_close(out.view(n, H, dv), normed * pv.silu(gate[:, pad:].double()).view(n, H, dv), dtype,
+                 "silu gate")
+    if dv <= 132:
+        wide = torch.rand(H * dv, generator=g) + 0.5
+        rk.head_gate(o.to(DEV), gate.to(DEV)[:, pad:], wide.to(DEV), out, H, dv, 1e-5, spanning=True)
+        want = normed * wide.double().view(H, dv) * torch.sigmoid(gate[:, pad:].double()).view(n, H, dv)
+        assert_close(out.view(n, H, dv), want, dtype, "spanning gate")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_head_gates_and_mean_of_normed(dtype):
     from distengine_b200.kernels import recurrent as rk
