@@ -20,7 +20,7 @@
 // A cut of a portion changes the order of float32 sums only.
 //
 // Figures below: 2,048 tokens of 16 heads of 128 x 128 on B200.  The scan takes 0.37 us a
-// token for the delta rule, 760 us in all, by chunks 221 us; under a decay per head a layer with its
+// token for the delta rule, 760 us in all, by chunks 205 us; under a decay per head a layer with its
 // products took 1,861 us by the scan, 200 us by chunks (105 of them here).
 
 #include "common.cuh"
@@ -536,151 +536,199 @@ delta_solve_kernel(const float* __restrict__ at, const float* __restrict__ v, in
 }
 
 // The chain from chunk to chunk: states[item] = the state before the chunk, u = X_v - X_k S0 in
-// X_v's place, then the state after it.  grid (portions, H, dv / 16), 2 DK threads: a block has 16
-// columns of a head's state, a warp 16 of its rows in registers.  For u every warp sums over its own
-// rows; the warps' parts meet in shared memory.  The next chunk's operands arrive meanwhile.
-// 106 us, 3.3 us a chunk: 62 % of what shared memory can pass (128 blocks, one an SM; columns in
-// slices of 16 are what gives the chain a block on most SMs).
-constexpr int PC = 16, PLD = PC + 4;
+// X_v's place, then the state after it.  grid (portions, H, dv / 16), 4 DK + 64 threads: a block has 16
+// columns of a head's state in two sides of eight, and each side's 2 DK threads go through the chunks by
+// themselves, a warp 16 rows of the state.  For u every warp sums over its own rows; the warps' parts
+// meet in shared memory.  Two warps more bring the chunks' operands, which both sides read, through two
+// stages, so that one side's multiply-adds fill the other's waits.  88 us, 2.8 us a chunk, shared
+// memory's pipe at work in 62 % of the cycles (128 blocks, one an SM; columns in slices of 16 are what
+// gives the chain a block on most SMs).  All 16 columns on eight warps that wait for one another three
+// times a chunk took 105 us, on 16 warps 109; four warps to bring the operands instead of two, 4 us more.
+constexpr int PC = 16, PS = PC / 2, BRING = 64;
 template <int DK> struct Pass {
     static constexpr int W = DK + 4;
-    static constexpr int STAGE = DK * LD + CH * W + CH * PLD;  // xkt, kh, xv
-    static constexpr int WARPS = DK / 16, THREADS = 2 * DK;
-    static constexpr size_t SMEM =
-        (size_t)(2 * STAGE + DK * PLD + CH * PLD + WARPS * CH * PLD) * sizeof(float);
+    static constexpr int STAGE = DK * LD + CH * W;             // xkt, kh
+    static constexpr int WARPS = DK / 16, SIDE = 2 * DK;       // of a side
+    static constexpr int THREADS = 2 * SIDE + BRING;
+    static constexpr int OWN = DK * PS + CH * PS + WARPS * CH * PS;      // floats of a side: S0, u, parts
+    static constexpr size_t SMEM = (size_t)(2 * STAGE + 2 * OWN) * sizeof(float);
 };
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
 
 template <int DK>
-__global__ void __launch_bounds__(2 * DK)
+__global__ void __launch_bounds__(4 * DK + BRING)
 delta_pass_kernel(const float* __restrict__ xkt, const float* __restrict__ kh,
                   const float* __restrict__ bn, float* __restrict__ xv, float* __restrict__ states,
                   const Portion* __restrict__ portions, int begin, int m,
                   float* __restrict__ state, long long slot_stride,
                   const int* __restrict__ seq_slot, int H, int dv) {
     constexpr int W = Pass<DK>::W, STAGE = Pass<DK>::STAGE, WARPS = Pass<DK>::WARPS;
-    constexpr int THREADS = Pass<DK>::THREADS;
+    constexpr int SIDE = Pass<DK>::SIDE;
     extern __shared__ __align__(16) float sh[];
-    float* ss = sh + 2 * STAGE;                      // [DK][PLD]: the state before the chunk
-    float* us = ss + DK * PLD;                       // [CH][PLD]
-    float* red = us + CH * PLD;                      // [WARPS][CH][PLD]
     const Portion p = part_of(portions[blockIdx.x], begin, m);
-    const int h = blockIdx.y, j0 = blockIdx.z * PC;
-    if (p.chunks == 0) {
-        pdl_wait();
+    const int h = blockIdx.y;
+    pdl_wait();
+    if (p.chunks == 0) return;
+    // named barriers: 1 + side within a side, 3 + 2 side + stage "landed", 7 + 2 side + stage "used"
+    if (threadIdx.x >= 2 * SIDE) {
+        const int tid = threadIdx.x - 2 * SIDE;
+        for (int n = 0; n < p.chunks; ++n) {
+            float* st = sh + (n & 1) * STAGE;
+            if (n >= 2) {
+                bar_sync(7 + (n & 1), SIDE + BRING);
+                bar_sync(9 + (n & 1), SIDE + BRING);
+            }
+            const size_t where = (size_t)(p.first + n) * H + h;
+            const float* a = xkt + where * DK * CH;
+            const float* b = kh + where * CH * DK;
+#pragma unroll 8
+            for (int e = tid; e < DK * 16; e += BRING)
+                cp16(st + (e >> 4) * LD + (e & 15) * 4, a + e * 4, true);
+#pragma unroll 8
+            for (int e = tid; e < CH * DK / 4; e += BRING)
+                cp16(st + DK * LD + e / (DK / 4) * W + e % (DK / 4) * 4, b + e * 4, true);
+            cp_commit();
+            cp_wait<0>();
+            __threadfence_block();
+            bar_arrive(3 + (n & 1), SIDE + BRING);
+            bar_arrive(5 + (n & 1), SIDE + BRING);
+        }
+        pdl_trigger();
         return;
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // for u: eight groups of four tokens (and four more 32 on) by four of four columns; for S: four
-    // groups of four rows by eight of two columns.  (Lanes l and l ^ 1, or l ^ 2, share one of the two.)
-    const int a4 = ((lane & 1) | ((lane >> 1) & 6)) * 4, j4 = (((lane >> 1) & 1) | ((lane >> 3) & 2)) * 4;
-    const int j2 = a4 / 2, c0 = warp * 16 + j4;
-    pdl_wait();
+    const int side = threadIdx.x >= SIDE, tid = threadIdx.x - side * SIDE;
+    const int warp = tid >> 5, lane = tid & 31, rows0 = warp * 16;
+    // [DK][PS]: the state before the chunk, of each 16 rows row r at r % 4 * 4 + r / 4
+    float* ss = sh + 2 * STAGE + side * Pass<DK>::OWN;
+    float* us = ss + DK * PS;                                  // [CH][PS], token t at place(t)
+    float* red = us + CH * PS;                                 // [WARPS][CH][PS], likewise
+    // place(t) = t % 4 * 16 + t / 4: what lanes side by side write or read lies side by side
+    const int j0 = blockIdx.z * PC + side * PS;
+    // for u: 16 groups of four tokens by two of four columns
+    const int tg = (lane & 1) | ((lane >> 1) & 14), j4 = ((lane >> 1) & 1) * 4;
+    // for S: four groups of four rows by two of four columns, and of 16 tokens four; the sums over the
+    // tokens meet, and a thread keeps four columns of one row
+    const int c4 = rows0 + ((lane & 1) | ((lane >> 1) & 2)) * 4, part = lane >> 3;
+    const int row = c4 + (lane >> 4) * 2 + ((lane >> 3) & 1);
+    const int row_place = rows0 + ((row & 3) * 4 + ((row & 15) >> 2));
+    // u's tokens: half of the warps' parts each on lanes 16 apart
+    const int e = warp * 16 + (lane & 15), upper = lane >> 4;
     float* slot = state + (size_t)seq_slot[p.seq] * slot_stride + (size_t)h * DK * dv + j0;
-    auto load = [&](int n) {
-        float* st = sh + (n & 1) * STAGE;
-        const size_t where = (size_t)(p.first + n) * H + h;
-        const float* a = xkt + where * DK * CH;
-        const float* b = kh + where * CH * DK;
-        const float* x = xv + where * CH * dv + j0;
-        for (int e = threadIdx.x; e < DK * 16; e += THREADS)
-            cp16(st + (e >> 4) * LD + (e & 15) * 4, a + e * 4, true);
-        for (int e = threadIdx.x; e < CH * DK / 4; e += THREADS)
-            cp16(st + DK * LD + e / (DK / 4) * W + e % (DK / 4) * 4, b + e * 4, true);
-        for (int e = threadIdx.x; e < CH * 4; e += THREADS)
-            cp16(st + DK * LD + CH * W + (e >> 2) * PLD + (e & 3) * 4,
-                 x + (size_t)(e >> 2) * dv + (e & 3) * 4, true);
-        cp_commit();
-    };
-    load(0);
-    float2 S[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        S[i] = *reinterpret_cast<const float2*>(slot + (size_t)(c0 + i) * dv + j2);
+    float4 S = four(slot + (size_t)row * dv + j4);
     for (int n = 0; n < p.chunks; ++n) {
         const size_t where = (size_t)(p.first + n) * H + h;
-        const float4 b = four(bn + where * DK + c0);
+        const float b = bn[where * DK + row];
+        float4 u[CH * PS / 4 / (WARPS * 16)];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            *reinterpret_cast<float2*>(states + (where * DK + c0 + i) * dv + j0 + j2) = S[i];
-            *reinterpret_cast<float2*>(ss + (c0 + i) * PLD + j2) = S[i];
+        for (int i = 0; i < CH * PS / 4 / (WARPS * 16); ++i) {
+            const int at = e + i * WARPS * 16, t = (at >> 1) % 16 * 4 + (at >> 5);
+            u[i] = four(xv + (where * CH + t) * dv + j0 + (at & 1) * 4);
         }
-        cp_wait<0>();
-        __syncthreads();                 // the chunk has landed, the one before it has been used
-        if (n + 1 < p.chunks) load(n + 1);
+        *reinterpret_cast<float4*>(states + (where * DK + row) * dv + j0 + j4) = S;
+        *reinterpret_cast<float4*>(ss + row_place * PS + j4) = S;
+        bar_sync(3 + 2 * side + (n & 1), SIDE + BRING);        // the chunk has landed, S0 is written
         const float* st = sh + (n & 1) * STAGE;
         {
             // X_k S0 over this warp's rows of the state
-            unsigned long long acc[8][2];
+            unsigned long long acc[4][2];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = 0ull;
-            const float* xa = st + warp * 16 * LD + a4;
-            const float* sb = ss + warp * 16 * PLD + j4;
-#pragma unroll 8
+            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
+            const float* xa = st + rows0 * LD + tg * 4;
+            const float* sb = ss + rows0 * PS + j4;
+#pragma unroll
             for (int c = 0; c < 16; ++c) {
-                const float4 t0 = four(xa + c * LD), t1 = four(xa + c * LD + 32);
-                const float4 y = four(sb + c * PLD);
-                const float v[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+                const float4 t = four(xa + c * LD), y = four(sb + (c % 4 * 4 + c / 4) * PS);
+                const float v[4] = {t.x, t.y, t.z, t.w};
                 const unsigned long long y0 = pair(y.x, y.y), y1 = pair(y.z, y.w);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     const unsigned long long vv = pair(v[i], v[i]);
                     fma2(acc[i][0], vv, y0);
                     fma2(acc[i][1], vv, y1);
                 }
             }
-            float* rd = red + warp * CH * PLD + j4;
+            float* rd = red + (warp * CH + tg) * PS + j4;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < 4; ++i) {
                 float4 r;
                 unpair(acc[i][0], r.x, r.y);
                 unpair(acc[i][1], r.z, r.w);
-                *reinterpret_cast<float4*>(rd + (a4 + (i & 3) + (i >> 2) * 32) * PLD) = r;
+                *reinterpret_cast<float4*>(rd + i * 16 * PS) = r;
             }
         }
-        __syncthreads();
-        for (int e = threadIdx.x; e < CH * 4; e += THREADS) {
-            const int t = e >> 2, c = (e & 3) * 4;
-            float4 u = four(st + DK * LD + CH * W + t * PLD + c);
-            float4 sum = four(red + t * PLD + c);
+        bar_sync(1 + side, SIDE);
 #pragma unroll
-            for (int w = 1; w < WARPS; ++w) {
-                const float4 r = four(red + (w * CH + t) * PLD + c);
+        for (int i = 0; i < CH * PS / 4 / (WARPS * 16); ++i) {
+            const int at = e + i * WARPS * 16, t = (at >> 1) % 16 * 4 + (at >> 5);
+            const float* from = red + upper * (WARPS / 2) * CH * PS + at * 4;
+            float4 sum = four(from);
+#pragma unroll
+            for (int w = 1; w < WARPS / 2; ++w) {
+                const float4 r = four(from + w * CH * PS);
                 sum.x += r.x; sum.y += r.y; sum.z += r.z; sum.w += r.w;
             }
-            u.x -= sum.x; u.y -= sum.y; u.z -= sum.z; u.w -= sum.w;
-            *reinterpret_cast<float4*>(us + t * PLD + c) = u;
-            *reinterpret_cast<float4*>(xv + (where * CH + t) * dv + j0 + c) = u;
+            sum.x += __shfl_xor_sync(0xffffffffu, sum.x, 16);
+            sum.y += __shfl_xor_sync(0xffffffffu, sum.y, 16);
+            sum.z += __shfl_xor_sync(0xffffffffu, sum.z, 16);
+            sum.w += __shfl_xor_sync(0xffffffffu, sum.w, 16);
+            const float4 out = make_float4(u[i].x - sum.x, u[i].y - sum.y, u[i].z - sum.z, u[i].w - sum.w);
+            *reinterpret_cast<float4*>(upper ? xv + (where * CH + t) * dv + j0 + (at & 1) * 4
+                                             : us + at * 4) = out;
         }
-        __syncthreads();
+        bar_sync(1 + side, SIDE);
         {
             // S <- diag(b_n) S + sum over the tokens of kh u
-            unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
-            const float bv[4] = {b.x, b.y, b.z, b.w};
-            const float* ka = st + DK * LD + c0;
-            const float* ub = us + j2;
-#pragma unroll 16
-            for (int s = 0; s < CH; ++s) {
-                const float4 kk = four(ka + s * W);
-                const unsigned long long u =
-                    *reinterpret_cast<const unsigned long long*>(ub + s * PLD);
-                fma2(acc[0], pair(kk.x, kk.x), u);
-                fma2(acc[1], pair(kk.y, kk.y), u);
-                fma2(acc[2], pair(kk.z, kk.z), u);
-                fma2(acc[3], pair(kk.w, kk.w), u);
-            }
+            unsigned long long acc[4][2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                float d0, d1;
-                unpair(acc[i], d0, d1);
-                S[i].x = fmaf(bv[i], S[i].x, d0);
-                S[i].y = fmaf(bv[i], S[i].y, d1);
+            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;
+            const float* ka = st + DK * LD + part * 4 * W + c4;
+            const float* ub = us + part * PS + j4;
+#pragma unroll
+            for (int s16 = 0; s16 < 4; ++s16)                  // tokens 16 s16 + 4 part + i
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 kk = four(ka + (s16 * 16 + i) * W);
+                    const float4 y = four(ub + (i * 16 + s16 * 4) * PS);
+                    const float v[4] = {kk.x, kk.y, kk.z, kk.w};
+                    const unsigned long long y0 = pair(y.x, y.y), y1 = pair(y.z, y.w);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const unsigned long long vv = pair(v[r], v[r]);
+                        fma2(acc[r][0], vv, y0);
+                        fma2(acc[r][1], vv, y1);
+                    }
+                }
+            if (n + 2 < p.chunks) bar_arrive(7 + 2 * side + (n & 1), SIDE + BRING);
+            float d[4][4], two[2][4], one[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                unpair(acc[r][0], d[r][0], d[r][1]);
+                unpair(acc[r][1], d[r][2], d[r][3]);
             }
+            const bool q = lane & 16, o = lane & 8;
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+                    two[r][x] = (q ? d[2 + r][x] : d[r][x]) +
+                                __shfl_xor_sync(0xffffffffu, q ? d[r][x] : d[2 + r][x], 16);
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+                one[x] = (o ? two[1][x] : two[0][x]) +
+                         __shfl_xor_sync(0xffffffffu, o ? two[0][x] : two[1][x], 8);
+            S.x = fmaf(b, S.x, one[0]);
+            S.y = fmaf(b, S.y, one[1]);
+            S.z = fmaf(b, S.z, one[2]);
+            S.w = fmaf(b, S.w, one[3]);
         }
     }
     pdl_trigger();
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<float2*>(slot + (size_t)(c0 + i) * dv + j2) = S[i];
+    *reinterpret_cast<float4*>(slot + (size_t)row * dv + j4) = S;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -862,7 +910,7 @@ DE_EXPORT int de_delta_chunks(const float* q, int ldq, const float* k, int ldk, 
         RUN(de_launch(delta_solve_kernel<DK>, sgrid, dim3(64), ssmem, s, (const float*)at, v,   \
                       ldv, (const float*)kd, beta, ldb, it, xv, xkt, H, dv));                   \
         RUN(need_smem((const void*)delta_pass_kernel<DK>, Pass<DK>::SMEM));             \
-        RUN(de_launch(delta_pass_kernel<DK>, pgrid, dim3(2 * DK), Pass<DK>::SMEM, s,            \
+        RUN(de_launch(delta_pass_kernel<DK>, pgrid, dim3(Pass<DK>::THREADS), Pass<DK>::SMEM, s, \
                       (const float*)xkt, (const float*)kh, (const float*)bn, xv, states, po,    \
                       begin, m, state, slot_stride, seq_slot, H, dv));                          \
     } while (0)
