@@ -394,29 +394,26 @@ __global__ void silu_rows_kernel(const T* __restrict__ proj, int ld, float* __re
     }
 }
 
-// The same in rows of whole groups of four: 2,048 rows of 6,144 columns 25 us (an element a
-// thread: 38).
+// The same in rows of whole groups of four: a block four rows of 1,024 columns, a thread one group of
+// each.  Bound by the instructions of the exponential and the quotient.  2,048 rows
+// of 6,144 columns 15 us (groups counted through all rows, a division each: 25; an element a thread: 31).
 template <typename T>
 __global__ void __launch_bounds__(256)
-silu_rows_vec_kernel(const T* __restrict__ proj, int ld, float* __restrict__ out, unsigned quads,
-                     unsigned total) {
+silu_rows_vec_kernel(const T* __restrict__ proj, int ld, float* __restrict__ out, int n, int cols) {
+    const int c = (int)(blockIdx.x * 256 + threadIdx.x) * 4;
     pdl_wait();
     pdl_trigger();
-    const unsigned step = gridDim.x * 256;
-    for (unsigned first = blockIdx.x * 256 + threadIdx.x; first < total; first += 4 * step) {
+    if (c >= cols) return;
+    for (int r0 = (int)blockIdx.y * 4; r0 < n; r0 += (int)gridDim.y * 4) {
         float4 v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const unsigned e = first + u * step;
-            if (e < total) v[u] = load_four(proj + (size_t)(e / quads) * ld + e % quads * 4);
-        }
+        for (int u = 0; u < 4; ++u)
+            if (r0 + u < n) v[u] = load_four(proj + (size_t)(r0 + u) * ld + c);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const unsigned e = first + u * step;
-            if (e < total)
-                store_four(out + (size_t)e * 4, make_float4(silu_f(v[u].x), silu_f(v[u].y),
-                                                            silu_f(v[u].z), silu_f(v[u].w)));
-        }
+        for (int u = 0; u < 4; ++u)
+            if (r0 + u < n)
+                store_four(out + (size_t)(r0 + u) * cols + c,
+                           make_float4(silu_f(v[u].x), silu_f(v[u].y), silu_f(v[u].z), silu_f(v[u].w)));
     }
 }
 
@@ -1081,19 +1078,18 @@ DE_EXPORT int de_silu_rows(int dtype, const void* proj, int ld, float* out, int 
     if (n <= 0 || cols <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t total = (size_t)n * cols;
-    // groups of four from 600,000 elements on (us, an element a thread and so: 8 rows of 6,144 1.5 and
-    // 3.1, 300 of 1,536 2.7 and 3.2, 100 of 6,144 3.4 and 3.4, 2,048 of 6,144 31 and 20): with few
-    // elements four loads a thread one after the other are a longer chain on fewer blocks
-    if (total >= 600000 && cols % 4 == 0 && ld % 4 == 0 &&
-        (uintptr_t)proj % (dtype == DE_BF16 ? 8 : 16) == 0 && (uintptr_t)out % 16 == 0 &&
-        total / 4 < (1u << 30)) {
-        const unsigned quads = (unsigned)(total / 4), fours = (quads + 1023) / 1024;
-        const dim3 grid(fours < 148 * 8 ? fours : 148 * 8);
+    // groups of four from 400,000 elements on (us, an element a thread and so: 8 rows of 6,144 1.3 and
+    // 2.1, 64 of 6,144 2.3 and 2.2, 300 of 1,536 2.5 and 2.3, 2,048 of 6,144 31 and 13): with few
+    // elements four loads a thread are a longer chain on fewer blocks
+    if (total >= 400000 && cols % 4 == 0 && ld % 4 == 0 &&
+        (uintptr_t)proj % (dtype == DE_BF16 ? 8 : 16) == 0 && (uintptr_t)out % 16 == 0) {
+        const int fours = n / 4 + (n % 4 != 0);
+        const dim3 grid((cols / 4 + 255) / 256, fours < 65535 ? fours : 65535);
         if (dtype == DE_BF16)
             return de_launch(silu_rows_vec_kernel<__nv_bfloat16>, grid, dim3(256), 0, s,
-                             (const __nv_bfloat16*)proj, ld, out, (unsigned)cols / 4, quads);
+                             (const __nv_bfloat16*)proj, ld, out, n, cols);
         return de_launch(silu_rows_vec_kernel<float>, grid, dim3(256), 0, s, (const float*)proj, ld,
-                         out, (unsigned)cols / 4, quads);
+                         out, n, cols);
     }
     size_t blocks = (total + 255) / 256;
     if (blocks > 148 * 32) blocks = 148 * 32;

@@ -211,6 +211,14 @@ def test_silu_of_many_rows(dtype, n, cols):
     assert (out.double().cpu() - want).abs().max().item() <= 8 * EPS * want.abs().max().item()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,cols", [(97, 4100), (100, 4000), (781, 516), (3, 140004)])
+def test_silu_of_rows_by_fours(dtype, n, cols):
+    """Around the 400,000 elements from which a thread takes a group of four of four rows, remainders of
+    four rows and of 1,024 columns among them."""
+    test_silu_of_many_rows(dtype, n, cols)
+
+
 def _walk(rule, lens, inputs, state, H, dk, dv, begin=0):
     """The tokens from ``begin`` on of one sequence, in steps of ``lens``: portions of 192 tokens and
     more by chunks, others by the scan.  Returns the read-outs."""
