@@ -189,24 +189,53 @@ __device__ __forceinline__ void angles(float* tab, const float* __restrict__ fre
     for (int i = threadIdx.x; i < half; i += blockDim.x)
         sincosf(pos * freq[i], tab + half + i, tab + i);
 }
-// four neighbouring pairs (i, i + half) of src turned into dst
-template <typename T>
-__device__ __forceinline__ void turn_four(const T* src, T* dst, const float* tab, int half, int i) {
-    const float4 a = load_four(src + i), b = load_four(src + i + half);
-    const float4 c = load_four(tab + i), s = load_four(tab + half + i);
-    float4 x, y;
-    rope_rotate(a.x, b.x, c.x, s.x, x.x, y.x);
-    rope_rotate(a.y, b.y, c.y, s.y, x.y, y.y);
-    rope_rotate(a.z, b.z, c.z, s.z, x.z, y.z);
-    rope_rotate(a.w, b.w, c.w, s.w, x.w, y.w);
-    store_four(dst + i, x);
-    store_four(dst + i + half, y);
+// E (4 or 8) neighbouring features, in 16-byte pieces (four of bfloat16: 8 bytes)
+template <int E, typename T> __device__ __forceinline__ void load_features(const T* p, float (&v)[E]) {
+    if constexpr (E == 8 && sizeof(T) == 2) {
+        const uint4 u = *reinterpret_cast<const uint4*>(p);
+        const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < E; ++i)
+            v[i] = __uint_as_float(i & 1 ? w[i / 2] & 0xffff0000u : w[i / 2] << 16);
+    } else {
+#pragma unroll
+        for (int i = 0; i < E; i += 4) {
+            const float4 f = load_four(p + i);
+            v[i] = f.x; v[i + 1] = f.y; v[i + 2] = f.z; v[i + 3] = f.w;
+        }
+    }
+}
+template <int E, typename T> __device__ __forceinline__ void store_features(T* p, const float (&v)[E]) {
+    if constexpr (E == 8 && sizeof(T) == 2) {
+        __nv_bfloat162 w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(w);
+    } else {
+#pragma unroll
+        for (int i = 0; i < E; i += 4) store_four(p + i, make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+    }
+}
+// E neighbouring pairs (i, i + half) of src turned into dst
+template <int E, typename T>
+__device__ __forceinline__ void turn_features(const T* src, T* dst, const float* tab, int half, int i) {
+    float a[E], b[E], c[E], s[E], x[E], y[E];
+    load_features<E>(src + i, a);
+    load_features<E>(src + i + half, b);
+    load_features<E>(tab + i, c);
+    load_features<E>(tab + half + i, s);
+#pragma unroll
+    for (int e = 0; e < E; ++e) rope_rotate(a[e], b[e], c[e], s[e], x[e], y[e]);
+    store_features<E>(dst + i, x);
+    store_features<E>(dst + i + half, y);
 }
 
-// The same in groups of four features, the token's angles formed once for all heads: where half the
+// The same in groups of E features, the token's angles formed once for all heads: where half the
 // turned part, the plain part and the values' (half) rows are whole groups, and everything lies at
-// such addresses.  2,048 tokens, 16 + 4 heads of 128: 13 us (23, each head forming its angles).
-template <typename T>
+// such addresses.  2,048 tokens, 16 + 4 heads of 128, a product before
+// it: 5.9 us in groups of eight, 7.3 in groups of four, whose last round is a quarter of the block (cold
+// 13, and 23 with each head forming its angles).
+template <typename T, int E>
 __global__ void kv_write_rotated_vec_kernel(
     T* __restrict__ proj, int ld, const int* __restrict__ positions,
     const int* __restrict__ token_slot, const float* __restrict__ fk, int rot,
@@ -232,23 +261,31 @@ __global__ void kv_write_rotated_vec_kernel(
     if (can_write && fv != nullptr) angles(vtab, fv, vhalf, (float)pos);
     __syncthreads();
     pdl_wait();
-    const int per = (dk - half) / 4;                 // groups of pairs, then plain groups
-    const int qk_heads = H + (can_write ? G : 0);
-    for (int idx = threadIdx.x; idx < qk_heads * per; idx += blockDim.x) {
-        const int h = idx / per, i = (idx - h * per) * 4;
-        T* src = row + h * dk;
-        T* dst = h < H ? src : k_pages + (at + (size_t)(h - H) * page) * dk;   // q in place
-        if (i < half) turn_four(src, dst, ktab, half, i);
-        else if (h >= H) store_four(dst + i + half, load_four(src + i + half));
-    }
-    if (can_write) {
-        const T* vs = row + (H + G) * dk;
-        const int vper = (fv != nullptr ? vhalf : dv) / 4;
-        for (int idx = threadIdx.x; idx < G * vper; idx += blockDim.x) {
-            const int h = idx / vper, i = (idx - h * vper) * 4;
+    // groups of pairs, then plain groups, of queries and keys; then the values'
+    const int per = (dk - half) / E, vper = (fv != nullptr ? vhalf : dv) / E;
+    const int of_qk = (H + (can_write ? G : 0)) * per, total = of_qk + (can_write ? G * vper : 0);
+    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+        float plain[E];
+        if (idx < of_qk) {
+            const int h = idx / per, i = (idx - h * per) * E;
+            T* src = row + h * dk;
+            T* dst = h < H ? src : k_pages + (at + (size_t)(h - H) * page) * dk;   // q in place
+            if (i < half) {
+                turn_features<E>(src, dst, ktab, half, i);
+            } else if (h >= H) {
+                load_features<E>(src + i + half, plain);
+                store_features<E>(dst + i + half, plain);
+            }
+        } else {
+            const int h = (idx - of_qk) / vper, i = (idx - of_qk - h * vper) * E;
+            const T* src = row + (H + G) * dk + h * dv;
             T* dst = v_pages + (at + (size_t)h * page) * dv;
-            if (fv != nullptr) turn_four(vs + h * dv, dst, vtab, vhalf, i);
-            else store_four(dst + i, load_four(vs + h * dv + i));
+            if (fv != nullptr) {
+                turn_features<E>(src, dst, vtab, vhalf, i);
+            } else {
+                load_features<E>(src + i, plain);
+                store_features<E>(dst + i, plain);
+            }
         }
     }
     pdl_trigger();
@@ -2726,18 +2763,25 @@ DE_EXPORT int de_kv_write_rotated(int dtype, void* proj, int ld, const int* posi
     cudaStream_t s = (cudaStream_t)stream;
     const int work = (H + G) * dk + G * dv;
     const int threads = n >= 512 ? 128 : (work >= 2048 ? 512 : 256);
-    const size_t four = dtype == DE_BF16 ? 8 : 16;   // bytes of a group of four
-    if (rot % 8 == 0 && (dk - rot) % 4 == 0 && dv % (fv != nullptr ? 8 : 4) == 0 && ld % 4 == 0 &&
-        dk <= MAX_D && dv <= MAX_D && (uintptr_t)proj % four == 0 && (uintptr_t)k_pages % four == 0 &&
-        (uintptr_t)v_pages % four == 0) {
-#define ROT(T)                                                                                  \
-    return de_launch(kv_write_rotated_vec_kernel<T>, dim3(n), dim3(work >= 1024 ? 256 : 128), 0, s, \
-                     (T*)proj, ld, positions, token_slot, fk, rot, fv, H, G, dk, dv, (T*)k_pages, \
-                     (T*)v_pages, block_table, table_stride, page, num_pages, write_kv, status)
-        if (dtype == DE_BF16) ROT(__nv_bfloat16);
-        ROT(float);
+    // a group's features: eight of bfloat16 where everything is whole groups of them, else four
+    auto groups = [&](int e, size_t bytes) {
+        return rot % (2 * e) == 0 && (dk - rot) % e == 0 && dv % (fv != nullptr ? 2 * e : e) == 0 &&
+               ld % e == 0 && dk <= MAX_D && dv <= MAX_D && (uintptr_t)proj % bytes == 0 &&
+               (uintptr_t)k_pages % bytes == 0 && (uintptr_t)v_pages % bytes == 0;
+    };
+#define ROT(T, E)                                                                               \
+    do {                                                                                        \
+        const int items = (H + G) * ((dk - rot / 2) / E) + G * ((fv != nullptr ? dv / 2 : dv) / E); \
+        const int block = items >= 256 ? 256 : (items + 31) / 32 * 32;                          \
+        return de_launch(kv_write_rotated_vec_kernel<T, E>, dim3(n), dim3(block), 0, s,         \
+                         (T*)proj, ld, positions, token_slot, fk, rot, fv, H, G, dk, dv,        \
+                         (T*)k_pages, (T*)v_pages, block_table, table_stride, page, num_pages,  \
+                         write_kv, status);                                                     \
+    } while (0)
+    if (dtype == DE_BF16 && groups(8, 16)) ROT(__nv_bfloat16, 8);
+    if (dtype == DE_BF16 && groups(4, 8)) ROT(__nv_bfloat16, 4);
+    if (dtype != DE_BF16 && groups(4, 16)) ROT(float, 4);
 #undef ROT
-    }
     if (dtype == DE_BF16)
         return de_launch(kv_write_rotated_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0, s,
                          (__nv_bfloat16*)proj, ld, positions, token_slot, fk, rot, fv, H, G, dk, dv,

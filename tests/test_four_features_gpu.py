@@ -50,6 +50,32 @@ def test_rotation_and_cache_write(dtype, H, G, dk, dv, rot, turned, write):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("H,G,dk,dv,rot,turned", [(3, 1, 64, 64, 64, True), (4, 2, 128, 48, 32, True),
+                                                   (2, 2, 24, 8, 16, False), (8, 4, 256, 256, 256, True),
+                                                   (1, 1, 24, 16, 0, False), (4, 4, 72, 40, 64, True)])
+@pytest.mark.parametrize("write", [True, False])
+def test_rotation_in_groups_of_eight(H, G, dk, dv, rot, turned, write):
+    """bfloat16 rows of whole groups of eight, and where only groups of four fit: the same bits."""
+    from distengine_b200.kernels import recurrent as rk
+    lens, page, g = (5, 1, 9), 8, _gen(dk)
+    ctx = _ctx(lens, (3, 900, 0), (1, 0, 2))
+    n = sum(lens)
+    proj = torch.randn(n, H * dk + G * (dk + dv), generator=g).to(torch.bfloat16)
+    fk, fv = torch.rand(rot // 2, generator=g).to(DEV), torch.rand(dv // 2, generator=g).to(DEV)
+    table = torch.full((3, 120), -1, dtype=torch.int32)
+    table[1, 0], table[0, 112], table[2, 0], table[2, 1] = 2, 0, 3, 1
+    results = []
+    for pad in (8 - proj.shape[1] % 8, 12 - proj.shape[1] % 8):
+        p = _rows(proj, pad)
+        kp = torch.zeros(4, G, page, dk, dtype=torch.bfloat16, device=DEV)
+        vp = torch.zeros(4, G, page, dv, dtype=torch.bfloat16, device=DEV)
+        rk.kv_write_rotated(p, fk, rot, fv if turned else None, H, G, dk, dv, kp, vp, table.to(DEV),
+                            write, ctx)
+        results.append((p.clone(), kp, vp))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("K", [1, 2, 4, 5])
 @pytest.mark.parametrize("biased", [True, False])
