@@ -21,7 +21,7 @@
 //
 // Figures below: 2,048 tokens of 16 heads of 128 x 128 on B200.  The scan takes 0.37 us a
 // token for the delta rule, 760 us in all, by chunks 205 us; under a decay per head a layer with its
-// products took 1,861 us by the scan, 200 us by chunks (105 of them here).
+// products took 1,861 us by the scan, 194 us by chunks (98 of them here).
 
 #include "common.cuh"
 
@@ -98,7 +98,7 @@ struct Tile {
     }
     // rows of a [k][LD] against columns of b [k][LD], n values of k
     template <int N> __device__ __forceinline__ void add(const float* a, const float* b) {
-#pragma unroll 8
+#pragma unroll 16
         for (int k = 0; k < N; ++k) {
             const float4 a0 = four(a + k * LD + row), a1 = four(a + k * LD + row + 16);
             const float4 b0 = four(b + k * LD + col);
@@ -192,7 +192,7 @@ decay_products_kernel(const float* __restrict__ q, int ldq, const float* __restr
         cp_commit();
         cp_wait<0>();
         __syncthreads();
-        tile.add<64>(ks, qs);
+        if (warp != 2) tile.add<64>(ks, qs);         // (its 32 s lie behind its 32 t: zeros)
         for (int e = threadIdx.x; e < 64 * CH / 4; e += 128) {
             const int c = e >> 4, t = (e & 15) * 4;
             const float4 v = four(qs + c * LD + t);
@@ -770,7 +770,8 @@ chunk_out_kernel(const float* __restrict__ xt, const float* __restrict__ states,
         cp_wait<1>();
         __syncthreads();
         const float* a = sh + (step & 1) * 2 * 32 * LD;
-        tile.add<32>(a, a + 32 * LD);
+        // (the last 32 u say nothing to the first 32 tokens, which are the first two warps' rows)
+        if (step + 1 < steps || threadIdx.x >= 64) tile.add<32>(a, a + 32 * LD);
         __syncthreads();
     }
     pdl_trigger();
