@@ -17,7 +17,8 @@
 //
 // Long key ranges of decoded tokens are cut into chunks that separate blocks work on; each writes
 // an unnormalised partial result (accumulator, maximum, sum) into scratch memory, and
-// `attn_combine` merges the chunks of a row in ascending order.
+// `attn_combine` merges the chunks of a row in ascending order (in float32 steps of single tokens the
+// block that finishes a row last does, after the rotation and the cache's write in the same kernel).
 
 #include "common.cuh"
 

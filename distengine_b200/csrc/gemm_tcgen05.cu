@@ -2,8 +2,8 @@
 // float32 accumulation in tensor memory, for prompt portions (many rows of x).
 //
 // A persistent kernel, one block per SM, each block walking over 128 x bn tiles of the output
-// (bn a multiple of 32 up to 256, chosen by the host so that the last round of tiles over the SMs
-// wastes least), with the roles split over warps:
+// (bn a multiple of 32 up to 256, chosen by the host: the fewest rounds of tiles over the SMs, then
+// the narrowest tile), with the roles split over warps:
 //   * warp 0, one thread: moves 128 x 64 tiles of x and bn x 64 tiles of w into shared memory with
 //     TMA (cp.async.bulk.tensor.2d, 128-byte swizzle, zero fill outside the matrices), 4 stages
 //     deep, each stage guarded by a "full" mbarrier with a transaction count;
@@ -11,7 +11,7 @@
 //     shared-memory descriptors), four per stage, hands the stage back with tcgen05.commit on its
 //     "empty" mbarrier, and after a tile's last stage commits on the accumulator's "full" mbarrier;
 //   * warps 2-5: the epilogue.  The accumulator is double-buffered in tensor memory (2 x 256
-//     columns), so these warps read one tile with tcgen05.ld, convert and store it while the
+//     columns), so these warps read one tile with tcgen05.ld, convert, turn and store it while the
 //     tensor core already works on the next.  The gated epilogue computes silu(gate) * up from the
 //     two halves of the accumulator (src/layers/activation.py:6-9), so the activation costs no
 //     pass over memory and the product's [gate | up] output is never written.
