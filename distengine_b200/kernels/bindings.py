@@ -2,10 +2,12 @@
 functions' signatures, that takes the arguments off the interpreter's stack and calls the C function by
 its exact prototype.
 
-A launch function takes up to 42 arguments; ctypes converts them through an object each, 2 to 4 us a call
-(0.2 here).  Eager layers of a few launches are bound by the host: 64 single tokens through sink
-attention 71 -> 66 us a pass, 8 through a window layer 39 -> 32, through the gated delta rule 95 -> 85.  As with ctypes, the interpreter's lock is
-released during the call, ``None`` is a null pointer and integers are cut to the parameter's width.
+A launch function takes up to 42 arguments; ctypes converts them through an object each, 2 to 4 us a
+call (0.2 here).  Eager layers of a few launches are bound by the host: 64 single tokens through sink
+attention 71 -> 66 us a pass, 8 through a window layer 39 -> 32, through the gated delta rule 95 -> 85.
+As with ctypes, the interpreter's lock is released during the call, ``None`` is a null pointer and
+integers are cut to the parameter's width.  Where the interpreter has no headers to compile it with,
+``library`` calls the functions through ctypes.
 """
 
 from __future__ import annotations

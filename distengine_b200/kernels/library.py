@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 from ctypes import c_float, c_int, c_void_p
 
 from . import bindings as _bindings
@@ -197,22 +198,38 @@ def bindings_source() -> str:
     return _bindings.source(_all_letters())
 
 
-_bind = None
+_bind = None         # of the bindings; False where they cannot be had
+
+
+def _bound():
+    """``bindings``' function that binds a C function, or False: an interpreter without its headers
+    cannot have the extension, and the functions are then called through ctypes."""
+    global _bind
+    if _bind is None:
+        try:
+            _bind = _bindings.load(_build.build_bindings(bindings_source())).bind
+        except (_build.BuildError, OSError, ImportError) as error:
+            _bind = False
+            print("[distengine_b200] kernels are called through ctypes (2 to 4 us more a call): "
+                  f"{error}", file=sys.stderr, flush=True)
+    return _bind
 
 
 class Library:
-    """A kernel library: the functions of ``SIGNATURES`` as ``bindings`` calls them; anything else
-    that it exports through ctypes."""
+    """A kernel library: the functions of ``SIGNATURES`` as ``bindings`` calls them, or through
+    ctypes where there are no bindings; anything else that it exports through ctypes."""
 
     def __init__(self, cdll: ctypes.CDLL, functions: dict[str, list]) -> None:
-        global _bind
+        bind = _bound()
         letters = _all_letters()
-        if _bind is None:
-            _bind = _bindings.load(_build.build_bindings(bindings_source())).bind
         self._cdll = cdll
         for name, argtypes in functions.items():
-            address = ctypes.cast(getattr(cdll, name), c_void_p).value
-            setattr(self, name, _bind(letters.index(_letters(argtypes)), address))
+            fn = getattr(cdll, name)
+            if bind:
+                fn = bind(letters.index(_letters(argtypes)), ctypes.cast(fn, c_void_p).value)
+            else:
+                fn.argtypes, fn.restype = argtypes, c_int
+            setattr(self, name, fn)
 
     def __getattr__(self, name: str):
         return getattr(self._cdll, name)
@@ -226,7 +243,7 @@ def load(module: str, defines: tuple[str, ...] = ()) -> Library:
     try:
         path = _build.build(module, defines)
         lib = Library(ctypes.CDLL(path), SIGNATURES[module])
-    except (_build.BuildError, OSError, ImportError) as error:
+    except (_build.BuildError, OSError) as error:
         raise KernelsUnavailable(
             f"the CUDA kernel library '{module}' of distengine_b200 could not be built or "
             f"loaded: {error}") from error

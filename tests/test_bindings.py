@@ -55,3 +55,26 @@ def test_kernel_functions_through_both():
         assert lib.de_gemm_f32_form(*sizes) == plain(*sizes)
     with pytest.raises(AttributeError):
         lib.no_such_function
+
+
+def test_without_the_interpreters_headers(tmp_path, monkeypatch):
+    """No Python.h: the extension cannot be made, and the functions come through ctypes."""
+    want = library.load("gemm_f32").de_gemm_f32_form(8, 131, 600, 1)
+    make, folder = build.build_bindings, build._build_dir
+
+    def make_anew(text):                     # (not the one that was made before)
+        monkeypatch.setattr(build, "_build_dir", lambda: str(tmp_path))
+        try:
+            return make(text)
+        finally:
+            monkeypatch.setattr(build, "_build_dir", folder)
+    monkeypatch.setattr(bindings, "include_dir", lambda: str(tmp_path))
+    monkeypatch.setattr(build, "build_bindings", make_anew)
+    monkeypatch.setattr(library, "_bind", None)
+    monkeypatch.setattr(library, "_loaded", {})
+    lib = library.load("gemm_f32")
+    assert lib.de_gemm_f32_form(8, 131, 600, 1) == want
+    with pytest.raises(ctypes.ArgumentError):
+        lib.de_gemm_f32_form(8, 131, 600, 1.5)
+    monkeypatch.setattr(build, "build_many", lambda requests, verbose: ["kernels"])
+    assert build.build_all(verbose=False) == ["kernels"]
