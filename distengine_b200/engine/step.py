@@ -218,7 +218,7 @@ class StepRunner:
                 count = self._portion_shapes[shape] = self._portion_shapes.get(shape, 0) + 1
                 if count > PORTION_REPEATS:
                     graph_shape = {"context_cap": cap}
-        prep = StepPrep(host, graph_shape)
+        prep = StepPrep(host, graph_shape, self.cache.page_size)
         self.model.prepare(prep)
         for name, array in (extra or {}).items():
             prep.add(name, array)

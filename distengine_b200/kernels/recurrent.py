@@ -440,7 +440,7 @@ def portion_kernels(dtype: torch.dtype, key_dim: int, value_dim: int) -> "tuple[
 def portion_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int, prep, heads: int,
                       kv_heads: int) -> int:
     """Rows of a tile of the chunk attention for a step with prompt portions: 128 (the tcgen05
-    kernel) or what ``chunk_rows_per_tile`` says.
+    kernel, where it takes the cache's pages) or what ``chunk_rows_per_tile`` says.
 
     A tile of 128 rows is two blocks of the tcgen05 kernel, two of which an SM holds.  It is the sooner
     one (us, heads of 128, 16 on 4, tiles of 32 / 64 / 128 rows) for one portion of 9 tokens behind
@@ -448,11 +448,13 @@ def portion_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int, prep, he
     500 43 / 53 / 39; with as many blocks as places also for 20 single tokens behind 600 keys beside a
     portion of 300 (46 / 59 / 43).  Not where tiles are mostly empty and take several rounds - 60
     single tokens beside it 54 / 62 / 77, 64 portions of 2 tokens 41 / 51 / 69 - or where many of
-    them have few keys each (16 portions of 40 tokens from position 0: 21 / 21 / 26)."""
+    them have few keys each (16 portions of 40 tokens from position 0: 21 / 21 / 26).  Where the pages
+    are not that kernel's, items of 128 rows would run on mma.sync in tiles of 64, whatever the step."""
     host = prep.host
     seq_qlen = host.seq_qlen
     wide = int(seq_qlen.max()) > 1
-    if wide and len(portion_kernels(dtype, key_dim, value_dim)) > 1:
+    if (wide and len(portion_kernels(dtype, key_dim, value_dim)) > 1
+            and (prep.page_size is None or _wide_ok(key_dim, value_dim, prep.page_size))):
         rows = seq_qlen.astype("int64") * (heads // kv_heads)
         tiles = int(((rows + WIDE_ROWS - 1) // WIDE_ROWS).sum())
         blocks, sms = 2 * tiles * kv_heads, _sms()

@@ -64,8 +64,12 @@ class Workspace:
 class StepPrep:
     """Host side of a step before upload: the batch's numpy arrays plus arrays that parts add."""
 
-    def __init__(self, host: SimpleNamespace, graph_shape: "dict[str, Any] | None" = None) -> None:
+    def __init__(self, host: SimpleNamespace, graph_shape: "dict[str, Any] | None" = None,
+                 page_size: "int | None" = None) -> None:
+        """``page_size``: tokens of a page of the step's cache; None: not known, then parts take it
+        for one that all kernels accept (the others run too, in tiles that suit them less)."""
         self.host = host
+        self.page_size = page_size
         self.extra: dict[str, np.ndarray] = {}
         self.notes: dict[str, Any] = {}
         # set when the step is being shaped for a replayed CUDA graph: parts must then produce

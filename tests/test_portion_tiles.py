@@ -1,0 +1,55 @@
+"""Rows of a tile of the attention with 32-bit weights, chosen from a step's lengths and the cache's page
+size alone, so it can be checked without a GPU (the kernel libraries are loaded, none of them runs)."""
+
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+import torch
+
+from distengine_b200.kernels import recurrent as rk
+from distengine_b200.parts.context import StepPrep
+
+
+def _prep(qlen, pos0, page, graph_shape=None):
+    host = SimpleNamespace(seq_qlen=np.array(qlen, dtype=np.int32),
+                           seq_pos0=np.array(pos0, dtype=np.int32))
+    return StepPrep(host, graph_shape, page)
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("qlen,pos0", [([9], [1900]), ([500], [0]), ([2048], [0]), ([30] * 4, [500] * 4),
+                                       ([300] + [1] * 20, [0] + [600] * 20), ([64], [0])])
+def test_pages_that_the_kernel_takes_and_others(dim, qlen, pos0, monkeypatch):
+    monkeypatch.setattr(rk, "_sms", lambda: 148)
+    host = _prep(qlen, pos0, None).host
+    without = rk.chunk_rows_per_tile(torch.bfloat16, dim, dim, True,
+                                     rk.long_portion_rows(host.seq_qlen, 16, 4))
+    for shape in (None, {"context_cap": 2048}):
+        for page in (1, 2, 4, 12, 20, 8, 16, 24, 64):
+            rows = rk.portion_tile_rows(torch.bfloat16, dim, dim, _prep(qlen, pos0, page, shape), 16, 4)
+            assert rows == (128 if page % 8 == 0 else without), page
+        assert rk.portion_tile_rows(torch.bfloat16, dim, dim, _prep(qlen, pos0, None, shape), 16, 4) == 128
+    assert without in (32, 64)
+    for dtype, size in ((torch.float32, dim), (torch.bfloat16, 96)):
+        rows = rk.portion_tile_rows(dtype, size, size, _prep(qlen, pos0, 16), 16, 4)
+        assert rows == rk.chunk_rows_per_tile(dtype, size, size, True,
+                                              rk.long_portion_rows(host.seq_qlen, 16, 4))
+
+
+@pytest.mark.parametrize("page", [4, 16])
+def test_a_steps_plan_knows_its_page_size(page, monkeypatch):
+    """``StepRunner`` tells the parts what pages its cache has."""
+    from distengine_b200.engine import step
+    from distengine_b200.kernels import ops
+    seen = []
+    monkeypatch.setattr(ops, "require_device", lambda device: None)
+    monkeypatch.setattr(torch.cuda, "Event", lambda: None)
+    monkeypatch.setattr(step.StepRunner, "_stage", lambda self, host, prep: ({}, [], 0, []))
+    model = SimpleNamespace(device=torch.device("cpu"), dtype=torch.float32,
+                            config=SimpleNamespace(vocabulary=10),
+                            prepare=lambda prep: seen.append(prep.page_size))
+    cache = SimpleNamespace(page_size=page, bindings=lambda: [], has=lambda r: True, reserve=lambda r: None,
+                            length=lambda r: 0, slot=lambda r: 0)
+    step.StepRunner(model, cache).prepare([step.StepEntry("a", [1, 2])])
+    assert seen == [page]
