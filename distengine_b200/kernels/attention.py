@@ -262,13 +262,15 @@ class AttentionLauncher:
                                      sm_count=self.sm_count())
             plan = build_plan(qlen, host.seq_pos0, self.group, self.kv_heads, shape.rows,
                               self.window, chunk, chunks_cap)
+            combine = plan.combine
             if prep.notes[self.key + "/decode"] is not None:
                 # (a tile a sequence: the items carry the token's position and slot instead of their
-                # rows and their tile)
+                # rows and their tile; the kernel merges by them)
                 seq = plan.items[:, 0]
                 plan.items[:, 1], plan.items[:, 7] = host.seq_pos0[seq], host.seq_slot[seq]
+                combine = combine[:0]
             prep.add(f"{self.key}/{shape.name}/items", plan.items)
-            prep.add(f"{self.key}/{shape.name}/combine", plan.combine)
+            prep.add(f"{self.key}/{shape.name}/combine", combine)
             notes[shape.name] = plan.num_partials
         prep.notes[self.key] = tuple(sorted(notes.items()))
 

@@ -130,3 +130,22 @@ def test_float32_tiles_by_the_blocks_of_a_step(qlen, pos0, heads, kv_heads, dim,
                 assert shape == "rows32" or not len(count["rows32"])
         assert arrays[1] == arrays[2]
 
+
+
+@pytest.mark.parametrize("graph_shape", [None, {"context_cap": 1536}])
+def test_float32_decode_steps_bring_no_list_of_merges(graph_shape):
+    """The one-launch kernel merges by its items; the kernels apart need the list."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from distengine_b200.kernels.attention import AttentionLauncher
+    from distengine_b200.parts.context import StepPrep
+    launcher = AttentionLauncher(torch.float32, 32, 4, 64, 1.0, None)
+    host = SimpleNamespace(seq_qlen=np.ones(3, dtype=np.int32), seq_slot=np.arange(3, dtype=np.int32),
+                           seq_pos0=np.array([5, 700, 1200], dtype=np.int32))
+    for fused in (True, False):
+        prep = StepPrep(host, graph_shape)
+        launcher.prepare(prep, allow_decode=fused)
+        assert (prep.notes[launcher.key + "/decode"] is not None) == fused
+        assert (len(prep.extra[f"{launcher.key}/rows8/combine"]) == 0) == fused
