@@ -31,8 +31,10 @@
 // 1,024 and a cap 156, 92, 96; prompts of 1,201 and 1,172 tokens 153, 100, 84; with distance slopes
 // 158, 139, 98; heads of 64 135, 86, 65.  Four threads a row instead of two: 134 instead of 114.
 //
-// Every wait is bounded (status 3; the block then runs to its end, waits for its own copies and frees
-// its tensor memory).
+// Every wait is bounded (status 3).  A thread whose wait ran out waits for nothing more but goes on to
+// the end; the issuer then issues nothing more, so that no other wait for it succeeds either and the
+// fetcher overwrites nothing.  The copies and products in flight are waited for, neither block of the
+// pair stores a result, and the tensor memory is freed.
 
 #include <cuda.h>
 
@@ -43,6 +45,10 @@
 #include "tensor_maps.cuh"
 
 DE_DEFINE_PDL_SWITCH
+
+#ifndef ROLE_SPINS                     // how often a wait of the tiles' loop looks before it gives up
+#define ROLE_SPINS tc5::SPIN_LIMIT
+#endif
 
 namespace {
 
@@ -112,6 +118,9 @@ __device__ __forceinline__ unsigned peer_address(const void* mine, int rank) {
     unsigned r;
     asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_u32(mine)), "r"(rank));
     return r;
+}
+__device__ __forceinline__ void store_peer(unsigned at, unsigned v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(at), "r"(v) : "memory");
 }
 __device__ __forceinline__ void store_peer(unsigned at, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(at), "f"(v) : "memory");
@@ -189,9 +198,11 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
     unsigned long long* s_done = bars + STAGES;                 // a tile's scores are complete
     unsigned long long* p_ready = bars + STAGES + 1;            // its weights are written (every thread arrives)
     unsigned long long* o_done = bars + STAGES + 2;             // its share of the results is complete
-    unsigned* gone_s = reinterpret_cast<unsigned*>(bars + STAGES + 3);   // [STAGES] boxes without a page
+    unsigned long long* drained = bars + STAGES + 3;            // the products of an issuer that gave up
+    unsigned* gone_s = reinterpret_cast<unsigned*>(bars + STAGES + 4);   // [STAGES] boxes without a page
     unsigned* spoilt_s = gone_s + STAGES;                       // [8]
     unsigned* tmem_slot = spoilt_s + 8;
+    volatile unsigned* gave_up_s = tmem_slot + 1;               // a wait of the pair ran out
 
     const int rank = blockIdx.x & 1;                            // in its pair of blocks
     const WorkItem it = items[(blockIdx.x >> 1) / kv_heads];
@@ -215,6 +226,8 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
         mbar_init(s_done, 1);
         mbar_init(p_ready, UTHREADS);
         mbar_init(o_done, 1);
+        mbar_init(drained, 1);
+        *gave_up_s = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == ISSUER) tmem_alloc(tmem_slot, UCOLS);
@@ -268,6 +281,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
     after_sync();
     const unsigned tmem = *tmem_slot;
     bool ok = true;
+    auto wait = [&](void* bar, unsigned parity) { return mbar_wait(bar, parity, status, ROLE_SPINS); };
 
     // a tile's pages, a box a lane (at most 8)
     auto fetch = [&](int t) {
@@ -298,7 +312,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
         }
     };
     auto scores = [&](int t) {
-        if (ok) ok = mbar_wait(&kv_full[t % STAGES], (t / STAGES) & 1, status);
+        if (ok) ok = wait(&kv_full[t % STAGES], (t / STAGES) & 1);
         after_sync();
         if (lane == 0) {
 #pragma unroll
@@ -310,13 +324,13 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
                 if (ok) umma_bf16(tmem + S_HALF * into, a, b, instr_desc(128, UKT),
                                   k % (D / 32) > 0);
             }
-            umma_commit(s_done);
+            if (ok) umma_commit(s_done);
         }
         __syncwarp();
     };
     // the products of tile t's weights, once they are written, and the next tile's scores behind them
     auto products = [&](int t) {
-        if (ok) ok = mbar_wait(p_ready, t & 1, status);
+        if (ok) ok = wait(p_ready, t & 1);
         after_sync();
         if (lane == 0) {
             // 16 keys of a term are 8 columns; 16 keys of the values 2 groups of 8 rows.  The values are
@@ -330,7 +344,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
                     if (ok) umma_a_tmem(tmem + O_COL, tmem + P_TERM * term + 8 * k,
                                         b + (unsigned long long)(k * 2048 >> 4), idesc_pv(D),
                                         term < 2 || k > 0);
-            umma_commit(o_done);
+            if (ok) umma_commit(o_done);
         }
         __syncwarp();
         if (t + 1 < n_tiles) scores(t + 1);
@@ -367,7 +381,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
 
     for (int t = 0; t < n_tiles; ++t) {
         const int kt = tile_at(t), stage = t % STAGES, k0 = kt + 32 * half;
-        if (ok) ok = mbar_wait(s_done, t & 1, status);
+        if (ok) ok = wait(s_done, t & 1);
         after_sync();
         const unsigned gone = gone_s[stage];
         float v[32];
@@ -479,7 +493,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
         if (kt + UKT > k_hi || (kt < k_lo && kt + UKT > k_first) || gone != 0) {
             const int j = tid >> 2, key = kt + j;
             if (key >= k_hi || (key < k_lo && key >= k_first) || ((gone >> (j / box)) & 1u)) {
-                if (ok) ok = mbar_wait(&kv_full[stage], (t / STAGES) & 1, status);
+                if (ok) ok = wait(&kv_full[stage], (t / STAGES) & 1);
                 constexpr int PIECES = KS * 2;           // of 16 bytes, a thread
                 const int c = (tid & 3) * PIECES;
                 uint4* row = reinterpret_cast<uint4*>(
@@ -493,7 +507,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
         before_sync();
         mbar_arrive(p_ready);
         if (warp == ISSUER) products(t);
-        if (ok) ok = mbar_wait(o_done, t & 1, status);
+        if (ok) ok = wait(o_done, t & 1);
         after_sync();
         if (warp == FETCHER && fetched < n_tiles && __all_sync(0xffffffffu, ok)) fetch(fetched++);
 #pragma unroll
@@ -510,9 +524,16 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
         }
         before_sync();
     }
-    if (warp == FETCHER && !__all_sync(0xffffffffu, ok))     // copies in flight end before the block does
+    // Copies and products in flight end before the block does (a fetcher whose waits all succeeded has
+    // seen every tile's products complete, which began after the tile's copies).
+    if (warp == FETCHER && !__all_sync(0xffffffffu, ok))
         for (int t = max(0, fetched - STAGES); t < fetched; ++t)
             mbar_wait(&kv_full[t % STAGES], (t / STAGES) & 1, status);
+    if (warp == ISSUER && !__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) umma_commit(drained);
+        __syncwarp();
+        mbar_wait(drained, 0, status);
+    }
     pdl_trigger();
 
     // back by position: cosines and sines of the block's tokens and this rank's pairs, where q was (all
@@ -536,6 +557,8 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
     float4* from_s = reinterpret_cast<float4*>(k_s);           // [HD / 4][128]
     float* from_ml = reinterpret_cast<float*>(from_s + HD / 4 * UROWS);   // [2][128]
     cluster_sync();                          // both blocks are through their tiles
+    if (!ok)
+        for (int b = 0; b < 2; ++b) store_peer(peer_address(const_cast<unsigned*>(gave_up_s), b), 1u);
     if (half != rank) {
         const unsigned to = peer_address(from_s + rowi, rank ^ 1);
         const unsigned to_ml = peer_address(from_ml + rowi, rank ^ 1);
@@ -545,6 +568,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
         store_peer(to_ml + UROWS * 4, l);
     }
     cluster_sync();
+    const bool whole = *gave_up_s == 0u;
     if (half == rank) {
         const float M_peer = from_ml[rowi], both = fmaxf(M, M_peer);
         const float ref = both == -INFINITY ? 0.0f : both;
@@ -579,7 +603,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
     const float head_gate =
         per_feature ? 1.0f : sight_gate<__nv_bfloat16>(sight, live ? token : 0, hq, D, 0);
     float zero = 0.0f;
-    if (live && ok && half == rank) {
+    if (live && whole && half == rank) {
 #pragma unroll
         for (int i = 0; i < HD / 2; ++i) acc[i] = mul_two(acc[i], two(inv, inv));
         if (fv != nullptr) {
@@ -633,7 +657,7 @@ attn_chunk_tcgen05_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, voi
             }
         }
     }
-    const unsigned met = __ballot_sync(0xffffffffu, live && ok && half == rank && !(zero == 0.0f));
+    const unsigned met = __ballot_sync(0xffffffffu, live && whole && half == rank && !(zero == 0.0f));
     if (lane == 0) spoilt_s[warp] = met;
     before_sync();
     __syncthreads();

@@ -24,9 +24,10 @@ __device__ __forceinline__ void mbar_arrive(void* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 // Bounded wait for the phase with the given parity; false when the limit ran out.
-__device__ __forceinline__ bool mbar_wait(void* bar, unsigned parity, int* status) {
+__device__ __forceinline__ bool mbar_wait(void* bar, unsigned parity, int* status,
+                                          unsigned limit = SPIN_LIMIT) {
     const unsigned addr = smem_u32(bar);
-    for (unsigned spins = 0; spins < SPIN_LIMIT; ++spins) {
+    for (unsigned spins = 0; spins < limit; ++spins) {
         unsigned done;
         asm volatile(
             "{\n"

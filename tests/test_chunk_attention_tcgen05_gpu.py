@@ -175,3 +175,27 @@ def test_results_turned_back(dim, heads, kv_heads, gated, spoilt):
     assert torch.equal(out.isnan(), want.isnan())
     assert torch.equal(out.nan_to_num(1.0), want.nan_to_num(1.0))
     assert bool(want.isnan().any()) == spoilt
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+def test_waits_that_run_out(dim, monkeypatch):
+    """Every wait of the tiles' loop gives up at once: status 3, no result is stored, the copies in flight
+    are waited for, and the launches after it find the GPU as before.  One to nine tiles a block."""
+    from distengine_b200.kernels import library
+    lens, qlen = [1100, 64, 130], [300, 64, 1]
+    fx = PagedFixture(lens, 2, dim, 16, torch.bfloat16, DEV, seed=dim)
+    q = torch.randn(sum(qlen), 6 * dim, generator=torch.Generator().manual_seed(dim))
+    q = q.to(torch.bfloat16).to(DEV)
+    want = torch.empty(sum(qlen), 6 * dim, device=DEV)
+    _run(fx, qlen, 6, 2, q, want, dim ** -0.5)
+    load = library.load
+    monkeypatch.setattr(library, "load", lambda module, defines=(): load(
+        module, ("ROLE_SPINS=0",) if module == "attention_chunk_tcgen05" else defines))
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.full_like(want, 55.0, dtype=dtype)
+        _run(fx, qlen, 6, 2, q, out, dim ** -0.5, status=3)
+        assert bool((out == 55.0).all())
+    monkeypatch.undo()
+    out = torch.full_like(want, 55.0)
+    _run(fx, qlen, 6, 2, q, out, dim ** -0.5)
+    assert torch.equal(out, want)
