@@ -42,6 +42,10 @@ struct CombineItem {           // 4 ints
     int seq, row0, first_partial, num_partials;
 };
 
+// A score as its row's maximum takes it: NaN as infinity, so that a tile of nothing but NaN is not one
+// that the row does not see (fmaxf leaves NaN out), and the row's result is NaN in tiles of any height.
+__device__ __forceinline__ float for_max(float s) { return s == s ? s : INFINITY; }
+
 template <typename T>
 __global__ void __launch_bounds__(ROWS * 32)
 attn_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int out_stride,
@@ -132,7 +136,7 @@ attn_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int
         float s = 0.0f;
         for (int dd = 0; dd < d; ++dd) s = fmaf(qr[dd], kr[dd], s);
         s = valid ? s * scale : -INFINITY;
-        const float m_new = fmaxf(m, warp_max(s));
+        const float m_new = fmaxf(m, warp_max(for_max(s)));
         if (m_new == -INFINITY) continue;             // nothing of this tile is visible to the row
         const float p = valid ? expf(s - m_new) : 0.0f;
         const float corr = expf(m - m_new);           // 0 when m was -inf
@@ -373,7 +377,7 @@ attn_simt_vec_kernel(const float* __restrict__ q, int q_stride, float* __restric
         for (int i = 0; i < RW; ++i) {
             const bool valid = kpos >= row_lo[i] && kpos < row_hi[i] && held;
             const float sc = valid ? s[i] * scale : -INFINITY;
-            const float m_new = fmaxf(m[i], warp_max(sc));
+            const float m_new = fmaxf(m[i], warp_max(for_max(sc)));
             p[i] = 0.0f;
             if (m_new == -INFINITY) continue;         // nothing of this tile is visible to the row
             p[i] = valid ? expf(sc - m_new) : 0.0f;
@@ -654,7 +658,7 @@ attn_simt_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
 #pragma unroll
             for (int t = 0; t < NT; ++t) sc[t] = Ps[warp * KEYS + t * TILE + lane];
 #pragma unroll
-            for (int t = 0; t < NT; ++t) top[t] = warp_max(sc[t]);
+            for (int t = 0; t < NT; ++t) top[t] = warp_max(for_max(sc[t]));
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 const float m_new = fmaxf(m, top[t]);
