@@ -219,6 +219,13 @@ def test_silu_of_rows_by_fours(dtype, n, cols):
     test_silu_of_many_rows(dtype, n, cols)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,cols", [(6251, 64), (100003, 4), (4001, 100), (1563, 256), (397, 1012), (394, 1020)])
+def test_silu_of_narrow_rows(dtype, n, cols):
+    """Fewer than 1,024 columns: a block takes as many fours of rows as it has threads for."""
+    test_silu_of_many_rows(dtype, n, cols)
+
+
 def _walk(rule, lens, inputs, state, H, dk, dv, begin=0):
     """The tokens from ``begin`` on of one sequence, in steps of ``lens``: portions of 192 tokens and
     more by chunks, others by the scan.  Returns the read-outs."""
