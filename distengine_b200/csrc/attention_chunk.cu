@@ -2792,6 +2792,26 @@ DE_EXPORT int de_kv_write_rotated(int dtype, void* proj, int ld, const int* posi
                      (float*)v_pages, block_table, table_stride, page, num_pages, write_kv, status);
 }
 
+// Whether a step of n tokens goes in runs, where its sizes are whole groups: `heads` of q, k and v
+// together.  Us, a token a block and in runs, a norm a head, what proj holds in the L2 as after its product:
+// always from 128 tokens on for heads of 64 (48 heads, 650 tokens, 11.5 and 7.3), with taps (24 heads of
+// 128, 128 tokens 6.2 and 4.9, 600 16.5 and 10.2) and in float32 (24 heads, 700 tokens 7.8 and 7.4).
+// bfloat16 heads of 128 without taps: not while the runs' blocks leave SMs without one or hardly one each
+// (20 heads, 128 tokens 3.2 and 4.0; 12 heads, 300 4.2 and 4.3, 400 5.0 and 4.4), nor where up to 24 heads'
+// runs are two rounds of blocks, three an SM, and the tokens one, five an SM (20 heads, 592 tokens 6.4
+// and 5.2, 600 6.5 and 7.2, 700 6.5 and 7.5, 750 9.1 and 7.7; with 48 heads 600 12.4 and 11.5).
+static bool prepare_in_runs(int dtype, int n, int heads, int dk, bool taps, int sms) {
+    if (n < 128) return false;
+    if (dk == 64 || taps || dtype == DE_F32) return true;
+    const int across = (heads + 7) / 8, blocks = (n + RUN - 1) / RUN * across;
+    // (blocks of 512 threads, two an SM, for fewer than 512 tokens of 16 heads and more)
+    if (n > (heads >= 16 && n < 512 ? 2 : 5) * sms) return true;
+    return 4 * blocks >= 5 * sms && !(across <= 3 && blocks > 3 * sms);
+}
+DE_EXPORT int de_qkv_prepare_in_runs(int dtype, int n, int heads, int dk, int taps, int sms) {
+    return prepare_in_runs(dtype, n, heads, dk, taps != 0, sms);
+}
+
 DE_EXPORT int de_qkv_prepare(int dtype, const void* proj, int ld, void* q_out,
                              const int* positions, const int* token_seq, const int* token_slot,
                              const int* seq_pos0, const float* bias, const float* taps, int by_tap, int K,
@@ -2817,13 +2837,11 @@ DE_EXPORT int de_qkv_prepare(int dtype, const void* proj, int ld, void* q_out,
     cudaStream_t s = (cudaStream_t)stream;
     const int C = (H + G) * dk + (v_from_k ? 0 : G * dv);
     const size_t four = dtype == DE_BF16 ? 8 : 16;   // bytes of a group of four
-    // (us a call, a token a block and in runs, 16 + 4 + 4 heads of 128, bfloat16: with three taps 128
-    // tokens 13.3 and 12.2, 400 19.5 and 13.3, 1,000 25.6 and 20.4; without taps 400 16.4 and 12.3, 700
-    // 13.3 and 16.4 - one round of blocks of 256 threads against two - 1,000 18.6 and 16.4)
-    if (n >= 128 && (taps != nullptr || n < 512 || n >= 800) && dk == dv && (dk == 64 || dk == 128) && norm != 2 && mix == 0 && !keep_here &&
+    if (dk == dv && (dk == 64 || dk == 128) && norm != 2 && mix == 0 && !keep_here &&
         (taps == nullptr || (K >= 2 && K <= 4)) && rot % (adjacent ? 4 : 8) == 0 && ld % 4 == 0 &&
         (uintptr_t)proj % four == 0 && (uintptr_t)q_out % four == 0 &&
-        (uintptr_t)k_pages % four == 0 && (uintptr_t)v_pages % four == 0) {
+        (uintptr_t)k_pages % four == 0 && (uintptr_t)v_pages % four == 0 &&
+        prepare_in_runs(dtype, n, C / dk, dk, taps != nullptr, sm_count())) {
         const int heads = C / dk, per_block = dk == 64 ? 16 : 8;
         const dim3 grid((n + RUN - 1) / RUN, (heads + per_block - 1) / per_block);
 #define PREP_RUNS(T, D, KK)                                                                     \

@@ -222,12 +222,11 @@ __device__ __forceinline__ void merge_row(T* o, const float* partial_acc, const 
 
 // The same attention for float32 pages whose rows are whole 16-byte pieces: tiles of keys and values
 // come through three stages of 16-byte cp.async (eight threads a key, which look its page up once
-// and a tile ahead), a warp takes RW rows and reads a key or a value from shared memory once for
+// and a tile ahead), a warp takes RW = 4 rows and reads a key or a value from shared memory once for
 // all of them.  A row's sums have the order of the kernel above - features ascending in a score,
-// keys ascending in a weighted sum - so the two, and any RW, give the same bits.  The kernel above
-// waited for one element's page and then its key at a time: a decode step of 8 sequences of 520 keys
-// (4 kv heads of 64, ranges of 128 keys) took 53 us and takes 22; a layer with a prompt of 400 tokens
-// takes 325 us (872), one of 64 sequences of 1,900 keys and 8 kv heads of 128 747 us (1,883).
+// keys ascending in a weighted sum - so the two give the same bits.  Portions in tiles of 32 rows come
+// here.  The kernel above waits for one element's page and then its key at a time: a layer with a prompt
+// of 400 tokens took 872 us by it, 325 by this one.
 constexpr int STAGES = 3;
 
 template <int RW, int VW, int NB>
@@ -889,8 +888,6 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
 #undef LAUNCH
 }
 
-// `rows_per_tile`: rows of a tile in the partial layout (8 for the kernel above; the tensor-core
-// kernel writes the same layout with its own tile height).
 // A step of single tokens in float32 in one launch: qkv rows [q heads | k heads | v heads] as the product
 // left them (`Fuse`); `items` as de_attn_simt takes them for tiles of 8 rows, up to 8 query heads a kv
 // head; `counters`: int32 [tiles * kv_heads], zero before and after.
@@ -909,6 +906,8 @@ DE_EXPORT int de_attn_simt_decode(const void* qkv, int qkv_stride, void* out, in
                        scale, window, status, stream, ROWS, Fuse{1, inv_freq, rot, writes, counters});
 }
 
+// `rows_per_tile`: rows of a tile in the partial layout (8 for the kernels above, 32 for the one of
+// portions; the tensor-core kernel writes the same layout with its own tile height).
 DE_EXPORT int de_attn_combine(int dtype, void* out, int out_stride, const int* seq_qstart,
                               const int* seq_qlen, const int* items, int num_items,
                               const float* partial_acc, const float* partial_ml, int heads,
