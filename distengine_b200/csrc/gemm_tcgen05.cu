@@ -339,16 +339,21 @@ int best_width(int m_rows, int n_out, bool gated, int fixed) {
     return best;
 }
 
-// A round hardly depends on the tiles' width: at k = 2,048 11.4 us for 128 columns, 12.2 for 192, 13.4 for
-// 256, at k = 4,096 23, 24.5 and 26.8, so the number of rounds decides and, among equals, the narrowest.
-// (By width + 16, as it was chosen: 1,300 rows against 2 x 5,632 gated 79 us in seven rounds of 128, 53
-// in four of 256; 2,048 against 2 x 11,008 with k = 4,096 336 and 268; 1,024 against 2 x 5,632 64 and 43.)
-int choose_bn(int m_rows, int n_out, bool gated) { return best_width(m_rows, n_out, gated, 600); }
+// From k = 256 on a round hardly depends on the tiles' width: at k = 2,048 11.4 us for 128 columns, 12.2
+// for 192, 13.4 for 256, at k = 4,096 23, 24.5 and 26.8, so the number of rounds decides and, among
+// equals, the narrowest.  (By width + 16: 1,300 rows against 2 x 5,632 gated 79 us in seven rounds of
+// 128, 53 in four of 256; 2,048 against 2 x 11,008 with k = 4,096 336 and 268; 1,024 against 2 x 5,632 64
+// and 43.)  Of a smaller k a round is mostly its epilogue, at k = 64 1.45, 2.0 and 2.5 us, at k = 128 1.6, 2.0
+// and 2.55: 1,300 rows against 12,288 in five rounds of 192 columns 11.8 and 12.3 us, in four of 256 12.4
+// and 13.1 (with k = 256 14.2 and 14.1).
+int choose_bn(int m_rows, int n_out, bool gated, int k_dim) {
+    return best_width(m_rows, n_out, gated, k_dim < 256 ? 48 : 600);
+}
 
 template <bool GATED, typename OutT>
 int launch(const void* x, int ldx, const void* w, int ldw, void* out, int ldo, int m_rows, int n_out,
            int k_dim, int* status, cudaStream_t s) {
-    const int bn = choose_bn(m_rows, n_out, GATED);
+    const int bn = choose_bn(m_rows, n_out, GATED, k_dim);
     CUtensorMap map_x, map_w, map_up;
     int code = make_map(&map_x, x, m_rows, k_dim, ldx, BM);
     if (code) return code;
@@ -379,9 +384,14 @@ int launch(const void* x, int ldx, const void* w, int ldw, void* out, int ldo, i
 
 }  // namespace
 
-// How wide the tiles would have to be if a tile took as long as its columns: the host decides with it
-// whether the shape suits the kernel better than the library's (by the width that the kernel really takes,
-// 2,048 rows against 4,096 x 4,096 would come here, 51 us against the library's 50).
+// How wide the tiles are for a product of these sizes.
+DE_EXPORT int de_gemm_tcgen05_width(int m_rows, int n_out, int k_dim, int gated) {
+    return choose_bn(m_rows, n_out, gated != 0, k_dim);
+}
+// How wide they would have to be if a tile took as long as its columns: the host decides with it whether
+// a shape comes here.  By the width that the kernel takes, shapes would come that fill their rounds only
+// so: 4,096 rows against 2,048 and 2,048 against 4,096, for which the library is the sooner one at every k
+// (us, here and there, k = 128 7.9 and 6.7, 512 10.9 and 10.3, 2,048 26.5 and 24.8, 4,096 50.3 and 45.7).
 DE_EXPORT int de_gemm_tcgen05_tile(int m_rows, int n_out, int gated) {
     return best_width(m_rows, n_out, gated != 0, 16);
 }

@@ -66,6 +66,7 @@ SIGNATURES: dict[str, dict[str, list]] = {
     "gemm_tcgen05": {
         "de_gemm_tcgen05": [P, I, P, I, P, I, I, I, I, I, I, P, P],
         "de_gemm_tcgen05_tile": [I, I, I], "de_gemm_tcgen05_sms": [],
+        "de_gemm_tcgen05_width": [I, I, I, I],
         "de_gemm_tcgen05_grouped": [P, I, P, P, I, P, P, I, I, I, I, I, I, P, P],
     },
     "attention_tcgen05": {

@@ -554,10 +554,11 @@ _tile_fits: dict[tuple[int, int], bool] = {}
 
 def _tcgen05_fits(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
     """Whether a plain product of this shape goes to this package's tcgen05 kernel: many rows, and
-    a shape whose tiles fill the SMs in whole rounds with wide tiles.  (Measured on B200 against
-    cuBLAS at 2,048 rows: equal or within 4% where this holds, up to a third slower where the
-    tiles have to be narrow or the last round is nearly empty; with few rows cuBLAS splits k,
-    which this kernel does not.)"""
+    a shape whose tiles fill the SMs in whole rounds with wide tiles.  (Us on B200, operands in the L2,
+    here and by cuBLAS: 2,048 rows against 2,048 columns with k = 128 5.2 and 5.0, k = 2,048 15.5 and
+    14.0, k = 4,096 25.9 and 23.8; against 12,288 with k = 4,096 156 and 150; up to a third slower where
+    the tiles have to be narrow or the last round is nearly empty, and 1,300 rows against 12,288, k =
+    2,048, 56 and 47; with few rows cuBLAS splits k, which this kernel does not.)"""
     m, n = x.shape[0], w.shape[0]
     if (m < TCGEN05_ROWS or x.shape[1] % 8 or x.stride(0) % 8 or w.stride(0) % 8 or x.stride(1) != 1
             or w.stride(1) != 1 or x.data_ptr() % 16 or w.data_ptr() % 16):

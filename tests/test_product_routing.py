@@ -39,3 +39,15 @@ def test_float32_and_unaligned_weights_keep_the_norm_kernel():
 def test_the_switch_turns_it_off(monkeypatch):
     monkeypatch.setattr(ops, "NORM_RIDE", False)
     assert ops.norm_ride_parts(8, _w(2048, 2048), torch.bfloat16) == 0
+
+
+@pytest.mark.parametrize("m,n,k,gated,width", [
+    # few rounds of wide tiles, but with a short sum a tile takes as long as its columns
+    (1300, 12288, 64, 0, 192), (1300, 12288, 128, 0, 192), (1300, 12288, 256, 0, 256),
+    (1300, 12288, 4096, 0, 256), (2048, 12288, 64, 0, 224), (2048, 12288, 4096, 0, 224),
+    (2048, 2048, 64, 0, 256), (2048, 2048, 2048, 0, 256), (2112, 8192, 128, 0, 192), (2112, 8192, 512, 0, 256),
+    (1024, 2048, 64, 0, 128), (1024, 2048, 4096, 0, 128), (1300, 5632, 2048, 1, 256), (2048, 11008, 4096, 1, 256),
+])
+def test_tile_width_of_a_tcgen05_product(m, n, k, gated, width):
+    from distengine_b200.kernels import library
+    assert library.load("gemm_tcgen05").de_gemm_tcgen05_width(m, n, k, gated) == width
