@@ -232,9 +232,11 @@ __device__ __forceinline__ void turn_features(const T* src, T* dst, const float*
 
 // The same in groups of E features, the token's angles formed once for all heads: where half the
 // turned part, the plain part and the values' (half) rows are whole groups, and everything lies at
-// such addresses.  2,048 tokens, 16 + 4 heads of 128, a product before
-// it: 5.9 us in groups of eight, 7.3 in groups of four, whose last round is a quarter of the block (cold
-// 13, and 23 with each head forming its angles).
+// such addresses.  2,048 tokens, 16 + 4 heads of 128, a product before it: 6.0 us in groups of eight, 7.4
+// in groups of four (cold 13, and 23 with each head forming its angles).  In bfloat16 the values go with
+// queries and keys in one pass over all groups, so that most threads have one (6.0 against 7.4 in two
+// passes, in groups of four at rot 120 7.35 and 7.8); in float32, several a thread, two passes are the
+// sooner ones (rot 64: 7.9 and 8.4).
 template <typename T, int E>
 __global__ void kv_write_rotated_vec_kernel(
     T* __restrict__ proj, int ld, const int* __restrict__ positions,
@@ -263,30 +265,39 @@ __global__ void kv_write_rotated_vec_kernel(
     pdl_wait();
     // groups of pairs, then plain groups, of queries and keys; then the values'
     const int per = (dk - half) / E, vper = (fv != nullptr ? vhalf : dv) / E;
-    const int of_qk = (H + (can_write ? G : 0)) * per, total = of_qk + (can_write ? G * vper : 0);
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        float plain[E];
-        if (idx < of_qk) {
-            const int h = idx / per, i = (idx - h * per) * E;
-            T* src = row + h * dk;
-            T* dst = h < H ? src : k_pages + (at + (size_t)(h - H) * page) * dk;   // q in place
-            if (i < half) {
-                turn_features<E>(src, dst, ktab, half, i);
-            } else if (h >= H) {
-                load_features<E>(src + i + half, plain);
-                store_features<E>(dst + i + half, plain);
-            }
-        } else {
-            const int h = (idx - of_qk) / vper, i = (idx - of_qk - h * vper) * E;
-            const T* src = row + (H + G) * dk + h * dv;
-            T* dst = v_pages + (at + (size_t)h * page) * dv;
-            if (fv != nullptr) {
-                turn_features<E>(src, dst, vtab, vhalf, i);
-            } else {
-                load_features<E>(src + i, plain);
-                store_features<E>(dst + i, plain);
-            }
+    const int of_qk = (H + (can_write ? G : 0)) * per, of_v = can_write ? G * vper : 0;
+    auto query_or_key = [&](int idx) {
+        const int h = idx / per, i = (idx - h * per) * E;
+        T* src = row + h * dk;
+        T* dst = h < H ? src : k_pages + (at + (size_t)(h - H) * page) * dk;   // q in place
+        if (i < half) {
+            turn_features<E>(src, dst, ktab, half, i);
+        } else if (h >= H) {
+            float plain[E];
+            load_features<E>(src + i + half, plain);
+            store_features<E>(dst + i + half, plain);
         }
+    };
+    auto value = [&](int idx) {
+        const int h = idx / vper, i = (idx - h * vper) * E;
+        const T* src = row + (H + G) * dk + h * dv;
+        T* dst = v_pages + (at + (size_t)h * page) * dv;
+        if (fv != nullptr) {
+            turn_features<E>(src, dst, vtab, vhalf, i);
+        } else {
+            float plain[E];
+            load_features<E>(src + i, plain);
+            store_features<E>(dst + i, plain);
+        }
+    };
+    if constexpr (sizeof(T) == 2) {
+        for (int idx = threadIdx.x; idx < of_qk + of_v; idx += blockDim.x) {
+            if (idx < of_qk) query_or_key(idx);
+            else value(idx - of_qk);
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < of_qk; idx += blockDim.x) query_or_key(idx);
+        for (int idx = threadIdx.x; idx < of_v; idx += blockDim.x) value(idx);
     }
     pdl_trigger();
 }
@@ -2763,7 +2774,10 @@ DE_EXPORT int de_kv_write_rotated(int dtype, void* proj, int ld, const int* posi
     cudaStream_t s = (cudaStream_t)stream;
     const int work = (H + G) * dk + G * dv;
     const int threads = n >= 512 ? 128 : (work >= 2048 ? 512 : 256);
-    // a group's features: eight of bfloat16 where everything is whole groups of them, else four
+    // A group's features: eight of bfloat16 where everything is whole groups of them, else four.  As many
+    // threads as groups, but at least four warps (8 + 2 heads of 64, 1,000 tokens 2.4 us; 3.1 by the two
+    // that have groups, 2.55 by four in groups of four); in float32, while the tokens are one round of
+    // six blocks of 256 an SM, more (12 + 2 heads of 64, 512 tokens 2.3 and 2.6, 999 tokens 3.5 and 3.1).
     auto groups = [&](int e, size_t bytes) {
         return rot % (2 * e) == 0 && (dk - rot) % e == 0 && dv % (fv != nullptr ? 2 * e : e) == 0 &&
                ld % e == 0 && dk <= MAX_D && dv <= MAX_D && (uintptr_t)proj % bytes == 0 &&
@@ -2772,7 +2786,8 @@ DE_EXPORT int de_kv_write_rotated(int dtype, void* proj, int ld, const int* posi
 #define ROT(T, E)                                                                               \
     do {                                                                                        \
         const int items = (H + G) * ((dk - rot / 2) / E) + G * ((fv != nullptr ? dv / 2 : dv) / E); \
-        const int block = items >= 256 ? 256 : (items + 31) / 32 * 32;                          \
+        const int fits = items >= 256 ? 256 : items <= 128 ? 128 : (items + 31) / 32 * 32;      \
+        const int block = sizeof(T) == 4 && n <= 6 * sm_count() && work >= 1024 ? 256 : fits;   \
         return de_launch(kv_write_rotated_vec_kernel<T, E>, dim3(n), dim3(block), 0, s,         \
                          (T*)proj, ld, positions, token_slot, fk, rot, fv, H, G, dk, dv,        \
                          (T*)k_pages, (T*)v_pages, block_table, table_stride, page, num_pages,  \
