@@ -437,32 +437,50 @@ def portion_kernels(dtype: torch.dtype, key_dim: int, value_dim: int) -> "tuple[
     return ("attention_chunk",) + (("attention_chunk_tcgen05",) if wide else ())
 
 
-def portion_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int, prep, heads: int,
-                      kv_heads: int) -> int:
-    """Rows of a tile of the chunk attention for a step with prompt portions: 128 (the tcgen05
-    kernel, where it takes the cache's pages) or what ``chunk_rows_per_tile`` says.
+def _wide_pays(key_dim: int, plain: bool, rounds: int, fill: float, keys: int) -> bool:
+    """Whether tiles of 128 rows are sooner than those of 32 or 64: ``plain`` scores (no cap, no
+    penalty), ``rounds`` of one block an SM, the rows' share of the tiles, the longest row's keys.
 
-    A tile of 128 rows is two blocks of the tcgen05 kernel, two of which an SM holds.  It is the sooner
-    one (us, heads of 128, 16 on 4, tiles of 32 / 64 / 128 rows) for one portion of 9 tokens behind
-    1,900 keys 113 / 152 / 77, of 500 tokens 43 / 51 / 33, of 2,048 238 / 213 / 88, four of 30 behind
-    500 43 / 53 / 39; with as many blocks as places also for 20 single tokens behind 600 keys beside a
-    portion of 300 (46 / 59 / 43).  Not where tiles are mostly empty and take several rounds - 60
-    single tokens beside it 54 / 62 / 77, 64 portions of 2 tokens 41 / 51 / 69 - or where many of
-    them have few keys each (16 portions of 40 tokens from position 0: 21 / 21 / 26).  Where the pages
-    are not that kernel's, items of 128 rows would run on mma.sync in tiles of 64, whatever the step."""
+    The tcgen05 kernel costs a block 6 to 9 us before its first 128 keys, a cap or a penalty costs it more
+    than the mma.sync kernel, the most at 64 features, and a third block on an SM waits; where keys are
+    many and tiles full, it makes up for it.  Us, tiles of 32 or 64 rows / of 128, 16 heads on 4.  Heads of
+    128, plain: from position 0 a portion of 2 tokens 8.5 / 12.5, of 96 14.6 / 13.9, of 512 36.9 / 22.7, 16
+    of 64 24.6 / 18.3, 8 of 160 25.0 / 32.6; 9 tokens behind 1,900 100 / 71; 2 tokens beside 20 single
+    ones behind 400 27.1 / 28.8, beside 60 30.3 / 57.3.  With slopes: four of 2 behind 160 14.9 / 19.0, one of
+    200 20.5 / 18.6.  Heads of 64 with slopes: 16 of 2 from position 0 6.2 / 11.1, one of 200 12.8 / 13.6, of
+    512 23.5 / 18.4.  Of 6,664 steps on B200 (1 to 61 sequences, 8 to 32 heads) the tiles chosen so are
+    0.7 % above the sooner ones on average, and 97 times more than 10 % above those of 32 or 64 rows."""
+    if key_dim == 64 and not plain:
+        return fill >= 0.75 and keys > (300 if rounds == 1 else 120 if rounds == 2 else 256)
+    if rounds > 2:
+        return fill >= 0.5 and keys > 200
+    if rounds == 2:
+        return keys > 32 if fill >= 0.75 else fill >= 0.25 and keys > (64 if plain else 200)
+    if fill < (0.25 if plain else 0.75):
+        return keys > (64 if plain and key_dim == 128 else 200)
+    return keys > (64 if plain else 128)
+
+
+def portion_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int, prep, heads: int,
+                      kv_heads: int, plain: bool = True, reach: int = 0) -> int:
+    """Rows of a tile of the chunk attention for a step with prompt portions: 128 (the tcgen05
+    kernel, where it takes the cache's pages and is the sooner one) or what ``chunk_rows_per_tile``
+    says.  ``plain``: the scores pass no cap and no penalty; ``reach``: a row sees that many keys at
+    most (0: all before it).  Where the pages are not that kernel's, items of 128 rows would run on
+    mma.sync in tiles of 64, whatever the step."""
     host = prep.host
     seq_qlen = host.seq_qlen
     wide = int(seq_qlen.max()) > 1
     if (wide and len(portion_kernels(dtype, key_dim, value_dim)) > 1
             and (prep.page_size is None or _wide_ok(key_dim, value_dim, prep.page_size))):
-        rows = seq_qlen.astype("int64") * (heads // kv_heads)
+        group = heads // kv_heads
+        rows = seq_qlen.astype("int64") * group
         tiles = int(((rows + WIDE_ROWS - 1) // WIDE_ROWS).sum())
-        blocks, sms = 2 * tiles * kv_heads, _sms()
-        # (in a step whose graph is replayed: by the batch's shape only)
-        longest = (int((host.seq_pos0 + seq_qlen).max()) if prep.graph_shape is None
-                   else int(prep.graph_shape["context_cap"]))
-        if blocks <= sms or (longest > 128 and (blocks <= 2 * sms
-                                                or 2 * int(rows.sum()) >= tiles * WIDE_ROWS)):
+        keys = int((host.seq_pos0 + seq_qlen).max())
+        if reach:
+            keys = min(keys, reach + WIDE_ROWS // group)
+        if _wide_pays(key_dim, plain, -(-2 * tiles * kv_heads // _sms()),
+                      int(rows.sum()) / (tiles * WIDE_ROWS), keys):
             return WIDE_ROWS
     return chunk_rows_per_tile(dtype, key_dim, value_dim, wide,
                                long_portion_rows(seq_qlen, heads, kv_heads))

@@ -84,7 +84,8 @@ class ChunkAttention(ProjectedMixer):
             prep.notes[self.key] = 0
             return
         # tiles of 32, 64 or 128 rows when the step brings prompt portions, of 8 for single tokens
-        rows = rk.portion_tile_rows(self.dtype, self.dk, self.dv, prep, self.heads, self.kv_heads)
+        rows = rk.portion_tile_rows(self.dtype, self.dk, self.dv, prep, self.heads, self.kv_heads,
+                                    plain=False, reach=self.chunk)
         plan = build_plan(host.seq_qlen, host.seq_pos0, self.heads // self.kv_heads,
                           self.kv_heads, rows, 0, chunk=0)
         prep.add(name, plan.items)

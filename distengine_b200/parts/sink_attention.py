@@ -227,7 +227,9 @@ class SinkAttention(ProjectedMixer):
             prep.add(name, np.zeros((0, 8), dtype=np.int32))
             prep.notes[self.key] = 0
             return
-        rows = rk.portion_tile_rows(self.dtype, self.dk, self.dv, prep, self.heads, self.kv_heads)
+        rows = rk.portion_tile_rows(self.dtype, self.dk, self.dv, prep, self.heads, self.kv_heads,
+                                    plain=not (self.slopes is not None or self.softcap),
+                                    reach=self.window or 0)
         plan = build_plan(host.seq_qlen, host.seq_pos0, self.heads // self.kv_heads,
                           self.kv_heads, rows, 0, chunk=0)
         prep.add(name, plan.items)

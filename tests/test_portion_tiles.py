@@ -19,7 +19,7 @@ def _prep(qlen, pos0, page, graph_shape=None):
 
 @pytest.mark.parametrize("dim", [64, 128])
 @pytest.mark.parametrize("qlen,pos0", [([9], [1900]), ([500], [0]), ([2048], [0]), ([30] * 4, [500] * 4),
-                                       ([300] + [1] * 20, [0] + [600] * 20), ([64], [0])])
+                                       ([300] + [1] * 20, [0] + [600] * 20), ([100], [0])])
 def test_pages_that_the_kernel_takes_and_others(dim, qlen, pos0, monkeypatch):
     monkeypatch.setattr(rk, "_sms", lambda: 148)
     host = _prep(qlen, pos0, None).host
@@ -53,3 +53,31 @@ def test_a_steps_plan_knows_its_page_size(page, monkeypatch):
                             length=lambda r: 0, slot=lambda r: 0)
     step.StepRunner(model, cache).prepare([step.StepEntry("a", [1, 2])])
     assert seen == [page]
+
+
+# (tokens, position of the first, plain scores?, heads, key/value heads, size, tiles of 128 rows?), measured on B200
+MEASURED = [
+    ([2], [0], True, 16, 4, 128, False), ([64], [0], True, 16, 4, 128, False), ([96], [0], True, 16, 4, 128, True),
+    ([96], [0], False, 16, 4, 128, False), ([200], [0], False, 16, 4, 128, True), ([9], [1900], True, 16, 4, 128, True),
+    ([64] * 16, [0] * 16, True, 16, 4, 128, True), ([160] * 8, [0] * 8, True, 16, 4, 128, False),
+    ([512] * 4, [0] * 4, False, 16, 4, 128, True), ([2] + [1] * 60, [50] + [400] * 60, True, 16, 4, 128, False),
+    ([2] * 4, [160] * 4, False, 16, 4, 128, False), ([2048], [0], False, 16, 4, 128, True),
+    ([1201, 1172], [0, 0], True, 16, 4, 128, True), ([2] * 16, [0] * 16, True, 16, 4, 64, False),
+    ([96], [0], True, 16, 4, 64, True), ([200], [0], False, 16, 4, 64, False), ([512], [0], False, 16, 4, 64, True),
+    ([9], [500], False, 16, 4, 64, False), ([9], [500], True, 16, 4, 64, True),
+    ([2] + [1] * 30, [50] + [400] * 30, False, 12, 4, 64, False), ([2] * 64, [300] * 64, True, 16, 2, 64, False),
+]
+
+
+@pytest.mark.parametrize("qlen,pos0,plain,heads,kv_heads,dim,wide", MEASURED)
+def test_tiles_of_128_rows_where_they_are_sooner(qlen, pos0, plain, heads, kv_heads, dim, wide, monkeypatch):
+    monkeypatch.setattr(rk, "_sms", lambda: 148)
+    rows = rk.portion_tile_rows(torch.bfloat16, dim, dim, _prep(qlen, pos0, 16), heads, kv_heads, plain)
+    assert (rows == 128) == wide
+
+
+def test_keys_out_of_a_windows_reach_do_not_count(monkeypatch):
+    monkeypatch.setattr(rk, "_sms", lambda: 148)
+    for reach, wide in ((0, True), (1024, True), (100, True), (20, False)):
+        rows = rk.portion_tile_rows(torch.bfloat16, 128, 128, _prep([40], [1900], 16), 16, 4, True, reach)
+        assert (rows == 128) == wide, reach
