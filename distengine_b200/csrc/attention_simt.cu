@@ -222,11 +222,12 @@ __device__ __forceinline__ void merge_row(T* o, const float* partial_acc, const 
 
 // The same attention for float32 pages whose rows are whole 16-byte pieces: tiles of keys and values
 // come through three stages of 16-byte cp.async (eight threads a key, which look its page up once
-// and a tile ahead), a warp takes RW = 4 rows and reads a key or a value from shared memory once for
+// and a tile ahead), a warp takes RW rows and reads a key or a value from shared memory once for
 // all of them.  A row's sums have the order of the kernel above - features ascending in a score,
-// keys ascending in a weighted sum - so the two give the same bits.  Portions in tiles of 32 rows come
-// here.  The kernel above waits for one element's page and then its key at a time: a layer with a prompt
-// of 400 tokens took 872 us by it, 325 by this one.
+// keys ascending in a weighted sum - so the two, and any RW, give the same bits.  Portions in tiles of
+// 32 rows come here (RW 4), and tiles of 8 rows over few keys (RW 1, de_attn_simt_by_tiles).  The kernel
+// above waits for one element's page and then its key at a time: a layer with a prompt of 400 tokens took
+// 872 us by it, 325 by this one.
 constexpr int STAGES = 3;
 
 template <int RW, int VW, int NB>
@@ -780,6 +781,30 @@ attn_combine_kernel(T* __restrict__ out, int out_stride, const int* __restrict__
 
 DE_EXPORT int de_attn_simt_rows_per_tile() { return ROWS; }
 
+// shared memory of attn_simt_vec_kernel
+static size_t vec_bytes(int d, int tile_rows) {
+    return (size_t)(STAGES * (TILE * (2 * d + 4) + TILE) + tile_rows * d) * sizeof(float);
+}
+// Whether `blocks` of tiles of 8 float32 rows whose longest sees `keys` keys are sooner through tiles of 32
+// keys (de_attn_simt with tile_rows -8) than a range at once, which costs a block some 1.5 us more before
+// its first scores (us, 32 heads on 4 of 64: one portion of 10 tokens 5.4 and 6.9, four of 17 6.3 and 9.7, 10
+// of 4 behind 1,000 58 and 46; 32 on 8 of 128, one of 10 5.9 and 6.7, one of 33 9.0 and 7.9) but then wins by
+// a quarter to two fifths.  Up to one tile of keys unless that takes more rounds of blocks over the SMs,
+// three of which an SM holds the other way; up to three tiles where it takes fewer (heads of 64: 480
+// blocks of 43 keys 13.3 and 18.1).
+DE_EXPORT int de_attn_simt_by_tiles(int d, int blocks, int keys) {
+    if (d <= 0 || d > MAX_D || d % 4 != 0 || keys > 3 * TILE) return 0;
+    int device = 0, sms = 148;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        sms = 148;
+    int places = (int)(227 * 1024 / (vec_bytes(d, ROWS) + 1024));
+    places = places < 1 ? 1 : places > 8 ? 8 : places;       // (256 threads each)
+    const int here = (blocks + places * sms - 1) / (places * sms);
+    const int at_once = (blocks + 3 * sms - 1) / (3 * sms);
+    return keys <= TILE ? here <= at_once : here < at_once;
+}
+
 static int launch_simt(int dtype, const void* q, int q_stride, void* out, int out_stride,
                        const void* k_pages, const void* v_pages, const int* block_table,
                        int table_stride, int num_pages, const int* seq_slot,
@@ -800,6 +825,7 @@ DE_EXPORT int de_attn_simt(int dtype, const void* q, int q_stride, void* out, in
                            const int* items, int num_items, float* partial_acc, float* partial_ml,
                            int heads, int kv_heads, int d, int page, float scale, int window,
                            int tile_rows, int* status, void* stream) {
+    // (tile_rows -8: tiles of 8 rows, see de_attn_simt_by_tiles)
     return launch_simt(dtype, q, q_stride, out, out_stride, k_pages, v_pages, block_table,
                        table_stride, num_pages, seq_slot, seq_qstart, seq_qlen, seq_pos0, items,
                        num_items, partial_acc, partial_ml, 0x7fffffff, heads, kv_heads, d, page,
@@ -820,10 +846,12 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
     cudaStream_t s = (cudaStream_t)stream;
     const bool vec = dtype == DE_F32 && d % 4 == 0;
     const int aligned = (uintptr_t)k_pages % 16 == 0 && (uintptr_t)v_pages % 16 == 0;
+    const bool by_tiles = tile_rows == -ROWS;        // tiles of 8 rows through the kernel for tiles of keys
+    if (by_tiles) tile_rows = ROWS;
+    if (by_tiles && (!vec || fuse.on)) return -5;
     if (tile_rows != ROWS && !(vec && tile_rows == 4 * ROWS)) return -5;
     if (vec) {
-        const size_t bytes = (size_t)(STAGES * (TILE * (2 * d + 4) + TILE) + tile_rows * d) *
-                             sizeof(float);
+        const size_t bytes = vec_bytes(d, tile_rows);
 #define LAUNCH_VEC(RW, VW, NB)                                                                  \
     do {                                                                                        \
         auto kernel = attn_simt_vec_kernel<RW, VW, NB>;                                         \
@@ -839,6 +867,11 @@ static int launch_simt(int dtype, const void* q, int q_stride, void* out, int ou
                          (const WorkItem*)items, partial_acc, partial_ml, partial_limit, heads, \
                          kv_heads, d, page, scale, window, aligned, status);                    \
     } while (0)
+        if (by_tiles) {
+            if (d <= 64) LAUNCH_VEC(1, 2, 1);
+            if (d <= 128) LAUNCH_VEC(1, 4, 1);
+            LAUNCH_VEC(1, 4, 2);
+        }
         if (tile_rows == ROWS) {
 #define LAUNCH_ROWS(VW, KEYS)                                                                   \
     do {                                                                                        \

@@ -269,6 +269,14 @@ class AttentionLauncher:
                 seq = plan.items[:, 0]
                 plan.items[:, 1], plan.items[:, 7] = host.seq_pos0[seq], host.seq_slot[seq]
                 combine = combine[:0]
+            elif shape.name == "rows8" and len(self.shapes) > 1:
+                # few keys: through tiles of them (the same bits)
+                blocks = int((plan.items[:, 3] > plan.items[:, 2]).sum()) * self.kv_heads
+                keys = int((host.seq_pos0 + qlen)[qlen > 0].max())
+                if self.window:
+                    keys = min(keys, self.window + int(qlen.max()))
+                prep.notes[self.key + "/by_tiles"] = bool(library.load(
+                    "attention_simt").de_attn_simt_by_tiles(self.head_dim, blocks, keys))
             prep.add(f"{self.key}/{shape.name}/items", plan.items)
             prep.add(f"{self.key}/{shape.name}/combine", combine)
             notes[shape.name] = plan.num_partials
@@ -307,7 +315,10 @@ class AttentionLauncher:
                 acc = ctx.buffer(f"attention.partial_acc.{shape.name}", (rows * d,), torch.float32)
                 ml = ctx.buffer(f"attention.partial_ml.{shape.name}", (rows * 2,), torch.float32)
             module = self.tcgen05_module if shape.code == 2 else self.module
-            launch_items(shape.code, module, q, out, k_pages, v_pages, block_table,
+            code = shape.code
+            if shape.name == "rows8" and ctx.notes.get(self.key + "/by_tiles"):
+                code = -2
+            launch_items(code, module, q, out, k_pages, v_pages, block_table,
                          ctx.seq_slot, ctx.seq_qstart, ctx.seq_qlen, ctx.seq_pos0, items, combine,
                          shape.rows, acc, ml, self.heads, self.kv_heads, d, self.scale, self.window,
                          getattr(ctx, "status", None), (float(softcap), sink, float(out_scale)))
@@ -399,7 +410,8 @@ def launch_items(code: int, module, q, out, k_pages, v_pages, block_table, seq_s
                  seq_qlen, seq_pos0, items, combine, tile_rows, partial_acc, partial_ml, heads,
                  kv_heads, head_dim, scale, window, status=None,
                  extras=(0.0, None, 1.0)) -> None:
-    """One launch of a kernel over ``items`` and, if any range was split, the merge.  ``extras``:
+    """One launch of a kernel over ``items`` and, if any range was split, the merge.  ``code``: -1
+    attn_simt, -2 the same for tiles of 8 rows over few keys, 0 and 1 mma.sync, 2 tcgen05.  ``extras``:
     (softcap, sink, factor of the results), for the mma.sync kernel only."""
     _need(code in (0, 1) or extras == (0.0, None, 1.0),
           "paged attention: this kernel takes no soft cap, sink or factor")
@@ -425,8 +437,8 @@ def launch_items(code: int, module, q, out, k_pages, v_pages, block_table, seq_s
             _status_fallback = torch.zeros(1, dtype=torch.int32, device=q.device)
         status = _status_fallback
     if code < 0:
-        _check(lib.de_attn_simt(_tag(q.dtype), *common, tile_rows, status.data_ptr(), _stream()),
-               "paged attention")
+        _check(lib.de_attn_simt(_tag(q.dtype), *common, -tile_rows if code == -2 else tile_rows,
+                                status.data_ptr(), _stream()), "paged attention")
     elif code == 2:
         _check(lib.de_attn_tcgen05(*common, status.data_ptr(), _stream()),
                "paged attention (tcgen05)")

@@ -48,7 +48,7 @@ SIGNATURES: dict[str, dict[str, list]] = {
     "attention_simt": {
         "de_attn_simt_decode": [P, I, P, I, P, P, P, I, I, P, P, P, P, P, I, P, P, P, P, I, I, I, I, I,
                                 I, F, I, P, P],
-        "de_attn_simt_rows_per_tile": [],
+        "de_attn_simt_rows_per_tile": [], "de_attn_simt_by_tiles": [I, I, I],
         "de_attn_simt": [I, P, I, P, I, P, P, P, I, I, P, P, P, P, P, I, P, P, I, I, I, I, F, I, I,
                          P, P],
         "de_attn_combine": [I, P, I, P, P, P, I, P, P, I, I, I, I, P],

@@ -149,3 +149,30 @@ def test_float32_decode_steps_bring_no_list_of_merges(graph_shape):
         launcher.prepare(prep, allow_decode=fused)
         assert (prep.notes[launcher.key + "/decode"] is not None) == fused
         assert (len(prep.extra[f"{launcher.key}/rows8/combine"]) == 0) == fused
+
+
+@pytest.mark.parametrize("dim,blocks,keys,by_tiles", [
+    (64, 4, 10, 1), (64, 480, 17, 1), (64, 2000, 32, 1), (64, 400, 33, 0), (64, 480, 43, 1), (64, 480, 96, 1),
+    (64, 480, 97, 0), (64, 700, 64, 0), (64, 1000, 64, 1), (128, 100, 32, 1), (128, 300, 32, 0), (128, 500, 20, 1),
+    (128, 500, 33, 0), (256, 100, 32, 1), (256, 149, 32, 0), (256, 10, 33, 0), (32, 460, 50, 1), (32, 400, 50, 0),
+    (66, 4, 10, 0)])
+def test_float32_tiles_of_8_rows_over_few_keys(dim, blocks, keys, by_tiles):
+    """Up to 32 keys, and up to 96 where it saves a round of blocks, tiles of 8 rows go through tiles of keys."""
+    from distengine_b200.kernels import library
+    assert library.load("attention_simt").de_attn_simt_by_tiles(dim, blocks, keys) == by_tiles
+
+
+def test_the_plan_says_how_tiles_of_8_rows_go():
+    from types import SimpleNamespace
+
+    import torch
+
+    from distengine_b200.kernels.attention import AttentionLauncher
+    from distengine_b200.parts.context import StepPrep
+    for dim, qlen, pos0, note in ((64, [10], [0], True), (64, [10], [500], False), (64, [3] * 40, [40] * 40, True),
+                                  (128, [3] * 40, [40] * 40, False), (64, [200], [0], None), (18, [10], [0], None)):
+        launcher = AttentionLauncher(torch.float32, 32, 4, dim, 1.0, None)
+        prep = StepPrep(SimpleNamespace(seq_qlen=np.array(qlen, dtype=np.int32),
+                                        seq_pos0=np.array(pos0, dtype=np.int32)))
+        launcher.prepare(prep)
+        assert prep.notes.get(launcher.key + "/by_tiles") is note

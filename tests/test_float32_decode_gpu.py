@@ -61,3 +61,23 @@ def test_decode_attention_in_one_kernel(heads, kv_heads, d, rot, page, window, w
     for a, b, name in zip(got, want, ("out", "k", "v")):
         assert torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0)), name     # (free pages hold NaN)
     assert torch.isfinite(got[0]).all()
+
+
+@pytest.mark.parametrize("heads,kv_heads,d,window", [(32, 4, 64, None), (6, 2, 20, 9), (8, 1, 128, None), (3, 3, 256, 40)])
+@pytest.mark.parametrize("lens,qlen", [((10, 32, 33, 1), (10, 17, 2, 1)), ((43,) * 9, (3,) * 9), ((200, 96), (5, 33))])
+def test_tiles_of_8_rows_through_tiles_of_keys(heads, kv_heads, d, window, lens, qlen, monkeypatch):
+    """Small portions by either kernel: the same bits, also where a range is cut and merged."""
+    from distengine_b200.kernels import library
+    from gpu_helpers import run_paged_attention
+    fx = PagedFixture(list(lens), kv_heads, d, 16, torch.float32, DEV, seed=d)
+    g = torch.Generator().manual_seed(heads)
+    q = [torch.randn(n, heads, d, generator=g) for n in qlen]
+    out = []
+    for by_tiles in (0, 1):
+        monkeypatch.setattr(library.load("attention_simt"), "de_attn_simt_by_tiles", lambda *sizes: by_tiles)
+        for chunk in (0, 32, None):
+            out.append(run_paged_attention(fx, q, heads, kv_heads, d, d ** -0.5, window, shape="rows8",
+                                           chunk=chunk)[0])
+    assert torch.isfinite(out[0]).all()
+    for i in range(3):
+        assert torch.equal(out[i], out[i + 3]), i
