@@ -130,9 +130,10 @@ static inline void de_prefer_carveout(F kernel, int percent) {
     value[at] = percent;
 }
 
+// `early` false: the kernel starts when the one before it is done.
 template <typename... KArgs, typename... Args>
-static inline int de_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                            cudaStream_t stream, Args... args) {
+static inline int de_launch_when(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                                 size_t smem, cudaStream_t stream, Args... args) {
     de_prefer_carveout(kernel, g_carveout);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -143,8 +144,13 @@ static inline int de_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_pdl ? 1 : 0;
+    cfg.numAttrs = early && g_pdl ? 1 : 0;
     return de_check(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
+}
+template <typename... KArgs, typename... Args>
+static inline int de_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                            cudaStream_t stream, Args... args) {
+    return de_launch_when(true, kernel, grid, block, smem, stream, args...);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -862,7 +862,7 @@ int launch_scan_cols(int R, dim3 grid, cudaStream_t s, const float* q, int ldq, 
                      int ldk, const VT* v, int ldv, const float* g, int ldg, const float* beta,
                      int ldb, const float* z, int ldz, const float* decay, float* state, long long slot_stride, float* out,
                      const int* seq_slot, const int* seq_qstart, const int* seq_qlen, int H,
-                     int rep, int dk, int dv, int vec16, int longest, ConvKeep keep) {
+                     int rep, int dk, int dv, int vec16, int longest, ConvKeep keep, bool early) {
 #define SCAN(RR)                                                                                \
     do {                                                                                        \
         const size_t smem = (size_t)2 * TB * (MODE + 2) * LANES * (RR + 4) * sizeof(float);     \
@@ -872,7 +872,7 @@ int launch_scan_cols(int R, dim3 grid, cudaStream_t s, const float* q, int ldq, 
                                                  (int)smem);                                    \
             if (e != cudaSuccess) return (int)e;                                                \
         }                                                                                       \
-        return de_launch(scan_kernel<VT, RR, MODE, COLS, LANES>, grid, dim3(COLS * LANES),      \
+        return de_launch_when(early, scan_kernel<VT, RR, MODE, COLS, LANES>, grid, dim3(COLS * LANES), \
                          smem, s, q, ldq, k, ldk, v, ldv, g, ldg, beta, ldb, z, ldz, decay, state, \
                          slot_stride, out, seq_slot, seq_qstart, seq_qlen, H, rep, dk, dv,      \
                          vec16, longest, keep);                                                          \
@@ -902,7 +902,7 @@ int launch_scan(cudaStream_t s, const float* q, int ldq, const float* k, int ldk
                 int ldz, const float* decay,
                 float* state, long long slot_stride, float* out, const int* seq_slot,
                 const int* seq_qstart, const int* seq_qlen, int n_seqs, int H, int rep, int dk,
-                int dv, int longest, ConvKeep keep) {
+                int dv, int longest, ConvKeep keep, bool early) {
     const int vec16 = (dk % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && (MODE == 0 || ldg % 4 == 0) &&
                        (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 &&
                        (MODE == 0 || (uintptr_t)g % 16 == 0) &&
@@ -912,7 +912,7 @@ int launch_scan(cudaStream_t s, const float* q, int ldq, const float* k, int ldk
     return launch_scan_cols<VT, MODE, CC, LL>(R, grid, s, q, ldq, k, ldk, v, ldv, g, ldg,       \
                                                beta, ldb, z, ldz, decay, state, slot_stride, out, \
                                                seq_slot, seq_qstart, seq_qlen, H, rep, dk, dv, \
-                                               vec16, longest, keep)
+                                               vec16, longest, keep, early)
     // (eight lanes a column - twice the warps, half the instructions a token and warp - was
     // measured for a single long prompt and is slower: 867 against 788 us for 2,048 tokens of 16
     // heads of 128 x 128; a token's time is its chain of dependent steps, which a third butterfly
@@ -1037,16 +1037,22 @@ DE_EXPORT int de_state_scan(int mode, int v_dtype, const float* q, int ldq, cons
                             const int* seq_slot, const int* seq_qstart, const int* seq_qlen,
                             int n_seqs, int H, int rep, int dk, int dv, const void* conv_proj,
                             int conv_ld, int conv_dtype, int conv_offset, int conv_channels,
-                            int conv_taps, int longest, void* stream) {
+                            int conv_taps, int longest, int portions, void* stream) {
     if (n_seqs <= 0) return 0;
     if (dk <= 0 || dk > 256 || dv <= 0 || H <= 0 || rep <= 0 || H % rep) return -2;
     if (mode < 0 || mode > 2) return -2;
     cudaStream_t s = (cudaStream_t)stream;
     ConvKeep keep = {conv_proj, conv_ld, conv_dtype == DE_BF16 ? 1 : 0, conv_offset,
                      conv_channels, conv_proj ? conv_taps : 0};
+    // `portions`: some sequence has more than one token.  Blocks that start while the kernel before them
+    // still runs land beside one another on the SMs that it leaves free, several blocks of one warp on a
+    // scheduler, and a decay's walk, a short chain a token, then takes two to three times as long (300 tokens
+    // of 8 heads of 64 165 us; 56 spread over the SMs).  Such a step's scan waits for that kernel's end; single
+    // tokens keep the microsecond, and the delta rules, whose chain is the longer one, theirs.
+    const bool early = mode != 0 || !portions;
 #define SCAN_ARGS(VT)                                                                           \
     s, q, ldq, k, ldk, (const VT*)v, ldv, g, ldg, beta, ldb, z, ldz, decay, state, slot_stride, \
-        out, seq_slot, seq_qstart, seq_qlen, n_seqs, H, rep, dk, dv, longest, keep
+        out, seq_slot, seq_qstart, seq_qlen, n_seqs, H, rep, dk, dv, longest, keep, early
     if (mode == 1) {
         if (v_dtype != DE_F32) return -4;
         return launch_scan<float, 1>(SCAN_ARGS(float));

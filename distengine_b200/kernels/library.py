@@ -105,7 +105,7 @@ SIGNATURES: dict[str, dict[str, list]] = {
         "de_conv_state": [I, P, I, P, L, I, P, P, P, I, I, I, P],
         "de_retention_prep": [I, P, I, P, P, I, I, I, P, P, I, P],
         "de_state_scan": [I, I, P, I, P, I, P, I, P, I, P, I, P, I, P, P, L, P, P, P, P, I, I, I,
-                          I, I, P, I, I, I, I, I, I, P],
+                          I, I, P, I, I, I, I, I, I, I, P],
         "de_gdelta_prep": [I, P, I, I, I, I, P, P, P, P, P, P, P, P, I, I, I, P],
         "de_silu_rows": [I, P, I, P, I, I, P],
         "de_head_gate": [I, P, P, I, P, P, I, I, I, F, I, P],

@@ -151,7 +151,7 @@ def state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
                              state.stride(0), out.data_ptr(), ctx.seq_slot.data_ptr(),
                              ctx.seq_qstart.data_ptr(), ctx.seq_qlen.data_ptr(), ctx.n_seqs, heads,
                              heads // qk_heads, key_dim, value_dim, *conv,
-                             int(longest) or 0x7fffffff, _stream()),
+                             int(longest) or 0x7fffffff, int(n > ctx.n_seqs), _stream()),
            "state_scan")
 
 
