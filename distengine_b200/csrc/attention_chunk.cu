@@ -863,7 +863,7 @@ qkv_prepare_runs_kernel(const T* __restrict__ proj, int ld, T* __restrict__ q_ou
 // pos0 + qlen - (K - 1) + i; a portion shorter than K - 1 moves the older rows up.  The layout is
 // the one that the state mixers' convolution keeps (recurrent.cu); a model whose only
 // convolution is this mixer's needs no other library for it.  grid (sequences, channels / 256): a
-// thread a channel, 2.9 us for two sequences of 3,072 channels (6.5 with a block a sequence).
+// thread a channel, 2.4 us in a layer of two sequences of 3,072 channels (6.5 with a block a sequence).
 template <typename T>
 __global__ void conv_keep_kernel(const T* __restrict__ proj, int ld, float* __restrict__ state,
                                  long long slot_stride, int conv_offset,

@@ -9,10 +9,10 @@
 // and warp 7 issues the products beside that: a warp more would leave a thread 96 registers instead of
 // 128.  A tile: s = q k^T into 64 columns of tensor memory for
 // either half of the features (added in float32: one sum over all of them is cut off at every
-// product, 2.1e-7 from 64 bits in the results instead of 1.5e-7); scale, penalty, cap, mask and maximum in registers; the weights over the scores' columns as three
-// bfloat16 terms (each the upper half of what the ones before it leave: their sum is the float32
-// weight), 32 columns each; three products with the values, the small terms first, into columns of the
-// tile's own.  The sums over tiles are float32 multiply-adds in registers (acc <- acc * correction +
+// product, 2.1e-7 from 64 bits in the results instead of 1.5e-7); scale, penalty, cap, mask and maximum
+// in registers; the weights over the scores' columns as three bfloat16 terms (each the upper half of what
+// the ones before it leave: their sum is the float32 weight), 32 columns each; three products with the
+// values, the small terms first, into columns of the tile's own.  The sums over tiles are float32 multiply-adds in registers (acc <- acc * correction +
 // tile's share), so that what the tensor cores add up is a tile's share only.
 //
 // Nothing loses precision against the kernels on mma.sync: products of bfloat16 operands are exact,
@@ -23,10 +23,11 @@
 // again on the CUDA cores once everything is stored.
 //
 // The pair of blocks: an item's tiles go by the parity of their place to two blocks of a cluster, which
-// exchange half of the features each through distributed shared memory at the end.  A block alone
-// takes 2.0 us a tile at 128 features (8,000 cycles: two products' latencies and some 800
-// instructions a warp between them at two to four warps a scheduler), which is what bounds it: the
-// longest rows' tiles one after the other.  Measured (us; mma.sync in tiles of 64 rows, one block a
+// exchange half of the features each through distributed shared memory at the end.  A pair alone on the
+// GPU takes 4.2 us a tile and block at 128 features (8,000 cycles: two products' latencies and some 800
+// instructions a warp between them at two to four warps a scheduler) and 2.5 at 64, which is what bounds
+// it: the longest rows' tiles one after the other.  On a full GPU an instruction is issued in 24 to 29 %
+// of the cycles, the tensor cores are at work in 13 to 15 %.  Measured (us; mma.sync in tiles of 64 rows, one block a
 // row tile, pairs): 2,048 tokens of 16 heads of 128 on 4 kv heads 213, 114, 88; under a window of
 // 1,024 and a cap 156, 92, 96; prompts of 1,201 and 1,172 tokens 153, 100, 84; with distance slopes
 // 158, 139, 98; heads of 64 135, 86, 65.  Four threads a row instead of two: 134 instead of 114.

@@ -171,13 +171,16 @@ def chunks_pay(delta: bool, heads: int, key_dim: int, value_dim: int, longest: i
 
     The scan costs the longest portion's chain and every (token, head)'s work, the chunks mostly a
     fixed time a (chunk, head).  In us, from layers of 1 to 32 portions of 192 to 4,096 tokens with 8,
-    16 and 64 heads on B200 (a bfloat16 layer by the scan / by chunks): delta rule 128 x 128, 16
-    heads, one portion of 512 tokens 234 / 132, ten of 200 517 / 436, 32 of 200 1,307 / 1,382; delta
-    rule 64 x 64, 16 heads, one of 512 149 / 86, ten of 200 181 / 207, 32 of 200 496 / 538, 64 heads,
-    ten of 400 1,044 / 1,110, four of 500 699 / 554; a decay per head gains at all of these.  The
-    chunks are four or five launches instead of one, and a step that runs launch by launch waits for
-    the host: what the scan does in less than that stays with it (delta 64 x 64, 8 heads, one
-    portion of 256: 122 against 147; a decay per head 64 x 64, 16 heads, the same 77 against 83)."""
+    16 and 64 heads on B200 (a bfloat16 layer by the scan / by chunks, as a graph): delta rule 128 x
+    128, 16 heads, one portion of 512 tokens 230 / 119, ten of 200 502 / 373; delta rule 64 x 64, 16
+    heads, one of 512 146 / 80, ten of 200 177 / 183, 32 of 200 471 / 498, 64 heads, ten of 400
+    1,000 / 1,065, four of 500 687 / 529; a decay per head gains at all of these.  The line was drawn
+    when a chunk took a tenth more than it does: just beyond it chunks are now 5 to 9 % the sooner
+    ones (delta rule 128 x 128, 16 heads, 32 of 200 1,233 / 1,159, 64 heads, ten of 200 1,564 /
+    1,425; 64 x 64, 64 heads, four of 400 564 / 438).  The chunks are four or five launches instead of
+    one, and a step that runs launch by launch waits for the host: what the scan does in less than
+    that stays with it (delta 64 x 64, 8 heads, one portion of 256: 135 against 150; a decay per head
+    64 x 64, 16 heads, the same 88 and 89)."""
     wide = key_dim == 128
     by = value_dim / key_dim
     if not delta:
