@@ -440,9 +440,11 @@ def portion_kernels(dtype: torch.dtype, key_dim: int, value_dim: int) -> "tuple[
     return ("attention_chunk",) + (("attention_chunk_tcgen05",) if wide else ())
 
 
-def _wide_pays(key_dim: int, plain: bool, rounds: int, fill: float, keys: int) -> bool:
+def _wide_pays(key_dim: int, plain: bool, rounds: int, fill: float, keys: int,
+               launch_saved: bool = False) -> bool:
     """Whether tiles of 128 rows are sooner than those of 32 or 64: ``plain`` scores (no cap, no
     penalty), ``rounds`` of one block an SM, the rows' share of the tiles, the longest row's keys.
+    ``launch_saved``: their kernel stands for two where small steps wait for the host, 5 us a launch.
 
     The tcgen05 kernel costs a block 6 to 9 us before its first 128 keys, a cap or a penalty costs it more
     than the mma.sync kernel, the most at 64 features, and a third block on an SM waits; where keys are
@@ -453,6 +455,9 @@ def _wide_pays(key_dim: int, plain: bool, rounds: int, fill: float, keys: int) -
     200 20.5 / 18.6.  Heads of 64 with slopes: 16 of 2 from position 0 6.2 / 11.1, one of 200 12.8 / 13.6, of
     512 23.5 / 18.4.  Of 6,664 steps on B200 (1 to 61 sequences, 8 to 32 heads) the tiles chosen so are
     0.7 % above the sooner ones on average, and 97 times more than 10 % above those of 32 or 64 rows."""
+    if launch_saved and rounds <= 2 and (rounds == 1 or fill >= 0.25 or plain
+                                         or (key_dim == 128 and keys > 200)):
+        return True
     if key_dim == 64 and not plain:
         return fill >= 0.75 and keys > (300 if rounds == 1 else 120 if rounds == 2 else 256)
     if rounds > 2:
@@ -465,11 +470,14 @@ def _wide_pays(key_dim: int, plain: bool, rounds: int, fill: float, keys: int) -
 
 
 def portion_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int, prep, heads: int,
-                      kv_heads: int, plain: bool = True, reach: int = 0) -> int:
+                      kv_heads: int, plain: bool = True, reach: int = 0,
+                      finishes: bool = False) -> int:
     """Rows of a tile of the chunk attention for a step with prompt portions: 128 (the tcgen05
     kernel, where it takes the cache's pages and is the sooner one) or what ``chunk_rows_per_tile``
     says.  ``plain``: the scores pass no cap and no penalty; ``reach``: a row sees that many keys at
-    most (0: all before it).  Where the pages are not that kernel's, items of 128 rows would run on
+    most (0: all before it); ``finishes``: that kernel also does what another would after it, which
+    counts where the step runs launch by launch (a layer of four portions of 30 tokens behind 500 55 us
+    instead of 60; as a graph it is the kernel's time that counts).  Where the pages are not that kernel's, items of 128 rows would run on
     mma.sync in tiles of 64, whatever the step."""
     host = prep.host
     seq_qlen = host.seq_qlen
@@ -483,7 +491,8 @@ def portion_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int, prep, he
         if reach:
             keys = min(keys, reach + WIDE_ROWS // group)
         if _wide_pays(key_dim, plain, -(-2 * tiles * kv_heads // _sms()),
-                      int(rows.sum()) / (tiles * WIDE_ROWS), keys):
+                      int(rows.sum()) / (tiles * WIDE_ROWS), keys,
+                      finishes and prep.graph_shape is None):
             return WIDE_ROWS
     return chunk_rows_per_tile(dtype, key_dim, value_dim, wide,
                                long_portion_rows(seq_qlen, heads, kv_heads))

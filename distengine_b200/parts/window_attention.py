@@ -138,7 +138,8 @@ class WindowAttention(ProjectedMixer):
             return
         rows = rk.portion_tile_rows(self.dtype, self.dk, self.dv, prep, self.heads, self.kv_heads,
                                     plain=not self.softcap,
-                                    reach=(self.window + self.keep_first) if self.window else 0)
+                                    reach=(self.window + self.keep_first) if self.window else 0,
+                                    finishes=self.fv is not None or self.gated)
         plan = build_plan(host.seq_qlen, host.seq_pos0, self.heads // self.kv_heads,
                           self.kv_heads, rows, 0, chunk=0)
         prep.add(name, plan.items)

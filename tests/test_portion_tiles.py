@@ -81,3 +81,14 @@ def test_keys_out_of_a_windows_reach_do_not_count(monkeypatch):
     for reach, wide in ((0, True), (1024, True), (100, True), (20, False)):
         rows = rk.portion_tile_rows(torch.bfloat16, 128, 128, _prep([40], [1900], 16), 16, 4, True, reach)
         assert (rows == 128) == wide, reach
+
+
+def test_a_launch_that_is_saved_counts_where_steps_go_launch_by_launch(monkeypatch):
+    monkeypatch.setattr(rk, "_sms", lambda: 148)
+    for qlen, pos0, plain, eager, replayed in (([33], [0], True, True, False), ([2048], [0], True, True, True),
+                                               ([2] + [1] * 60, [50] + [400] * 60, True, False, False),
+                                               ([2] + [1] * 30, [50] + [100] * 30, False, False, False)):
+        for shape, wide in ((None, eager), ({"context_cap": 2048}, replayed)):
+            rows = rk.portion_tile_rows(torch.bfloat16, 128, 128, _prep(qlen, pos0, 16, shape), 16, 4, plain,
+                                        finishes=True)
+            assert (rows == 128) == wide, (qlen, shape)
