@@ -12,8 +12,9 @@
 // product, 2.1e-7 from 64 bits in the results instead of 1.5e-7); scale, penalty, cap, mask and maximum
 // in registers; the weights over the scores' columns as three bfloat16 terms (each the upper half of what
 // the ones before it leave: their sum is the float32 weight), 32 columns each; three products with the
-// values, the small terms first, into columns of the tile's own.  The sums over tiles are float32 multiply-adds in registers (acc <- acc * correction +
-// tile's share), so that what the tensor cores add up is a tile's share only.
+// values, the small terms first, into columns of the tile's own.  The sums over tiles are float32
+// multiply-adds in registers (acc <- acc * correction + tile's share), so that what the tensor cores add
+// up is a tile's share only.
 //
 // Nothing loses precision against the kernels on mma.sync: products of bfloat16 operands are exact,
 // a weight has its 24 bits.  exp(score - maximum) is 2^(v U - M), one multiply-add and ex2.approx, with

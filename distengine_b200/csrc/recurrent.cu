@@ -952,9 +952,9 @@ DE_EXPORT int de_delta_prep(int dtype, const void* proj, int ld, const float* a,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    // steps with portions: four channels a thread, eight tokens a block (us by the general kernel and so:
-    // 128 tokens of 8 + 8 + 8 heads of 64 5.9 and 6.2 in bfloat16, 5.0 and 7.2 in float32, whose norms
-    // are a longer chain; 300 of them 8.2 and 6.3, 8.2 and 7.4)
+    // steps with portions: four channels a thread, four tokens a block (us by the general kernel at 127
+    // tokens and so at 128: 8 + 8 + 8 heads of 64, bfloat16, 7.3 and 4.6, of 16 of 128 11.7 and 5.4, in
+    // float32, whose norms are a longer chain, 11.7 and 10.2; float32, 8 of 64, 300 tokens 8.1 and 5.8)
     const int esize = dtype == DE_BF16 ? 2 : 4;
     const bool many = n >= 128 && (dtype == DE_BF16 || (long long)n * (2 * G * dk + H * dv) >= 420000);
     if (many && K <= 4 && (dk == 64 || dk == 128) && (G * dk) % 128 == 0 && (H * dv) % 128 == 0 &&

@@ -476,9 +476,9 @@ def portion_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int, prep, he
     kernel, where it takes the cache's pages and is the sooner one) or what ``chunk_rows_per_tile``
     says.  ``plain``: the scores pass no cap and no penalty; ``reach``: a row sees that many keys at
     most (0: all before it); ``finishes``: that kernel also does what another would after it, which
-    counts where the step runs launch by launch (a layer of four portions of 30 tokens behind 500 55 us
-    instead of 60; as a graph it is the kernel's time that counts).  Where the pages are not that kernel's, items of 128 rows would run on
-    mma.sync in tiles of 64, whatever the step."""
+    counts where the step runs launch by launch (a layer of four portions of 30 tokens behind 500 55
+    us instead of 60; as a graph it is the kernel's time that counts).  Where the pages are not that
+    kernel's, items of 128 rows would run on mma.sync in tiles of 64, whatever the step."""
     host = prep.host
     seq_qlen = host.seq_qlen
     wide = int(seq_qlen.max()) > 1
